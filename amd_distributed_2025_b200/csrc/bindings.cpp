@@ -4,6 +4,7 @@
 // (all2all/hipv8.py:20-40,229-237), with host-side validation of dtypes, shapes and
 // contiguity and launches on the caller's current stream instead of the default stream.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <pybind11/stl.h>
 #include <torch/extension.h>
@@ -233,6 +234,7 @@ class MoeDedupEngine {
                 "expert_y must be a contiguous [E_local, max_recv, hidden] tensor of the layer's dtype");
     c10::cuda::CUDAGuard guard(heap_->device());
     combine_blocks_ = b200::moe_dedup_combine_max_blocks(heap_->device());
+    sms_ = at::cuda::getDeviceProperties(heap_->device())->multiProcessorCount;
     TORCH_CHECK(blk_hist_.scalar_type() == at::kInt && blk_hist_.is_contiguous(), "blk_hist must be contiguous int32");
   }
 
@@ -271,6 +273,11 @@ class MoeDedupEngine {
     c10::cuda::CUDAGuard guard(heap_->device());
     const int ws = heap_->world_size();
     const int n = (int)(T * k_);
+    if (ws == 1 && b200::moe_local_dispatch_applies(n, (int)E_)) {
+      TORCH_CHECK(!fuse_scale, "one rank: forward() fuses the expert op");
+      local_dispatch(x, indices, nullptr, nullptr, 1.0f);
+      return 0;
+    }
     const int bulk = (bulk_landing && ws > 1 && (H_ * elem_) % 16 == 0) ? 1 : 0;
     const int max_blocks = b200::moe_dedup_dispatch_max_blocks(heap_->device(), (int)E_, n, bulk);
     TORCH_CHECK(blk_hist_.numel() >= (int64_t)max_blocks * E_, "blk_hist scratch too small");
@@ -341,6 +348,10 @@ class MoeDedupEngine {
     }
     c10::cuda::CUDAGuard guard(heap_->device());
     const int ws = heap_->world_size();
+    if (ws == 1) {
+      local_combine(out, weights, ey);
+      return 0;
+    }
     b200::MoeDedupCombineParams p;
     p.out = out.data_ptr();
     p.weights = weights.data_ptr<float>();
@@ -379,11 +390,96 @@ class MoeDedupEngine {
 
   // dispatch (carrying the weights, applying expert_y = expert_x * scale on the way) + combine
   int forward(const at::Tensor& x, const at::Tensor& indices, const at::Tensor& weights, at::Tensor out, double scale) {
+    if (local_ready(x, indices) && b200::moe_local_dispatch_applies(x.size(0) * k_, (int)E_) &&
+        rows_of(weights, at::kFloat, x.size(0), k_, true) && rows_of(out, dtype_, x.size(0), H_, false)) {
+      c10::cuda::CUDAGuard guard(heap_->device());
+      local_dispatch(x, indices, weights.const_data_ptr<float>(), out.mutable_data_ptr(), (float)scale);
+      ++combine_epoch_;
+      return 0;
+    }
     if (const int rc = dispatch(x, indices, weights, true, scale)) return rc;
     return combine(out, weights, c10::nullopt);
   }
 
+  // One rank, everything as the kernels want it (types, shapes, contiguity, no failure on record): the whole
+  // call without another look at it from Python, whose checks cost as much as a short kernel.  None / false:
+  // nothing was done, take the checked path.
+  c10::optional<at::Tensor> try_forward(const at::Tensor& x, const at::Tensor& indices, const at::Tensor& weights, double scale) {
+    if (!local_ready(x, indices) || !b200::moe_local_dispatch_applies(x.size(0) * k_, (int)E_) ||
+        !rows_of(weights, at::kFloat, x.size(0), k_, true))
+      return c10::nullopt;
+    c10::cuda::CUDAGuard guard(heap_->device());
+    at::Tensor out = at::detail::empty_cuda({x.size(0), H_}, dtype_, x.device(), c10::nullopt);
+    local_dispatch(x, indices, weights.const_data_ptr<float>(), out.mutable_data_ptr(), (float)scale);
+    ++combine_epoch_;
+    return out;
+  }
+  bool try_dispatch(const at::Tensor& x, const at::Tensor& indices) {
+    if (!local_ready(x, indices) || !b200::moe_local_dispatch_applies(x.size(0) * k_, (int)E_)) return false;
+    c10::cuda::CUDAGuard guard(heap_->device());
+    local_dispatch(x, indices, nullptr, nullptr, 1.0f);
+    return true;
+  }
+  bool try_combine(const at::Tensor& out, const at::Tensor& weights, const at::Tensor& expert_y, int64_t num_tokens) {
+    if (heap_->world_size() != 1 || heap_->status_host().code != 0 || (num_tokens >= 0 && num_tokens != num_tokens_) ||
+        !rows_of(out, dtype_, num_tokens_, H_, false) || !rows_of(weights, at::kFloat, num_tokens_, k_, false) ||
+        !expert_y.is_cuda() || expert_y.get_device() != heap_->device() || expert_y.scalar_type() != dtype_ ||
+        !expert_y.is_contiguous() || expert_y.sizes() != expert_y_.sizes())
+      return false;
+    c10::cuda::CUDAGuard guard(heap_->device());
+    local_combine(out, weights, expert_y.const_data_ptr());
+    return true;
+  }
+
  private:
+  // a contiguous [rows or more, cols] CUDA tensor of this type on the layer's device
+  bool rows_of(const at::Tensor& t, at::ScalarType type, int64_t rows, int64_t cols, bool exact) const {
+    return t.is_cuda() && t.dim() == 2 && t.scalar_type() == type && t.size(1) == cols &&
+           (exact ? t.size(0) == rows : t.size(0) >= rows) && t.is_contiguous() && t.get_device() == heap_->device();
+  }
+  bool local_ready(const at::Tensor& x, const at::Tensor& indices) const {
+    return heap_->world_size() == 1 && heap_->status_host().code == 0 && x.dim() == 2 && x.size(0) <= max_tokens_ &&
+           rows_of(x, dtype_, x.size(0), H_, true) && rows_of(indices, at::kInt, x.size(0), k_, true);
+  }
+  void local_dispatch(const at::Tensor& x, const at::Tensor& indices, const float* weights, void* out, float scale) {
+    b200::MoeLocalDispatchParams p;
+    const uint64_t base = heap_->peer_base(0);
+    p.x = x.const_data_ptr();
+    p.indices = indices.const_data_ptr<int32_t>();
+    p.weights = weights;
+    p.out = out;
+    p.expert_x = reinterpret_cast<void*>(base + lay_.off_expert_x);
+    p.expert_meta = reinterpret_cast<int32_t*>(base + lay_.off_expert_meta);
+    p.route = reinterpret_cast<int2*>(route_.mutable_data_ptr<int32_t>());
+    p.expert_num_tokens = expert_num_tokens_.mutable_data_ptr<int32_t>();
+    p.num_tokens = (int32_t)x.size(0);
+    p.k = (int32_t)k_;
+    p.num_experts = (int32_t)E_;
+    p.max_recv = (int32_t)max_recv_;
+    p.dtype = dtype_code_;
+    p.row_bytes = (uint32_t)(H_ * elem_);
+    p.scale = scale;
+    p.epoch = (uint64_t)(++dispatch_epoch_);
+    p.status = heap_->status_device();
+    p.trace_d = trace_d_;
+    p.trace_c = trace_c_;
+    num_tokens_ = p.num_tokens;
+    cuda_check(b200::launch_moe_local_dispatch(p, sms_, at::cuda::getCurrentCUDAStream()), "moe_local_dispatch launch");
+  }
+  void local_combine(const at::Tensor& out, const at::Tensor& weights, const void* expert_y) {
+    b200::MoeLocalCombineParams p;
+    p.out = out.mutable_data_ptr();
+    p.weights = weights.const_data_ptr<float>();
+    p.route = reinterpret_cast<const int2*>(route_.const_data_ptr<int32_t>());
+    p.expert_y = expert_y;
+    p.num_tokens = num_tokens_;
+    p.k = (int32_t)k_;
+    p.dtype = dtype_code_;
+    p.row_bytes = (uint32_t)(H_ * elem_);
+    p.trace = trace_c_;
+    ++combine_epoch_;
+    cuda_check(b200::launch_moe_local_combine(p, sms_, at::cuda::getCurrentCUDAStream()), "moe_local_combine launch");
+  }
   uint64_t* check_trace(const c10::optional<at::Tensor>& t) {
     if (!t.has_value() || !t->defined()) return nullptr;
     TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kLong && t->is_contiguous() && t->numel() >= 8,
@@ -415,6 +511,7 @@ class MoeDedupEngine {
   int64_t timeout_ns_;
   int64_t dispatch_epoch_ = 0, combine_epoch_ = 0;
   int combine_blocks_ = 1;
+  int sms_ = 1;
   bool weights_sent_ = false;
   int num_tokens_ = 0;
   uint64_t* trace_d_ = nullptr;
@@ -1108,6 +1205,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            py::arg("fuse_scale") = false, py::arg("scale") = 1.0)
       .def("combine", &MoeDedupEngine::combine, py::arg("out"), py::arg("weights"), py::arg("expert_y") = py::none())
       .def("forward", &MoeDedupEngine::forward)
+      .def("try_forward", &MoeDedupEngine::try_forward)
+      .def("try_dispatch", &MoeDedupEngine::try_dispatch)
+      .def("try_combine", &MoeDedupEngine::try_combine)
       .def("set_trace", &MoeDedupEngine::set_trace, py::arg("dispatch_trace") = py::none(), py::arg("combine_trace") = py::none())
       .def("set_timeout_ns", &MoeDedupEngine::set_timeout_ns)
       .def_readwrite("bulk_landing", &MoeDedupEngine::bulk_landing)

@@ -153,4 +153,43 @@ int moe_dedup_combine_max_blocks(int device);
 cudaError_t launch_moe_dedup_dispatch(const MoeDedupDispatchParams& p, int grid, cudaStream_t stream);
 cudaError_t launch_moe_dedup_combine(const MoeDedupCombineParams& p, int grid, cudaStream_t stream);
 
+// ---------------------------------------------------------------------------------------
+// One rank (moe_local.cu): every expert is here, nothing crosses a link
+// ---------------------------------------------------------------------------------------
+struct MoeLocalDispatchParams {
+  const void* x;             // [T, hidden]
+  const int32_t* indices;    // [T, k]
+  const float* weights;      // [T, k]; only with `out`
+  void* out;                 // not null: also out[t] = sum over k of w * (x * scale rounded to the row type)
+  void* expert_x;            // [E][max_recv][hidden]
+  int32_t* expert_meta;      // [E][max_recv][5]
+  int2* route;               // [T*k] (0, row) or (-1, -1)
+  int32_t* expert_num_tokens;
+  int32_t num_tokens, k, num_experts, max_recv;
+  int32_t dtype;             // 0 = fp16, 1 = bf16, 2 = fp32
+  uint32_t row_bytes;
+  float scale;
+  uint64_t epoch;
+  StatusBlock* status;
+  uint64_t* trace_d;         // optional stamps, slots as in the multi-rank kernels
+  uint64_t* trace_c;
+  int32_t vec, pieces, piece_vecs, cap;  // filled in by the launcher
+};
+
+struct MoeLocalCombineParams {
+  void* out;                 // [T, hidden]
+  const float* weights;      // [T, k]
+  const int2* route;
+  const void* expert_y;      // [E][max_recv][hidden]
+  int32_t num_tokens, k;
+  int32_t dtype;
+  uint32_t row_bytes;
+  uint64_t* trace;
+  int32_t vec, pieces, piece_vecs;  // filled in by the launcher
+};
+
+bool moe_local_dispatch_applies(int64_t num_entries, int num_experts);
+cudaError_t launch_moe_local_dispatch(MoeLocalDispatchParams p, int sms, cudaStream_t stream);
+cudaError_t launch_moe_local_combine(MoeLocalCombineParams p, int sms, cudaStream_t stream);
+
 }  // namespace b200

@@ -24,6 +24,9 @@
 //        w * expert_y[row], pushed as ONE row into the source's return buffer
 //     2  last CTA raises RET; source side: out[t] = sum over the owners it used
 //
+// One rank has kernels of its own (moe_local.cu); of these it only reaches dispatch with more than
+// 32768 entries.
+//
 // Calls must alternate dispatch, combine: a rank enters call n+1 only after every owner's
 // RET flag of call n, i.e. after every rank finished reading what call n+1 overwrites.
 // All cross-GPU waits are bounded (signal.cuh); row indices read from memory that peers
@@ -751,7 +754,6 @@ __global__ void __launch_bounds__(kThreads) moe_dedup_combine_kernel(const MoeDe
   const int32_t* tok_rec = peer_ptr<const int32_t>(my_base, p.layout.off_tok_rec);
   const uint8_t* ey = reinterpret_cast<const uint8_t*>(p.expert_y);
   const int total_rows = p.num_local_experts * p.max_recv;
-  const bool direct_out = p.world_size == 1;  // the only owner is the source: write the result itself
   bool warp_ok = true;
   for (int j = 0; j < p.world_size && alive && warp_ok; ++j) {
     int s = p.rank + 1 + j;  // remote sources first, rotated so that the ranks do not all push to the same one
@@ -781,15 +783,13 @@ __global__ void __launch_bounds__(kThreads) moe_dedup_combine_kernel(const MoeDe
       const int from = __fns(valid, 0, lane + 1);  // lane of the (lane+1)-th valid entry, or -1
       const int crow = __shfl_sync(0xffffffffu, row, from < 0 ? 0 : from);
       const float cw = __shfl_sync(0xffffffffu, w, from < 0 ? 0 : from);
-      uint8_t* dst_row = direct_out
-                             ? reinterpret_cast<uint8_t*>(p.out) + (size_t)t * row_bytes
-                             : peer_ptr<uint8_t>(p.peer_base[s], p.layout.off_ret) +
-                                   ((uint64_t)p.rank * p.max_tokens + t) * ret_row_bytes;
+      uint8_t* dst_row = peer_ptr<uint8_t>(p.peer_base[s], p.layout.off_ret) +
+                         ((uint64_t)p.rank * p.max_tokens + t) * ret_row_bytes;
       if (vec16) {
         const int v_lo = piece * pv, v_hi = min(nv, (piece + 1) * pv);
         const uint8_t* my_row = ey + (size_t)(lane < cnt ? crow : 0) * row_bytes;
         bool ok;
-        if (p.partial_fp32 && !direct_out) {
+        if (p.partial_fp32) {
           ok = warp_weighted_sum_bulk<T, true>(my_row, cw, cnt, v_lo, v_hi, dst_row, stage, stage_u32, bar, parity, lane,
                                                p.timeout_ns, p.status);
         } else {
@@ -811,7 +811,7 @@ __global__ void __launch_bounds__(kThreads) moe_dedup_combine_kernel(const MoeDe
             if (h < p.hidden) acc = fmaf(to_f32(__ldcg(reinterpret_cast<const T*>(ey + (size_t)r * row_bytes) + h)), wc, acc);
           }
           if (h < p.hidden) {
-            if (p.partial_fp32 && !direct_out) reinterpret_cast<float*>(dst_row)[h] = acc;
+            if (p.partial_fp32) reinterpret_cast<float*>(dst_row)[h] = acc;
             else reinterpret_cast<T*>(dst_row)[h] = from_f32<T>(acc);
           }
         }
@@ -819,19 +819,6 @@ __global__ void __launch_bounds__(kThreads) moe_dedup_combine_kernel(const MoeDe
     }
   }
   stamp(p.trace, 2);
-
-  if (direct_out) {
-    // tokens none of whose entries was delivered still get a defined (zero) row
-    for (int t = gw; t < p.num_tokens; t += W) {
-      bool any = false;
-      if (lane < k) any = __ldg(p.route + (size_t)t * k + lane).y >= 0;
-      if (__ballot_sync(0xffffffffu, any) != 0) continue;
-      T* o = reinterpret_cast<T*>(p.out) + (size_t)t * p.hidden;
-      for (int h = lane; h < p.hidden; h += 32) o[h] = from_f32<T>(0.f);
-    }
-    if (p.trace != nullptr && tid == 0) atomicMax(reinterpret_cast<unsigned long long*>(p.trace + 7), global_timer_ns());
-    return;
-  }
 
   // ---- phase 2: all partial rows pushed -> tell the sources; add up what came back ----------
   if (last_cta_arrives(&p.sync_counters[3])) {

@@ -85,6 +85,29 @@ __device__ __forceinline__ void prefetch_tensormap(const void* tensor_map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tensor_map) : "memory");
 }
 
+// ---- programmatic dependent launch ------------------------------------------------------------
+// A kernel launched with launch_dependent() may start while the previous kernel of its stream still runs;
+// grid_dep_wait() returns once that one is complete and its writes are visible, and stands before the first
+// access to anything it may have written or read.  grid_dep_launch() lets the next such kernel start.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), int grid, int threads, size_t smem, cudaStream_t stream,
+                             const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // ---- tensor memory ----------------------------------------------------------------------
 // Whole-warp operations (.sync.aligned): call with all 32 lanes converged.
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_result, uint32_t ncols) {

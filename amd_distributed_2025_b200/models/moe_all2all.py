@@ -77,6 +77,7 @@ def moe_slab_layout(cfg: MoEConfig, world_size: int, header_bytes: int, mode: st
 
 class MoEAllToAll:
     META_DIM = META_DIM
+    _native = None  # the engine, where a whole call can be handed to it unchecked (one rank)
 
     def __init__(
         self,
@@ -153,6 +154,9 @@ class MoEAllToAll:
             self.engine.chunks = max(1, min(8, int(os.environ.get("B200_MOE_CHUNKS", "4"))))
             self.engine.chunk_min_ranks = int(os.environ.get("B200_MOE_CHUNK_MIN_RANKS", "4"))
             self.engine.chunk_min_bytes = int(os.environ.get("B200_MOE_CHUNK_MIN_BYTES", str(8 << 20)))
+            if world_size == 1:
+                self._native = self.engine
+        self._dispatched = (self.expert_num_tokens, self.expert_x, self.expert_meta)
         self.trace: Optional[Tuple[torch.Tensor, torch.Tensor]] = None
 
     def _guard(self) -> None:
@@ -195,6 +199,10 @@ class MoEAllToAll:
 
     # -- dispatch ----------------------------------------------------------------------
     def dispatch(self, dp_x: torch.Tensor, indices: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+        if self._native is not None and self.monitor is None and self._native.try_dispatch(dp_x, indices):
+            self._num_tokens = dp_x.shape[0]
+            self._dispatch_pending = True
+            return self._dispatched
         cfg = self.cfg
         if dp_x.shape[0] > cfg.max_num_tokens:
             raise ValueError(f"{dp_x.shape[0]} tokens exceed max_num_tokens={cfg.max_num_tokens}")
@@ -257,6 +265,10 @@ class MoEAllToAll:
         ``[0, num_tokens)`` of ``out_tokens`` are overwritten (``accumulate=True`` adds
         instead, which equals the reference's ``+=`` onto a caller-provided buffer).
         """
+        if (self._native is not None and self.monitor is None and not accumulate
+                and self._native.try_combine(out_tokens, weights, expert_y, -1 if num_tokens is None else num_tokens)):
+            self._dispatch_pending = False
+            return out_tokens
         n = self._num_tokens if num_tokens is None else int(num_tokens)
         if n != self._num_tokens:
             raise ValueError("num_tokens differs from the preceding dispatch")
@@ -306,8 +318,15 @@ class MoEAllToAll:
     def forward(self, dp_x: torch.Tensor, indices: torch.Tensor, weights: torch.Tensor, scale: float) -> torch.Tensor:
         """dispatch -> ``expert_y = expert_x * scale`` -> combine, launched back to back from
         one native call.  In "dedup" mode the scale is applied while the landed rows are
-        replicated into the expert buffers (two launches); in "direct" mode it is the three
-        kernels of the separate methods."""
+        replicated into the expert buffers (two launches); on one rank it and the weighted sum are
+        formed from the rows as they are stored to ``expert_x`` (one launch, ``expert_y`` is not
+        written); in "direct" mode it is the three kernels of the separate methods."""
+        if self._native is not None and self.monitor is None:
+            y = self._native.try_forward(dp_x, indices, weights, scale)
+            if y is not None:
+                self._num_tokens = dp_x.shape[0]
+                self._dispatch_pending = False
+                return y
         cfg = self.cfg
         if dp_x.shape[0] > cfg.max_num_tokens or dp_x.shape[1] != cfg.hidden_dim or dp_x.dtype != cfg.in_dtype:
             raise ValueError("dp_x does not match the configuration")
