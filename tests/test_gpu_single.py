@@ -86,6 +86,46 @@ def test_moe_world1_matches_oracle(E, k, H, T, dtype, fixed, mode):
         assert oracle.relative_error(y, oracle.moe_expected_output(cfg, data, 1, acc_dtype=torch.float64)) < 5e-3
 
 
+@pytest.mark.parametrize(
+    "E,k,H,T,M,dtype",
+    [
+        (8, 1, 64, 1, 3, torch.float16),  # one entry, one piece
+        (5, 5, 520, 7, 7, torch.bfloat16),  # every expert gets every token; last piece of a row is short
+        (64, 6, 1000, 395, 400, torch.float32),  # pieces shared between CTAs, just above 16 warps per SM
+        (1030, 3, 24, 1366, 1366, torch.float16),  # more experts than the replicated counts take, rows of 3 vectors
+        (16, 8, 256, 4096, 4096, torch.bfloat16),  # the most entries the single launch takes ...
+        (16, 8, 256, 4097, 4097, torch.bfloat16),  # ... and one token more
+    ],
+)
+def test_moe_one_rank_kernels_at_the_edges_of_their_ranges(E, k, H, T, M, dtype):
+    from amd_distributed_2025_b200.models import moe_all2all
+
+    cfg, data, _, _ = contract.make_moe_inputs(E, k, H, M, 5, 0, 1, device="cuda", dtype=dtype, fixed_num_tokens=T,
+                                               routing="zipf", weights="rand")
+    layer = moe_all2all.MoEAllToAll(cfg, 0, 1, mode="dedup")
+    for scale in (1.0, 3.0):  # the second forward must not see anything of the first
+        y = layer.forward(data.x, data.indices, data.weights, scale)
+        want = (data.x * scale).double() * data.weights.double().sum(1, keepdim=True)
+        assert oracle.relative_error(y, want) < 5e-3
+    counts, ex, meta = layer.dispatch(data.x, data.indices)
+    ids = data.indices.long().flatten()
+    order = torch.sort(ids, stable=True).indices  # entries by expert, (token, k) order inside an expert
+    assert torch.equal(counts.long(), torch.bincount(ids, minlength=E))
+    slot = torch.arange(T * k, device="cuda") - (torch.cumsum(counts.long(), 0) - counts.long())[ids[order]]
+    assert torch.equal(ex[ids[order], slot], data.x[order // k])
+    got = meta[ids[order], slot].long()
+    assert torch.equal(got, torch.stack([ids[order], 0 * order, order // k, order % k, 0 * order], dim=1))
+    ey = torch.randn(ex.shape, device="cuda").to(dtype)
+    out = torch.empty(T, H, dtype=dtype, device="cuda")
+    layer.combine(out, data.weights, meta, ey, counts, T)
+    rows = torch.empty(T * k, H, dtype=torch.float64, device="cuda")
+    rows[order] = ey[ids[order], slot].double()
+    want = (rows.view(T, k, H) * data.weights.double()[:, :, None]).sum(1)
+    assert oracle.relative_error(out, want) < 5e-3
+    layer.check()
+    layer.close()
+
+
 def test_moe_dedup_fp32_partial_rows_and_phase_stamps():
     from amd_distributed_2025_b200.models import moe_all2all
 
