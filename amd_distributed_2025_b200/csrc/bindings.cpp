@@ -596,6 +596,7 @@ class GemmRsEngine {
       off_stage_[i] = (uint64_t)stage_offsets[i];
       off_counters_[i] = (uint64_t)counter_offsets[i];
     }
+    sms_ = at::cuda::getDeviceProperties(heap_->device())->multiProcessorCount;
   }
 
   // knobs (0 / -1 = chosen from the shape); see GemmRsArgs
@@ -657,6 +658,10 @@ class GemmRsEngine {
       bias_ptr = bias->data_ptr();
     }
     c10::cuda::CUDAGuard guard(heap_->device());
+    if (local_applies(a, w, out) && (reinterpret_cast<uintptr_t>(bias_ptr) & 15u) == 0) {
+      run_local(a, w, bias_ptr, out, bias_at_source, bias_scale);
+      return 0;
+    }
     const b200::GemmRsPlan plan = cached_plan((int)M, (int)N, (int)K);
     TORCH_CHECK((int64_t)plan.stage_bytes <= stage_bytes_ && (int64_t)plan.counter_bytes <= counter_bytes_, "problem ", M, "x",
                 N, "x", K, " needs ", plan.stage_bytes, " staging bytes, the workspace has ", stage_bytes_);
@@ -703,7 +708,84 @@ class GemmRsEngine {
     return 0;
   }
 
+  // One rank, everything as the kernel wants it: the whole call without another look at it from Python.  None:
+  // nothing was done, take the checked path.
+  c10::optional<at::Tensor> try_run(const at::Tensor& a, const at::Tensor& w, const c10::optional<at::Tensor>& bias,
+                                    bool bias_at_source) {
+    if (heap_->world_size() != 1 || heap_->status_host().code != 0 || !a.is_cuda() || !w.is_cuda() || a.dim() != 2 || w.dim() != 2 ||
+        a.scalar_type() != at::kBFloat16 || w.scalar_type() != at::kBFloat16 || !a.is_contiguous() || !w.is_contiguous() ||
+        a.get_device() != heap_->device() || w.get_device() != heap_->device())
+      return c10::nullopt;
+    const int64_t M = a.size(0), N = w.size(0), K = a.size(1);
+    if (M <= 0 || N <= 0 || K <= 0 || K != w.size(1) || K % 8 != 0 || N % 8 != 0) return c10::nullopt;
+    const void* bias_ptr = nullptr;
+    if (bias.has_value() && bias->defined()) {
+      if (!bias->is_cuda() || bias->scalar_type() != at::kBFloat16 || bias->numel() != N || !bias->is_contiguous()) return c10::nullopt;
+      bias_ptr = bias->const_data_ptr();
+    }
+    c10::cuda::CUDAGuard guard(heap_->device());
+    if (!local_applies(a, w, a) || (reinterpret_cast<uintptr_t>(bias_ptr) & 15u) != 0) return c10::nullopt;
+    at::Tensor out = at::detail::empty_cuda({M, N}, at::kBFloat16, a.device(), c10::nullopt);
+    run_local(a, w, bias_ptr, out, bias_at_source, 1.0);
+    return out;
+  }
+
  private:
+  static bool aligned16(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15u) == 0; }
+  // the one-rank kernel plans for itself: any knob set by hand means the multi-rank kernel
+  bool local_applies(const at::Tensor& a, const at::Tensor& w, const at::Tensor& out) const {
+    return heap_->world_size() == 1 && !force_staged && max_ctas == 0 && block_n == 0 && cta_pair < 0 && splits == 0 && debug == 0 &&
+           aligned16(a) && aligned16(w) && aligned16(out);
+  }
+  void run_local(const at::Tensor& a, const at::Tensor& w, const void* bias, const at::Tensor& out, bool bias_at_source, double bias_scale) {
+    b200::GemmLocalArgs g;
+    g.a = a.const_data_ptr();
+    g.w = w.const_data_ptr();
+    g.bias = bias;
+    g.out = out.mutable_data_ptr();
+    g.M = (int)a.size(0);
+    g.N = (int)w.size(0);
+    g.K = (int)a.size(1);
+    g.bias_scale = (float)bias_scale;
+    g.bias_at_source = bias_at_source ? 1 : 0;
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
+    const LocalWorkspace* ws = local_workspace(stream);
+    g.partials = ws ? ws->partials : nullptr;
+    g.counters = ws ? ws->counters : nullptr;
+    g.timeout_ns = (uint64_t)timeout_ns_;
+    g.status = heap_->status_device();
+    g.trace = trace_;
+    g.sms = sms_;
+    ++epoch_;
+    cuda_check(b200::launch_gemm_local(g, stream), "gemm_local launch");
+  }
+  // Cut tiles meet in a workspace, one per stream because calls on two streams may overlap; at most four, kept with
+  // the operator.  Null (no tile is cut then) for further streams, and for a stream first seen while it is being
+  // captured: zeroing the counters would become part of the graph.
+  struct LocalWorkspace {
+    cudaStream_t stream;
+    at::Tensor keep;
+    float* partials;
+    uint32_t* counters;
+  };
+  const LocalWorkspace* local_workspace(cudaStream_t stream) {
+    for (const auto& ws : workspaces_)
+      if (ws.stream == stream) return &ws;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (workspaces_.size() >= 4 || cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
+      return nullptr;
+    LocalWorkspace ws;
+    ws.stream = stream;
+    ws.keep = at::detail::empty_cuda({(int64_t)(b200::kGemmLocalPartialBytes + 4 * b200::kGemmLocalCounters)}, at::kByte,
+                                     at::Device(at::kCUDA, (c10::DeviceIndex)heap_->device()), c10::nullopt);
+    uint8_t* base = ws.keep.mutable_data_ptr<uint8_t>();
+    ws.partials = reinterpret_cast<float*>(base);
+    ws.counters = reinterpret_cast<uint32_t*>(base + b200::kGemmLocalPartialBytes);
+    cuda_check(cudaMemsetAsync(ws.counters, 0, 4 * b200::kGemmLocalCounters, stream), "gemm_local workspace");
+    workspaces_.push_back(std::move(ws));
+    return &workspaces_.back();
+  }
+
   b200::GemmRsPlan cached_plan(int M, int N, int K) {
     for (const auto& e : plans_)
       if (e.M == M && e.N == N && e.K == K && e.block_n == block_n && e.cta_pair == cta_pair && e.splits == splits) return e.plan;
@@ -725,6 +807,8 @@ class GemmRsEngine {
   uint64_t* trace_ = nullptr;
   at::Tensor trace_keep_;
   std::vector<PlanEntry> plans_;
+  std::vector<LocalWorkspace> workspaces_;
+  int sms_ = 148;
   std::shared_ptr<b200::McastRegion> mcast_;
 };
 
@@ -1227,6 +1311,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            py::arg("counter_bytes"), py::arg("timeout_ns"))
       .def("run", &GemmRsEngine::run, py::arg("a"), py::arg("w"), py::arg("bias"), py::arg("out"),
            py::arg("bias_at_source") = true, py::arg("bias_scale") = 1.0)
+      .def("try_run", &GemmRsEngine::try_run)
       .def("plan", &GemmRsEngine::plan)
       .def("set_trace", &GemmRsEngine::set_trace)
       .def("restart_epochs", &GemmRsEngine::restart_epochs)

@@ -1,0 +1,964 @@
+// GEMM (+ bias) of one rank for sm_100a: out[M, N] = A[M, K] . W[N, K]^T, bf16 in and out, fp32 accumulation.
+//
+// Both kernels multiply rows of one operand (the "P side", a tensor-memory lane per row) by rows of the other (the
+// "Q side", accumulator columns):
+//   normal   P = A (tokens), Q = W (features): a lane holds a run of one output row
+//   swapped  P = W, Q = A: for few tokens, so that the 128-row side is full and the tile is as wide as the batch
+// The width `bn` of the Q side is a runtime value (a multiple of 32): the instruction descriptor, the copy boxes and
+// the number of pipeline stages follow it.
+//
+//   gemm_tile_kernel   problems of about one wave: one CTA per tile of 128 or 256 P rows; where there are fewer tiles
+//                      than SMs, a cluster of CTAs shares a tile, each with a part of K, and adds the parts up through
+//                      distributed shared memory.
+//   gemm_pair_kernel   larger ones: persistent CTA pairs (cta_group::2) on tiles of 256 P rows; the last wave, which
+//                      would leave pairs idle, is dealt out by k-blocks instead of by tiles.
+//
+// Warp roles of both (320 threads, one CTA per SM): 0 TMA producer, 1 MMA issuer, 2..9 epilogue, two per
+// tensor-memory lane quarter.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+
+#include "gemm_rs.h"
+#include "signal.cuh"
+#include "sm100_ptx.cuh"
+#include "tensor_map.h"
+
+namespace b200 {
+
+namespace {
+
+constexpr int kPRows = 128;                  // P rows per CTA
+constexpr int kBK = 64;                      // 64 bf16 = one 128-byte swizzled row
+constexpr int kPBytes = kPRows * kBK * 2;
+constexpr int kEpiWarps = 8;
+constexpr int kThreads = 64 + 32 * kEpiWarps;
+constexpr int kMaxStages = 12;
+constexpr int kSlabBytes = 4096;             // per epilogue warp: 32 rows x 128 bytes on their way to global memory
+constexpr int kTailBytes = kEpiWarps * kSlabBytes + kEpiWarps * 64 * 2 + 256;  // slabs, bias values, barriers
+constexpr int kMaxDynamicSmem = 232448 - 256;  // 227 KiB less what is static
+constexpr int kAccCols = 256;                // tensor-memory columns between the two accumulators
+constexpr int kTmemCols = 512;
+
+// CTA tiles of gemm_tile_kernel: 128 P rows, 256 P rows, or half of a pair's 256.
+constexpr int kOne = 1, kTwo = 2, kPair = 3;
+
+struct LocalParams {
+  const __nv_bfloat16* bias;
+  float bias_scale;
+  int bias_mode;      // 0 none, 1 added to the rounded product (then rounded again), 2 added in fp32
+  __nv_bfloat16* out; // [M, N]
+  int N;
+  int P, Q;           // rows of the two operands
+  int num_kb;
+  int p_tiles, q_tiles, band, bn, stages;
+  int rows;           // tile kernel: P rows of a CTA's tile (kTwo: of each half), at most 128
+  int splits;         // tile kernel: CTAs (or pairs) of a cluster that share a tile
+  int part_bytes;     // tile kernel: shared memory of its own for their parts (0: they take the pipeline's)
+  int sk_tiles, total_tiles;  // pair kernel
+  float* partials;    // pair kernel: [2][pair][cta][bn / 32][8][128 rows] float4
+  int64_t far_part;   // float4s between the two halves of `partials`
+  uint32_t* counters; // pair kernel: [sk_tiles][cta][epilogue warp], zero between launches
+  uint64_t timeout_ns;
+  StatusBlock* status;
+  uint64_t* trace;    // optional [gridDim.x][8]: 0 start, 1 ready, 2 tiles done, 3 exit
+};
+
+__device__ __forceinline__ void stamp(const LocalParams& p, int slot) {
+  if (p.trace != nullptr) p.trace[(size_t)blockIdx.x * 8 + slot] = global_timer_ns();
+}
+
+__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* abort, const LocalParams& p, int detail) {
+  if (ptx::mbar_try_wait(bar, parity)) return true;
+  const uint64_t t0 = global_timer_ns();
+  uint32_t spins = 0;
+  while (!ptx::mbar_try_wait(bar, parity)) {
+    if ((++spins & 255u) == 0) {
+      if (*abort) return false;
+      if (global_timer_ns() - t0 > p.timeout_ns) {
+        record_status(p.status, STATUS_TIMEOUT, PHASE_GEMM_PIPELINE, -1, detail, 0, parity);
+        *abort = 1;
+        return false;
+      }
+    }
+  }
+  return true;
+}
+
+// The k-block runs of one pair, in the order in which every warp role goes through them: first its share of the cut
+// tiles (so that their reductions hide behind the whole tiles), then its whole tiles.
+struct Segments {
+  int tile, kb0, kb1;
+  int u, u1, next_whole;
+  __device__ __forceinline__ void init(const LocalParams& p, int pair, int pairs) {
+    const long long units = (long long)p.sk_tiles * p.num_kb;
+    u = (int)(units * pair / pairs);
+    u1 = (int)(units * (pair + 1) / pairs);
+    next_whole = p.sk_tiles + pair;
+  }
+  __device__ __forceinline__ bool next(const LocalParams& p, int pairs) {
+    if (u < u1) {
+      tile = u / p.num_kb;
+      kb0 = u - tile * p.num_kb;
+      kb1 = min(p.num_kb, kb0 + (u1 - u));
+      u += kb1 - kb0;
+      return true;
+    }
+    tile = next_whole;
+    kb0 = 0;
+    kb1 = p.num_kb;
+    next_whole += pairs;
+    return tile < p.total_tiles;
+  }
+};
+
+// Tiles are visited in bands of `band` P tiles, Q tile by Q tile, so that pairs at work at the same time share operands in L2.
+__device__ __forceinline__ void tile_coords(const LocalParams& p, int tile, int& pt, int& qt) {
+  const int per_band = p.band * p.q_tiles;
+  const int b = tile / per_band;
+  const int start = b * p.band;
+  const int size = min(p.band, p.p_tiles - start);
+  const int within = tile - start * p.q_tiles;
+  qt = within / size;
+  pt = start + within - qt * size;
+}
+
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+__device__ __forceinline__ float with_bias(float v, float b, int mode) {
+  if (mode == 1) return __bfloat162float(__float2bfloat16_rn(v)) + b;
+  return v + b;
+}
+
+// Where an epilogue warp stands: its slab and bias values in shared memory, and how many groups it has sent off.
+struct Emit {
+  uint32_t slab, bias;
+  uint32_t stores = 0;
+};
+
+__device__ __forceinline__ float bias_of_lane(const LocalParams& p, int feature) {
+  if (p.bias_mode == 0 || feature >= p.N) return 0.f;
+  const float b = __bfloat162float(p.bias[feature]);
+  return p.bias_mode == 2 ? b * p.bias_scale : b;
+}
+
+// bias value e of packed bf16 words
+__device__ __forceinline__ float bias_of_word(const LocalParams& p, const uint32_t* words, int e) {
+  const float b = __uint_as_float((e & 1) ? (words[e >> 1] & 0xffff0000u) : (words[e >> 1] << 16));
+  return p.bias_mode == 2 ? b * p.bias_scale : b;
+}
+
+// One column group of a warp's 32 rows -- 64 columns, or 32 when swapped -- from fp32 to the result: bias, rounding,
+// through the warp's slab, out by TMA (which clips what lies outside the result).  chunk(c, v) gives 32 columns.
+template <bool SWAP, typename F>
+__device__ __forceinline__ void emit_group(const LocalParams& p, const CUtensorMap* map_out, Emit& em, int g, int prow, int qrow,
+                                           float lane_bias, int lane, F&& chunk) {
+  constexpr int kGroupChunks = SWAP ? 1 : 2;
+  const uint32_t buf = SWAP ? em.slab + (em.stores & 1u) * (kSlabBytes / 2) : em.slab;
+  ++em.stores;
+  if (!SWAP && p.bias_mode != 0) {
+    const int n = qrow + g * 64 + 2 * lane;  // N is a multiple of 8: both values or none
+    const uint32_t two = n < p.Q ? *reinterpret_cast<const uint32_t*>(p.bias + n) : 0u;
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(em.bias + (uint32_t)lane * 4u), "r"(two) : "memory");
+  }
+  if (lane == 0) {  // the store that used this buffer has read it
+    if (SWAP) ptx::bulk_wait_group_read<1>();
+    else ptx::bulk_wait_group_read<0>();
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int cc = 0; cc < kGroupChunks; ++cc) {
+    float v[32];
+    chunk(g * kGroupChunks + cc, v);
+    if (SWAP) {
+      // lane = feature, v[j] = token j of the chunk.  Two lanes exchange values so that each writes the feature
+      // pair of one of two tokens: rows of 64 bytes, 16 words per token, no bank conflict.
+      if (p.bias_mode != 0) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = with_bias(v[j], lane_bias, p.bias_mode);
+      }
+      const bool odd = lane & 1;
+#pragma unroll
+      for (int j = 0; j < 32; j += 2) {
+        const float mine = odd ? v[j + 1] : v[j];
+        const float other = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+        const uint32_t word = odd ? pack2(other, mine) : pack2(mine, other);
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(buf + (uint32_t)(j + (odd ? 1 : 0)) * 64u + (uint32_t)(lane >> 1) * 4u), "r"(word)
+                     : "memory");
+      }
+    } else {
+      if (p.bias_mode != 0) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          uint32_t two[2];
+          asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];"
+                       : "=r"(two[0]), "=r"(two[1])
+                       : "r"(em.bias + (uint32_t)(cc * 32 + j) * 2u));
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[j + e] = with_bias(v[j + e], bias_of_word(p, two, e), p.bias_mode);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {  // 16-byte piece cc * 4 + j of row `lane`, at the place the 128-byte swizzle wants it
+        const uint32_t at = buf + (uint32_t)lane * 128u + (uint32_t)(((cc * 4 + j) ^ (lane & 7)) << 4);
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(pack2(v[8 * j], v[8 * j + 1])),
+                     "r"(pack2(v[8 * j + 2], v[8 * j + 3])), "r"(pack2(v[8 * j + 4], v[8 * j + 5])),
+                     "r"(pack2(v[8 * j + 6], v[8 * j + 7]))
+                     : "memory");
+      }
+    }
+  }
+  ptx::fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    const int x = SWAP ? prow : qrow + g * 64;
+    const int y = SWAP ? qrow + g * 32 : prow;
+    if (x < (SWAP ? p.P : p.Q) && y < (SWAP ? p.Q : p.P)) ptx::tma_store_2d(map_out, buf, x, y);
+    ptx::bulk_commit_group();
+  }
+}
+
+__device__ __forceinline__ void load_chunk(uint32_t taddr, float (&v)[32]) {
+  uint32_t raw[32];
+  ptx::tmem_ld_32x32b_x32(taddr, raw);
+  ptx::tmem_ld_wait();
+#pragma unroll
+  for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
+}
+
+// After an abort: give copies still in flight time to land before shared memory is released.
+__device__ __forceinline__ void drain_after_abort() {
+  const uint64_t t0 = global_timer_ns();
+  while (global_timer_ns() - t0 < 200000) __nanosleep(1000);
+}
+
+}  // namespace
+
+template <bool SWAP>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
+                  const __grid_constant__ CUtensorMap map_out, const LocalParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ volatile int abort_flag;
+  __shared__ uint32_t tmem_base_shared;
+  const int tid = threadIdx.x;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform for the compiler too
+  const int lane = tid & 31;
+  if (tid == 0) stamp(p, 0);
+  const uint32_t cta = ptx::cluster_ctarank();
+  const bool leader = cta == 0;
+  const int pair = (int)blockIdx.x >> 1;
+  const int pairs = (int)gridDim.x >> 1;
+
+  const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t stage_bytes = kPBytes + (uint32_t)p.bn * (kBK * 2 / 2);  // this CTA's half of the Q rows
+  const uint32_t slabs = base + (uint32_t)p.stages * stage_bytes;
+  const uint32_t bias_smem = slabs + kEpiWarps * kSlabBytes;
+  const uint32_t bars = bias_smem + kEpiWarps * 64 * 2;
+  auto full_bar = [&](uint32_t s) { return bars + 8u * s; };
+  auto empty_bar = [&](uint32_t s) { return bars + 8u * (kMaxStages + s); };
+  auto tfull_bar = [&](uint32_t s) { return bars + 8u * (2 * kMaxStages + s); };
+  auto tempty_bar = [&](uint32_t s) { return bars + 8u * (2 * kMaxStages + 2 + s); };
+
+  if (tid == 0) {
+    abort_flag = 0;
+    for (int s = 0; s < p.stages; ++s) {
+      ptx::mbar_init(full_bar(s), 1);
+      ptx::mbar_init(empty_bar(s), 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      ptx::mbar_init(tfull_bar(s), 1);
+      ptx::mbar_init(tempty_bar(s), 2 * kEpiWarps);
+    }
+    ptx::fence_mbar_init();
+    ptx::fence_proxy_async_smem();
+    ptx::prefetch_tensormap(&map_p);
+    ptx::prefetch_tensormap(&map_q);
+    ptx::prefetch_tensormap(&map_out);
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc_pair(ptx::smem_u32(&tmem_base_shared), kTmemCols);
+    ptx::tmem_relinquish_pair();
+  }
+  ptx::tcgen05_fence_before();
+  __syncthreads();
+  ptx::cluster_sync_all();  // the other CTA's barriers exist before anything signals them
+  ptx::tcgen05_fence_after();
+  const uint32_t tmem_base = tmem_base_shared;
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
+  if (tid == 0) stamp(p, 1);
+
+  Segments seg;
+  seg.init(p, pair, pairs);
+
+  if (warp == 0) {
+    // ---- TMA producer: this CTA's 128 P rows and half of the Q rows of every k-block -----------------
+    uint32_t stage = 0, phase = 0;
+    while (!abort_flag && seg.next(p, pairs)) {
+      int pt, qt;
+      tile_coords(p, seg.tile, pt, qt);
+      const int py = pt * 256 + (int)cta * kPRows;
+      const int qy = qt * p.bn + (int)cta * (p.bn / 2);
+      for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
+        if (!wait_bar(empty_bar(stage), phase ^ 1u, &abort_flag, p, 100 + (int)stage)) break;
+        const uint32_t sp = base + stage * stage_bytes;
+        if (ptx::elect_one()) {
+          if (leader) ptx::mbar_arrive_expect_tx(full_bar(stage), 2 * stage_bytes);
+          ptx::tma_load_2d_pair(sp, &map_p, full_bar(stage), kb * kBK, py);
+          ptx::tma_load_2d_pair(sp + kPBytes, &map_q, full_bar(stage), kb * kBK, qy);
+        }
+        __syncwarp();
+        if (++stage == (uint32_t)p.stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---- MMA issuer: one lane of the leader drives both CTAs' tensor cores -----------------------------
+    if (leader) {
+      const uint32_t idesc = ptx::make_idesc_bf16_f32(256, p.bn);
+      uint32_t stage = 0, phase = 0, it = 0;
+      for (; !abort_flag && seg.next(p, pairs); ++it) {
+        const uint32_t acc = it & 1u;
+        if (!wait_bar(tempty_bar(acc), ((it >> 1) & 1u) ^ 1u, &abort_flag, p, 200 + (int)acc)) break;
+        ptx::tcgen05_fence_after();
+        const uint32_t d = tmem_base + acc * kAccCols;
+        bool ok = true;
+        for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
+          if (!wait_bar(full_bar(stage), phase, &abort_flag, p, 300 + (int)stage)) {
+            ok = false;
+            break;
+          }
+          ptx::tcgen05_fence_after();
+          const uint32_t sp = base + stage * stage_bytes;
+          const uint64_t dp = ptx::make_smem_desc_k_sw128(sp);
+          const uint64_t dq = ptx::make_smem_desc_k_sw128(sp + kPBytes);
+          if (ptx::elect_one()) {
+#pragma unroll
+            for (int j = 0; j < kBK / 16; ++j)  // 16 bf16 of K = 32 bytes = 2 descriptor address units
+              ptx::umma_bf16_pair(d, dp + 2u * j, dq + 2u * j, idesc, (kb > seg.kb0 || j > 0) ? 1u : 0u);
+            ptx::umma_commit_pair(empty_bar(stage), 3);
+          }
+          __syncwarp();
+          if (++stage == (uint32_t)p.stages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+        if (!ok) break;
+        if (ptx::elect_one()) ptx::umma_commit_pair(tfull_bar(acc), 3);
+        __syncwarp();
+      }
+    }
+  } else {
+    // ---- epilogue ----------------------------------------------------------------------------------------
+    const int ew = warp - 2;
+    const int q = warp & 3;       // tensor-memory lane quarter this warp may read
+    const int half = ew >> 2;
+    const int chunks = p.bn / 32;
+    // column groups: 2 chunks of 32 (normal), 1 (swapped); this warp takes every second one
+    constexpr int kGroupChunks = SWAP ? 1 : 2;
+    Emit em{slabs + (uint32_t)ew * kSlabBytes, bias_smem + (uint32_t)ew * 128u};
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
+    const size_t part_vecs = (size_t)chunks * 8 * kPRows;  // float4s of one CTA's half of a tile
+    uint32_t it = 0;
+    for (; !abort_flag && seg.next(p, pairs); ++it) {
+      const uint32_t acc = it & 1u;
+      int pt, qt;
+      tile_coords(p, seg.tile, pt, qt);
+      const int prow = pt * 256 + (int)cta * kPRows + q * 32;
+      const int qrow = qt * p.bn;
+      const float lane_bias = SWAP ? bias_of_lane(p, prow + lane) : 0.f;
+      // A cut tile has two contributors: the pair that starts it, as its last piece of cut work, and the next pair,
+      // as its first.  Whoever comes second, warp by warp, finds the other's accumulator in the workspace and
+      // finishes the tile; nobody waits.  (A sum of two terms is the same in either order.)
+      const bool cut = seg.kb1 - seg.kb0 < p.num_kb;
+      const int starter = pair - (seg.kb0 > 0 ? 1 : 0);
+      uint32_t* ctr = p.counters + ((size_t)(cut ? seg.tile : 0) * 2 + cta) * kEpiWarps + ew;
+      float4* part = reinterpret_cast<float4*>(p.partials) + ((size_t)(cut ? starter : 0) * 2 + cta) * part_vecs + q * 32 + lane;
+      int second = 0;
+      if (cut) {  // as a rule the starter is second, and this is known before its accumulator is complete
+        if (lane == 0) second = ld_acquire_gpu_u32(ctr) != 0;
+        second = __shfl_sync(0xffffffffu, second, 0);
+      }
+      if (!wait_bar(tfull_bar(acc), (it >> 1) & 1u, &abort_flag, p, 400 + (int)acc)) break;
+      ptx::tcgen05_fence_after();
+      const uint32_t acc_addr = lane_addr + acc * kAccCols;
+      auto release = [&]() {  // all reads of this accumulator are done
+        ptx::tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_cluster(tempty_bar(acc), 0);
+      };
+      bool own_in_tmem = true;
+      if (cut && !second) {
+        // Leave the accumulator: at the far end of the starter's block if it is the next pair's, so that both can
+        // be there at once.
+        float4* dst = part + (seg.kb0 > 0 ? 0 : (size_t)p.far_part);
+        for (int c = 0; c < chunks; ++c) {
+          if (((c / kGroupChunks) & 1) != half) continue;
+          float v[32];
+          load_chunk(acc_addr + c * 32, v);
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            __stcg(dst + (size_t)(c * 8 + j) * kPRows, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
+        }
+        release();
+        own_in_tmem = false;
+        __syncwarp();
+        if (lane == 0) {
+          __threadfence();
+          second = atomicAdd(ctr, 1u) != 0;  // the other one came meanwhile
+        }
+        second = __shfl_sync(0xffffffffu, second, 0);
+        if (!second) continue;
+      }
+      if (cut) {
+        if (lane == 0) {
+          __threadfence();  // what the other wrote before it counted itself in
+          *ctr = 0;
+        }
+        __syncwarp();
+      }
+      const float4* theirs = part + (seg.kb0 > 0 ? (size_t)p.far_part : 0);
+      const float4* mine = part + (seg.kb0 > 0 ? 0 : (size_t)p.far_part);
+      float4 ahead[8];
+      auto ask = [&](int c) {  // the other's share of a chunk, one chunk ahead of its use
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ahead[j] = __ldcg(theirs + (size_t)(c * 8 + j) * kPRows);
+      };
+      if (cut && half * kGroupChunks < chunks) ask(half * kGroupChunks);
+#pragma unroll 1
+      for (int g = half; g * kGroupChunks < chunks; g += 2) {
+        emit_group<SWAP>(p, &map_out, em, g, prow, qrow, lane_bias, lane, [&](int c, float (&v)[32]) {
+          if (own_in_tmem) {
+            load_chunk(acc_addr + c * 32, v);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(&v[4 * j]) = __ldcg(mine + (size_t)(c * 8 + j) * kPRows);
+          }
+          if (cut) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              v[4 * j] += ahead[j].x;
+              v[4 * j + 1] += ahead[j].y;
+              v[4 * j + 2] += ahead[j].z;
+              v[4 * j + 3] += ahead[j].w;
+            }
+            const int next = (c + 1) / kGroupChunks == g ? c + 1 : (g + 2) * kGroupChunks;
+            if (next < chunks) ask(next);
+          }
+        });
+      }
+      if (own_in_tmem) release();
+    }
+    if (lane == 0) ptx::bulk_wait_group_read<0>();
+    if (tid == 64) stamp(p, 2);
+  }
+
+  if (abort_flag) drain_after_abort();
+  __syncwarp();
+  ptx::tcgen05_fence_before();
+  __syncthreads();
+  ptx::cluster_sync_all();  // neither CTA retires while the other may still signal its barriers or read its memory
+  ptx::tcgen05_fence_after();
+  if (warp == 1) ptx::tmem_dealloc_pair(tmem_base, kTmemCols);
+  if (tid == 0) stamp(p, 3);
+}
+
+// One tile per CTA, 128 P rows by bn columns (kOne) or 256 (kTwo), or per CTA pair, 256 rows (kPair).  With `splits` > 1
+// a cluster shares the tile, each CTA or pair over its part of K.  When its part is complete, a CTA stores the
+// columns that other members finish straight into their shared memory; after one cluster barrier every member adds
+// up its columns in the order of K and writes them.  No workspace, no flags in global memory.
+template <bool SWAP, int SHAPE>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
+                 const __grid_constant__ CUtensorMap map_out, const LocalParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ volatile int abort_flag;
+  __shared__ uint32_t tmem_base_shared;
+  const int tid = threadIdx.x;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform for the compiler too
+  const int lane = tid & 31;
+  if (tid == 0) stamp(p, 0);
+  constexpr int RB = SHAPE == kTwo ? 2 : 1;
+  constexpr bool PAIR = SHAPE == kPair;
+  const int splits = p.splits;
+  const int cluster_rank = PAIR || splits > 1 ? (int)ptx::cluster_ctarank() : 0;
+  const int rank = PAIR ? cluster_rank >> 1 : cluster_rank;  // which part of K
+  const int cta = PAIR ? cluster_rank & 1 : 0;               // which half of the pair's rows
+  const int tile = (int)blockIdx.x / (PAIR ? 2 * splits : splits);
+  const int kb0 = (int)((int64_t)p.num_kb * rank / splits);
+  const int kb1 = (int)((int64_t)p.num_kb * (rank + 1) / splits);
+
+  const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+  const int q_rows = PAIR ? p.bn / 2 : p.bn;  // Q rows that this CTA brings in
+  const uint32_t p_bytes = (uint32_t)p.rows * (kBK * 2);
+  const uint32_t stage_bytes = RB * p_bytes + (uint32_t)q_rows * (kBK * 2);
+  const uint32_t slabs = base + (uint32_t)p.stages * stage_bytes;
+  const uint32_t bias_smem = slabs + kEpiWarps * kSlabBytes;
+  const uint32_t bars = bias_smem + kEpiWarps * 64 * 2;
+  const uint32_t parts = p.part_bytes > 0 ? bars + 256u : base;  // what the other members of the cluster send here
+  auto full_bar = [&](uint32_t s) { return bars + 8u * s; };
+  auto empty_bar = [&](uint32_t s) { return bars + 8u * (kMaxStages + s); };
+  const uint32_t done_bar = bars + 8u * (2 * kMaxStages);
+
+  if (tid == 0) {
+    abort_flag = 0;
+    for (int s = 0; s < p.stages; ++s) {
+      ptx::mbar_init(full_bar(s), 1);
+      ptx::mbar_init(empty_bar(s), 1);
+    }
+    ptx::mbar_init(done_bar, 1);
+    ptx::fence_mbar_init();
+    ptx::fence_proxy_async_smem();
+    ptx::prefetch_tensormap(&map_p);
+    ptx::prefetch_tensormap(&map_q);
+    ptx::prefetch_tensormap(&map_out);
+  }
+  if (warp == 1) {
+    if (PAIR) {
+      ptx::tmem_alloc_pair(ptx::smem_u32(&tmem_base_shared), kTmemCols);
+      ptx::tmem_relinquish_pair();
+    } else {
+      ptx::tmem_alloc(ptx::smem_u32(&tmem_base_shared), kTmemCols);
+      ptx::tmem_relinquish();
+    }
+  }
+  ptx::tcgen05_fence_before();
+  __syncthreads();
+  if (PAIR || splits > 1) ptx::cluster_sync_all();  // every member runs before anything is stored into its memory
+  ptx::tcgen05_fence_after();
+  const uint32_t tmem_base = tmem_base_shared;
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
+  if (tid == 0) stamp(p, 1);
+
+  int pt, qt;
+  tile_coords(p, tile, pt, qt);
+  const int p0 = (pt * (PAIR ? 2 : RB) + cta) * p.rows;
+  const int p_end = min(p.P, p0 + RB * p.rows);
+  const int q0 = qt * p.bn;
+
+  if (warp == 0) {
+    uint32_t stage = 0, phase = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (!wait_bar(empty_bar(stage), phase ^ 1u, &abort_flag, p, 100 + (int)stage)) break;
+      const uint32_t sp = base + stage * stage_bytes;
+      if (ptx::elect_one()) {
+        if (PAIR) {
+          if (cta == 0) ptx::mbar_arrive_expect_tx(full_bar(stage), 2 * stage_bytes);
+          ptx::tma_load_2d_pair(sp, &map_p, full_bar(stage), kb * kBK, p0);
+          ptx::tma_load_2d_pair(sp + p_bytes, &map_q, full_bar(stage), kb * kBK, q0 + cta * q_rows);
+        } else {
+          ptx::mbar_arrive_expect_tx(full_bar(stage), stage_bytes);
+#pragma unroll
+          for (int r = 0; r < RB; ++r) ptx::tma_load_2d(sp + r * p_bytes, &map_p, full_bar(stage), kb * kBK, p0 + r * p.rows);
+          ptx::tma_load_2d(sp + RB * p_bytes, &map_q, full_bar(stage), kb * kBK, q0);
+        }
+      }
+      __syncwarp();
+      if (++stage == (uint32_t)p.stages) {
+        stage = 0;
+        phase ^= 1u;
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (cta == 0) {
+      const uint32_t idesc = ptx::make_idesc_bf16_f32(PAIR ? 256 : kPRows, p.bn);
+      const uint16_t both = (uint16_t)(3u << (2 * rank));  // the pair's CTAs in the cluster
+      uint32_t stage = 0, phase = 0;
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        ok = wait_bar(full_bar(stage), phase, &abort_flag, p, 300 + (int)stage);
+        if (!ok) break;
+        ptx::tcgen05_fence_after();
+        const uint32_t sp = base + stage * stage_bytes;
+        // (a tile of fewer than 128 rows is followed by other data: it gives rows of the accumulator nobody reads)
+        const uint64_t dq = ptx::make_smem_desc_k_sw128(sp + RB * p_bytes);
+        if (ptx::elect_one()) {
+#pragma unroll
+          for (int r = 0; r < RB; ++r) {
+            const uint64_t dp = ptx::make_smem_desc_k_sw128(sp + r * p_bytes);
+#pragma unroll
+            for (int j = 0; j < kBK / 16; ++j) {  // 16 bf16 of K = 32 bytes = 2 descriptor address units
+              const uint32_t more = (kb > kb0 || j > 0) ? 1u : 0u;
+              if (PAIR) ptx::umma_bf16_pair(tmem_base, dp + 2u * j, dq + 2u * j, idesc, more);
+              else ptx::umma_bf16(tmem_base + r * kAccCols, dp + 2u * j, dq + 2u * j, idesc, more);
+            }
+          }
+          if (PAIR) ptx::umma_commit_pair(empty_bar(stage), both);
+          else ptx::umma_commit(empty_bar(stage));
+        }
+        __syncwarp();
+        if (++stage == (uint32_t)p.stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+      if (ok && ptx::elect_one()) {
+        if (PAIR) ptx::umma_commit_pair(done_bar, both);
+        else ptx::umma_commit(done_bar);
+        stamp(p, 5);
+      }
+    }
+    __syncwarp();
+  }
+
+  const int ew = warp - 2;
+  const int q = warp & 3;
+  const int half = ew >> 2;
+  const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
+  bool alive = true;
+  if (warp >= 2) {
+    // RB == 2: a warp takes all columns of one row block; else every second column group
+    const int row_block = RB == 2 ? half : 0;
+    const int prow = p0 + row_block * p.rows + q * 32;
+    const float lane_bias = SWAP ? bias_of_lane(p, prow + lane) : 0.f;
+    alive = wait_bar(done_bar, 0, &abort_flag, p, 400);
+    ptx::tcgen05_fence_after();
+    if (tid == 64) stamp(p, 6);
+    if (splits == 1 && alive && q * 32 < p.rows) {  // not split: whole groups of 32 rows
+      Emit em{slabs + (uint32_t)ew * kSlabBytes, bias_smem + (uint32_t)ew * 128u};
+      for (int g = RB == 2 ? 0 : half; g * (SWAP ? 1 : 2) < p.bn / 32; g += RB == 2 ? 1 : 2)
+        emit_group<SWAP>(p, &map_out, em, g, prow, q0, lane_bias, lane, [&](int c, float (&v)[32]) {
+          load_chunk(lane_addr + row_block * kAccCols + c * 32, v);
+        });
+      if (lane == 0) ptx::bulk_wait_group_read<0>();
+    }
+  }
+
+  if (SHAPE != kTwo && splits > 1) {
+    // columns [r * per, (r + 1) * per) are finished by member r; its memory holds [member][per / 4][128 rows] float4
+    const int per = ((p.bn / 8 + splits - 1) / splits) * 8;
+    if (p.part_bytes == 0) ptx::cluster_sync_all();  // every member is done with the stages that the parts go into
+    if (warp >= 2 && alive && q * 32 < p.rows) {
+      for (int c = half; c < p.bn / 32; c += 2) {
+        float v[32];
+        load_chunk(lane_addr + c * 32, v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int col = c * 32 + j * 8;
+          const int owner = col / per;
+          const uint32_t to = (uint32_t)(PAIR ? 2 * owner + cta : owner);
+          const uint32_t at = parts + (uint32_t)((rank * (per / 4) + (col - owner * per) / 4) * kPRows + q * 32 + lane) * 16u;
+          ptx::st_cluster_v4(at, to, v[8 * j], v[8 * j + 1], v[8 * j + 2], v[8 * j + 3]);
+          ptx::st_cluster_v4(at + kPRows * 16u, to, v[8 * j + 4], v[8 * j + 5], v[8 * j + 6], v[8 * j + 7]);
+        }
+      }
+    }
+    __syncwarp();
+    ptx::cluster_sync_all();
+    if (warp >= 2 && alive && q * 32 < p.rows) {
+      const int c_lo = rank * per;
+      const int c_hi = min(p.bn, c_lo + per);
+      const int prow = p0 + q * 32 + lane;
+      const float lane_bias = SWAP ? bias_of_lane(p, prow) : 0.f;
+      for (int col = c_lo + half * 8; col < c_hi; col += 16) {
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = 0.f;
+        const uint32_t at = parts + (uint32_t)(((col - c_lo) / 4) * kPRows + q * 32 + lane) * 16u;
+        for (int m = 0; m < splits; ++m) {  // ascending k
+          const uint32_t from = at + (uint32_t)m * (uint32_t)(per / 4) * kPRows * 16u;
+          float f[8];
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]) : "r"(from));
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "r"(from + kPRows * 16u));
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] += f[e];
+        }
+        if (prow >= p_end) continue;
+        const int qc = q0 + col;
+        if (SWAP) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            if (qc + e >= p.Q) break;
+            p.out[(size_t)(qc + e) * p.N + prow] = __float2bfloat16_rn(p.bias_mode ? with_bias(v[e], lane_bias, p.bias_mode) : v[e]);
+          }
+        } else if (qc < p.Q) {  // N is a multiple of 8: all eight or none
+          if (p.bias_mode != 0) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(p.bias + qc);
+            const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = with_bias(v[e], bias_of_word(p, words, e), p.bias_mode);
+          }
+          *reinterpret_cast<uint4*>(p.out + (size_t)prow * p.N + qc) =
+              make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+        }
+      }
+    }
+  }
+  if (tid == 64) stamp(p, 2);
+
+  if (abort_flag) drain_after_abort();
+  __syncwarp();
+  ptx::tcgen05_fence_before();
+  __syncthreads();
+  // neither CTA of a pair retires while the other may still signal its barriers or read its memory
+  if (PAIR && splits == 1) ptx::cluster_sync_all();
+  ptx::tcgen05_fence_after();
+  if (warp == 1) {
+    if (PAIR) ptx::tmem_dealloc_pair(tmem_base, kTmemCols);
+    else ptx::tmem_dealloc(tmem_base, kTmemCols);
+  }
+  if (tid == 0) stamp(p, 3);
+}
+
+// ---------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------
+namespace {
+
+int env_int(const char* name, int dflt) {
+  const char* v = getenv(name);
+  return v ? atoi(v) : dflt;
+}
+
+constexpr int kMaxSplits = 16;
+
+struct Plan {
+  bool persistent = false, swap = false;
+  int shape = kOne, rows = 128, bn = 256, splits = 1;  // tile kernel
+  int pairs = 1, sk_tiles = 0;             // pair kernel
+  int p_tiles = 0, q_tiles = 0;
+  double ns = 1e300;
+};
+
+int ctas_of(const Plan& p) { return p.splits * (p.shape == kPair ? 2 : 1); }  // CTAs that share a tile
+
+// How many clusters of `size` tile-kernel CTAs are resident at once (all of a CTA's shared memory in use).
+int cluster_capacity(int size) {
+  struct PerDevice {
+    int n[kMaxSplits + 1] = {0};
+  };
+  static thread_local PerDevice cache[16];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int& n = cache[dev & 15].n[size];
+  if (n > 0) return n;
+  auto kernel = gemm_tile_kernel<true, kOne>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(size * 16));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kMaxDynamicSmem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)size;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    n = size <= 8 ? std::max(1, 100 / size) : 1;
+  }
+  return n;
+}
+
+// Time model in ns.  What it charges, measured on a B200: a 128-byte row of a k-block takes an SM 1 ns to bring in from
+// L2 and 2.4 ns from HBM (the copy engine of an SM keeps about 500 rows in flight); 128 x 256 x 64 takes a tensor core
+// 270 ns, and all of them together 1.6 PFLOP/s (the power limit); 6.3 TB/s of HBM; a launch, the first operands' way
+// in and the result's way out 5 us.
+Plan make_local_plan(int M, int N, int K, int sms) {
+  const int num_kb = (K + kBK - 1) / kBK;
+  const double dram_ns = 2.0 * ((double)M * K + (double)N * K + (double)M * N) / 6300.0;
+  Plan best;
+  auto keep = [&](const Plan& p) {
+    if (p.ns < best.ns) best = p;
+  };
+  // ns for a CTA to bring in one k-block of a tile
+  auto load_ns = [](const Plan& p, double p_rows, double q_rows) {
+    return p_rows * (1.0 + 1.4 / p.q_tiles) + q_rows * (1.0 + 1.4 / p.p_tiles);
+  };
+  const int f_pair = env_int("GL_PAIR", -1), f_swap = env_int("GL_SWAP", -1), f_bn = env_int("GL_BN", 0), f_rb = env_int("GL_RB", 0),
+            f_s = env_int("GL_S", 0), f_sk = env_int("GL_SK", -1), f_r = env_int("GL_R", 0);
+  auto consider_tile = [&](bool swap, int shape, int bn) {
+    if (f_pair == 1 || (f_swap >= 0 && swap != (f_swap != 0)) || (f_bn && bn != f_bn) || (f_rb && shape != f_rb)) return;
+    Plan p;
+    p.swap = swap;
+    p.shape = shape;
+    p.bn = bn;
+    const int P = swap ? N : M;
+    const int ctas = shape == kOne ? 1 : 2;  // tile height in units of `rows`
+    p.q_tiles = ((swap ? M : N) + bn - 1) / bn;
+    for (int s = 1; s <= (shape == kTwo ? 1 : shape == kPair ? kMaxSplits / 2 : kMaxSplits); ++s) {
+      if ((s > 1 && s > num_kb) || (f_s && s != f_s)) continue;
+      p.splits = s;
+      const int cap = ctas_of(p) == 1 ? sms : cluster_capacity(ctas_of(p));
+      // Lower tiles when that many clusters fit at once and full ones would leave SMs without work: a share of the
+      // weight for everybody.  (Not split, tiles end on the 32 rows of an epilogue warp.)
+      p.rows = 128;
+      if (swap && shape != kTwo) {
+        const int step = s == 1 ? 32 : 8;
+        const int fit = (P + ctas * std::max(cap / p.q_tiles, 1) - 1) / (ctas * std::max(cap / p.q_tiles, 1));
+        p.rows = std::min(128, (fit + step - 1) / step * step);
+        if (f_r) p.rows = f_r;
+      }
+      p.p_tiles = (P + ctas * p.rows - 1) / (ctas * p.rows);
+      const int64_t tiles = (int64_t)p.p_tiles * p.q_tiles;
+      const double waves = std::ceil((double)tiles / cap);
+      if (waves > 4) continue;
+      const int kbs = (num_kb + s - 1) / s;
+      const double kb_ns = std::max(load_ns(p, (shape == kTwo ? 2.0 : 1.0) * p.rows, shape == kPair ? bn / 2 : bn),
+                                    270.0 * (shape == kTwo ? 2 : 1) * bn / 256.0);
+      const double power_ns = 2.0 * tiles * ctas * 128.0 * bn * (double)num_kb * kBK / 1.6e6;
+      const double out_ns = s == 1 ? 5.0 * bn : 600.0 + 5.0 * bn + 40.0 * s;
+      p.ns = std::max(std::max(waves * kbs * kb_ns, power_ns), dram_ns) + 5000.0 + waves * out_ns + (waves - 1) * 4000.0;
+      keep(p);
+    }
+  };
+  auto consider_pair = [&](bool swap, int bn) {
+    if (f_pair == 0 || (f_swap >= 0 && swap != (f_swap != 0)) || (f_bn && bn != f_bn)) return;
+    const int max_pairs = std::min(sms / 2, kGemmLocalMaxPairs);
+    Plan p;
+    p.persistent = true;
+    p.swap = swap;
+    p.bn = bn;
+    p.p_tiles = ((swap ? N : M) + 255) / 256;
+    p.q_tiles = ((swap ? M : N) + bn - 1) / bn;
+    const int64_t tiles = (int64_t)p.p_tiles * p.q_tiles;
+    p.pairs = (int)std::min<int64_t>(tiles, max_pairs);
+    const double power_ns = 2.0 * tiles * 256 * bn * (double)num_kb * kBK / 1.6e6;
+    const double kb_ns = std::max(load_ns(p, 128, bn / 2), 270.0 * bn / 256.0);
+    const double fixed = 5000.0 + 5.0 * bn;
+    p.sk_tiles = 0;
+    p.ns = std::max(std::max(std::ceil((double)tiles / p.pairs) * num_kb * kb_ns, power_ns), dram_ns) + fixed;
+    if (f_sk != 1) keep(p);
+    if (tiles > p.pairs && tiles % p.pairs != 0 && f_sk != 0) {
+      p.sk_tiles = (int)(tiles % p.pairs) + p.pairs;
+      p.ns = std::max(std::max((double)tiles / p.pairs * num_kb * kb_ns * 1.05, power_ns), dram_ns) + fixed + 2500.0;
+      keep(p);
+    }
+  };
+  for (int bn : {64, 128, 192, 256}) {
+    for (int shape : {kOne, kTwo, kPair}) consider_tile(false, shape, bn);
+    consider_pair(false, bn);
+  }
+  const int fewest = (M + 255) / 256;
+  for (int parts = fewest; parts <= std::min(fewest + 3, (M + 31) / 32); ++parts) {
+    const int bn = ((M + parts - 1) / parts + 31) / 32 * 32;
+    for (int shape : {kOne, kTwo, kPair}) consider_tile(true, shape, bn);
+    consider_pair(true, bn);
+  }
+  return best;
+}
+
+bool common_params(LocalParams& p, const GemmLocalArgs& a, const Plan& plan, int p_rows, int q_rows, CUtensorMap* map_p,
+                   CUtensorMap* map_q, CUtensorMap* map_out) {
+  const bool swap = plan.swap;
+  p = LocalParams{};
+  p.bias = reinterpret_cast<const __nv_bfloat16*>(a.bias);
+  p.bias_scale = a.bias_scale;
+  p.bias_mode = a.bias == nullptr ? 0 : (a.bias_at_source ? 1 : 2);
+  p.out = reinterpret_cast<__nv_bfloat16*>(a.out);
+  p.N = a.N;
+  p.P = swap ? a.N : a.M;
+  p.Q = swap ? a.M : a.N;
+  p.num_kb = (a.K + kBK - 1) / kBK;
+  p.p_tiles = plan.p_tiles;
+  p.q_tiles = plan.q_tiles;
+  p.band = std::min(env_int("GL_BAND", 8), plan.p_tiles);
+  p.bn = plan.bn;
+  p.rows = plan.rows;
+  p.splits = plan.splits;
+  p.timeout_ns = a.timeout_ns;
+  p.status = a.status;
+  p.trace = a.trace;
+  return make_tensor_map(map_p, swap ? a.w : a.a, (uint64_t)p.P, (uint64_t)a.K, 2, (uint32_t)p_rows, kBK, true) &&
+         make_tensor_map(map_q, swap ? a.a : a.w, (uint64_t)p.Q, (uint64_t)a.K, 2, (uint32_t)q_rows, kBK, true) &&
+         make_tensor_map(map_out, a.out, (uint64_t)a.M, (uint64_t)a.N, 2, 32, swap ? 32 : 64, !swap);
+}
+
+template <typename K>
+cudaError_t launch(K kernel, const LocalParams& p, int ctas, int cluster, size_t smem, cudaStream_t stream, const CUtensorMap& map_p,
+                   const CUtensorMap& map_q, const CUtensorMap& map_out) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, map_p, map_q, map_out, p);
+}
+
+template <bool SWAP>
+cudaError_t launch_pair(const GemmLocalArgs& a, const Plan& plan, cudaStream_t stream) {
+  LocalParams p;
+  CUtensorMap map_p, map_q, map_out;
+  if (!common_params(p, a, plan, kPRows, plan.bn / 2, &map_p, &map_q, &map_out)) return cudaErrorInvalidValue;
+  const int stage_bytes = kPBytes + plan.bn * kBK;
+  p.stages = std::min(kMaxStages, (kMaxDynamicSmem - 1024 - kTailBytes) / stage_bytes);
+  p.sk_tiles = plan.sk_tiles;
+  p.total_tiles = plan.p_tiles * plan.q_tiles;
+  p.partials = a.partials;
+  p.far_part = (int64_t)(kGemmLocalPartialBytes / 2 / 16);
+  p.counters = a.counters;
+  static const cudaError_t opted =
+      cudaFuncSetAttribute(gemm_pair_kernel<SWAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+  if (opted != cudaSuccess) return opted;
+  return launch(gemm_pair_kernel<SWAP>, p, 2 * plan.pairs, 2, 1024 + (size_t)p.stages * stage_bytes + kTailBytes, stream, map_p, map_q, map_out);
+}
+
+template <bool SWAP, int SHAPE>
+cudaError_t launch_tile(const GemmLocalArgs& a, const Plan& plan, cudaStream_t stream) {
+  LocalParams p;
+  CUtensorMap map_p, map_q, map_out;
+  const int q_rows = SHAPE == kPair ? plan.bn / 2 : plan.bn;
+  if (!common_params(p, a, plan, plan.rows, q_rows, &map_p, &map_q, &map_out)) return cudaErrorInvalidValue;
+  const int stage_bytes = ((SHAPE == kTwo ? 2 : 1) * plan.rows + q_rows) * kBK * 2;
+  int room = kMaxDynamicSmem - 1024 - kTailBytes;
+  if (plan.splits > 1) {
+    const int per = ((plan.bn / 8 + plan.splits - 1) / plan.splits) * 8;
+    p.part_bytes = plan.splits * per * kPRows * 4;
+    if ((room - p.part_bytes) / stage_bytes < 5) p.part_bytes = 0;  // too little left for the pipeline: share its memory
+    room -= p.part_bytes;
+  }
+  p.stages = std::min(env_int("GL_ST", kMaxStages), room / stage_bytes);
+  static const cudaError_t opted =
+      cudaFuncSetAttribute(gemm_tile_kernel<SWAP, SHAPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+  static const cudaError_t opted2 = cudaFuncSetAttribute(gemm_tile_kernel<SWAP, SHAPE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (opted != cudaSuccess || opted2 != cudaSuccess) return opted != cudaSuccess ? opted : opted2;
+  return launch(gemm_tile_kernel<SWAP, SHAPE>, p, plan.p_tiles * plan.q_tiles * ctas_of(plan), ctas_of(plan),
+                1024 + (size_t)p.stages * stage_bytes + kTailBytes + p.part_bytes, stream, map_p, map_q, map_out);
+}
+
+}  // namespace
+
+cudaError_t launch_gemm_local(const GemmLocalArgs& a, cudaStream_t stream) {
+  if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.K % 8 != 0 || a.N % 8 != 0) return cudaErrorInvalidValue;
+  Plan plan = make_local_plan(a.M, a.N, a.K, a.sms);
+  if (plan.ns > 1e299) return cudaErrorInvalidValue;
+  if (env_int("SHOW_GL", 0)) printf("plan persistent %d swap %d shape %d rows %d bn %d s %d pairs %d sk %d tiles %dx%d est %.1f us\n", plan.persistent, plan.swap, plan.shape, plan.rows, plan.bn, plan.splits, plan.pairs, plan.sk_tiles, plan.p_tiles, plan.q_tiles, plan.ns/1e3), fflush(stdout);
+  if (plan.persistent) {
+    if (a.partials == nullptr) plan.sk_tiles = 0;
+    return plan.swap ? launch_pair<true>(a, plan, stream) : launch_pair<false>(a, plan, stream);
+  }
+  switch (plan.shape) {
+    case kOne: return plan.swap ? launch_tile<true, kOne>(a, plan, stream) : launch_tile<false, kOne>(a, plan, stream);
+    case kTwo: return plan.swap ? launch_tile<true, kTwo>(a, plan, stream) : launch_tile<false, kTwo>(a, plan, stream);
+    default: return plan.swap ? launch_tile<true, kPair>(a, plan, stream) : launch_tile<false, kPair>(a, plan, stream);
+  }
+}
+
+}  // namespace b200

@@ -74,4 +74,29 @@ GemmRsPlan gemm_rs_plan(int M, int N, int K, int world_size, int block_n, int ct
 
 cudaError_t launch_gemm_rs(const GemmRsArgs& args, cudaStream_t stream);
 
+// One rank: nothing to scatter, so a GEMM without staging, signalling or reducers (gemm_local_sm100.cu).
+struct GemmLocalArgs {
+  const void* a;     // [M, K] bf16
+  const void* w;     // [N, K] bf16
+  const void* bias;  // [N] bf16 or nullptr
+  void* out;         // [M, N] bf16; all four 16-byte aligned
+  int M, N, K;
+  float bias_scale;
+  int bias_at_source;
+  float* partials;     // kGemmLocalPartialBytes, or nullptr: no tile is cut along K
+  uint32_t* counters;  // kGemmLocalCounters words, zero between launches; calls in flight at once need their own
+  uint64_t timeout_ns;
+  StatusBlock* status;
+  uint64_t* trace;
+  int sms;
+};
+
+constexpr int kGemmLocalMaxPairs = 80;
+// per CTA pair: two cut tiles, 256 rows x 256 columns of fp32
+constexpr uint64_t kGemmLocalPartialBytes = (uint64_t)kGemmLocalMaxPairs * 2 * 256 * 256 * 4;
+// per cut tile (at most two per pair): one per CTA and epilogue warp
+constexpr int kGemmLocalCounters = kGemmLocalMaxPairs * 2 * 2 * 8;
+
+cudaError_t launch_gemm_local(const GemmLocalArgs& args, cudaStream_t stream);
+
 }  // namespace b200

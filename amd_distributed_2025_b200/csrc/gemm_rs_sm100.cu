@@ -42,6 +42,7 @@
 #include "gemm_rs.h"
 #include "signal.cuh"
 #include "sm100_ptx.cuh"
+#include "tensor_map.h"
 
 namespace b200 {
 
@@ -1046,64 +1047,9 @@ gemm_rs_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
 // ---------------------------------------------------------------------------------------
 namespace {
 
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess ||
-        qres != cudaDriverEntryPointSuccess) {
-      return nullptr;
-    }
-    fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
-}
-
-// Row-major bf16 [rows, cols] tensor, box = [box_rows, 64 columns], 128-byte swizzle,
-// out-of-range elements read as zero.  Encoded maps are kept in a small per-thread cache:
-// a serving loop calls with the same weight (and often the same activation buffer) again
-// and again, and the driver call is a visible part of a short launch.
-bool make_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-  struct Entry {
-    const void* base;
-    uint64_t rows, cols;
-    uint32_t box_rows;
-    CUtensorMap map;
-  };
-  constexpr int kEntries = 64;
-  thread_local Entry cache[kEntries];
-  thread_local int used = 0, next = 0;
-  for (int i = 0; i < used; ++i) {
-    const Entry& e = cache[i];
-    if (e.base == base && e.rows == rows && e.cols == cols && e.box_rows == box_rows) {
-      *map = e.map;
-      return true;
-    }
-  }
-  EncodeTiledFn fn = get_encode_fn();
-  if (fn == nullptr) return false;
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {cols * 2};
-  cuuint32_t box[2] = {(cuuint32_t)BK, box_rows};
-  cuuint32_t elem_strides[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem_strides,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return false;
-  Entry& slot = cache[next];
-  slot.base = base;
-  slot.rows = rows;
-  slot.cols = cols;
-  slot.box_rows = box_rows;
-  slot.map = *map;
-  next = (next + 1) % kEntries;
-  if (used < kEntries) ++used;
-  return true;
+// Row-major bf16 [rows, cols] tensor, box = [box_rows, 64 columns], 128-byte swizzle.
+bool make_bf16_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+  return make_tensor_map(map, base, rows, cols, 2, box_rows, BK, true);
 }
 
 // Tile shape and K slicing from the problem size.  Cost model: waves of work items times
@@ -1160,8 +1106,8 @@ template <int BN, int CTAS>
 cudaError_t launch_typed(const GemmRsArgs& a, int sms, int splits, cudaStream_t stream) {
   using C = Cfg<BN, CTAS>;
   CUtensorMap map_a, map_b;
-  if (!make_tensor_map(&map_a, a.a, (uint64_t)a.M, (uint64_t)a.K, BM)) return cudaErrorInvalidValue;
-  if (!make_tensor_map(&map_b, a.w, (uint64_t)a.N, (uint64_t)a.K, C::kBRows)) return cudaErrorInvalidValue;
+  if (!make_bf16_map(&map_a, a.a, (uint64_t)a.M, (uint64_t)a.K, BM)) return cudaErrorInvalidValue;
+  if (!make_bf16_map(&map_b, a.w, (uint64_t)a.N, (uint64_t)a.K, C::kBRows)) return cudaErrorInvalidValue;
 
   KernelParams p;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(a.bias);
@@ -1214,14 +1160,14 @@ cudaError_t launch_typed(const GemmRsArgs& a, int sms, int splits, cudaStream_t 
   p.tma_store = 0;
   if (p.nvls && a.tma_store != 0) {
     p.tma_store = 1;
-    if (!make_tensor_map(&maps.m[0], reinterpret_cast<const void*>(a.nvls_local), (uint64_t)a.M, (uint64_t)a.N, 32))
+    if (!make_bf16_map(&maps.m[0], reinterpret_cast<const void*>(a.nvls_local), (uint64_t)a.M, (uint64_t)a.N, 32))
       return cudaErrorInvalidValue;
   } else if (a.world_size <= kMaxStageMaps && splits == 1 && !p.direct && p.rows_per_rank % 32 == 0 && a.tma_store != 0) {
     p.tma_store = 1;
     for (int o = 0; o < a.world_size; ++o) {
       const uint8_t* base = reinterpret_cast<const uint8_t*>(a.peer_base[o]) + a.off_stage +
                             (uint64_t)a.rank * p.rows_per_rank * a.N * 2ull;
-      if (!make_tensor_map(&maps.m[o], base, (uint64_t)p.rows_per_rank, (uint64_t)a.N, 32)) return cudaErrorInvalidValue;
+      if (!make_bf16_map(&maps.m[o], base, (uint64_t)p.rows_per_rank, (uint64_t)a.N, 32)) return cudaErrorInvalidValue;
     }
   }
 

@@ -12,6 +12,19 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// True in one lane of a converged warp.  Tensor-core and copy instructions take their operands from uniform
+// registers: a warp that runs its loop with all lanes and lets an elected lane issue has them there already, a
+// single lane in divergent code moves every operand over first (a 128 x 32 x 64 k-block: 300 ns, elected 100).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
+}
+
 // ---- mbarrier -------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -217,6 +230,15 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, uint32_t cta) 
       "mapa.shared::cluster.u32 remote, %0, %1;\n\t"
       "mbarrier.arrive.shared::cluster.b64 _, [remote];\n\t}"
       ::"r"(bar), "r"(cta)
+      : "memory");
+}
+// 16 bytes to the same shared-memory offset of CTA `cta` of the cluster.
+__device__ __forceinline__ void st_cluster_v4(uint32_t smem_addr, uint32_t cta, float a, float b, float c, float d) {
+  asm volatile(
+      "{\n\t.reg .b32 remote;\n\t"
+      "mapa.shared::cluster.u32 remote, %0, %1;\n\t"
+      "st.shared::cluster.v4.f32 [remote], {%2, %3, %4, %5};\n\t}"
+      ::"r"(smem_addr), "r"(cta), "f"(a), "f"(b), "f"(c), "f"(d)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_result, uint32_t ncols) {

@@ -1,0 +1,70 @@
+#include "tensor_map.h"
+
+#include <cuda_runtime.h>
+
+namespace b200 {
+
+namespace {
+
+using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_fn() {
+  static const EncodeTiledFn fn = [] {
+    void* ptr = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess ||
+        qres != cudaDriverEntryPointSuccess)
+      ptr = nullptr;
+    return reinterpret_cast<EncodeTiledFn>(ptr);
+  }();
+  return fn;
+}
+
+struct Key {
+  const void* base;
+  uint64_t rows, cols;
+  uint32_t elem_bytes, box_rows, box_cols, swizzle;
+  bool operator==(const Key& o) const {
+    return base == o.base && rows == o.rows && cols == o.cols && elem_bytes == o.elem_bytes && box_rows == o.box_rows &&
+           box_cols == o.box_cols && swizzle == o.swizzle;
+  }
+};
+
+}  // namespace
+
+bool make_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t elem_bytes, uint32_t box_rows,
+                     uint32_t box_cols, bool swizzle128) {
+  struct Entry {
+    Key key;
+    CUtensorMap map;
+  };
+  constexpr int kEntries = 64;
+  thread_local Entry cache[kEntries];
+  thread_local int used = 0, next = 0;
+  const Key key{base, rows, cols, elem_bytes, box_rows, box_cols, swizzle128 ? 1u : 0u};
+  for (int i = 0; i < used; ++i) {
+    if (cache[i].key == key) {
+      *map = cache[i].map;
+      return true;
+    }
+  }
+  const EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr || (elem_bytes != 1 && elem_bytes != 2)) return false;
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {cols * elem_bytes};
+  const cuuint32_t box[2] = {box_cols, box_rows};
+  const cuuint32_t elem_strides[2] = {1, 1};
+  const CUresult r = fn(map, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
+                        const_cast<void*>(base), dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return false;
+  cache[next] = Entry{key, *map};
+  next = (next + 1) % kEntries;
+  if (used < kEntries) ++used;
+  return true;
+}
+
+}  // namespace b200
