@@ -7,9 +7,9 @@
 // The width `bn` of the Q side is a runtime value (a multiple of 32): the instruction descriptor, the copy boxes and
 // the number of pipeline stages follow it.
 //
-//   gemm_tile_kernel   problems of about one wave: one CTA per tile of 128 or 256 P rows; where there are fewer tiles
-//                      than SMs, a cluster of CTAs shares a tile, each with a part of K, and adds the parts up through
-//                      distributed shared memory.
+//   gemm_tile_kernel   problems of about one wave: one CTA per tile of up to 128 P rows, or a pair (cta_group::2) per
+//                      256; where there are fewer tiles than SMs, a cluster of them shares a tile, each with a part of
+//                      K, and adds the parts up through distributed shared memory.
 //   gemm_pair_kernel   larger ones: persistent CTA pairs (cta_group::2) on tiles of 256 P rows; the last wave, which
 //                      would leave pairs idle, is dealt out by k-blocks instead of by tiles.
 //
@@ -22,8 +22,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstdio>
-#include <cstdlib>
 
 #include "gemm_rs.h"
 #include "signal.cuh"
@@ -46,9 +44,6 @@ constexpr int kMaxDynamicSmem = 232448 - 256;  // 227 KiB less what is static
 constexpr int kAccCols = 256;                // tensor-memory columns between the two accumulators
 constexpr int kTmemCols = 512;
 
-// CTA tiles of gemm_tile_kernel: 128 P rows, 256 P rows, or half of a pair's 256.
-constexpr int kOne = 1, kTwo = 2, kPair = 3;
-
 struct LocalParams {
   const __nv_bfloat16* bias;
   float bias_scale;
@@ -58,9 +53,10 @@ struct LocalParams {
   int P, Q;           // rows of the two operands
   int num_kb;
   int p_tiles, q_tiles, band, bn, stages;
-  int rows;           // tile kernel: P rows of a CTA's tile (kTwo: of each half), at most 128
+  int rows;           // tile kernel: P rows of a CTA's tile, at most 128
   int splits;         // tile kernel: CTAs (or pairs) of a cluster that share a tile
   int part_bytes;     // tile kernel: shared memory of its own for their parts (0: they take the pipeline's)
+  int stage_area;     // tile kernel: bytes of the pipeline's stages, and of the parts where these share them
   int sk_tiles, total_tiles;  // pair kernel
   float* partials;    // pair kernel: [2][pair][cta][bn / 32][8][128 rows] float4
   int64_t far_part;   // float4s between the two halves of `partials`
@@ -476,11 +472,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
   if (tid == 0) stamp(p, 3);
 }
 
-// One tile per CTA, 128 P rows by bn columns (kOne) or 256 (kTwo), or per CTA pair, 256 rows (kPair).  With `splits` > 1
-// a cluster shares the tile, each CTA or pair over its part of K.  When its part is complete, a CTA stores the
+// One tile per CTA, up to 128 P rows by bn columns, or per CTA pair, twice the rows.  With `splits` > 1 a cluster
+// shares the tile, each CTA or pair over its part of K.  When its part is complete, a CTA stores the
 // columns that other members finish straight into their shared memory; after one cluster barrier every member adds
 // up its columns in the order of K and writes them.  No workspace, no flags in global memory.
-template <bool SWAP, int SHAPE>
+template <bool SWAP, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
                  const __grid_constant__ CUtensorMap map_out, const LocalParams p) {
@@ -491,8 +487,6 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform for the compiler too
   const int lane = tid & 31;
   if (tid == 0) stamp(p, 0);
-  constexpr int RB = SHAPE == kTwo ? 2 : 1;
-  constexpr bool PAIR = SHAPE == kPair;
   const int splits = p.splits;
   const int cluster_rank = PAIR || splits > 1 ? (int)ptx::cluster_ctarank() : 0;
   const int rank = PAIR ? cluster_rank >> 1 : cluster_rank;  // which part of K
@@ -504,8 +498,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
   const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
   const int q_rows = PAIR ? p.bn / 2 : p.bn;  // Q rows that this CTA brings in
   const uint32_t p_bytes = (uint32_t)p.rows * (kBK * 2);
-  const uint32_t stage_bytes = RB * p_bytes + (uint32_t)q_rows * (kBK * 2);
-  const uint32_t slabs = base + (uint32_t)p.stages * stage_bytes;
+  const uint32_t stage_bytes = p_bytes + (uint32_t)q_rows * (kBK * 2);
+  const uint32_t slabs = base + (uint32_t)p.stage_area;
   const uint32_t bias_smem = slabs + kEpiWarps * kSlabBytes;
   const uint32_t bars = bias_smem + kEpiWarps * 64 * 2;
   const uint32_t parts = p.part_bytes > 0 ? bars + 256u : base;  // what the other members of the cluster send here
@@ -546,8 +540,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
 
   int pt, qt;
   tile_coords(p, tile, pt, qt);
-  const int p0 = (pt * (PAIR ? 2 : RB) + cta) * p.rows;
-  const int p_end = min(p.P, p0 + RB * p.rows);
+  const int p0 = (pt * (PAIR ? 2 : 1) + cta) * p.rows;
+  const int p_end = min(p.P, p0 + p.rows);
   const int q0 = qt * p.bn;
 
   if (warp == 0) {
@@ -562,9 +556,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
           ptx::tma_load_2d_pair(sp + p_bytes, &map_q, full_bar(stage), kb * kBK, q0 + cta * q_rows);
         } else {
           ptx::mbar_arrive_expect_tx(full_bar(stage), stage_bytes);
-#pragma unroll
-          for (int r = 0; r < RB; ++r) ptx::tma_load_2d(sp + r * p_bytes, &map_p, full_bar(stage), kb * kBK, p0 + r * p.rows);
-          ptx::tma_load_2d(sp + RB * p_bytes, &map_q, full_bar(stage), kb * kBK, q0);
+          ptx::tma_load_2d(sp, &map_p, full_bar(stage), kb * kBK, p0);
+          ptx::tma_load_2d(sp + p_bytes, &map_q, full_bar(stage), kb * kBK, q0);
         }
       }
       __syncwarp();
@@ -586,17 +579,14 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
         ptx::tcgen05_fence_after();
         const uint32_t sp = base + stage * stage_bytes;
         // (a tile of fewer than 128 rows is followed by other data: it gives rows of the accumulator nobody reads)
-        const uint64_t dq = ptx::make_smem_desc_k_sw128(sp + RB * p_bytes);
+        const uint64_t dq = ptx::make_smem_desc_k_sw128(sp + p_bytes);
+        const uint64_t dp = ptx::make_smem_desc_k_sw128(sp);
         if (ptx::elect_one()) {
 #pragma unroll
-          for (int r = 0; r < RB; ++r) {
-            const uint64_t dp = ptx::make_smem_desc_k_sw128(sp + r * p_bytes);
-#pragma unroll
-            for (int j = 0; j < kBK / 16; ++j) {  // 16 bf16 of K = 32 bytes = 2 descriptor address units
-              const uint32_t more = (kb > kb0 || j > 0) ? 1u : 0u;
-              if (PAIR) ptx::umma_bf16_pair(tmem_base, dp + 2u * j, dq + 2u * j, idesc, more);
-              else ptx::umma_bf16(tmem_base + r * kAccCols, dp + 2u * j, dq + 2u * j, idesc, more);
-            }
+          for (int j = 0; j < kBK / 16; ++j) {  // 16 bf16 of K = 32 bytes = 2 descriptor address units
+            const uint32_t more = (kb > kb0 || j > 0) ? 1u : 0u;
+            if (PAIR) ptx::umma_bf16_pair(tmem_base, dp + 2u * j, dq + 2u * j, idesc, more);
+            else ptx::umma_bf16(tmem_base, dp + 2u * j, dq + 2u * j, idesc, more);
           }
           if (PAIR) ptx::umma_commit_pair(empty_bar(stage), both);
           else ptx::umma_commit(empty_bar(stage));
@@ -610,7 +600,6 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
       if (ok && ptx::elect_one()) {
         if (PAIR) ptx::umma_commit_pair(done_bar, both);
         else ptx::umma_commit(done_bar);
-        stamp(p, 5);
       }
     }
     __syncwarp();
@@ -622,24 +611,20 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
   const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
   bool alive = true;
   if (warp >= 2) {
-    // RB == 2: a warp takes all columns of one row block; else every second column group
-    const int row_block = RB == 2 ? half : 0;
-    const int prow = p0 + row_block * p.rows + q * 32;
+    const int prow = p0 + q * 32;
     const float lane_bias = SWAP ? bias_of_lane(p, prow + lane) : 0.f;
     alive = wait_bar(done_bar, 0, &abort_flag, p, 400);
     ptx::tcgen05_fence_after();
-    if (tid == 64) stamp(p, 6);
     if (splits == 1 && alive && q * 32 < p.rows) {  // not split: whole groups of 32 rows
       Emit em{slabs + (uint32_t)ew * kSlabBytes, bias_smem + (uint32_t)ew * 128u};
-      for (int g = RB == 2 ? 0 : half; g * (SWAP ? 1 : 2) < p.bn / 32; g += RB == 2 ? 1 : 2)
-        emit_group<SWAP>(p, &map_out, em, g, prow, q0, lane_bias, lane, [&](int c, float (&v)[32]) {
-          load_chunk(lane_addr + row_block * kAccCols + c * 32, v);
-        });
+      for (int g = half; g * (SWAP ? 1 : 2) < p.bn / 32; g += 2)
+        emit_group<SWAP>(p, &map_out, em, g, prow, q0, lane_bias, lane,
+                         [&](int c, float (&v)[32]) { load_chunk(lane_addr + c * 32, v); });
       if (lane == 0) ptx::bulk_wait_group_read<0>();
     }
   }
 
-  if (SHAPE != kTwo && splits > 1) {
+  if (splits > 1) {
     // columns [r * per, (r + 1) * per) are finished by member r; its memory holds [member][per / 4][128 rows] float4
     const int per = ((p.bn / 8 + splits - 1) / splits) * 8;
     if (p.part_bytes == 0) ptx::cluster_sync_all();  // every member is done with the stages that the parts go into
@@ -720,22 +705,18 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
 // ---------------------------------------------------------------------------------------
 namespace {
 
-int env_int(const char* name, int dflt) {
-  const char* v = getenv(name);
-  return v ? atoi(v) : dflt;
-}
-
 constexpr int kMaxSplits = 16;
 
 struct Plan {
   bool persistent = false, swap = false;
-  int shape = kOne, rows = 128, bn = 256, splits = 1;  // tile kernel
-  int pairs = 1, sk_tiles = 0;             // pair kernel
+  bool pair = false;                  // tile kernel: a CTA pair per tile
+  int rows = 128, bn = 256, splits = 1;
+  int pairs = 1, sk_tiles = 0;        // pair kernel
   int p_tiles = 0, q_tiles = 0;
   double ns = 1e300;
 };
 
-int ctas_of(const Plan& p) { return p.splits * (p.shape == kPair ? 2 : 1); }  // CTAs that share a tile
+int ctas_of(const Plan& p) { return p.splits * (p.pair ? 2 : 1); }  // CTAs that share a tile
 
 // How many clusters of `size` tile-kernel CTAs are resident at once (all of a CTA's shared memory in use).
 int cluster_capacity(int size) {
@@ -747,7 +728,7 @@ int cluster_capacity(int size) {
   cudaGetDevice(&dev);
   int& n = cache[dev & 15].n[size];
   if (n > 0) return n;
-  auto kernel = gemm_tile_kernel<true, kOne>;
+  auto kernel = gemm_tile_kernel<true, false>;
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
   cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cudaLaunchConfig_t cfg = {};
@@ -768,61 +749,54 @@ int cluster_capacity(int size) {
   return n;
 }
 
-// Time model in ns.  What it charges, measured on a B200: a 128-byte row of a k-block takes an SM 1 ns to bring in from
-// L2 and 2.4 ns from HBM (the copy engine of an SM keeps about 500 rows in flight); 128 x 256 x 64 takes a tensor core
-// 270 ns, and all of them together 1.6 PFLOP/s (the power limit); 6.3 TB/s of HBM; a launch, the first operands' way
-// in and the result's way out 5 us.
+// Time model in ns.  What it charges, measured on a B200:
+//   a 128-byte row of a k-block takes an SM 1 ns to bring in, 1.6 when the rows of the matrix do not start on cache lines;
+//   128 x 256 x 64 takes a tensor core 280 ns, all tensor cores together do 1.55 PFLOP/s (the power limit); a k-block
+//   costs its issuing warp 150 ns and comes back for a stage after 1.7 us at the earliest; 6.6 TB/s of HBM; then what a launch costs before and after its k-blocks.
 Plan make_local_plan(int M, int N, int K, int sms) {
   const int num_kb = (K + kBK - 1) / kBK;
-  const double dram_ns = 2.0 * ((double)M * K + (double)N * K + (double)M * N) / 6300.0;
+  const double dram_ns = 2.0 * ((double)M * K + (double)N * K + (double)M * N) / 6600.0;
+  const double row_ns = K % kBK == 0 ? 1.0 : 1.6;
+  auto power_ns = [&](double rows, double cols) { return 2.0 * rows * cols * num_kb * kBK / 1.55e6; };
   Plan best;
   auto keep = [&](const Plan& p) {
     if (p.ns < best.ns) best = p;
   };
-  // ns for a CTA to bring in one k-block of a tile
-  auto load_ns = [](const Plan& p, double p_rows, double q_rows) {
-    return p_rows * (1.0 + 1.4 / p.q_tiles) + q_rows * (1.0 + 1.4 / p.p_tiles);
-  };
-  const int f_pair = env_int("GL_PAIR", -1), f_swap = env_int("GL_SWAP", -1), f_bn = env_int("GL_BN", 0), f_rb = env_int("GL_RB", 0),
-            f_s = env_int("GL_S", 0), f_sk = env_int("GL_SK", -1), f_r = env_int("GL_R", 0);
-  auto consider_tile = [&](bool swap, int shape, int bn) {
-    if (f_pair == 1 || (f_swap >= 0 && swap != (f_swap != 0)) || (f_bn && bn != f_bn) || (f_rb && shape != f_rb)) return;
+  auto consider_tile = [&](bool swap, bool pair, int bn) {
     Plan p;
     p.swap = swap;
-    p.shape = shape;
+    p.pair = pair;
     p.bn = bn;
     const int P = swap ? N : M;
-    const int ctas = shape == kOne ? 1 : 2;  // tile height in units of `rows`
+    const int halves = pair ? 2 : 1;  // tile height in units of `rows`
     p.q_tiles = ((swap ? M : N) + bn - 1) / bn;
-    for (int s = 1; s <= (shape == kTwo ? 1 : shape == kPair ? kMaxSplits / 2 : kMaxSplits); ++s) {
-      if ((s > 1 && s > num_kb) || (f_s && s != f_s)) continue;
+    for (int s = 1; s <= kMaxSplits / halves; ++s) {
+      if (s > 1 && s > num_kb) continue;
       p.splits = s;
       const int cap = ctas_of(p) == 1 ? sms : cluster_capacity(ctas_of(p));
       // Lower tiles when that many clusters fit at once and full ones would leave SMs without work: a share of the
       // weight for everybody.  (Not split, tiles end on the 32 rows of an epilogue warp.)
       p.rows = 128;
-      if (swap && shape != kTwo) {
+      if (swap) {
         const int step = s == 1 ? 32 : 8;
-        const int fit = (P + ctas * std::max(cap / p.q_tiles, 1) - 1) / (ctas * std::max(cap / p.q_tiles, 1));
-        p.rows = std::min(128, (fit + step - 1) / step * step);
-        if (f_r) p.rows = f_r;
+        const int fit = halves * std::max(cap / p.q_tiles, 1);
+        p.rows = std::min(128, ((P + fit - 1) / fit + step - 1) / step * step);
       }
-      p.p_tiles = (P + ctas * p.rows - 1) / (ctas * p.rows);
+      p.p_tiles = (P + halves * p.rows - 1) / (halves * p.rows);
       const int64_t tiles = (int64_t)p.p_tiles * p.q_tiles;
       const double waves = std::ceil((double)tiles / cap);
       if (waves > 4) continue;
       const int kbs = (num_kb + s - 1) / s;
-      const double kb_ns = std::max(load_ns(p, (shape == kTwo ? 2.0 : 1.0) * p.rows, shape == kPair ? bn / 2 : bn),
-                                    270.0 * (shape == kTwo ? 2 : 1) * bn / 256.0);
-      const double power_ns = 2.0 * tiles * ctas * 128.0 * bn * (double)num_kb * kBK / 1.6e6;
-      const double out_ns = s == 1 ? 5.0 * bn : 600.0 + 5.0 * bn + 40.0 * s;
-      p.ns = std::max(std::max(waves * kbs * kb_ns, power_ns), dram_ns) + 5000.0 + waves * out_ns + (waves - 1) * 4000.0;
+      const int q_rows = bn / halves;
+      const int stages = std::min(kMaxStages, (kMaxDynamicSmem - 1024 - kTailBytes) / ((p.rows + q_rows) * kBK * 2));
+      const double kb_ns = std::max({row_ns * (p.rows + q_rows), 280.0 * bn / 256.0, 150.0, 1700.0 / stages});
+      const double ends_ns = (s == 1 ? 3000.0 + 9.0 * bn : 4800.0 + 28.0 * std::max(bn - 64, 0) + 50.0 * s) + (pair ? 400.0 : 0.0);
+      p.ns = std::max({waves * kbs * kb_ns, power_ns((double)p.p_tiles * halves * 128, (double)p.q_tiles * bn), dram_ns}) + ends_ns +
+             (waves - 1) * 4000.0;
       keep(p);
     }
   };
   auto consider_pair = [&](bool swap, int bn) {
-    if (f_pair == 0 || (f_swap >= 0 && swap != (f_swap != 0)) || (f_bn && bn != f_bn)) return;
-    const int max_pairs = std::min(sms / 2, kGemmLocalMaxPairs);
     Plan p;
     p.persistent = true;
     p.swap = swap;
@@ -830,30 +804,43 @@ Plan make_local_plan(int M, int N, int K, int sms) {
     p.p_tiles = ((swap ? N : M) + 255) / 256;
     p.q_tiles = ((swap ? M : N) + bn - 1) / bn;
     const int64_t tiles = (int64_t)p.p_tiles * p.q_tiles;
-    p.pairs = (int)std::min<int64_t>(tiles, max_pairs);
-    const double power_ns = 2.0 * tiles * 256 * bn * (double)num_kb * kBK / 1.6e6;
-    const double kb_ns = std::max(load_ns(p, 128, bn / 2), 270.0 * bn / 256.0);
-    const double fixed = 5000.0 + 5.0 * bn;
+    p.pairs = (int)std::min<int64_t>(tiles, std::min(sms / 2, kGemmLocalMaxPairs));
+    const double power = power_ns(p.p_tiles * 256.0, (double)p.q_tiles * bn);
+    const double kb_ns = std::max({row_ns * (128 + bn / 2), 280.0 * bn / 256.0, 150.0});
     p.sk_tiles = 0;
-    p.ns = std::max(std::max(std::ceil((double)tiles / p.pairs) * num_kb * kb_ns, power_ns), dram_ns) + fixed;
-    if (f_sk != 1) keep(p);
-    if (tiles > p.pairs && tiles % p.pairs != 0 && f_sk != 0) {
+    p.ns = std::max({std::ceil((double)tiles / p.pairs) * num_kb * kb_ns, power, dram_ns}) + 3400.0 + 9.0 * bn;
+    keep(p);
+    if (tiles > p.pairs && tiles % p.pairs != 0) {
       p.sk_tiles = (int)(tiles % p.pairs) + p.pairs;
-      p.ns = std::max(std::max((double)tiles / p.pairs * num_kb * kb_ns * 1.05, power_ns), dram_ns) + fixed + 2500.0;
+      p.ns = std::max({(double)tiles / p.pairs * num_kb * kb_ns * 1.05, power, dram_ns}) + 3400.0 + 9.0 * bn + 2500.0;
       keep(p);
     }
   };
   for (int bn : {64, 128, 192, 256}) {
-    for (int shape : {kOne, kTwo, kPair}) consider_tile(false, shape, bn);
+    for (bool pair : {false, true}) consider_tile(false, pair, bn);
     consider_pair(false, bn);
   }
   const int fewest = (M + 255) / 256;
   for (int parts = fewest; parts <= std::min(fewest + 3, (M + 31) / 32); ++parts) {
     const int bn = ((M + parts - 1) / parts + 31) / 32 * 32;
-    for (int shape : {kOne, kTwo, kPair}) consider_tile(true, shape, bn);
+    for (bool pair : {false, true}) consider_tile(true, pair, bn);
     consider_pair(true, bn);
   }
   return best;
+}
+
+// A program comes back with the same few shapes: the search above costs more than a short kernel.
+const Plan& cached_plan(int M, int N, int K, int sms) {
+  struct Entry {
+    int M = 0, N = 0, K = 0, sms = 0, dev = -1;
+    Plan plan;
+  };
+  static thread_local Entry cache[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  Entry& e = cache[((uint32_t)M * 31u + (uint32_t)N * 7u + (uint32_t)K) * 2654435761u >> 26];
+  if (e.M != M || e.N != N || e.K != K || e.sms != sms || e.dev != dev) e = Entry{M, N, K, sms, dev, make_local_plan(M, N, K, sms)};
+  return e.plan;
 }
 
 bool common_params(LocalParams& p, const GemmLocalArgs& a, const Plan& plan, int p_rows, int q_rows, CUtensorMap* map_p,
@@ -870,7 +857,7 @@ bool common_params(LocalParams& p, const GemmLocalArgs& a, const Plan& plan, int
   p.num_kb = (a.K + kBK - 1) / kBK;
   p.p_tiles = plan.p_tiles;
   p.q_tiles = plan.q_tiles;
-  p.band = std::min(env_int("GL_BAND", 8), plan.p_tiles);
+  p.band = std::min(8, plan.p_tiles);
   p.bn = plan.bn;
   p.rows = plan.rows;
   p.splits = plan.splits;
@@ -920,45 +907,40 @@ cudaError_t launch_pair(const GemmLocalArgs& a, const Plan& plan, cudaStream_t s
   return launch(gemm_pair_kernel<SWAP>, p, 2 * plan.pairs, 2, 1024 + (size_t)p.stages * stage_bytes + kTailBytes, stream, map_p, map_q, map_out);
 }
 
-template <bool SWAP, int SHAPE>
+template <bool SWAP, bool PAIR>
 cudaError_t launch_tile(const GemmLocalArgs& a, const Plan& plan, cudaStream_t stream) {
   LocalParams p;
   CUtensorMap map_p, map_q, map_out;
-  const int q_rows = SHAPE == kPair ? plan.bn / 2 : plan.bn;
+  const int q_rows = PAIR ? plan.bn / 2 : plan.bn;
   if (!common_params(p, a, plan, plan.rows, q_rows, &map_p, &map_q, &map_out)) return cudaErrorInvalidValue;
-  const int stage_bytes = ((SHAPE == kTwo ? 2 : 1) * plan.rows + q_rows) * kBK * 2;
-  int room = kMaxDynamicSmem - 1024 - kTailBytes;
-  if (plan.splits > 1) {
-    const int per = ((plan.bn / 8 + plan.splits - 1) / plan.splits) * 8;
-    p.part_bytes = plan.splits * per * kPRows * 4;
-    if ((room - p.part_bytes) / stage_bytes < 5) p.part_bytes = 0;  // too little left for the pipeline: share its memory
-    room -= p.part_bytes;
-  }
-  p.stages = std::min(env_int("GL_ST", kMaxStages), room / stage_bytes);
+  const int stage_bytes = (plan.rows + q_rows) * kBK * 2;
+  const int room = kMaxDynamicSmem - 1024 - kTailBytes;
+  const int parts = plan.splits > 1 ? plan.splits * ((plan.bn / 8 + plan.splits - 1) / plan.splits) * 8 * kPRows * 4 : 0;
+  // the parts of a split tile in memory of their own, unless too little would be left for the pipeline
+  p.part_bytes = (room - parts) / stage_bytes >= 5 ? parts : 0;
+  p.stages = std::min(kMaxStages, (room - p.part_bytes) / stage_bytes);
+  p.stage_area = p.stages * stage_bytes;  // (a multiple of 1024, as the slabs behind it need)
+  if (p.part_bytes == 0) p.stage_area = std::max(p.stage_area, parts);
+  if (p.stages < 2 || p.stage_area + p.part_bytes > room) return cudaErrorInvalidValue;
   static const cudaError_t opted =
-      cudaFuncSetAttribute(gemm_tile_kernel<SWAP, SHAPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
-  static const cudaError_t opted2 = cudaFuncSetAttribute(gemm_tile_kernel<SWAP, SHAPE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      cudaFuncSetAttribute(gemm_tile_kernel<SWAP, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+  static const cudaError_t opted2 = cudaFuncSetAttribute(gemm_tile_kernel<SWAP, PAIR>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (opted != cudaSuccess || opted2 != cudaSuccess) return opted != cudaSuccess ? opted : opted2;
-  return launch(gemm_tile_kernel<SWAP, SHAPE>, p, plan.p_tiles * plan.q_tiles * ctas_of(plan), ctas_of(plan),
-                1024 + (size_t)p.stages * stage_bytes + kTailBytes + p.part_bytes, stream, map_p, map_q, map_out);
+  return launch(gemm_tile_kernel<SWAP, PAIR>, p, plan.p_tiles * plan.q_tiles * ctas_of(plan), ctas_of(plan),
+                1024 + (size_t)p.stage_area + kTailBytes + p.part_bytes, stream, map_p, map_q, map_out);
 }
 
 }  // namespace
 
 cudaError_t launch_gemm_local(const GemmLocalArgs& a, cudaStream_t stream) {
   if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.K % 8 != 0 || a.N % 8 != 0) return cudaErrorInvalidValue;
-  Plan plan = make_local_plan(a.M, a.N, a.K, a.sms);
-  if (plan.ns > 1e299) return cudaErrorInvalidValue;
-  if (env_int("SHOW_GL", 0)) printf("plan persistent %d swap %d shape %d rows %d bn %d s %d pairs %d sk %d tiles %dx%d est %.1f us\n", plan.persistent, plan.swap, plan.shape, plan.rows, plan.bn, plan.splits, plan.pairs, plan.sk_tiles, plan.p_tiles, plan.q_tiles, plan.ns/1e3), fflush(stdout);
+  Plan plan = cached_plan(a.M, a.N, a.K, a.sms);
   if (plan.persistent) {
     if (a.partials == nullptr) plan.sk_tiles = 0;
     return plan.swap ? launch_pair<true>(a, plan, stream) : launch_pair<false>(a, plan, stream);
   }
-  switch (plan.shape) {
-    case kOne: return plan.swap ? launch_tile<true, kOne>(a, plan, stream) : launch_tile<false, kOne>(a, plan, stream);
-    case kTwo: return plan.swap ? launch_tile<true, kTwo>(a, plan, stream) : launch_tile<false, kTwo>(a, plan, stream);
-    default: return plan.swap ? launch_tile<true, kPair>(a, plan, stream) : launch_tile<false, kPair>(a, plan, stream);
-  }
+  if (plan.pair) return plan.swap ? launch_tile<true, true>(a, plan, stream) : launch_tile<false, true>(a, plan, stream);
+  return plan.swap ? launch_tile<true, false>(a, plan, stream) : launch_tile<false, false>(a, plan, stream);
 }
 
 }  // namespace b200

@@ -40,15 +40,15 @@ bool make_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t
     Key key;
     CUtensorMap map;
   };
-  constexpr int kEntries = 64;
-  thread_local Entry cache[kEntries];
-  thread_local int used = 0, next = 0;
+  constexpr uint32_t kEntries = 256;  // direct mapped
+  thread_local Entry cache[kEntries] = {};
   const Key key{base, rows, cols, elem_bytes, box_rows, box_cols, swizzle128 ? 1u : 0u};
-  for (int i = 0; i < used; ++i) {
-    if (cache[i].key == key) {
-      *map = cache[i].map;
-      return true;
-    }
+  const uint32_t hash = (uint32_t)(reinterpret_cast<uintptr_t>(base) >> 8) * 2654435761u + (uint32_t)rows * 40503u +
+                        (uint32_t)cols * 2246822519u + box_rows * 3266489917u + box_cols;
+  Entry& slot = cache[(hash ^ (hash >> 15)) % kEntries];
+  if (slot.key == key) {  // (a null base is never asked for)
+    *map = slot.map;
+    return true;
   }
   const EncodeTiledFn fn = encode_fn();
   if (fn == nullptr || (elem_bytes != 1 && elem_bytes != 2)) return false;
@@ -61,9 +61,7 @@ bool make_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t
                         swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return false;
-  cache[next] = Entry{key, *map};
-  next = (next + 1) % kEntries;
-  if (used < kEntries) ++used;
+  slot = Entry{key, *map};
   return true;
 }
 

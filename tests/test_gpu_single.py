@@ -208,6 +208,41 @@ def test_gemm_world1_matches_fp32_reference(m, n, k, has_bias):
     assert oracle.relative_error(out, truth) < 5e-3
 
 
+@pytest.mark.parametrize(
+    "m,n,k",
+    [
+        (1, 512, 64),  # one token, one k-block
+        (33, 520, 1032),  # ragged in all three: rows of W start between cache lines
+        (30, 512, 29568),  # a few tiles, K shared by a large cluster
+        (90, 2048, 2752),  # ... by a small one
+        (256, 5120, 6400),  # CTA pairs, K shared, the parts in the pipeline's memory
+        (700, 2208, 1112),  # several tiles along M, short last ones
+        (129, 8192, 264),  # one row more than a tile
+        (2048, 2880, 2880),  # persistent pairs, whole tiles
+        (2560, 4096, 1032),  # ... and tiles cut along K, ragged
+        (3000, 3000, 512),
+    ],
+)
+def test_gemm_one_rank_schedules(m, n, k):
+    """Every schedule of the one-rank kernels against fp32, with both orders of the bias, call after call."""
+    from amd_distributed_2025_b200.models import gemm_rs
+
+    a, w, bias = contract.make_gemm_rs_inputs(0, 1, m, n, k, True, 17, device="cuda")
+    op = gemm_rs.get_op(m, n, k)
+    truth = a.float() @ w.float().T
+    cases = [(None, "per_rank", truth), (bias, "per_rank", truth.bfloat16().float() + bias.float()),
+             (bias, "once", truth + bias.float())]
+    for b, mode, want in cases:
+        first = op(a, w, b, mode)
+        for _ in range(3):
+            again = op(a, w, b, mode)
+        torch.cuda.synchronize()
+        op.check()
+        assert torch.equal(first, again)
+        assert oracle.relative_error(first, want) < 5e-3
+        assert float((first.float() - want).abs().max()) < 1e-2 * float(want.abs().max())
+
+
 @pytest.mark.parametrize("m,n,k,has_bias", [(64, 2880, 360, True), (512, 4096, 1536, True), (2048, 2880, 360, True)])
 def test_gemm_world1_reference_inputs_pass_reference_checker(m, n, k, has_bias):
     """Operands from the reference generator (uniform +-0.01) against the library path."""
