@@ -703,23 +703,9 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
 // ---------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------
-namespace {
-
 constexpr int kMaxSplits = 16;
 
-struct Plan {
-  bool persistent = false, swap = false;
-  bool pair = false;                  // tile kernel: a CTA pair per tile
-  int rows = 128, bn = 256, splits = 1;
-  int pairs = 1, sk_tiles = 0;        // pair kernel
-  int p_tiles = 0, q_tiles = 0;
-  double ns = 1e300;
-};
-
-int ctas_of(const Plan& p) { return p.splits * (p.pair ? 2 : 1); }  // CTAs that share a tile
-
-// How many clusters of `size` tile-kernel CTAs are resident at once (all of a CTA's shared memory in use).
-int cluster_capacity(int size) {
+int gemm_cluster_capacity(int size) {
   struct PerDevice {
     int n[kMaxSplits + 1] = {0};
   };
@@ -748,6 +734,18 @@ int cluster_capacity(int size) {
   }
   return n;
 }
+namespace {
+
+struct Plan {
+  bool persistent = false, swap = false;
+  bool pair = false;                  // tile kernel: a CTA pair per tile
+  int rows = 128, bn = 256, splits = 1;
+  int pairs = 1, sk_tiles = 0;        // pair kernel
+  int p_tiles = 0, q_tiles = 0;
+  double ns = 1e300;
+};
+
+int ctas_of(const Plan& p) { return p.splits * (p.pair ? 2 : 1); }  // CTAs that share a tile
 
 // Time model in ns.  What it charges, measured on a B200:
 //   a 128-byte row of a k-block takes an SM 1 ns to bring in, 1.6 when the rows of the matrix do not start on cache lines;
@@ -757,7 +755,11 @@ Plan make_local_plan(int M, int N, int K, int sms) {
   const int num_kb = (K + kBK - 1) / kBK;
   const double dram_ns = 2.0 * ((double)M * K + (double)N * K + (double)M * N) / 6600.0;
   const double row_ns = K % kBK == 0 ? 1.0 : 1.6;
-  auto power_ns = [&](double rows, double cols) { return 2.0 * rows * cols * num_kb * kBK / 1.55e6; };
+  // ... and the narrower the tile, the more of the power goes into moving operands: `rows_per_col` is what a CTA brings
+  // in per k-block, relative to a pair's 256 rows for 256 columns
+  auto power_ns = [&](double rows, double cols, double rows_per_col) {
+    return 2.0 * rows * cols * num_kb * kBK / 1.55e6 * (1.0 + 0.26 * (rows_per_col - 1.0));
+  };
   Plan best;
   auto keep = [&](const Plan& p) {
     if (p.ns < best.ns) best = p;
@@ -773,7 +775,7 @@ Plan make_local_plan(int M, int N, int K, int sms) {
     for (int s = 1; s <= kMaxSplits / halves; ++s) {
       if (s > 1 && s > num_kb) continue;
       p.splits = s;
-      const int cap = ctas_of(p) == 1 ? sms : cluster_capacity(ctas_of(p));
+      const int cap = ctas_of(p) == 1 ? sms : gemm_cluster_capacity(ctas_of(p));
       // Lower tiles when that many clusters fit at once and full ones would leave SMs without work: a share of the
       // weight for everybody.  (Not split, tiles end on the 32 rows of an epilogue warp.)
       p.rows = 128;
@@ -791,7 +793,7 @@ Plan make_local_plan(int M, int N, int K, int sms) {
       const int stages = std::min(kMaxStages, (kMaxDynamicSmem - 1024 - kTailBytes) / ((p.rows + q_rows) * kBK * 2));
       const double kb_ns = std::max({row_ns * (p.rows + q_rows), 280.0 * bn / 256.0, 150.0, 1700.0 / stages});
       const double ends_ns = (s == 1 ? 3000.0 + 9.0 * bn : 4800.0 + 28.0 * std::max(bn - 64, 0) + 50.0 * s) + (pair ? 400.0 : 0.0);
-      p.ns = std::max({waves * kbs * kb_ns, power_ns((double)p.p_tiles * halves * 128, (double)p.q_tiles * bn), dram_ns}) + ends_ns +
+      p.ns = std::max({waves * kbs * kb_ns, power_ns((double)p.p_tiles * halves * 128, (double)p.q_tiles * bn, (128.0 + q_rows) / bn), dram_ns}) + ends_ns +
              (waves - 1) * 4000.0;
       keep(p);
     }
@@ -805,7 +807,7 @@ Plan make_local_plan(int M, int N, int K, int sms) {
     p.q_tiles = ((swap ? M : N) + bn - 1) / bn;
     const int64_t tiles = (int64_t)p.p_tiles * p.q_tiles;
     p.pairs = (int)std::min<int64_t>(tiles, std::min(sms / 2, kGemmLocalMaxPairs));
-    const double power = power_ns(p.p_tiles * 256.0, (double)p.q_tiles * bn);
+    const double power = power_ns(p.p_tiles * 256.0, (double)p.q_tiles * bn, (128.0 + bn / 2) / bn);
     const double kb_ns = std::max({row_ns * (128 + bn / 2), 280.0 * bn / 256.0, 150.0});
     p.sk_tiles = 0;
     p.ns = std::max({std::ceil((double)tiles / p.pairs) * num_kb * kb_ns, power, dram_ns}) + 3400.0 + 9.0 * bn;
@@ -864,9 +866,9 @@ bool common_params(LocalParams& p, const GemmLocalArgs& a, const Plan& plan, int
   p.timeout_ns = a.timeout_ns;
   p.status = a.status;
   p.trace = a.trace;
-  return make_tensor_map(map_p, swap ? a.w : a.a, (uint64_t)p.P, (uint64_t)a.K, 2, (uint32_t)p_rows, kBK, true) &&
-         make_tensor_map(map_q, swap ? a.a : a.w, (uint64_t)p.Q, (uint64_t)a.K, 2, (uint32_t)q_rows, kBK, true) &&
-         make_tensor_map(map_out, a.out, (uint64_t)a.M, (uint64_t)a.N, 2, 32, swap ? 32 : 64, !swap);
+  return make_tensor_map(map_p, swap ? a.w : a.a, (uint64_t)p.P, (uint64_t)a.K, 2, (uint32_t)p_rows, kBK, 128) &&
+         make_tensor_map(map_q, swap ? a.a : a.w, (uint64_t)p.Q, (uint64_t)a.K, 2, (uint32_t)q_rows, kBK, 128) &&
+         make_tensor_map(map_out, a.out, (uint64_t)a.M, (uint64_t)a.N, 2, 32, swap ? 32 : 64, swap ? 0 : 128);
 }
 
 template <typename K>

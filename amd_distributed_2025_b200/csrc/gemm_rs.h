@@ -99,4 +99,7 @@ constexpr int kGemmLocalCounters = kGemmLocalMaxPairs * 2 * 2 * 8;
 
 cudaError_t launch_gemm_local(const GemmLocalArgs& args, cudaStream_t stream);
 
+// How many clusters of `size` (1..16) CTAs that each fill an SM's shared memory are resident at once.
+int gemm_cluster_capacity(int size);
+
 }  // namespace b200

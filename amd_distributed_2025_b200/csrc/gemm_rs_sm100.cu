@@ -1049,7 +1049,7 @@ namespace {
 
 // Row-major bf16 [rows, cols] tensor, box = [box_rows, 64 columns], 128-byte swizzle.
 bool make_bf16_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-  return make_tensor_map(map, base, rows, cols, 2, box_rows, BK, true);
+  return make_tensor_map(map, base, rows, cols, 2, box_rows, BK, 128);
 }
 
 // Tile shape and K slicing from the problem size.  Cost model: waves of work items times

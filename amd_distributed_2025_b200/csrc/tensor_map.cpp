@@ -35,14 +35,14 @@ struct Key {
 }  // namespace
 
 bool make_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t elem_bytes, uint32_t box_rows,
-                     uint32_t box_cols, bool swizzle128) {
+                     uint32_t box_cols, int swizzle) {
   struct Entry {
     Key key;
     CUtensorMap map;
   };
   constexpr uint32_t kEntries = 256;  // direct mapped
   thread_local Entry cache[kEntries] = {};
-  const Key key{base, rows, cols, elem_bytes, box_rows, box_cols, swizzle128 ? 1u : 0u};
+  const Key key{base, rows, cols, elem_bytes, box_rows, box_cols, (uint32_t)swizzle};
   const uint32_t hash = (uint32_t)(reinterpret_cast<uintptr_t>(base) >> 8) * 2654435761u + (uint32_t)rows * 40503u +
                         (uint32_t)cols * 2246822519u + box_rows * 3266489917u + box_cols;
   Entry& slot = cache[(hash ^ (hash >> 15)) % kEntries];
@@ -58,7 +58,7 @@ bool make_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t
   const cuuint32_t elem_strides[2] = {1, 1};
   const CUresult r = fn(map, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
                         const_cast<void*>(base), dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                        swizzle == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : swizzle == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return false;
   slot = Entry{key, *map};

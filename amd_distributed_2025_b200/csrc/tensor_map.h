@@ -5,11 +5,11 @@
 
 namespace b200 {
 
-// Rows x cols elements of `elem_bytes` (1 or 2), box of box_rows x box_cols elements; swizzle128: 128-byte swizzle, else
-// none.  Out-of-range elements read as zero and are not written.  Encoded maps are kept in a small per-thread
+// Rows x cols elements of `elem_bytes` (1 or 2), box of box_rows x box_cols elements, whose rows are stored with a swizzle
+// of 128 or 64 bytes or (0) none.  Out-of-range elements read as zero and are not written.  Encoded maps are kept in a small per-thread
 // cache: a serving loop calls with the same weight (and often the same activation buffer) again and again, and the
 // driver call is a visible part of a short launch.  False if the driver refuses the map.
 bool make_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t elem_bytes, uint32_t box_rows,
-                     uint32_t box_cols, bool swizzle128);
+                     uint32_t box_cols, int swizzle);
 
 }  // namespace b200
