@@ -814,8 +814,37 @@ class GemmRsEngine {
 
 // ------------------------------------------------------------------------ fp8 GEMM ----
 
+int device_sms(int device) {
+  static const std::vector<int> sms = [] {
+    std::vector<int> v;
+    for (int d = 0; d < (int)at::cuda::device_count(); ++d) v.push_back(at::cuda::getDeviceProperties(d)->multiProcessorCount);
+    return v;
+  }();
+  return sms.at((size_t)device);
+}
+
+void run_fp8_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& a_scale, const at::Tensor& b_scale,
+                  const at::Tensor& c, int64_t timeout_ns) {
+  b200::Fp8GemmArgs g;
+  g.a = a.const_data_ptr();
+  g.b = b.const_data_ptr();
+  g.a_scale = a_scale.const_data_ptr<float>();
+  g.b_scale = b_scale.const_data_ptr<float>();
+  g.c = c.mutable_data_ptr();
+  g.M = (int)a.size(0);
+  g.N = (int)b.size(0);
+  g.K = (int)a.size(1);
+  g.as_stride_m = a_scale.stride(0);
+  g.as_stride_k = a_scale.stride(1);
+  g.bs_stride_n = b_scale.stride(0);
+  g.bs_stride_k = b_scale.stride(1);
+  g.timeout_ns = (uint64_t)timeout_ns;
+  g.sms = device_sms(a.get_device());
+  cuda_check(b200::launch_fp8_gemm(g, at::cuda::getCurrentCUDAStream()), "fp8_gemm launch");
+}
+
 void fp8_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& a_scale, const at::Tensor& b_scale,
-              at::Tensor c, at::Tensor error_flag, int64_t timeout_ns) {
+              at::Tensor c, int64_t timeout_ns) {
   TORCH_CHECK(a.is_cuda() && b.is_cuda() && a.dim() == 2 && b.dim() == 2 && a.size(1) == b.size(1),
               "a [M, K] and b [N, K] must be CUDA matrices with equal K");
   TORCH_CHECK(a.scalar_type() == at::kFloat8_e4m3fn && b.scalar_type() == at::kFloat8_e4m3fn, "a and b must be float8_e4m3fn");
@@ -828,24 +857,28 @@ void fp8_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& a_scal
               "b_scale must be fp32 [ceil(N/128), ceil(K/128)]");
   TORCH_CHECK(c.scalar_type() == at::kBFloat16 && c.is_contiguous() && c.size(0) == M && c.size(1) == N, "c must be bf16 [M, N]");
   TORCH_CHECK(K % 16 == 0, "K must be a multiple of 16");
-  TORCH_CHECK(error_flag.scalar_type() == at::kInt && error_flag.numel() >= 1, "error_flag must be an int32 tensor");
   c10::cuda::CUDAGuard guard(a.device());
-  b200::Fp8GemmArgs g;
-  g.a = a.data_ptr();
-  g.b = b.data_ptr();
-  g.a_scale = a_scale.data_ptr<float>();
-  g.b_scale = b_scale.data_ptr<float>();
-  g.c = c.data_ptr();
-  g.M = (int)M;
-  g.N = (int)N;
-  g.K = (int)K;
-  g.as_stride_m = a_scale.stride(0);
-  g.as_stride_k = a_scale.stride(1);
-  g.bs_stride_n = b_scale.stride(0);
-  g.bs_stride_k = b_scale.stride(1);
-  g.timeout_ns = (uint64_t)timeout_ns;
-  g.error_flag = error_flag.data_ptr<int32_t>();
-  cuda_check(b200::launch_fp8_gemm(g, at::cuda::getCurrentCUDAStream()), "fp8_gemm launch");
+  run_fp8_gemm(a, b, a_scale, b_scale, c, timeout_ns);
+}
+
+// The common call (operands and scales as the kernel wants them, result to be allocated) without a look at it from
+// Python.  None: nothing was done, take the checked path.
+c10::optional<at::Tensor> fp8_gemm_try(const at::Tensor& a, const at::Tensor& b, const at::Tensor& a_scale, const at::Tensor& b_scale,
+                                       int64_t timeout_ns) {
+  if (!a.is_cuda() || !b.is_cuda() || !a_scale.is_cuda() || !b_scale.is_cuda() || a.dim() != 2 || b.dim() != 2 || a_scale.dim() != 2 ||
+      b_scale.dim() != 2 || a.scalar_type() != at::kFloat8_e4m3fn || b.scalar_type() != at::kFloat8_e4m3fn || !a.is_contiguous() ||
+      !b.is_contiguous() || a_scale.scalar_type() != at::kFloat || b_scale.scalar_type() != at::kFloat)
+    return c10::nullopt;
+  const int64_t M = a.size(0), N = b.size(0), K = a.size(1);
+  const int64_t kb = (K + 127) / 128;
+  if (M <= 0 || N <= 0 || K <= 0 || K != b.size(1) || K % 16 != 0 || a_scale.size(0) != M || a_scale.size(1) != kb ||
+      b_scale.size(0) != (N + 127) / 128 || b_scale.size(1) != kb || b.get_device() != a.get_device() ||
+      a_scale.get_device() != a.get_device() || b_scale.get_device() != a.get_device())
+    return c10::nullopt;
+  c10::cuda::CUDAGuard guard(a.device());
+  at::Tensor c = at::detail::empty_cuda({M, N}, at::kBFloat16, a.device(), c10::nullopt);
+  run_fp8_gemm(a, b, a_scale, b_scale, c, timeout_ns);
+  return c;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1381,6 +1414,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_forward", &moe_forward);
   m.def("gemm_rs", &gemm_rs);
   m.def("fp8_gemm", &fp8_gemm);
+  m.def("fp8_gemm_try", &fp8_gemm_try);
   m.def("gemm_rs_plan", [](int64_t M, int64_t N, int64_t K, int64_t ws, int64_t block_n, int64_t cta_pair, int64_t splits) {
     const b200::GemmRsPlan p = b200::gemm_rs_plan((int)M, (int)N, (int)K, (int)ws, (int)block_n, (int)cta_pair, (int)splits);
     py::dict d;

@@ -15,7 +15,7 @@ struct Fp8GemmArgs {
   int M, N, K;
   long long as_stride_m, as_stride_k, bs_stride_n, bs_stride_k;  // element strides of the scale tensors
   uint64_t timeout_ns;
-  int* error_flag;       // device int, set to 1 if a pipeline wait expired (may be nullptr)
+  int sms;
 };
 
 cudaError_t launch_fp8_gemm(const Fp8GemmArgs& args, cudaStream_t stream);

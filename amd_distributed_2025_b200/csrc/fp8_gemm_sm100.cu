@@ -4,231 +4,452 @@
 // its two tasks (all2all/hip.py:17-59, identical copy in gemm-rs/hip.py): one thread per
 // output element, K walked in blocks of 128, the block's partial product multiplied by a
 // per-row scale of A and a per-128x128-block scale of B, bf16 result.  Here the block
-// products run on the tensor cores: per 128-wide K block four tcgen05.mma.kind::f8f6f4
-// instructions (K = 32 each) write a fresh 128 x 128 fp32 partial into one of two
-// tensor-memory buffers, and the four epilogue warps pull it out, multiply by the
-// block's scales and accumulate in registers while the next block is being multiplied.
-// Operands are K-major (row-major [m, k] and [n, k]); TMA stages them with the 128-byte
-// swizzle exactly as in the bf16 GEMM (a 128-byte row now holds 128 fp8 values).
+// products run on the tensor cores.  Operands are K-major (row-major [m, k] and [n, k]); TMA stages
+// them with the 128-byte swizzle exactly as in the bf16 GEMM (a 128-byte row now holds 128 fp8 values).
+//
+// A CTA pair (cta_group::2) owns a tile of 256 rows of A by `bn` (64 or 128) rows of B.  Every 128-wide K block is
+// multiplied into a tensor-memory buffer of its own, one of four; eight epilogue warps, two per tensor-memory lane
+// quarter, pull it out, multiply by the block's scales and accumulate in fp32 registers while the next blocks are
+// being multiplied.  Two warps bring the scales in, sixteen blocks ahead: a row's scales lie in a line of their own,
+// and fetched by the epilogue itself they took longer than the products.  Pairs are persistent; where there are fewer
+// tiles than pairs, a cluster of pairs shares a tile, each over its part of K, and the parts meet in distributed
+// shared memory.
+//
+// Why 128 columns and four buffers: a buffer comes back after multiplication, signal, read-out and signal, some 1100
+// cycles in all, of which the multiplication is 256; two buffers of 256 columns left the tensor cores waiting.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "fp8_gemm.h"
+#include "gemm_rs.h"
 #include "signal.cuh"
 #include "sm100_ptx.cuh"
+#include "tensor_map.h"
 
 namespace b200 {
 
 namespace {
 
-constexpr int FBM = 128, FBN = 128, FBK = 128;  // FBK = the scale block of the operation
-constexpr int kFp8Threads = 192;                // producer, MMA issuer, 4 epilogue warps
-constexpr int kFp8Stages = 6;
-constexpr int kFp8ABytes = FBM * FBK;           // 16 KiB
-constexpr int kFp8BBytes = FBN * FBK;
-constexpr int kFp8StageBytes = kFp8ABytes + kFp8BBytes;
-constexpr int kFp8SmemBytes = 1024 + kFp8Stages * kFp8StageBytes + 1024;
+constexpr int kRows = 128;                // rows of A per CTA
+constexpr int kBlockK = 128;              // the scale block of the operation: one 128-byte row
+constexpr int kABytes = kRows * kBlockK;
+constexpr int kEpiWarps = 8;
+constexpr int kScaleWarps = 2;
+constexpr int kThreads = 64 + 32 * (kEpiWarps + kScaleWarps);
+constexpr int kMaxStages = 12;
+constexpr int kSlabBytes = 2 * 2048;      // per epilogue warp: two buffers of 32 rows x 64 bytes
+constexpr int kGroup = 4;                 // K blocks whose scales come in together
+constexpr int kScaleSlots = 4;
+constexpr int kScaleBytes = kGroup * (kRows + 4) * 4;  // [block][row], then [block][half of the columns][chunk]
+constexpr int kTailBytes = kEpiWarps * kSlabBytes + kScaleSlots * kScaleBytes + 512;
+constexpr int kBufs = 4;
+constexpr int kMaxDynamicSmem = 232448 - 256;
+constexpr int kTmemCols = 512;
+constexpr int kMaxChunks = 2;             // 32-column chunks of an epilogue warp
 
 struct Fp8Params {
   const float* a_scale;  // [m, k_blocks], element (m, kb) at m * as_stride_m + kb * as_stride_k
   const float* b_scale;  // [n_blocks, k_blocks], element (nb, kb) at nb * bs_stride_n + kb * bs_stride_k
   __nv_bfloat16* c;      // [m, n] row-major
-  int M, N, K, k_blocks;
+  int M, N, k_blocks;
   long long as_stride_m, as_stride_k, bs_stride_n, bs_stride_k;
-  uint64_t timeout_ns;
-  int* error_flag;  // set to 1 if a pipeline wait expired
+  int m_tiles, n_tiles, band, bn, stages, stage_area;
+  int splits;            // pairs of a cluster that share a tile
+  int tma_out;           // 1: rows of C are whole 16-byte pieces: results leave through TMA
+  uint64_t timeout_ns;   // of a pipeline wait
 };
 
 // Instruction descriptor of tcgen05.mma.kind::f8f6f4 with e4m3 A and B (both K-major) and fp32
 // accumulation: bits [4,6) D format (1 = f32), [7,10) A format (0 = e4m3), [10,13) B format,
 // [17,23) N >> 3, [24,29) M >> 4.
-constexpr uint32_t make_idesc_e4m3_f32(int m, int n) {
+__device__ __forceinline__ uint32_t make_idesc_e4m3_f32(int m, int n) {
   return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma_fp8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                         uint32_t accumulate) {
+__device__ __forceinline__ void umma_fp8_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                              uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
-__device__ __forceinline__ bool fp8_wait(uint32_t bar, uint32_t parity, volatile int* abort, uint64_t limit_ns,
-                                         int* error_flag) {
+__device__ __forceinline__ bool fp8_wait(uint32_t bar, uint32_t parity, volatile int* abort, const Fp8Params& p) {
   if (ptx::mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = global_timer_ns();
   uint32_t spins = 0;
-  while (true) {
-    if (ptx::mbar_try_wait(bar, parity)) return true;
+  while (!ptx::mbar_try_wait(bar, parity)) {
     if ((++spins & 255u) == 0) {
       if (*abort) return false;
-      if (global_timer_ns() - t0 > limit_ns) {
+      if (global_timer_ns() - t0 > p.timeout_ns) {
         *abort = 1;
-        if (error_flag != nullptr) *error_flag = 1;
         return false;
       }
     }
   }
+  return true;
+}
+
+// acc[0..1] += v[0..1] * s
+__device__ __forceinline__ void fma2(float2& acc, uint32_t v0, uint32_t v1, float2 ss) {
+  const float2 v = make_float2(__uint_as_float(v0), __uint_as_float(v1));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;"
+      : "+l"(reinterpret_cast<unsigned long long&>(acc))
+      : "l"(reinterpret_cast<const unsigned long long&>(v)), "l"(reinterpret_cast<const unsigned long long&>(ss)));
+}
+
+__device__ __forceinline__ uint32_t pack2(float2 f) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y);
+  return *reinterpret_cast<const uint32_t*>(&h);
 }
 
 }  // namespace
 
-__global__ void __launch_bounds__(kFp8Threads, 1)
-fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                const Fp8Params p) {
+__global__ void __launch_bounds__(kThreads, 1)
+fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                const __grid_constant__ CUtensorMap map_c, const Fp8Params p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ volatile int abort_flag;
   __shared__ uint32_t tmem_base_shared;
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
-  const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t bar_base = smem_base + kFp8Stages * kFp8StageBytes;
-  auto full_bar = [&](uint32_t s) { return bar_base + 8u * s; };
-  auto empty_bar = [&](uint32_t s) { return bar_base + 8u * (kFp8Stages + s); };
-  auto tfull_bar = [&](uint32_t s) { return bar_base + 8u * (2 * kFp8Stages + s); };
-  auto tempty_bar = [&](uint32_t s) { return bar_base + 8u * (2 * kFp8Stages + 2 + s); };
+  const int splits = p.splits;
+  const int cluster_rank = (int)ptx::cluster_ctarank();
+  const int rank = cluster_rank >> 1;  // which part of K
+  const int cta = cluster_rank & 1;    // which half of the pair's rows
+  const int kb0 = (int)((int64_t)p.k_blocks * rank / splits);
+  const int kb1 = (int)((int64_t)p.k_blocks * (rank + 1) / splits);
+  const int first_tile = (int)blockIdx.x / (2 * splits);
+  const int tile_step = (int)gridDim.x / (2 * splits);
+  const int total = p.m_tiles * p.n_tiles;
+  const int b_rows = p.bn / 2;  // rows of B that this CTA brings in
+  constexpr uint32_t buf_cols = kTmemCols / kBufs;
+
+  const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t stage_bytes = kABytes + (uint32_t)b_rows * kBlockK;
+  const uint32_t slabs = base + (uint32_t)p.stage_area;
+  const uint32_t scales = slabs + kEpiWarps * kSlabBytes;
+  const uint32_t bars = scales + kScaleSlots * kScaleBytes;
+  auto full_bar = [&](uint32_t s) { return bars + 8u * s; };
+  auto empty_bar = [&](uint32_t s) { return bars + 8u * (kMaxStages + s); };
+  auto tfull_bar = [&](uint32_t s) { return bars + 8u * (2 * kMaxStages + s); };
+  auto tempty_bar = [&](uint32_t s) { return bars + 8u * (2 * kMaxStages + kBufs + s); };
+  auto sfull_bar = [&](uint32_t s) { return bars + 8u * (2 * kMaxStages + 2 * kBufs + s); };
+  auto sempty_bar = [&](uint32_t s) { return bars + 8u * (2 * kMaxStages + 2 * kBufs + kScaleSlots + s); };
 
   if (tid == 0) {
     abort_flag = 0;
-    for (int s = 0; s < kFp8Stages; ++s) {
+    for (int s = 0; s < p.stages; ++s) {
       ptx::mbar_init(full_bar(s), 1);
       ptx::mbar_init(empty_bar(s), 1);
     }
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < kBufs; ++s) {
       ptx::mbar_init(tfull_bar(s), 1);
-      ptx::mbar_init(tempty_bar(s), 4);
+      ptx::mbar_init(tempty_bar(s), 2 * kEpiWarps);
+    }
+    for (int s = 0; s < kScaleSlots; ++s) {
+      ptx::mbar_init(sfull_bar(s), kScaleWarps);
+      ptx::mbar_init(sempty_bar(s), kEpiWarps);
     }
     ptx::fence_mbar_init();
     ptx::fence_proxy_async_smem();
+    ptx::prefetch_tensormap(&map_a);
+    ptx::prefetch_tensormap(&map_b);
+    ptx::prefetch_tensormap(&map_c);
   }
   if (warp == 1) {
-    ptx::tmem_alloc(ptx::smem_u32(&tmem_base_shared), 2 * FBN);
-    ptx::tmem_relinquish();
+    ptx::tmem_alloc_pair(ptx::smem_u32(&tmem_base_shared), kTmemCols);
+    ptx::tmem_relinquish_pair();
   }
   ptx::tcgen05_fence_before();
   __syncthreads();
+  ptx::cluster_sync_all();
   ptx::tcgen05_fence_after();
   const uint32_t tmem_base = tmem_base_shared;
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
 
-  const int m_tiles = (p.M + FBM - 1) / FBM;
-  const int n_tiles = (p.N + FBN - 1) / FBN;
-  const int total = m_tiles * n_tiles;
-  const int G = gridDim.x;
-  const uint64_t limit = p.timeout_ns;
+  // bands of row tiles, column tile by column tile: pairs at work at the same time share operands in L2
+  auto tile_coords = [&](int tile, int& mt, int& nt) {
+    const int per_band = p.band * p.n_tiles;
+    const int b = tile / per_band;
+    const int start = b * p.band;
+    const int size = min(p.band, p.m_tiles - start);
+    const int within = tile - start * p.n_tiles;
+    nt = within / size;
+    mt = start + within - nt * size;
+  };
+
+  float2 acc[kMaxChunks][16];  // epilogue warps: this lane's row, chunk i of the warp's half of the columns
+  bool alive = true;
+  const int ew = warp - 2;
+  const int q = warp & 3;
+  const int half = ew >> 2;
+  const int chunks = p.bn / 64;  // of one warp
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0;
-      for (int t = blockIdx.x; t < total && !abort_flag; t += G) {
-        const int mb = t / n_tiles, nb = t % n_tiles;
-        for (int kb = 0; kb < p.k_blocks; ++kb) {
-          if (!fp8_wait(empty_bar(stage), phase ^ 1u, &abort_flag, limit, p.error_flag)) break;
-          const uint32_t sa = smem_base + stage * kFp8StageBytes;
-          ptx::mbar_arrive_expect_tx(full_bar(stage), kFp8StageBytes);
-          ptx::tma_load_2d(sa, &tma_a, full_bar(stage), kb * FBK, mb * FBM);
-          ptx::tma_load_2d(sa + kFp8ABytes, &tma_b, full_bar(stage), kb * FBK, nb * FBN);
-          if (++stage == kFp8Stages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+    uint32_t stage = 0, phase = 0;
+    for (int tile = first_tile; tile < total && !abort_flag; tile += tile_step) {
+      int mt, nt;
+      tile_coords(tile, mt, nt);
+      const int ay = mt * 256 + cta * kRows;
+      const int by = nt * p.bn + cta * b_rows;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!fp8_wait(empty_bar(stage), phase ^ 1u, &abort_flag, p)) break;
+        const uint32_t sa = base + stage * stage_bytes;
+        if (ptx::elect_one()) {
+          if (cta == 0) ptx::mbar_arrive_expect_tx(full_bar(stage), 2 * stage_bytes);
+          ptx::tma_load_2d_pair(sa, &map_a, full_bar(stage), kb * kBlockK, ay);
+          ptx::tma_load_2d_pair(sa + kABytes, &map_b, full_bar(stage), kb * kBlockK, by);
+        }
+        __syncwarp();
+        if (++stage == (uint32_t)p.stages) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_e4m3_f32(FBM, FBN);
-      uint32_t stage = 0, phase = 0, it = 0;  // `it` counts K blocks over all tiles: one TMEM buffer each
-      for (int t = blockIdx.x; t < total && !abort_flag; t += G) {
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
-          const uint32_t acc = it & 1u;
-          if (!fp8_wait(tempty_bar(acc), ((it >> 1) & 1u) ^ 1u, &abort_flag, limit, p.error_flag)) break;
-          if (!fp8_wait(full_bar(stage), phase, &abort_flag, limit, p.error_flag)) break;
+    if (cta == 0) {
+      const uint32_t idesc = make_idesc_e4m3_f32(256, p.bn);
+      const uint16_t both = (uint16_t)(3u << (2 * rank));
+      uint32_t stage = 0, phase = 0, buf = 0, buf_phase = 0;
+      for (int tile = first_tile; tile < total && !abort_flag; tile += tile_step) {
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!fp8_wait(tempty_bar(buf), buf_phase ^ 1u, &abort_flag, p)) break;
+          if (!fp8_wait(full_bar(stage), phase, &abort_flag, p)) break;
           ptx::tcgen05_fence_after();
-          const uint32_t sa = smem_base + stage * kFp8StageBytes;
+          const uint32_t sa = base + stage * stage_bytes;
           const uint64_t da = ptx::make_smem_desc_k_sw128(sa);
-          const uint64_t db = ptx::make_smem_desc_k_sw128(sa + kFp8ABytes);
+          const uint64_t db = ptx::make_smem_desc_k_sw128(sa + kABytes);
+          const uint32_t d = tmem_base + buf * buf_cols;
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int j = 0; j < FBK / 32; ++j) {
-            // 32 fp8 = 32 bytes of K per instruction = 2 descriptor address units
-            umma_fp8(tmem_base + acc * FBN, da + 2u * j, db + 2u * j, idesc, j > 0 ? 1u : 0u);
+            for (int j = 0; j < kBlockK / 32; ++j)  // 32 fp8 of K = 32 bytes = 2 descriptor address units
+              umma_fp8_pair(d, da + 2u * j, db + 2u * j, idesc, j > 0 ? 1u : 0u);
+            ptx::umma_commit_pair(empty_bar(stage), both);
+            ptx::umma_commit_pair(tfull_bar(buf), both);
           }
-          ptx::umma_commit(empty_bar(stage));
-          ptx::umma_commit(tfull_bar(acc));
-          if (++stage == kFp8Stages) {
+          __syncwarp();
+          if (++stage == (uint32_t)p.stages) {
             stage = 0;
             phase ^= 1u;
+          }
+          if (++buf == (uint32_t)kBufs) {
+            buf = 0;
+            buf_phase ^= 1u;
           }
         }
       }
     }
-  } else {
-    const int q = warp & 3;
-    uint32_t it = 0;
-    for (int t = blockIdx.x; t < total && !abort_flag; t += G) {
-      const int mb = t / n_tiles, nb = t % n_tiles;
-      const int m = mb * FBM + q * 32 + lane;
-      float accum[FBN];
+  } else if (warp >= 2 + kEpiWarps) {
+    // ---- scales: two rows per lane, four K blocks at a time ------------------------------------------------
+    const int l = (warp - 2 - kEpiWarps) * 32 + lane;
+    const bool vec = p.as_stride_k == 1 && p.as_stride_m % 4 == 0 && kb0 % 4 == 0 && p.k_blocks % 4 == 0 &&
+                     (reinterpret_cast<uintptr_t>(p.a_scale) & 15u) == 0;
+    uint32_t slot = 0, phase = 0;
+    for (int tile = first_tile; tile < total && !abort_flag && alive; tile += tile_step) {
+      int mt, nt;
+      tile_coords(tile, mt, nt);
+      const int m0 = mt * 256 + cta * kRows;
+      const float* as[2];
 #pragma unroll
-      for (int j = 0; j < FBN; ++j) accum[j] = 0.f;
-      bool ok = true;
-      for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
-        const uint32_t acc = it & 1u;
-        if (!fp8_wait(tfull_bar(acc), (it >> 1) & 1u, &abort_flag, limit, p.error_flag)) {
-          ok = false;
-          break;
-        }
-        ptx::tcgen05_fence_after();
-        float scale = 0.f;
-        if (m < p.M) {
-          scale = p.a_scale[(long long)m * p.as_stride_m + (long long)kb * p.as_stride_k] *
-                  p.b_scale[(long long)nb * p.bs_stride_n + (long long)kb * p.bs_stride_k];
-        }
+      for (int r = 0; r < 2; ++r) as[r] = p.a_scale + (long long)min(m0 + l + 64 * r, p.M - 1) * p.as_stride_m;
+      for (int kb = kb0; kb < kb1; kb += kGroup) {
+        float v[2][kGroup];
+        float sb = 0.f;
+        if (vec) {  // (kb + 3 < k_blocks)
 #pragma unroll
-        for (int c = 0; c < FBN / 32; ++c) {
-          uint32_t v[32];
-          ptx::tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * FBN + c * 32, v);
-          ptx::tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 32; ++j) accum[c * 32 + j] = fmaf(__uint_as_float(v[j]), scale, accum[c * 32 + j]);
-        }
-        ptx::tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(tempty_bar(acc));
-        __syncwarp();
-      }
-      if (ok && m < p.M) {
-        __nv_bfloat16* row = p.c + (size_t)m * p.N + (size_t)nb * FBN;
-        const int ncols = min(FBN, p.N - nb * FBN);
-        if ((p.N & 7) == 0) {
-#pragma unroll
-          for (int j = 0; j < FBN; j += 8) {
-            if (j < ncols) {
-              uint4 o;
-              __nv_bfloat162 h;
-              h = __floats2bfloat162_rn(accum[j], accum[j + 1]);
-              o.x = *reinterpret_cast<uint32_t*>(&h);
-              h = __floats2bfloat162_rn(accum[j + 2], accum[j + 3]);
-              o.y = *reinterpret_cast<uint32_t*>(&h);
-              h = __floats2bfloat162_rn(accum[j + 4], accum[j + 5]);
-              o.z = *reinterpret_cast<uint32_t*>(&h);
-              h = __floats2bfloat162_rn(accum[j + 6], accum[j + 7]);
-              o.w = *reinterpret_cast<uint32_t*>(&h);
-              *reinterpret_cast<uint4*>(row + j) = o;
-            }
-          }
+          for (int r = 0; r < 2; ++r) *reinterpret_cast<float4*>(v[r]) = __ldcg(reinterpret_cast<const float4*>(as[r] + kb));
         } else {
 #pragma unroll
-          for (int j = 0; j < FBN; ++j)
-            if (j < ncols) row[j] = __float2bfloat16_rn(accum[j]);
+          for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int i = 0; i < kGroup; ++i) v[r][i] = __ldcg(as[r] + (long long)min(kb + i, kb1 - 1) * p.as_stride_k);
+        }
+        if (l < 4 * kGroup) {  // block l / 4, chunk l % 4 of the tile's columns
+          const int n = min(nt * p.bn + (l & 3) * (p.bn / 4), p.N - 1);
+          sb = __ldcg(p.b_scale + (long long)(n >> 7) * p.bs_stride_n + (long long)min(kb + (l >> 2), kb1 - 1) * p.bs_stride_k);
+        }
+        alive = __all_sync(0xffffffffu, fp8_wait(sempty_bar(slot), phase ^ 1u, &abort_flag, p));
+        if (!alive) break;
+        const uint32_t at = scales + slot * kScaleBytes;
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int i = 0; i < kGroup; ++i)
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + (uint32_t)(i * kRows + l + 64 * r) * 4u), "f"(v[r][i]) : "memory");
+        if (l < 4 * kGroup) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + (uint32_t)(kGroup * kRows + l) * 4u), "f"(sb) : "memory");
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(sfull_bar(slot));
+        if (++slot == kScaleSlots) {
+          slot = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+  } else {
+    const uint32_t slab = slabs + (uint32_t)ew * kSlabBytes;
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * chunks * 32);
+    uint32_t buf = 0, buf_phase = 0, slot = 0, slot_phase = 0, stores = 0;
+    for (int tile = first_tile; tile < total && !abort_flag && alive; tile += tile_step) {
+      int mt, nt;
+      tile_coords(tile, mt, nt);
+      const int row0 = mt * 256 + cta * kRows + q * 32;
+      const int n0 = nt * p.bn + half * chunks * 32;
+      const int m = row0 + lane;
+      const bool rows_in = row0 < p.M;
+#pragma unroll
+      for (int i = 0; i < kMaxChunks; ++i)
+#pragma unroll
+        for (int j = 0; j < 16; ++j) acc[i][j] = make_float2(0.f, 0.f);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const int in_group = (kb - kb0) % kGroup;
+        if (in_group == 0) {
+          alive = __all_sync(0xffffffffu, fp8_wait(sfull_bar(slot), slot_phase, &abort_flag, p));
+          if (!alive) break;
+        }
+        float sa, sb[2];
+        const uint32_t at = scales + slot * kScaleBytes;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sa) : "r"(at + (uint32_t)(in_group * kRows + q * 32 + lane) * 4u));
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
+                     : "=f"(sb[0]), "=f"(sb[1])
+                     : "r"(at + (uint32_t)(kGroup * kRows + in_group * 4 + half * 2) * 4u));
+        alive = __all_sync(0xffffffffu, fp8_wait(tfull_bar(buf), buf_phase, &abort_flag, p));
+        if (!alive) break;
+        ptx::tcgen05_fence_after();
+        if (rows_in) {
+          uint32_t v[kMaxChunks][32];
+          ptx::tmem_ld_32x32b_x32(lane_addr + buf * buf_cols, v[0]);
+          if (chunks == 2) ptx::tmem_ld_32x32b_x32(lane_addr + buf * buf_cols + 32, v[1]);
+          ptx::tmem_ld_wait();
+          ptx::tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_cluster(tempty_bar(buf), (uint32_t)(2 * rank));  // the pair's leader
+#pragma unroll
+          for (int i = 0; i < kMaxChunks; ++i) {
+            if (i < chunks) {
+              const float s = sa * sb[i];
+              const float2 ss = make_float2(s, s);
+#pragma unroll
+              for (int j = 0; j < 16; ++j) fma2(acc[i][j], v[i][2 * j], v[i][2 * j + 1], ss);
+            }
+          }
+        } else if (lane == 0) {
+          ptx::mbar_arrive_cluster(tempty_bar(buf), (uint32_t)(2 * rank));
+        }
+        if (++buf == (uint32_t)kBufs) {
+          buf = 0;
+          buf_phase ^= 1u;
+        }
+        if (in_group == kGroup - 1 || kb + 1 == kb1) {
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(sempty_bar(slot));
+          if (++slot == kScaleSlots) {
+            slot = 0;
+            slot_phase ^= 1u;
+          }
+        }
+      }
+      if (!alive || !rows_in || splits > 1) continue;
+      // ---- result: rounded, through the slab by TMA, or element by element where rows are ragged ------------
+#pragma unroll
+      for (int i = 0; i < kMaxChunks; ++i) {
+        if (i < chunks) {
+          const int n = n0 + i * 32;
+          if (p.tma_out) {
+            const uint32_t out = slab + (stores++ & 1u) * 2048u;
+            if (lane == 0) ptx::bulk_wait_group_read<1>();  // the store that used this buffer has read it
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {  // 16-byte piece j of row `lane`, at the place the 64-byte swizzle wants it
+              const uint32_t at = out + (uint32_t)lane * 64u + (uint32_t)((j ^ ((lane >> 1) & 3)) << 4);
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(pack2(acc[i][4 * j])), "r"(pack2(acc[i][4 * j + 1])),
+                           "r"(pack2(acc[i][4 * j + 2])), "r"(pack2(acc[i][4 * j + 3]))
+                           : "memory");
+            }
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (n < p.N) ptx::tma_store_2d(&map_c, out, n, row0);
+              ptx::bulk_commit_group();
+            }
+          } else if (m < p.M) {
+            __nv_bfloat16* row = p.c + (size_t)m * p.N;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              if (n + 2 * j < p.N) row[n + 2 * j] = __float2bfloat16_rn(acc[i][j].x);
+              if (n + 2 * j + 1 < p.N) row[n + 2 * j + 1] = __float2bfloat16_rn(acc[i][j].y);
+            }
+          }
+        }
+      }
+    }
+    if (lane == 0) ptx::bulk_wait_group_read<0>();
+  }
+
+  if (splits > 1) {
+    // One tile per cluster.  Columns [r * per, (r + 1) * per) are finished by member r; its pipeline memory, no longer in
+    // use anywhere in the cluster after the first barrier, holds [member][per / 4][128 rows] float4.
+    int mt, nt;
+    tile_coords(first_tile, mt, nt);
+    const int row0 = mt * 256 + cta * kRows + q * 32;
+    const int per = ((p.bn / 8 + splits - 1) / splits) * 8;
+    __syncwarp();
+    ptx::cluster_sync_all();
+    if (warp >= 2 && warp < 2 + kEpiWarps && alive && row0 < p.M) {
+#pragma unroll
+      for (int i = 0; i < kMaxChunks; ++i) {
+        if (i < chunks) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int col = (half * chunks + i) * 32 + j * 8;
+            const int owner = col / per;
+            const uint32_t to = (uint32_t)(2 * owner + cta);
+            const uint32_t at = base + (uint32_t)((rank * (per / 4) + (col - owner * per) / 4) * kRows + q * 32 + lane) * 16u;
+            ptx::st_cluster_v4(at, to, acc[i][4 * j].x, acc[i][4 * j].y, acc[i][4 * j + 1].x, acc[i][4 * j + 1].y);
+            ptx::st_cluster_v4(at + kRows * 16u, to, acc[i][4 * j + 2].x, acc[i][4 * j + 2].y, acc[i][4 * j + 3].x, acc[i][4 * j + 3].y);
+          }
+        }
+      }
+    }
+    __syncwarp();
+    ptx::cluster_sync_all();
+    const int m = row0 + lane;
+    if (warp >= 2 && warp < 2 + kEpiWarps && alive && m < p.M) {
+      const int c_lo = rank * per;
+      const int c_hi = min(p.bn, c_lo + per);
+      for (int col = c_lo + half * 8; col < c_hi; col += 16) {
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = 0.f;
+        for (int r = 0; r < splits; ++r) {  // ascending k
+          const uint32_t from = base + (uint32_t)((r * (per / 4) + (col - c_lo) / 4) * kRows + q * 32 + lane) * 16u;
+          float f[8];
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]) : "r"(from));
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "r"(from + kRows * 16u));
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] += f[e];
+        }
+        const int n = nt * p.bn + col;
+        if (p.tma_out) {  // (rows of whole 16-byte pieces: all eight or none)
+          if (n < p.N)
+            *reinterpret_cast<uint4*>(p.c + (size_t)m * p.N + n) =
+                make_uint4(pack2(make_float2(v[0], v[1])), pack2(make_float2(v[2], v[3])), pack2(make_float2(v[4], v[5])),
+                           pack2(make_float2(v[6], v[7])));
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (n + e < p.N) p.c[(size_t)m * p.N + n + e] = __float2bfloat16_rn(v[e]);
         }
       }
     }
@@ -238,70 +459,117 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     const uint64_t t0 = global_timer_ns();
     while (global_timer_ns() - t0 < 200000) __nanosleep(1000);
   }
+  __syncwarp();
   ptx::tcgen05_fence_before();
   __syncthreads();
+  ptx::cluster_sync_all();  // no CTA retires while another may still signal its barriers or read its memory
   ptx::tcgen05_fence_after();
-  if (warp == 1) {
-    __syncwarp();
-    ptx::tmem_dealloc(tmem_base, 2 * FBN);
-  }
+  if (warp == 1) ptx::tmem_dealloc_pair(tmem_base, kTmemCols);
 }
 
+// ---------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------
 namespace {
 
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+struct Fp8Plan {
+  int bn = 128, splits = 1, clusters = 1;
+  double ns = 1e300;
+};
 
-bool make_fp8_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess ||
-        qres != cudaDriverEntryPointSuccess)
-      return false;
-    fn = reinterpret_cast<EncodeTiledFn>(ptr);
+// The time model of the bf16 kernels (gemm_local_sm100.cu) with fp8's numbers: a 128-byte row is 128 values.
+Fp8Plan make_fp8_plan(int M, int N, int K, int sms) {
+  const int k_blocks = (K + kBlockK - 1) / kBlockK;
+  const double dram_ns = ((double)M * K + (double)N * K + 2.0 * M * N) / 6600.0;
+  const double row_ns = K % kBlockK == 0 ? 1.0 : 1.6;
+  Fp8Plan best;
+  for (int bn : {64, 128}) {
+    const int64_t tiles = (int64_t)((M + 255) / 256) * ((N + bn - 1) / bn);
+    for (int s = 1; s <= 8 && s <= k_blocks; ++s) {
+      Fp8Plan p;
+      p.bn = bn;
+      p.splits = s;
+      const int cap = std::min(gemm_cluster_capacity(2 * s), sms / (2 * s));
+      const double waves = std::ceil((double)tiles / cap);
+      if (s > 1 && waves > 1) break;
+      p.clusters = (int)std::min<int64_t>(tiles, cap);
+      const int kbs = (k_blocks + s - 1) / s;
+      const double kb_ns = std::max({row_ns * (std::min(M, 128) + bn / 2), 280.0 * bn / 256.0, 170.0});
+      const double power_ns = 2.0 * ((M + 255) / 256) * 256.0 * ((N + bn - 1) / bn) * bn * (double)k_blocks * kBlockK / 2.6e6;
+      p.ns = std::max({waves * kbs * kb_ns, power_ns, dram_ns}) +
+             (s == 1 ? 3400.0 + 9.0 * bn : 5200.0 + 28.0 * std::max(bn - 64, 0) + 50.0 * s) + (waves - 1) * 4.0 * bn;
+      if (p.ns < best.ns) best = p;
+    }
   }
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {cols};
-  cuuint32_t box[2] = {(cuuint32_t)FBK, box_rows};
-  cuuint32_t elem_strides[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, elem_strides,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return best;
+}
+
+const Fp8Plan& cached_plan(int M, int N, int K, int sms) {
+  struct Entry {
+    int M = 0, N = 0, K = 0, sms = 0, dev = -1;
+    Fp8Plan plan;
+  };
+  static thread_local Entry cache[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  Entry& e = cache[((uint32_t)M * 31u + (uint32_t)N * 7u + (uint32_t)K) * 2654435761u >> 26];
+  if (e.M != M || e.N != N || e.K != K || e.sms != sms || e.dev != dev) e = Entry{M, N, K, sms, dev, make_fp8_plan(M, N, K, sms)};
+  return e.plan;
 }
 
 }  // namespace
 
 cudaError_t launch_fp8_gemm(const Fp8GemmArgs& a, cudaStream_t stream) {
   if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.K % 16 != 0) return cudaErrorInvalidValue;
-  CUtensorMap map_a, map_b;
-  if (!make_fp8_map(&map_a, a.a, (uint64_t)a.M, (uint64_t)a.K, FBM)) return cudaErrorInvalidValue;
-  if (!make_fp8_map(&map_b, a.b, (uint64_t)a.N, (uint64_t)a.K, FBN)) return cudaErrorInvalidValue;
-  Fp8Params p;
+  const Fp8Plan& plan = cached_plan(a.M, a.N, a.K, a.sms);
+  Fp8Params p = {};
   p.a_scale = a.a_scale;
   p.b_scale = a.b_scale;
   p.c = reinterpret_cast<__nv_bfloat16*>(a.c);
   p.M = a.M;
   p.N = a.N;
-  p.K = a.K;
-  p.k_blocks = (a.K + FBK - 1) / FBK;
+  p.k_blocks = (a.K + kBlockK - 1) / kBlockK;
   p.as_stride_m = a.as_stride_m;
   p.as_stride_k = a.as_stride_k;
   p.bs_stride_n = a.bs_stride_n;
   p.bs_stride_k = a.bs_stride_k;
+  p.bn = plan.bn;
+  p.splits = plan.splits;
+  p.m_tiles = (a.M + 255) / 256;
+  p.n_tiles = (a.N + plan.bn - 1) / plan.bn;
+  p.band = std::min(8, p.m_tiles);
+  p.tma_out = (a.N % 8 == 0 && (reinterpret_cast<uintptr_t>(a.c) & 15u) == 0) ? 1 : 0;
   p.timeout_ns = a.timeout_ns;
-  p.error_flag = a.error_flag;
-  cudaError_t e = cudaFuncSetAttribute(fp8_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFp8SmemBytes);
-  if (e != cudaSuccess) return e;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int total = ((a.M + FBM - 1) / FBM) * ((a.N + FBN - 1) / FBN);
-  const int grid = std::max(1, std::min(total, sms));
-  fp8_gemm_kernel<<<grid, kFp8Threads, kFp8SmemBytes, stream>>>(map_a, map_b, p);
-  return cudaGetLastError();
+  const int stage_bytes = kABytes + plan.bn / 2 * kBlockK;
+  const int room = kMaxDynamicSmem - 1024 - kTailBytes;
+  const int parts = plan.splits > 1 ? plan.splits * ((plan.bn / 8 + plan.splits - 1) / plan.splits) * 8 * kRows * 4 : 0;
+  p.stages = std::min(kMaxStages, room / stage_bytes);
+  p.stage_area = std::max(p.stages * stage_bytes, parts);  // multiples of 1024
+  if (p.stage_area > room) return cudaErrorInvalidValue;
+  CUtensorMap map_a, map_b, map_c = {};
+  if (!make_tensor_map(&map_a, a.a, (uint64_t)a.M, (uint64_t)a.K, 1, kRows, kBlockK, 128) ||
+      !make_tensor_map(&map_b, a.b, (uint64_t)a.N, (uint64_t)a.K, 1, (uint32_t)plan.bn / 2, kBlockK, 128) ||
+      (p.tma_out && !make_tensor_map(&map_c, a.c, (uint64_t)a.M, (uint64_t)a.N, 2, 32, 32, 64)))
+    return cudaErrorInvalidValue;
+  static const cudaError_t opted = cudaFuncSetAttribute(fp8_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+  static const cudaError_t opted2 = cudaFuncSetAttribute(fp8_gemm_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (opted != cudaSuccess || opted2 != cudaSuccess) return opted != cudaSuccess ? opted : opted2;
+  const int total = p.m_tiles * p.n_tiles;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * plan.splits * (plan.splits > 1 ? total : plan.clusters)));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = 1024 + (size_t)p.stage_area + kTailBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)(2 * plan.splits);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, fp8_gemm_kernel, map_a, map_b, map_c, p);
 }
 
 }  // namespace b200

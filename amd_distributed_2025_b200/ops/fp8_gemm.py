@@ -47,14 +47,17 @@ def fp8_gemm(
     from . import _ext
 
     ext = _ext.load()
+    if c is None:
+        c = ext.fp8_gemm_try(a, b, a_scale, b_scale, int(timeout_ms * 1e6))
+        if c is not None:
+            return c
     if not a.is_contiguous():  # e.g. the template's column-major storage, a [K, M] buffer viewed as [M, K]
         a = a.contiguous()
     if not b.is_contiguous():
         b = b.contiguous()
     if c is None:
         c = torch.empty((a.shape[0], b.shape[0]), dtype=torch.bfloat16, device=a.device)
-    flag = torch.zeros(1, dtype=torch.int32, device=a.device)
-    ext.fp8_gemm(a, b, a_scale, b_scale, c, flag, int(timeout_ms * 1e6))
+    ext.fp8_gemm(a, b, a_scale, b_scale, c, int(timeout_ms * 1e6))
     return c
 
 

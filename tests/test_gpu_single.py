@@ -302,6 +302,24 @@ def test_fp8_block_scaled_gemm_matches_fp32_reference(m, n, k):
     assert torch.allclose(c.float(), want, rtol=2e-2, atol=2e-2 * float(want.abs().max()))
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 8, 16), (257, 200, 1040), (64, 1024, 4096), (300, 619, 400), (129, 136, 1408), (4100, 3000, 640)])
+def test_fp8_gemm_schedules(m, n, k):
+    """Shared and whole tiles, ragged rows, columns and K, scales by rows (four at a time where aligned), with and without ``c``."""
+    from amd_distributed_2025_b200.ops.fp8_gemm import fp8_gemm, fp8_gemm_reference
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randn(m, k, device="cuda", generator=g).to(torch.float8_e4m3fn)
+    b = torch.randn(n, k, device="cuda", generator=g).to(torch.float8_e4m3fn)
+    a_scale = torch.rand(m, (k + 127) // 128, device="cuda", generator=g) + 0.5
+    b_scale = torch.rand((n + 127) // 128, (k + 127) // 128, device="cuda", generator=g) + 0.5
+    out = fp8_gemm(a, b, a_scale, b_scale)
+    again = fp8_gemm(a, b, a_scale, b_scale, c=torch.empty_like(out))
+    want = fp8_gemm_reference(a, b, a_scale, b_scale)
+    assert torch.equal(out, again)
+    assert oracle.relative_error(out, want) < 5e-3
+    assert float((out.float() - want).abs().max()) < 1e-2 * float(want.abs().max())
+
+
 @pytest.mark.parametrize("tma_store", [True, False])
 @pytest.mark.parametrize("fuse_own", [True, False])
 @pytest.mark.parametrize("m,n,k,block_n,cta_pair", [(2048, 2048, 1024, 256, 1), (1024, 2880, 512, 192, 1), (512, 1024, 256, 128, 0),
