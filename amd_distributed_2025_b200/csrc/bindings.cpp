@@ -749,7 +749,7 @@ class GemmRsEngine {
     g.bias_scale = (float)bias_scale;
     g.bias_at_source = bias_at_source ? 1 : 0;
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
-    const LocalWorkspace* ws = local_workspace(stream);
+    const LocalWorkspace* ws = b200::gemm_local_cuts_tiles(g.M, g.N, g.K, sms_) ? local_workspace(stream) : nullptr;
     g.partials = ws ? ws->partials : nullptr;
     g.counters = ws ? ws->counters : nullptr;
     g.timeout_ns = (uint64_t)timeout_ns_;
@@ -759,23 +759,35 @@ class GemmRsEngine {
     ++epoch_;
     cuda_check(b200::launch_gemm_local(g, stream), "gemm_local launch");
   }
-  // Cut tiles meet in a workspace, one per stream because calls on two streams may overlap; at most four, kept with
-  // the operator.  Null (no tile is cut then) for further streams, and for a stream first seen while it is being
-  // captured: zeroing the counters would become part of the graph.
+  // Cut tiles meet in a workspace, one per stream because calls on two streams may overlap, and one more per graph
+  // that a stream is captured into, because the graph may be replayed on another (its counters are then zeroed by the
+  // graph itself).  At most four of either kind are kept with the operator; null (no tile is cut then) beyond them.
   struct LocalWorkspace {
     cudaStream_t stream;
+    unsigned long long capture;  // 0: calls that run at once
     at::Tensor keep;
     float* partials;
     uint32_t* counters;
   };
   const LocalWorkspace* local_workspace(cudaStream_t stream) {
-    for (const auto& ws : workspaces_)
-      if (ws.stream == stream) return &ws;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (workspaces_.size() >= 4 || cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
-      return nullptr;
+    unsigned long long capture = 0;
+    if (cudaStreamGetCaptureInfo(stream, &capturing, &capture) != cudaSuccess || capturing == cudaStreamCaptureStatusInvalidated) return nullptr;
+    if (capturing == cudaStreamCaptureStatusNone) capture = 0;
+    for (const auto& ws : workspaces_)
+      if (ws.stream == stream && ws.capture == capture) return &ws;
+    const auto same_kind = [&](const LocalWorkspace& ws) { return (ws.capture != 0) == (capture != 0); };
+    if (std::count_if(workspaces_.begin(), workspaces_.end(), same_kind) >= 4) {
+      if (capture == 0) return nullptr;
+      // graphs captured before keep theirs alive in their own memory pool
+      workspaces_.erase(std::remove_if(workspaces_.begin(), workspaces_.end(),
+                                       [&](const LocalWorkspace& ws) { return ws.capture != 0 && ws.capture != capture; }),
+                        workspaces_.end());
+      if (std::count_if(workspaces_.begin(), workspaces_.end(), same_kind) >= 4) return nullptr;
+    }
     LocalWorkspace ws;
     ws.stream = stream;
+    ws.capture = capture;
     ws.keep = at::detail::empty_cuda({(int64_t)(b200::kGemmLocalPartialBytes + 4 * b200::kGemmLocalCounters)}, at::kByte,
                                      at::Device(at::kCUDA, (c10::DeviceIndex)heap_->device()), c10::nullopt);
     uint8_t* base = ws.keep.mutable_data_ptr<uint8_t>();

@@ -934,6 +934,11 @@ cudaError_t launch_tile(const GemmLocalArgs& a, const Plan& plan, cudaStream_t s
 
 }  // namespace
 
+bool gemm_local_cuts_tiles(int M, int N, int K, int sms) {
+  const Plan& plan = cached_plan(M, N, K, sms);
+  return plan.persistent && plan.sk_tiles > 0;
+}
+
 cudaError_t launch_gemm_local(const GemmLocalArgs& a, cudaStream_t stream) {
   if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.K % 8 != 0 || a.N % 8 != 0) return cudaErrorInvalidValue;
   Plan plan = cached_plan(a.M, a.N, a.K, a.sms);

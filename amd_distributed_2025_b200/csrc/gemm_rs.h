@@ -98,6 +98,7 @@ constexpr uint64_t kGemmLocalPartialBytes = (uint64_t)kGemmLocalMaxPairs * 2 * 2
 constexpr int kGemmLocalCounters = kGemmLocalMaxPairs * 2 * 2 * 8;
 
 cudaError_t launch_gemm_local(const GemmLocalArgs& args, cudaStream_t stream);
+bool gemm_local_cuts_tiles(int M, int N, int K, int sms);  // whether the launch has a use for `partials`
 
 // How many clusters of `size` (1..16) CTAs that each fill an SM's shared memory are resident at once.
 int gemm_cluster_capacity(int size);

@@ -205,6 +205,8 @@ class GemmRS:
 
 
 _OPS: Dict[tuple, GemmRS] = {}
+# The operator of a program of one process and one GPU: its calls need neither the lookup nor a workspace of their size.
+_one_rank: Optional[GemmRS] = None
 
 
 def get_op(m: int, n: int, k: int = 0, group=None, splits_hint: int = 8) -> GemmRS:
@@ -219,6 +221,8 @@ def get_op(m: int, n: int, k: int = 0, group=None, splits_hint: int = 8) -> Gemm
     op = _OPS.get(key)
     if op is not None and (m, n, k) in op._fits:
         return op
+    global _one_rank
+    _one_rank = None
     from ..ops import _ext
 
     ext = _ext.load()
@@ -235,6 +239,8 @@ def get_op(m: int, n: int, k: int = 0, group=None, splits_hint: int = 8) -> Gemm
     if op is not None:
         if need_stage <= op.stage_bytes and need_counters <= op.counter_bytes:
             op._fits.add((m, n, k))
+            if not initialized and torch.cuda.device_count() == 1:
+                _one_rank = op
             return op
         torch.cuda.synchronize()
         if initialized:
@@ -244,6 +250,8 @@ def get_op(m: int, n: int, k: int = 0, group=None, splits_hint: int = 8) -> Gemm
     op = GemmRS(need_stage, need_counters, group=group)
     op._fits.add((m, n, k))
     _OPS[key] = op
+    if not initialized and torch.cuda.device_count() == 1:
+        _one_rank = op
     return op
 
 
@@ -265,6 +273,8 @@ def reserve(shapes, group=None) -> GemmRS:
 
 def release_ops() -> None:
     """Free every cached workspace (collective: all ranks must call it while idle)."""
+    global _one_rank
+    _one_rank = None
     for op in _OPS.values():
         op.close(collective=True)
     _OPS.clear()
@@ -283,6 +293,12 @@ def custom_kernel(data: GemmRsInput, bias_mode: str = "per_rank", backend: str =
     (models/host_ops.py) for CPU tensors when all ranks share a machine, library collectives
     otherwise; "shm" and "torch" force the latter two."""
     a, w, bias = data
+    op = _one_rank
+    if (op is not None and backend == "auto" and op.monitor is None and not dist.is_initialized()
+            and (bias_mode == "per_rank" or bias_mode == "once")):
+        out = op.engine.try_run(a, w, bias, bias_mode == "per_rank")
+        if out is not None:
+            return out
     if backend == "shm" or (backend == "auto" and not a.is_cuda and _cpu_ranks_share_a_node()):
         from . import host_ops
 
