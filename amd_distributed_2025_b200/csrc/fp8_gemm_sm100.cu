@@ -8,15 +8,20 @@
 // them with the 128-byte swizzle exactly as in the bf16 GEMM (a 128-byte row now holds 128 fp8 values).
 //
 // A CTA pair (cta_group::2) owns a tile of 256 rows of A by `bn` (64 or 128) rows of B.  Every 128-wide K block is
-// multiplied into a tensor-memory buffer of its own, one of four; eight epilogue warps, two per tensor-memory lane
-// quarter, pull it out, multiply by the block's scales and accumulate in fp32 registers while the next blocks are
-// being multiplied.  Two warps bring the scales in, sixteen blocks ahead: a row's scales lie in a line of their own,
-// and fetched by the epilogue itself they took longer than the products.  Pairs are persistent; where there are fewer
-// tiles than pairs, a cluster of pairs shares a tile, each over its part of K, and the parts meet in distributed
-// shared memory.
+// multiplied into tensor memory of its own, two neighbouring blocks to a buffer, two buffers; eight epilogue warps, two
+// per tensor-memory lane quarter, pull the products out, multiply by the blocks' scales and accumulate in fp32
+// registers while the next two blocks are being multiplied.  Two warps bring the scales in by asynchronous copies,
+// sixteen blocks ahead: a row's scales lie in a line of their own, and fetched by the epilogue itself they took longer
+// than the products.  Pairs are persistent; where there are fewer tiles than pairs, a cluster of pairs shares a tile,
+// each over its part of K, and the parts meet in distributed shared memory.
 //
-// Why 128 columns and four buffers: a buffer comes back after multiplication, signal, read-out and signal, some 1100
-// cycles in all, of which the multiplication is 256; two buffers of 256 columns left the tensor cores waiting.
+// What bounds it: the epilogue.  For a K block a warp spends some 300 cycles on reading and scaling 64 columns, 130 on
+// the signal that frees the buffer and 130 on the wait for the next, against 256 cycles of multiplication; meeting once
+// for two blocks halves the last two, and the read of a chunk runs beside the sums of the one before.  Tried and slower
+// at 4096 x 4096 x 2048: 256 columns in halves with split registers (40.6 us; few tiles, long ends), sixteen epilogue
+// warps (52 us; the waits doubled), warp-wide waits (40.8 us).
+// On a B200, us, with one block a buffer and scales through registers -> now: 4096 x 4096 x 2048 40.9 -> 37.8,
+// 8192 x 8192 x 4096 293 -> 268, 2048^3 14.5 -> 13.0, 512 x 512 x 8192 12.6 -> 10.7, 64 x 4096 x 4096 11.6 -> 10.2.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -45,9 +50,10 @@ constexpr int kMaxStages = 12;
 constexpr int kSlabBytes = 2 * 2048;      // per epilogue warp: two buffers of 32 rows x 64 bytes
 constexpr int kGroup = 4;                 // K blocks whose scales come in together
 constexpr int kScaleSlots = 4;
-constexpr int kScaleBytes = kGroup * (kRows + 4) * 4;  // [block][row], then [block][half of the columns][chunk]
+constexpr int kScaleBytes = kGroup * (kRows + 4) * 4;  // [row][block], then [half of the columns][block][chunk]
 constexpr int kTailBytes = kEpiWarps * kSlabBytes + kScaleSlots * kScaleBytes + 512;
-constexpr int kBufs = 4;
+constexpr int kBufs = 2;                  // tensor-memory buffers, each of
+constexpr int kStep = 2;                  // K blocks
 constexpr int kMaxDynamicSmem = 232448 - 256;
 constexpr int kTmemCols = 512;
 constexpr int kMaxChunks = 2;             // 32-column chunks of an epilogue warp
@@ -82,13 +88,13 @@ __device__ __forceinline__ void umma_fp8_pair(uint32_t tmem_d, uint64_t desc_a, 
 }
 
 __device__ __forceinline__ bool fp8_wait(uint32_t bar, uint32_t parity, volatile int* abort, const Fp8Params& p) {
-  if (ptx::mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = global_timer_ns();
-  uint32_t spins = 0;
-  while (!ptx::mbar_try_wait(bar, parity)) {
-    if ((++spins & 255u) == 0) {
+  uint64_t t0 = 0;  // (the clock takes longer to read than most waits last)
+  for (uint32_t spins = 1; !ptx::mbar_try_wait(bar, parity); ++spins) {
+    if ((spins & 255u) == 0) {
       if (*abort) return false;
-      if (global_timer_ns() - t0 > p.timeout_ns) {
+      const uint64_t now = global_timer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > p.timeout_ns) {
         *abort = 1;
         return false;
       }
@@ -100,9 +106,24 @@ __device__ __forceinline__ bool fp8_wait(uint32_t bar, uint32_t parity, volatile
 // acc[0..1] += v[0..1] * s
 __device__ __forceinline__ void fma2(float2& acc, uint32_t v0, uint32_t v1, float2 ss) {
   const float2 v = make_float2(__uint_as_float(v0), __uint_as_float(v1));
-  asm("fma.rn.f32x2 %0, %1, %2, %0;"
+  // (volatile: not before the wait for the tensor memory load that brings v)
+  asm volatile("fma.rn.f32x2 %0, %1, %2, %0;"
       : "+l"(reinterpret_cast<unsigned long long&>(acc))
       : "l"(reinterpret_cast<const unsigned long long&>(v)), "l"(reinterpret_cast<const unsigned long long&>(ss)));
+}
+
+template <int BYTES>
+__device__ __forceinline__ void cp_async(uint32_t to, const float* from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(to), "l"(from), "n"(BYTES) : "memory");
+}
+
+// Arrives on `bar` when this thread's copies so far have landed.
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void ld_shared_f4(float* to, uint32_t from) {
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(to[0]), "=f"(to[1]), "=f"(to[2]), "=f"(to[3]) : "r"(from) : "memory");
 }
 
 __device__ __forceinline__ uint32_t pack2(float2 f) {
@@ -126,13 +147,16 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   const int cluster_rank = (int)ptx::cluster_ctarank();
   const int rank = cluster_rank >> 1;  // which part of K
   const int cta = cluster_rank & 1;    // which half of the pair's rows
-  const int kb0 = (int)((int64_t)p.k_blocks * rank / splits);
-  const int kb1 = (int)((int64_t)p.k_blocks * (rank + 1) / splits);
+  // parts of K; even bounds where that is little of a part, so that scales still come in by pieces of 8 bytes
+  const int round = p.k_blocks >= 4 * splits ? ~1 : ~0;
+  const int kb0 = (int)((int64_t)p.k_blocks * rank / splits) & round;
+  const int kb1 = rank + 1 == splits ? p.k_blocks : (int)((int64_t)p.k_blocks * (rank + 1) / splits) & round;
   const int first_tile = (int)blockIdx.x / (2 * splits);
   const int tile_step = (int)gridDim.x / (2 * splits);
   const int total = p.m_tiles * p.n_tiles;
   const int b_rows = p.bn / 2;  // rows of B that this CTA brings in
   constexpr uint32_t buf_cols = kTmemCols / kBufs;
+  constexpr uint32_t block_cols = buf_cols / kStep;
 
   const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t stage_bytes = kABytes + (uint32_t)b_rows * kBlockK;
@@ -157,7 +181,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       ptx::mbar_init(tempty_bar(s), 2 * kEpiWarps);
     }
     for (int s = 0; s < kScaleSlots; ++s) {
-      ptx::mbar_init(sfull_bar(s), kScaleWarps);
+      ptx::mbar_init(sfull_bar(s), 32 * kScaleWarps);
       ptx::mbar_init(sempty_bar(s), kEpiWarps);
     }
     ptx::fence_mbar_init();
@@ -224,73 +248,77 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const uint16_t both = (uint16_t)(3u << (2 * rank));
       uint32_t stage = 0, phase = 0, buf = 0, buf_phase = 0;
       for (int tile = first_tile; tile < total && !abort_flag; tile += tile_step) {
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!fp8_wait(tempty_bar(buf), buf_phase ^ 1u, &abort_flag, p)) break;
-          if (!fp8_wait(full_bar(stage), phase, &abort_flag, p)) break;
+        bool ok = true;
+        for (int kb = kb0; kb < kb1 && ok; kb += kStep) {
+          ok = fp8_wait(tempty_bar(buf), buf_phase ^ 1u, &abort_flag, p);
           ptx::tcgen05_fence_after();
-          const uint32_t sa = base + stage * stage_bytes;
-          const uint64_t da = ptx::make_smem_desc_k_sw128(sa);
-          const uint64_t db = ptx::make_smem_desc_k_sw128(sa + kABytes);
-          const uint32_t d = tmem_base + buf * buf_cols;
-          if (ptx::elect_one()) {
 #pragma unroll
-            for (int j = 0; j < kBlockK / 32; ++j)  // 32 fp8 of K = 32 bytes = 2 descriptor address units
-              umma_fp8_pair(d, da + 2u * j, db + 2u * j, idesc, j > 0 ? 1u : 0u);
-            ptx::umma_commit_pair(empty_bar(stage), both);
-            ptx::umma_commit_pair(tfull_bar(buf), both);
-          }
-          __syncwarp();
-          if (++stage == (uint32_t)p.stages) {
-            stage = 0;
-            phase ^= 1u;
+          for (int i = 0; i < kStep; ++i) {
+            if (kb + i >= kb1) break;
+            ok = ok && fp8_wait(full_bar(stage), phase, &abort_flag, p);
+            if (!ok) break;
+            ptx::tcgen05_fence_after();
+            const uint32_t sa = base + stage * stage_bytes;
+            const uint64_t da = ptx::make_smem_desc_k_sw128(sa);
+            const uint64_t db = ptx::make_smem_desc_k_sw128(sa + kABytes);
+            const uint32_t d = tmem_base + buf * buf_cols + i * block_cols;
+            if (ptx::elect_one()) {
+#pragma unroll
+              for (int j = 0; j < kBlockK / 32; ++j)  // 32 fp8 of K = 32 bytes = 2 descriptor address units
+                umma_fp8_pair(d, da + 2u * j, db + 2u * j, idesc, j > 0 ? 1u : 0u);
+              ptx::umma_commit_pair(empty_bar(stage), both);
+              if (i == kStep - 1 || kb + i + 1 == kb1) ptx::umma_commit_pair(tfull_bar(buf), both);
+            }
+            __syncwarp();
+            if (++stage == (uint32_t)p.stages) {
+              stage = 0;
+              phase ^= 1u;
+            }
           }
           if (++buf == (uint32_t)kBufs) {
             buf = 0;
             buf_phase ^= 1u;
           }
         }
+        if (!ok) break;
       }
     }
   } else if (warp >= 2 + kEpiWarps) {
-    // ---- scales: two rows per lane, four K blocks at a time ------------------------------------------------
+    // ---- scales: two rows per lane, four K blocks at a time, sixteen under way ------------------------------
     const int l = (warp - 2 - kEpiWarps) * 32 + lane;
-    const bool vec = p.as_stride_k == 1 && p.as_stride_m % 4 == 0 && kb0 % 4 == 0 && p.k_blocks % 4 == 0 &&
-                     (reinterpret_cast<uintptr_t>(p.a_scale) & 15u) == 0;
+    // how many neighbouring scales of a row one copy may take: addresses, group starts and the end of the row allow it
+    const uint64_t ends = reinterpret_cast<uintptr_t>(p.a_scale) / 4 | (uint64_t)p.as_stride_m | (uint64_t)kb0 | (uint64_t)p.k_blocks;
+    const int wide = p.as_stride_k != 1 || ends % 2 != 0 ? 1 : ends % 4 != 0 ? 2 : 4;
     uint32_t slot = 0, phase = 0;
-    for (int tile = first_tile; tile < total && !abort_flag && alive; tile += tile_step) {
+    for (int tile = first_tile; tile < total && !abort_flag; tile += tile_step) {
       int mt, nt;
       tile_coords(tile, mt, nt);
       const int m0 = mt * 256 + cta * kRows;
-      const float* as[2];
-#pragma unroll
-      for (int r = 0; r < 2; ++r) as[r] = p.a_scale + (long long)min(m0 + l + 64 * r, p.M - 1) * p.as_stride_m;
       for (int kb = kb0; kb < kb1; kb += kGroup) {
-        float v[2][kGroup];
-        float sb = 0.f;
-        if (vec) {  // (kb + 3 < k_blocks)
+        if (!fp8_wait(sempty_bar(slot), phase ^ 1u, &abort_flag, p)) break;
+        const uint32_t at = scales + slot * kScaleBytes;
 #pragma unroll
-          for (int r = 0; r < 2; ++r) *reinterpret_cast<float4*>(v[r]) = __ldcg(reinterpret_cast<const float4*>(as[r] + kb));
-        } else {
+        for (int r = 0; r < 2; ++r) {
+          const int row = l + 64 * r;
+          if (m0 + row >= p.M) break;  // (nobody reads what such a row multiplies)
+          const float* as = p.a_scale + (long long)(m0 + row) * p.as_stride_m;
+          const uint32_t to = at + (uint32_t)row * 16u;
+          if (wide == 4) {  // (kb + 3 < k_blocks)
+            cp_async<16>(to, as + kb);
+          } else if (wide == 2) {
+            cp_async<8>(to, as + kb);
+            cp_async<8>(to + 8u, as + min(kb + 2, p.k_blocks - 2));
+          } else {
 #pragma unroll
-          for (int r = 0; r < 2; ++r)
-#pragma unroll
-            for (int i = 0; i < kGroup; ++i) v[r][i] = __ldcg(as[r] + (long long)min(kb + i, kb1 - 1) * p.as_stride_k);
+            for (int i = 0; i < kGroup; ++i) cp_async<4>(to + 4u * i, as + (long long)min(kb + i, p.k_blocks - 1) * p.as_stride_k);
+          }
         }
         if (l < 4 * kGroup) {  // block l / 4, chunk l % 4 of the tile's columns
           const int n = min(nt * p.bn + (l & 3) * (p.bn / 4), p.N - 1);
-          sb = __ldcg(p.b_scale + (long long)(n >> 7) * p.bs_stride_n + (long long)min(kb + (l >> 2), kb1 - 1) * p.bs_stride_k);
+          cp_async<4>(at + (uint32_t)(kGroup * kRows + (l & 2) * kGroup + (l >> 2) * 2 + (l & 1)) * 4u,
+                     p.b_scale + (long long)(n >> 7) * p.bs_stride_n + (long long)min(kb + (l >> 2), p.k_blocks - 1) * p.bs_stride_k);
         }
-        alive = __all_sync(0xffffffffu, fp8_wait(sempty_bar(slot), phase ^ 1u, &abort_flag, p));
-        if (!alive) break;
-        const uint32_t at = scales + slot * kScaleBytes;
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-#pragma unroll
-          for (int i = 0; i < kGroup; ++i)
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + (uint32_t)(i * kRows + l + 64 * r) * 4u), "f"(v[r][i]) : "memory");
-        if (l < 4 * kGroup) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + (uint32_t)(kGroup * kRows + l) * 4u), "f"(sb) : "memory");
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(sfull_bar(slot));
+        cp_async_arrive(sfull_bar(slot));
         if (++slot == kScaleSlots) {
           slot = 0;
           phase ^= 1u;
@@ -301,66 +329,78 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const uint32_t slab = slabs + (uint32_t)ew * kSlabBytes;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * chunks * 32);
     uint32_t buf = 0, buf_phase = 0, slot = 0, slot_phase = 0, stores = 0;
-    for (int tile = first_tile; tile < total && !abort_flag && alive; tile += tile_step) {
+    for (int tile = first_tile; tile < total && !abort_flag; tile += tile_step) {
       int mt, nt;
       tile_coords(tile, mt, nt);
       const int row0 = mt * 256 + cta * kRows + q * 32;
       const int n0 = nt * p.bn + half * chunks * 32;
       const int m = row0 + lane;
       const bool rows_in = row0 < p.M;
+      uint32_t v[kMaxChunks][32];
 #pragma unroll
       for (int i = 0; i < kMaxChunks; ++i)
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc[i][j] = make_float2(0.f, 0.f);
-      for (int kb = kb0; kb < kb1; ++kb) {
-        const int in_group = (kb - kb0) % kGroup;
-        if (in_group == 0) {
-          alive = __all_sync(0xffffffffu, fp8_wait(sfull_bar(slot), slot_phase, &abort_flag, p));
-          if (!alive) break;
+        for (int j = 0; j < 16; ++j) {
+          acc[i][j] = make_float2(0.f, 0.f);
+          v[i][2 * j] = v[i][2 * j + 1] = 0;
         }
-        float sa, sb[2];
+      float2 last = make_float2(0.f, 0.f);  // scale of v[1]: it is added while the next block's v[0] is on its way
+      for (int kb = kb0; kb < kb1; kb += kGroup) {
+        // (where a wait expires, the numbers are of no use any more; the loop still ends, and `alive` is asked after it)
+        alive &= fp8_wait(sfull_bar(slot), slot_phase, &abort_flag, p);
+        __syncwarp();
+        float sa[kGroup], sb[2 * kGroup];
         const uint32_t at = scales + slot * kScaleBytes;
-        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sa) : "r"(at + (uint32_t)(in_group * kRows + q * 32 + lane) * 4u));
-        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
-                     : "=f"(sb[0]), "=f"(sb[1])
-                     : "r"(at + (uint32_t)(kGroup * kRows + in_group * 4 + half * 2) * 4u));
-        alive = __all_sync(0xffffffffu, fp8_wait(tfull_bar(buf), buf_phase, &abort_flag, p));
-        if (!alive) break;
-        ptx::tcgen05_fence_after();
-        if (rows_in) {
-          uint32_t v[kMaxChunks][32];
-          ptx::tmem_ld_32x32b_x32(lane_addr + buf * buf_cols, v[0]);
-          if (chunks == 2) ptx::tmem_ld_32x32b_x32(lane_addr + buf * buf_cols + 32, v[1]);
-          ptx::tmem_ld_wait();
-          ptx::tcgen05_fence_before();
+        ld_shared_f4(sa, at + (uint32_t)(q * 32 + lane) * 16u);
+        ld_shared_f4(sb, at + (uint32_t)(kGroup * kRows + half * 2 * kGroup) * 4u);
+        ld_shared_f4(sb + 4, at + (uint32_t)(kGroup * kRows + half * 2 * kGroup + 4) * 4u);
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(sempty_bar(slot));
+        if (++slot == kScaleSlots) {
+          slot = 0;
+          slot_phase ^= 1u;
+        }
+#pragma unroll
+        for (int i0 = 0; i0 < kGroup; i0 += kStep) {
+          if (kb + i0 >= kb1) break;
+          alive &= fp8_wait(tfull_bar(buf), buf_phase, &abort_flag, p);
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive_cluster(tempty_bar(buf), (uint32_t)(2 * rank));  // the pair's leader
+          ptx::tcgen05_fence_after();
+          if (rows_in) {
 #pragma unroll
-          for (int i = 0; i < kMaxChunks; ++i) {
-            if (i < chunks) {
-              const float s = sa * sb[i];
-              const float2 ss = make_float2(s, s);
+            for (int i = i0; i < i0 + kStep; ++i) {
+              if (kb + i >= kb1) break;
+              const uint32_t from = lane_addr + buf * buf_cols + (i - i0) * block_cols;
+              ptx::tmem_ld_32x32b_x32(from, v[0]);
+              if (chunks == 2) {
 #pragma unroll
-              for (int j = 0; j < 16; ++j) fma2(acc[i][j], v[i][2 * j], v[i][2 * j + 1], ss);
+                for (int j = 0; j < 16; ++j) fma2(acc[1][j], v[1][2 * j], v[1][2 * j + 1], last);
+              }
+              ptx::tmem_ld_wait();
+              if (chunks == 2) ptx::tmem_ld_32x32b_x32(from + 32, v[1]);
+              const float2 first = make_float2(sa[i] * sb[2 * i], sa[i] * sb[2 * i]);
+#pragma unroll
+              for (int j = 0; j < 16; ++j) fma2(acc[0][j], v[0][2 * j], v[0][2 * j + 1], first);
+              last = make_float2(sa[i] * sb[2 * i + 1], sa[i] * sb[2 * i + 1]);
+              ptx::tmem_ld_wait();
             }
+            ptx::tcgen05_fence_before();
+            __syncwarp();
           }
-        } else if (lane == 0) {
-          ptx::mbar_arrive_cluster(tempty_bar(buf), (uint32_t)(2 * rank));
-        }
-        if (++buf == (uint32_t)kBufs) {
-          buf = 0;
-          buf_phase ^= 1u;
-        }
-        if (in_group == kGroup - 1 || kb + 1 == kb1) {
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(sempty_bar(slot));
-          if (++slot == kScaleSlots) {
-            slot = 0;
-            slot_phase ^= 1u;
+          if (lane == 0) ptx::mbar_arrive_cluster(tempty_bar(buf), (uint32_t)(2 * rank));  // the pair's leader
+          if (++buf == (uint32_t)kBufs) {
+            buf = 0;
+            buf_phase ^= 1u;
           }
         }
       }
-      if (!alive || !rows_in || splits > 1) continue;
+      if (chunks == 2) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) fma2(acc[1][j], v[1][2 * j], v[1][2 * j + 1], last);
+      }
+      alive = __all_sync(0xffffffffu, alive);
+      if (!alive) break;
+      if (!rows_in || splits > 1) continue;
       // ---- result: rounded, through the slab by TMA, or element by element where rows are ragged ------------
 #pragma unroll
       for (int i = 0; i < kMaxChunks; ++i) {
@@ -435,8 +475,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         for (int r = 0; r < splits; ++r) {  // ascending k
           const uint32_t from = base + (uint32_t)((r * (per / 4) + (col - c_lo) / 4) * kRows + q * 32 + lane) * 16u;
           float f[8];
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]) : "r"(from));
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "r"(from + kRows * 16u));
+          ld_shared_f4(f, from);
+          ld_shared_f4(f + 4, from + kRows * 16u);
 #pragma unroll
           for (int e = 0; e < 8; ++e) v[e] += f[e];
         }
