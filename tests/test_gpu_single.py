@@ -302,7 +302,7 @@ def test_fp8_block_scaled_gemm_matches_fp32_reference(m, n, k):
     assert torch.allclose(c.float(), want, rtol=2e-2, atol=2e-2 * float(want.abs().max()))
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 8, 16), (257, 200, 1040), (64, 1024, 4096), (300, 619, 400), (129, 136, 1408), (4100, 3000, 640)])
+@pytest.mark.parametrize("m,n,k", [(1, 8, 16), (257, 200, 1040), (64, 1024, 4096), (200, 264, 1280), (300, 619, 400), (129, 136, 1408), (4100, 3000, 640)])
 def test_fp8_gemm_schedules(m, n, k):
     """Shared and whole tiles, ragged rows, columns and K, scales by rows (four at a time where aligned), with and without ``c``."""
     from amd_distributed_2025_b200.ops.fp8_gemm import fp8_gemm, fp8_gemm_reference
