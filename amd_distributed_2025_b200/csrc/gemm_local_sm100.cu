@@ -11,7 +11,10 @@
 //                      256; where there are fewer tiles than SMs, a cluster of them shares a tile, each with a part of
 //                      K, and adds the parts up through distributed shared memory.
 //   gemm_pair_kernel   larger ones: persistent CTA pairs (cta_group::2) on tiles of 256 P rows; the last wave, which
-//                      would leave pairs idle, is dealt out by k-blocks instead of by tiles.
+//                      would leave pairs idle, is dealt out by k-blocks instead of by tiles.  The largest ones run
+//                      against the power limit: there a tile is 512 columns, both accumulators wide, and a quarter
+//                      less operand traffic buys clock (8192 x 8192 x 28672 in a row of calls: 2980 us at 1100 MHz with
+//                      256 columns, 2846 us at 1280 MHz with 512; cuBLAS 2863 us at 1245 MHz).
 //
 // Warp roles of both (320 threads, one CTA per SM): 0 TMA producer, 1 MMA issuer, 2..9 epilogue, two per
 // tensor-memory lane quarter.
@@ -58,6 +61,7 @@ struct LocalParams {
   int part_bytes;     // tile kernel: shared memory of its own for their parts (0: they take the pipeline's)
   int stage_area;     // tile kernel: bytes of the pipeline's stages, and of the parts where these share them
   int sk_tiles, total_tiles;  // pair kernel
+  int halves;         // pair kernel: 2 = a tile is twice `bn` columns, one accumulator for each half
   float* partials;    // pair kernel: [2][pair][cta][bn / 32][8][128 rows] float4
   int64_t far_part;   // float4s between the two halves of `partials`
   uint32_t* counters; // pair kernel: [sk_tiles][cta][epilogue warp], zero between launches
@@ -256,7 +260,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
   const int pairs = (int)gridDim.x >> 1;
 
   const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t stage_bytes = kPBytes + (uint32_t)p.bn * (kBK * 2 / 2);  // this CTA's half of the Q rows
+  const uint32_t q_bytes = (uint32_t)p.bn * (kBK * 2 / 2);  // this CTA's part of the Q rows
+  const uint32_t stage_bytes = kPBytes + (uint32_t)p.halves * q_bytes;
   const uint32_t slabs = base + (uint32_t)p.stages * stage_bytes;
   const uint32_t bias_smem = slabs + kEpiWarps * kSlabBytes;
   const uint32_t bars = bias_smem + kEpiWarps * 64 * 2;
@@ -304,7 +309,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
       int pt, qt;
       tile_coords(p, seg.tile, pt, qt);
       const int py = pt * 256 + (int)cta * kPRows;
-      const int qy = qt * p.bn + (int)cta * (p.bn / 2);
+      const int qy = qt * p.halves * p.bn + (int)cta * (p.bn / 2);
       for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
         if (!wait_bar(empty_bar(stage), phase ^ 1u, &abort_flag, p, 100 + (int)stage)) break;
         const uint32_t sp = base + stage * stage_bytes;
@@ -312,6 +317,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
           if (leader) ptx::mbar_arrive_expect_tx(full_bar(stage), 2 * stage_bytes);
           ptx::tma_load_2d_pair(sp, &map_p, full_bar(stage), kb * kBK, py);
           ptx::tma_load_2d_pair(sp + kPBytes, &map_q, full_bar(stage), kb * kBK, qy);
+          if (p.halves == 2) ptx::tma_load_2d_pair(sp + kPBytes + q_bytes, &map_q, full_bar(stage), kb * kBK, qy + p.bn);
         }
         __syncwarp();
         if (++stage == (uint32_t)p.stages) {
@@ -325,32 +331,84 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
     if (leader) {
       const uint32_t idesc = ptx::make_idesc_bf16_f32(256, p.bn);
       uint32_t stage = 0, phase = 0, it = 0;
-      for (; !abort_flag && seg.next(p, pairs); ++it) {
-        const uint32_t acc = it & 1u;
-        if (!wait_bar(tempty_bar(acc), ((it >> 1) & 1u) ^ 1u, &abort_flag, p, 200 + (int)acc)) break;
+      auto wait_acc = [&](uint32_t acc, uint32_t use) {
+        const bool ok = wait_bar(tempty_bar(acc), (use & 1u) ^ 1u, &abort_flag, p, 200 + (int)acc);
         ptx::tcgen05_fence_after();
+        return ok;
+      };
+      auto wait_full = [&](uint32_t s, uint32_t ph) {
+        const bool ok = wait_bar(full_bar(s), ph, &abort_flag, p, 300 + (int)s);
+        ptx::tcgen05_fence_after();
+        return ok;
+      };
+      auto multiply = [&](uint32_t s, uint32_t half, uint32_t acc, bool first) {  // (one lane)
+        const uint32_t sp = base + s * stage_bytes;
+        const uint64_t dp = ptx::make_smem_desc_k_sw128(sp);
+        const uint64_t dq = ptx::make_smem_desc_k_sw128(sp + kPBytes + half * q_bytes);
         const uint32_t d = tmem_base + acc * kAccCols;
-        bool ok = true;
-        for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
-          if (!wait_bar(full_bar(stage), phase, &abort_flag, p, 300 + (int)stage)) {
-            ok = false;
-            break;
-          }
-          ptx::tcgen05_fence_after();
-          const uint32_t sp = base + stage * stage_bytes;
-          const uint64_t dp = ptx::make_smem_desc_k_sw128(sp);
-          const uint64_t dq = ptx::make_smem_desc_k_sw128(sp + kPBytes);
-          if (ptx::elect_one()) {
 #pragma unroll
-            for (int j = 0; j < kBK / 16; ++j)  // 16 bf16 of K = 32 bytes = 2 descriptor address units
-              ptx::umma_bf16_pair(d, dp + 2u * j, dq + 2u * j, idesc, (kb > seg.kb0 || j > 0) ? 1u : 0u);
+        for (int j = 0; j < kBK / 16; ++j)  // 16 bf16 of K = 32 bytes = 2 descriptor address units
+          ptx::umma_bf16_pair(d, dp + 2u * j, dq + 2u * j, idesc, (!first || j > 0) ? 1u : 0u);
+      };
+      auto advance = [&](uint32_t& s, uint32_t& ph) {
+        if (++s == (uint32_t)p.stages) {
+          s = 0;
+          ph ^= 1u;
+        }
+      };
+      for (; !abort_flag && seg.next(p, pairs); ++it) {
+        bool ok = true;
+        int kb = seg.kb0;
+        if (p.halves == 2) {
+          // As many k-blocks as the pipeline holds go into the first half's accumulator before the second half's is
+          // waited for: the epilogue of the tile before is still reading that one.
+          const int held = min(p.stages, p.num_kb);
+          ok = wait_acc(0, it);
+          uint32_t s = stage, ph = phase;
+          for (int i = 0; i < held && ok; ++i) {
+            ok = wait_full(s, ph);
+            if (ok && ptx::elect_one()) multiply(s, 0, 0, i == 0);
+            __syncwarp();
+            advance(s, ph);
+          }
+          ok = ok && wait_acc(1, it);
+          for (; kb < held && ok; ++kb) {
+            if (ptx::elect_one()) {
+              multiply(stage, 1, 1, kb == 0);
+              ptx::umma_commit_pair(empty_bar(stage), 3);
+            }
+            __syncwarp();
+            advance(stage, phase);
+          }
+          for (; kb < seg.kb1 && ok; ++kb) {
+            ok = wait_full(stage, phase);
+            if (ok && ptx::elect_one()) {
+              multiply(stage, 0, 0, false);
+              if (kb + 1 == seg.kb1) ptx::umma_commit_pair(tfull_bar(0), 3);
+              multiply(stage, 1, 1, false);
+              ptx::umma_commit_pair(empty_bar(stage), 3);
+            }
+            __syncwarp();
+            advance(stage, phase);
+          }
+          if (!ok) break;
+          if (ptx::elect_one()) {
+            if (held == p.num_kb) ptx::umma_commit_pair(tfull_bar(0), 3);
+            ptx::umma_commit_pair(tfull_bar(1), 3);
+          }
+          __syncwarp();
+          continue;
+        }
+        const uint32_t acc = it & 1u;
+        ok = wait_acc(acc, it >> 1);
+        for (; kb < seg.kb1 && ok; ++kb) {
+          ok = wait_full(stage, phase);
+          if (ok && ptx::elect_one()) {
+            multiply(stage, 0, acc, kb == seg.kb0);
             ptx::umma_commit_pair(empty_bar(stage), 3);
           }
           __syncwarp();
-          if (++stage == (uint32_t)p.stages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          advance(stage, phase);
         }
         if (!ok) break;
         if (ptx::elect_one()) ptx::umma_commit_pair(tfull_bar(acc), 3);
@@ -369,12 +427,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     const size_t part_vecs = (size_t)chunks * 8 * kPRows;  // float4s of one CTA's half of a tile
     uint32_t it = 0;
-    for (; !abort_flag && seg.next(p, pairs); ++it) {
+    for (;; ++it) {
       const uint32_t acc = it & 1u;
+      if (abort_flag || ((p.halves == 1 || acc == 0) && !seg.next(p, pairs))) break;
       int pt, qt;
       tile_coords(p, seg.tile, pt, qt);
       const int prow = pt * 256 + (int)cta * kPRows + q * 32;
-      const int qrow = qt * p.bn;
+      const int qrow = p.halves == 1 ? qt * p.bn : (2 * qt + (int)acc) * p.bn;
       const float lane_bias = SWAP ? bias_of_lane(p, prow + lane) : 0.f;
       // A cut tile has two contributors: the pair that starts it, as its last piece of cut work, and the next pair,
       // as its first.  Whoever comes second, warp by warp, finds the other's accumulator in the workspace and
@@ -740,7 +799,7 @@ struct Plan {
   bool persistent = false, swap = false;
   bool pair = false;                  // tile kernel: a CTA pair per tile
   int rows = 128, bn = 256, splits = 1;
-  int pairs = 1, sk_tiles = 0;        // pair kernel
+  int pairs = 1, sk_tiles = 0, halves = 1;  // pair kernel
   int p_tiles = 0, q_tiles = 0;
   double ns = 1e300;
 };
@@ -798,21 +857,28 @@ Plan make_local_plan(int M, int N, int K, int sms) {
       keep(p);
     }
   };
-  auto consider_pair = [&](bool swap, int bn) {
+  auto consider_pair = [&](bool swap, int bn, int halves) {
     Plan p;
     p.persistent = true;
     p.swap = swap;
     p.bn = bn;
     p.p_tiles = ((swap ? N : M) + 255) / 256;
-    p.q_tiles = ((swap ? M : N) + bn - 1) / bn;
+    p.halves = halves;
+    const int cols = halves * bn;
+    p.q_tiles = ((swap ? M : N) + cols - 1) / cols;
     const int64_t tiles = (int64_t)p.p_tiles * p.q_tiles;
     p.pairs = (int)std::min<int64_t>(tiles, std::min(sms / 2, kGemmLocalMaxPairs));
-    const double power = power_ns(p.p_tiles * 256.0, (double)p.q_tiles * bn, (128.0 + bn / 2) / bn);
-    const double kb_ns = std::max({row_ns * (128 + bn / 2), 280.0 * bn / 256.0, 150.0});
+    const double power = power_ns(p.p_tiles * 256.0, (double)p.q_tiles * cols, (128.0 + cols / 2) / cols);
+    const double kb_ns = std::max({row_ns * (128 + cols / 2), 280.0 * cols / 256.0, 150.0});
+    const double waves = std::ceil((double)tiles / p.pairs);
     p.sk_tiles = 0;
-    p.ns = std::max({std::ceil((double)tiles / p.pairs) * num_kb * kb_ns, power, dram_ns}) + 3400.0 + 9.0 * bn;
+    p.ns = std::max({waves * num_kb * kb_ns, power, dram_ns}) + 3400.0 + 9.0 * cols;
+    // With both accumulators in one tile, 5.5 us of its epilogue do not run beside products (all pairs store at once), and
+    // the long tiles of a last wave that is not full cost more than the power its idle pairs leave to the others:
+    // 4096 x 8192 x 14336, 3.5 waves, takes 647 us this way and 620 us with 256 columns.
+    if (halves == 2) p.ns = std::max(waves * num_kb * kb_ns, power * waves * p.pairs / tiles) + waves * 5500.0 + 3400.0 + 9.0 * cols;
     keep(p);
-    if (tiles > p.pairs && tiles % p.pairs != 0) {
+    if (halves == 1 && tiles > p.pairs && tiles % p.pairs != 0) {
       p.sk_tiles = (int)(tiles % p.pairs) + p.pairs;
       p.ns = std::max({(double)tiles / p.pairs * num_kb * kb_ns * 1.05, power, dram_ns}) + 3400.0 + 9.0 * bn + 2500.0;
       keep(p);
@@ -820,14 +886,16 @@ Plan make_local_plan(int M, int N, int K, int sms) {
   };
   for (int bn : {64, 128, 192, 256}) {
     for (bool pair : {false, true}) consider_tile(false, pair, bn);
-    consider_pair(false, bn);
+    consider_pair(false, bn, 1);
   }
+  consider_pair(false, 256, 2);
   const int fewest = (M + 255) / 256;
   for (int parts = fewest; parts <= std::min(fewest + 3, (M + 31) / 32); ++parts) {
     const int bn = ((M + parts - 1) / parts + 31) / 32 * 32;
     for (bool pair : {false, true}) consider_tile(true, pair, bn);
-    consider_pair(true, bn);
+    consider_pair(true, bn, 1);
   }
+  consider_pair(true, 256, 2);
   return best;
 }
 
@@ -896,7 +964,9 @@ cudaError_t launch_pair(const GemmLocalArgs& a, const Plan& plan, cudaStream_t s
   LocalParams p;
   CUtensorMap map_p, map_q, map_out;
   if (!common_params(p, a, plan, kPRows, plan.bn / 2, &map_p, &map_q, &map_out)) return cudaErrorInvalidValue;
-  const int stage_bytes = kPBytes + plan.bn * kBK;
+  const int stage_bytes = kPBytes + plan.halves * plan.bn * kBK;
+  p.halves = plan.halves;
+  if (plan.halves == 2) p.band = std::min(12, plan.p_tiles);  // 12 x 6 tiles of 256 x 512: as square as 74 pairs come
   p.stages = std::min(kMaxStages, (kMaxDynamicSmem - 1024 - kTailBytes) / stage_bytes);
   p.sk_tiles = plan.sk_tiles;
   p.total_tiles = plan.p_tiles * plan.q_tiles;

@@ -221,6 +221,7 @@ def test_gemm_world1_matches_fp32_reference(m, n, k, has_bias):
         (2048, 2880, 2880),  # persistent pairs, whole tiles
         (2560, 4096, 1032),  # ... and tiles cut along K, ragged
         (3000, 3000, 512),
+        (7990, 7688, 12296),  # tiles of two accumulators, the last ones ragged
     ],
 )
 def test_gemm_one_rank_schedules(m, n, k):
