@@ -219,7 +219,8 @@ def test_gemm_world1_matches_fp32_reference(m, n, k, has_bias):
         (700, 2208, 1112),  # several tiles along M, short last ones
         (129, 8192, 264),  # one row more than a tile
         (2048, 2880, 2880),  # persistent pairs, whole tiles
-        (2560, 4096, 1032),  # ... and tiles cut along K, ragged
+        (2560, 4096, 1032),  # ... ragged along K
+        (4162, 1248, 4280),  # ... and tiles cut along K, ragged
         (3000, 3000, 512),
         (7990, 7688, 12296),  # tiles of two accumulators, the last ones ragged
     ],
