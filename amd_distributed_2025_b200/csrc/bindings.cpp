@@ -57,6 +57,7 @@ py::dict status_to_dict(const b200::StatusWord& w) {
 }
 
 at::Tensor heap_view(SymmHeap& heap, int64_t offset, std::vector<int64_t> shape, at::ScalarType dtype) {
+  TORCH_CHECK(heap.local_base() != nullptr, "symmetric heap: closed");
   int64_t numel = 1;
   for (auto s : shape) numel *= s;
   const int64_t nbytes = numel * (int64_t)c10::elementSize(dtype);
@@ -72,7 +73,7 @@ void moe_dispatch(SymmHeap& heap, const at::Tensor& x, const at::Tensor& indices
                   int64_t max_recv, int64_t off_counts, int64_t off_expert_x, int64_t off_expert_meta,
                   at::Tensor blk_hist, at::Tensor local_rank, at::Tensor route, at::Tensor expert_num_tokens,
                   int64_t epoch, int64_t timeout_ns) {
-  TORCH_CHECK(heap.peers_open(), "symmetric heap: peers are not mapped yet");
+  TORCH_CHECK(heap.peers_open(), "symmetric heap: peers are not mapped, or it was closed");
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.is_contiguous(), "x must be a contiguous [T, H] CUDA tensor");
   TORCH_CHECK(indices.is_cuda() && indices.dim() == 2 && indices.is_contiguous() && indices.scalar_type() == at::kInt,
               "indices must be a contiguous [T, k] int32 CUDA tensor");
@@ -156,7 +157,7 @@ void moe_expert_scale(const at::Tensor& expert_x, at::Tensor expert_y, const at:
 
 void moe_combine(SymmHeap& heap, at::Tensor out, const at::Tensor& weights, const at::Tensor& route,
                  int64_t num_tokens, int64_t max_recv, int64_t off_expert_y, int64_t epoch, int64_t timeout_ns) {
-  TORCH_CHECK(heap.peers_open(), "symmetric heap: peers are not mapped yet");
+  TORCH_CHECK(heap.peers_open(), "symmetric heap: peers are not mapped, or it was closed");
   TORCH_CHECK(out.is_cuda() && out.dim() == 2 && out.is_contiguous(), "out must be a contiguous [T, H] CUDA tensor");
   TORCH_CHECK(weights.scalar_type() == at::kFloat && weights.is_contiguous() && weights.dim() == 2,
               "weights must be contiguous fp32 [T, k]");
@@ -210,7 +211,7 @@ class MoeDedupEngine {
       : heap_(std::move(heap)), E_(num_experts), k_(topk), H_(hidden), max_tokens_(max_tokens), max_recv_(max_recv),
         dtype_(dtype), partial_fp32_(partial_fp32), expert_y_(std::move(expert_y)), blk_hist_(std::move(blk_hist)),
         route_(std::move(route)), expert_num_tokens_(std::move(expert_num_tokens)), timeout_ns_(timeout_ns) {
-    TORCH_CHECK(heap_->peers_open(), "symmetric heap: peers are not mapped yet");
+    TORCH_CHECK(heap_->peers_open(), "symmetric heap: peers are not mapped, or it was closed");
     const int ws = heap_->world_size();
     TORCH_CHECK(E_ > 0 && E_ % ws == 0, "num_experts must be divisible by world_size");
     TORCH_CHECK(k_ >= 1 && k_ <= 15, "experts_per_token must be in 1..15 (one 32-lane store per token record)");
@@ -254,6 +255,7 @@ class MoeDedupEngine {
   // kernel recorded (nothing is launched then; the caller turns the record into an exception).
   int dispatch(const at::Tensor& x, const at::Tensor& indices, const c10::optional<at::Tensor>& weights,
                bool fuse_scale, double scale) {
+    TORCH_CHECK(heap_->peers_open(), "symmetric heap: peers are not mapped, or it was closed");
     if (const uint32_t code = heap_->status_host().code) return (int)code;
     TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.is_contiguous() && x.scalar_type() == dtype_ && x.size(1) == H_,
                 "x must be a contiguous [T, hidden] CUDA tensor of the layer's dtype");
@@ -331,6 +333,7 @@ class MoeDedupEngine {
   }
 
   int combine(at::Tensor out, const at::Tensor& weights, const c10::optional<at::Tensor>& expert_y) {
+    TORCH_CHECK(heap_->peers_open(), "symmetric heap: peers are not mapped, or it was closed");
     if (const uint32_t code = heap_->status_host().code) return (int)code;
     const int64_t T = num_tokens_;
     TORCH_CHECK(out.is_cuda() && out.dim() == 2 && out.is_contiguous() && out.scalar_type() == dtype_ &&
@@ -401,8 +404,8 @@ class MoeDedupEngine {
     return combine(out, weights, c10::nullopt);
   }
 
-  // One rank, everything as the kernels want it (types, shapes, contiguity, no failure on record): the whole
-  // call without another look at it from Python, whose checks cost as much as a short kernel.  None / false:
+  // One rank, everything as the kernels want it (types, shapes, contiguity, an open slab, no failure on record): the
+  // whole call without another look at it from Python, whose checks cost as much as a short kernel.  None / false:
   // nothing was done, take the checked path.
   c10::optional<at::Tensor> try_forward(const at::Tensor& x, const at::Tensor& indices, const at::Tensor& weights, double scale) {
     if (!local_ready(x, indices) || !b200::moe_local_dispatch_applies(x.size(0) * k_, (int)E_) ||
@@ -421,7 +424,7 @@ class MoeDedupEngine {
     return true;
   }
   bool try_combine(const at::Tensor& out, const at::Tensor& weights, const at::Tensor& expert_y, int64_t num_tokens) {
-    if (heap_->world_size() != 1 || heap_->status_host().code != 0 || (num_tokens >= 0 && num_tokens != num_tokens_) ||
+    if (!one_rank_ready() || (num_tokens >= 0 && num_tokens != num_tokens_) ||
         !rows_of(out, dtype_, num_tokens_, H_, false) || !rows_of(weights, at::kFloat, num_tokens_, k_, false) ||
         !expert_y.is_cuda() || expert_y.get_device() != heap_->device() || expert_y.scalar_type() != dtype_ ||
         !expert_y.is_contiguous() || expert_y.sizes() != expert_y_.sizes())
@@ -437,8 +440,10 @@ class MoeDedupEngine {
     return t.is_cuda() && t.dim() == 2 && t.scalar_type() == type && t.size(1) == cols &&
            (exact ? t.size(0) == rows : t.size(0) >= rows) && t.is_contiguous() && t.get_device() == heap_->device();
   }
+  // A closed slab has no address and no status record: nothing may be launched on it.
+  bool one_rank_ready() const { return heap_->world_size() == 1 && heap_->peers_open() && heap_->status_host().code == 0; }
   bool local_ready(const at::Tensor& x, const at::Tensor& indices) const {
-    return heap_->world_size() == 1 && heap_->status_host().code == 0 && x.dim() == 2 && x.size(0) <= max_tokens_ &&
+    return one_rank_ready() && x.dim() == 2 && x.size(0) <= max_tokens_ &&
            rows_of(x, dtype_, x.size(0), H_, true) && rows_of(indices, at::kInt, x.size(0), k_, true);
   }
   void local_dispatch(const at::Tensor& x, const at::Tensor& indices, const float* weights, void* out, float scale) {
@@ -526,7 +531,7 @@ void gemm_rs(SymmHeap& heap, const at::Tensor& a, const at::Tensor& w, const c10
              int64_t timeout_ns, int64_t max_ctas, int64_t block_n, int64_t cta_pair, int64_t splits,
              const c10::optional<at::Tensor>& trace, int64_t debug, bool fuse_own, bool tma_store, bool force_staged,
              bool checked, int64_t stage_capacity) {
-  TORCH_CHECK(heap.peers_open(), "symmetric heap: peers are not mapped yet");
+  TORCH_CHECK(heap.peers_open(), "symmetric heap: peers are not mapped, or it was closed");
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16,
               "input and weight must be bf16 CUDA tensors");
   TORCH_CHECK(a.dim() == 2 && w.dim() == 2 && a.size(1) == w.size(1), "input [M, K] and weight [N, K] disagree on K");
@@ -640,7 +645,7 @@ class GemmRsEngine {
   // launched then; the caller turns the record into an exception).
   int run(const at::Tensor& a, const at::Tensor& w, const c10::optional<at::Tensor>& bias, at::Tensor out,
           bool bias_at_source, double bias_scale) {
-    TORCH_CHECK(heap_->peers_open(), "symmetric heap: peers are not mapped yet");
+    TORCH_CHECK(heap_->peers_open(), "symmetric heap: peers are not mapped, or it was closed");
     if (const uint32_t code = heap_->status_host().code) return (int)code;
     TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16,
                 "input and weight must be bf16 CUDA tensors");
@@ -712,7 +717,7 @@ class GemmRsEngine {
   // nothing was done, take the checked path.
   c10::optional<at::Tensor> try_run(const at::Tensor& a, const at::Tensor& w, const c10::optional<at::Tensor>& bias,
                                     bool bias_at_source) {
-    if (heap_->world_size() != 1 || heap_->status_host().code != 0 || !a.is_cuda() || !w.is_cuda() || a.dim() != 2 || w.dim() != 2 ||
+    if (heap_->world_size() != 1 || !heap_->peers_open() || heap_->status_host().code != 0 || !a.is_cuda() || !w.is_cuda() || a.dim() != 2 || w.dim() != 2 ||
         a.scalar_type() != at::kBFloat16 || w.scalar_type() != at::kBFloat16 || !a.is_contiguous() || !w.is_contiguous() ||
         a.get_device() != heap_->device() || w.get_device() != heap_->device())
       return c10::nullopt;
@@ -1266,6 +1271,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("reset_status", &SymmHeap::reset_status)
       .def("barrier",
            [](SymmHeap& h, int64_t epoch, int64_t timeout_ns) {
+             TORCH_CHECK(h.peers_open(), "symmetric heap: peers are not mapped, or it was closed");
              c10::cuda::CUDAGuard guard(h.device());
              cuda_check(b200::launch_symm_barrier(h, (uint64_t)epoch, (uint64_t)timeout_ns,
                                                   at::cuda::getCurrentCUDAStream()),
@@ -1274,12 +1280,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("link_probe",
            [](SymmHeap& h, int peer, int64_t src_offset, int64_t dst_offset, int64_t bytes, int mode, int chunk, int grid,
               int64_t timeout_ns) {
+             TORCH_CHECK(h.peers_open(), "symmetric heap: peers are not mapped, or it was closed");
              c10::cuda::CUDAGuard guard(h.device());
              cuda_check(b200::launch_link_probe(h, peer, (uint64_t)src_offset, (uint64_t)dst_offset, (uint64_t)bytes, mode,
                                                 chunk, grid, (uint64_t)timeout_ns, at::cuda::getCurrentCUDAStream()),
                         "link_probe launch");
            })
       .def("wait_selftest", [](SymmHeap& h, int slot, int64_t want, int64_t timeout_ns) {
+        TORCH_CHECK(h.local_base() != nullptr, "symmetric heap: closed");
         c10::cuda::CUDAGuard guard(h.device());
         cuda_check(b200::launch_wait_selftest(h, slot, (uint64_t)want, (uint64_t)timeout_ns,
                                               at::cuda::getCurrentCUDAStream()),

@@ -78,6 +78,7 @@ def moe_slab_layout(cfg: MoEConfig, world_size: int, header_bytes: int, mode: st
 class MoEAllToAll:
     META_DIM = META_DIM
     _native = None  # the engine, where a whole call can be handed to it unchecked (one rank)
+    _closed = False
 
     def __init__(
         self,
@@ -159,9 +160,15 @@ class MoEAllToAll:
         self._dispatched = (self.expert_num_tokens, self.expert_x, self.expert_meta)
         self.trace: Optional[Tuple[torch.Tensor, torch.Tensor]] = None
 
+    def _require_open(self) -> None:
+        """The buffers went with the workspace: a kernel on them would write to freed memory."""
+        if self._closed:
+            raise RuntimeError("the layer is closed")
+
     def _guard(self) -> None:
         """Host-side checks before a launch that waits on peers: an earlier device failure, and
         (with a monitor) peers that announced their departure or stopped their heartbeat."""
+        self._require_open()
         self.ws.check()
         if self.monitor is not None:
             self.monitor.beat()
@@ -242,6 +249,7 @@ class MoEAllToAll:
     def expert_scale(self, scale: float) -> torch.Tensor:
         """``expert_y = expert_x * scale`` on the rows dispatch delivered
         (all2all/reference.py:262 with ``scale = 1 + rank``)."""
+        self._require_open()
         self.ext.moe_expert_scale(self.expert_x, self.expert_y, self.expert_num_tokens, float(scale))
         return self.expert_y
 
@@ -332,6 +340,7 @@ class MoEAllToAll:
             raise ValueError("dp_x does not match the configuration")
         if indices.shape[1] != cfg.experts_per_token:
             raise ValueError("indices do not match the configuration")
+        self._require_open()
         if self.monitor is not None:
             self.monitor.beat()
             self.monitor.assert_all_alive()
@@ -360,7 +369,10 @@ class MoEAllToAll:
         self.ws.check_canaries()
 
     def close(self, collective: bool = False) -> None:
-        self.engine = None
+        """Release the workspace; later calls raise.  (A CUDA graph that holds calls of this layer must not be
+        replayed any more.)"""
+        self._closed = True
+        self.engine = self._native = None
         self.ws.close(collective)
 
 

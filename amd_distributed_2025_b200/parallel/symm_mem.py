@@ -238,6 +238,7 @@ class SymmetricWorkspace:
         if self._closed:
             return
         self._closed = True
+        self._canary_views = []
         if collective and self.world_size > 1 and dist.is_initialized():
             self.heap.close_peers()
             dist.barrier(group=self.group)

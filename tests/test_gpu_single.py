@@ -346,3 +346,32 @@ def test_gemm_staged_path_on_one_gpu(tma_store, fuse_own, m, n, k, block_n, cta_
     want = oracle.gemm_rs_fused_rounding([a], [w], bias, 0)
     assert oracle.outlier_fraction(out, want, oracle.GEMM_RS_RTOL, oracle.GEMM_RS_ATOL) < 1e-4
     assert oracle.relative_error(out, a.float() @ w.float().T + bias.float()) < 5e-3
+
+
+def test_closed_operators_launch_nothing():
+    """After close() there is no slab and no status record: native entry points refuse by themselves, whoever holds them."""
+    from amd_distributed_2025_b200.models import gemm_rs, moe_all2all
+
+    cfg, data, _, _ = contract.make_moe_inputs(16, 2, 256, 8, 3, 0, 1, device="cuda", fixed_num_tokens=8)
+    layer = moe_all2all.MoEAllToAll(cfg, 0, 1, mode="dedup")
+    engine, heap, y = layer.engine, layer.ws.heap, torch.zeros(8, 256, dtype=cfg.out_dtype, device="cuda")
+    ey = torch.zeros(layer.expert_y.shape, dtype=cfg.out_dtype, device="cuda")
+    layer.forward(data.x, data.indices, data.weights, 1.0)
+    layer.close()
+    assert engine.try_forward(data.x, data.indices, data.weights, 1.0) is None
+    assert not engine.try_dispatch(data.x, data.indices) and not engine.try_combine(y, data.weights, ey, 8)
+    for call in (lambda: engine.forward(data.x, data.indices, data.weights, y, 1.0), lambda: engine.dispatch(data.x, data.indices),
+                 lambda: engine.combine(y, data.weights, ey), lambda: heap.view(4096, [16], torch.uint8),
+                 lambda: heap.barrier(1, 1000), lambda: heap.wait_selftest(0, 1, 1000),
+                 lambda: layer.forward(data.x, data.indices, data.weights, 1.0)):
+        with pytest.raises(RuntimeError):
+            call()
+    a, w, bias = contract.make_gemm_rs_inputs(0, 1, 64, 512, 256, True, 5, device="cuda")
+    op = gemm_rs.GemmRS(1 << 20, 1 << 12, rank=0, world_size=1)
+    op(a, w, bias)
+    op.close()
+    assert op.engine.try_run(a, w, bias, True) is None
+    with pytest.raises(RuntimeError):
+        op(a, w, bias)
+    torch.cuda.synchronize()
+    assert float(torch.ones(4, device="cuda").sum()) == 4.0

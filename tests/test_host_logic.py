@@ -365,3 +365,41 @@ def test_second_dedup_dispatch_without_combine_waits_for_all_ranks(monkeypatch):
     layer.world_size = 1
     layer.dispatch(x, idx)  # a single rank has no peers to wait for
     assert calls[6:] == ["dispatch"]
+
+
+@pytest.mark.parametrize("mode", ["dedup", "direct"])
+def test_closed_moe_layer_raises_and_hands_nothing_to_the_engine(mode):
+    """The workspace of a closed layer is freed memory: no call may reach a launch."""
+    from amd_distributed_2025_b200.models import moe_all2all as m
+    from amd_distributed_2025_b200.parallel.symm_mem import SlabLayout, SymmetricWorkspace
+
+    launched = []
+
+    class Engine:
+        def __getattr__(self, name):
+            return lambda *a, **k: launched.append(name) or True
+
+    class Heap:
+        def status_code(self):
+            return 0
+
+        def close(self):
+            pass
+
+    layer = m.MoEAllToAll.__new__(m.MoEAllToAll)
+    layer.cfg = contract.MoEConfig(num_experts=8, experts_per_token=2, hidden_dim=16, max_num_tokens=4,
+                                   in_dtype=torch.float32, out_dtype=torch.float32)
+    layer.world_size, layer.rank, layer.group, layer.device, layer.monitor = 1, 0, None, torch.device("cpu"), None
+    layer.ext = Engine()
+    layer.engine = layer._native = Engine() if mode == "dedup" else None
+    layer.ws = SymmetricWorkspace(SlabLayout(4096), heap=Heap())
+    layer._num_tokens, layer._dispatch_pending, layer._dispatched = 4, False, ()
+    layer.expert_num_tokens = layer.expert_meta = None
+    layer.expert_x = layer.expert_y = torch.zeros(8, 4, 16)
+    x, idx, w, y = torch.zeros(4, 16), torch.zeros(4, 2, dtype=torch.int32), torch.zeros(4, 2), torch.zeros(4, 16)
+    layer.close()
+    for call in (lambda: layer.expert_scale(2.0), lambda: layer.forward(x, idx, w, 1.0), lambda: layer.dispatch(x, idx),
+                 lambda: layer.combine(y, w, None, torch.zeros(8, 4, 16), None, 4)):
+        with pytest.raises(RuntimeError):
+            call()
+    assert launched == []
