@@ -1435,6 +1435,20 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_rs", &gemm_rs);
   m.def("fp8_gemm", &fp8_gemm);
   m.def("fp8_gemm_try", &fp8_gemm_try);
+  // (shared memory, tensor-memory columns) of a CTA, by tile
+  m.def("gemm_tile_share", [](int rows, int bn, int splits, bool pair) {
+    const b200::SmShare s = b200::gemm_tile_share(rows, bn, splits, pair);
+    return py::make_tuple(s.smem, s.tmem_cols);
+  });
+  m.def("gemm_pair_share", [](int bn, int halves) {
+    const b200::SmShare s = b200::gemm_pair_share(bn, halves);
+    return py::make_tuple(s.smem, s.tmem_cols);
+  });
+  m.def("gemm_rs_share", [](int block_n, bool cta_pair) {
+    const b200::SmShare s = b200::gemm_rs_share(block_n, cta_pair);
+    return py::make_tuple(s.smem, s.tmem_cols);
+  });
+  m.def("fp8_gemm_share", [](int bn, int splits) { return py::make_tuple(b200::fp8_gemm_smem(bn, splits), 512); });
   m.def("gemm_rs_plan", [](int64_t M, int64_t N, int64_t K, int64_t ws, int64_t block_n, int64_t cta_pair, int64_t splits) {
     const b200::GemmRsPlan p = b200::gemm_rs_plan((int)M, (int)N, (int)K, (int)ws, (int)block_n, (int)cta_pair, (int)splits);
     py::dict d;

@@ -18,6 +18,9 @@ struct Fp8GemmArgs {
   int sms;
 };
 
+// Shared memory of a CTA (it takes all of the tensor memory).
+int fp8_gemm_smem(int bn, int splits);
+
 cudaError_t launch_fp8_gemm(const Fp8GemmArgs& args, cudaStream_t stream);
 
 }  // namespace b200

@@ -517,6 +517,18 @@ struct Fp8Plan {
   double ns = 1e300;
 };
 
+struct Fp8Memory {
+  int stages, stage_area;  // multiples of 1024
+};
+Fp8Memory fp8_memory(int bn, int splits) {
+  const int stage_bytes = kABytes + bn / 2 * kBlockK;
+  const int parts = splits > 1 ? splits * ((bn / 8 + splits - 1) / splits) * 8 * kRows * 4 : 0;
+  Fp8Memory m;
+  m.stages = std::min(kMaxStages, (kMaxDynamicSmem - 1024 - kTailBytes) / stage_bytes);
+  m.stage_area = std::max(m.stages * stage_bytes, parts);
+  return m;
+}
+
 // The time model of the bf16 kernels (gemm_local_sm100.cu) with fp8's numbers: a 128-byte row is 128 values.
 Fp8Plan make_fp8_plan(int M, int N, int K, int sms) {
   const int k_blocks = (K + kBlockK - 1) / kBlockK;
@@ -559,6 +571,11 @@ const Fp8Plan& cached_plan(int M, int N, int K, int sms) {
 
 }  // namespace
 
+int fp8_gemm_smem(int bn, int splits) {
+  const Fp8Memory m = fp8_memory(bn, splits);
+  return 1024 + m.stage_area + kTailBytes;
+}
+
 cudaError_t launch_fp8_gemm(const Fp8GemmArgs& a, cudaStream_t stream) {
   if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.K % 16 != 0) return cudaErrorInvalidValue;
   const Fp8Plan& plan = cached_plan(a.M, a.N, a.K, a.sms);
@@ -580,12 +597,10 @@ cudaError_t launch_fp8_gemm(const Fp8GemmArgs& a, cudaStream_t stream) {
   p.band = std::min(8, p.m_tiles);
   p.tma_out = (a.N % 8 == 0 && (reinterpret_cast<uintptr_t>(a.c) & 15u) == 0) ? 1 : 0;
   p.timeout_ns = a.timeout_ns;
-  const int stage_bytes = kABytes + plan.bn / 2 * kBlockK;
-  const int room = kMaxDynamicSmem - 1024 - kTailBytes;
-  const int parts = plan.splits > 1 ? plan.splits * ((plan.bn / 8 + plan.splits - 1) / plan.splits) * 8 * kRows * 4 : 0;
-  p.stages = std::min(kMaxStages, room / stage_bytes);
-  p.stage_area = std::max(p.stages * stage_bytes, parts);  // multiples of 1024
-  if (p.stage_area > room) return cudaErrorInvalidValue;
+  const Fp8Memory mem = fp8_memory(plan.bn, plan.splits);
+  p.stages = mem.stages;
+  p.stage_area = mem.stage_area;
+  if (1024 + p.stage_area + kTailBytes > kMaxDynamicSmem) return cudaErrorInvalidValue;
   CUtensorMap map_a, map_b, map_c = {};
   if (!make_tensor_map(&map_a, a.a, (uint64_t)a.M, (uint64_t)a.K, 1, kRows, kBlockK, 128) ||
       !make_tensor_map(&map_b, a.b, (uint64_t)a.N, (uint64_t)a.K, 1, (uint32_t)plan.bn / 2, kBlockK, 128) ||

@@ -20,8 +20,10 @@
 // and its call), 64 x 7168 x 18432 71 -> 49 (memory, 5.9 TB/s while cool), 256 x 5120 x 12800 58 -> 41 (34 while cool:
 // memory, then the meeting of the parts), 2048 x 2880 x 2880 45 -> 34 (power), 8192 x 8192 x 28672 3040 -> 2770 (power).
 //
-// Warp roles of both (320 threads, one CTA per SM): 0 TMA producer, 1 MMA issuer, 2..9 epilogue, two per
-// tensor-memory lane quarter.
+// Warp roles of both (320 threads): 0 TMA producer, 1 MMA issuer, 2..9 epilogue, two per tensor-memory lane quarter.
+// Shared memory keeps CTAs of the pair kernel, which take all of the tensor memory, alone on their SM.  Small tiles of
+// the tile kernel leave room for a second CTA, so a CTA takes no more tensor memory than its accumulator: whatever fits
+// on an SM by shared memory has its columns too, and no CTA ever waits for another one's.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -49,7 +51,7 @@ constexpr int kSlabBytes = 4096;             // per epilogue warp: 32 rows x 128
 constexpr int kTailBytes = kEpiWarps * kSlabBytes + kEpiWarps * 64 * 2 + 256;  // slabs, bias values, barriers
 constexpr int kMaxDynamicSmem = 232448 - 256;  // 227 KiB less what is static
 constexpr int kAccCols = 256;                // tensor-memory columns between the two accumulators
-constexpr int kTmemCols = 512;
+constexpr int kTmemCols = 512;               // pair kernel: both accumulators
 
 struct LocalParams {
   const __nv_bfloat16* bias;
@@ -63,6 +65,7 @@ struct LocalParams {
   int rows;           // tile kernel: P rows of a CTA's tile, at most 128
   int splits;         // tile kernel: CTAs (or pairs) of a cluster that share a tile
   int part_bytes;     // tile kernel: shared memory of its own for their parts (0: they take the pipeline's)
+  int tmem_cols;      // tile kernel: tensor-memory columns of its one accumulator
   int stage_area;     // tile kernel: bytes of the pipeline's stages, and of the parts where these share them
   int sk_tiles, total_tiles;  // pair kernel
   int halves;         // pair kernel: 2 = a tile is twice `bn` columns, one accumulator for each half
@@ -585,10 +588,10 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
   }
   if (warp == 1) {
     if (PAIR) {
-      ptx::tmem_alloc_pair(ptx::smem_u32(&tmem_base_shared), kTmemCols);
+      ptx::tmem_alloc_pair(ptx::smem_u32(&tmem_base_shared), (uint32_t)p.tmem_cols);
       ptx::tmem_relinquish_pair();
     } else {
-      ptx::tmem_alloc(ptx::smem_u32(&tmem_base_shared), kTmemCols);
+      ptx::tmem_alloc(ptx::smem_u32(&tmem_base_shared), (uint32_t)p.tmem_cols);
       ptx::tmem_relinquish();
     }
   }
@@ -757,8 +760,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
   if (PAIR && splits == 1) ptx::cluster_sync_all();
   ptx::tcgen05_fence_after();
   if (warp == 1) {
-    if (PAIR) ptx::tmem_dealloc_pair(tmem_base, kTmemCols);
-    else ptx::tmem_dealloc(tmem_base, kTmemCols);
+    if (PAIR) ptx::tmem_dealloc_pair(tmem_base, (uint32_t)p.tmem_cols);
+    else ptx::tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
   }
   if (tid == 0) stamp(p, 3);
 }
@@ -807,6 +810,30 @@ struct Plan {
   int p_tiles = 0, q_tiles = 0;
   double ns = 1e300;
 };
+
+// How a CTA of the tile kernel divides its shared memory, and the tensor memory it takes.
+struct TileMemory {
+  int stages, part_bytes, stage_area, smem, tmem_cols;  // (see LocalParams)
+};
+TileMemory tile_memory(int rows, int bn, int splits, bool pair) {
+  TileMemory t;
+  const int stage_bytes = (rows + (pair ? bn / 2 : bn)) * kBK * 2;
+  const int room = kMaxDynamicSmem - 1024 - kTailBytes;
+  const int parts = splits > 1 ? splits * ((bn / 8 + splits - 1) / splits) * 8 * kPRows * 4 : 0;
+  // the parts of a split tile in memory of their own, unless too little would be left for the pipeline
+  t.part_bytes = (room - parts) / stage_bytes >= 5 ? parts : 0;
+  t.stages = std::min(kMaxStages, (room - t.part_bytes) / stage_bytes);
+  t.stage_area = t.stages * stage_bytes;  // (a multiple of 1024, as the slabs behind it need)
+  if (t.part_bytes == 0) t.stage_area = std::max(t.stage_area, parts);
+  t.smem = 1024 + t.stage_area + kTailBytes + t.part_bytes;
+  t.tmem_cols = 32;  // an allocation is a power of two, at least 32
+  while (t.tmem_cols < bn) t.tmem_cols *= 2;
+  return t;
+}
+
+int pair_stage_bytes(int bn, int halves) { return kPBytes + halves * bn * kBK; }
+int pair_stages(int bn, int halves) { return std::min(kMaxStages, (kMaxDynamicSmem - 1024 - kTailBytes) / pair_stage_bytes(bn, halves)); }
+int pair_smem(int bn, int halves) { return 1024 + pair_stages(bn, halves) * pair_stage_bytes(bn, halves) + kTailBytes; }
 
 int ctas_of(const Plan& p) { return p.splits * (p.pair ? 2 : 1); }  // CTAs that share a tile
 
@@ -980,10 +1007,9 @@ cudaError_t launch_pair(const GemmLocalArgs& a, const Plan& plan, cudaStream_t s
   LocalParams p;
   CUtensorMap map_p, map_q, map_out;
   if (!common_params(p, a, plan, kPRows, plan.bn / 2, &map_p, &map_q, &map_out)) return cudaErrorInvalidValue;
-  const int stage_bytes = kPBytes + plan.halves * plan.bn * kBK;
   p.halves = plan.halves;
   if (plan.halves == 2) p.band = std::min(12, plan.p_tiles);  // 12 x 6 tiles of 256 x 512: as square as 74 pairs come
-  p.stages = std::min(kMaxStages, (kMaxDynamicSmem - 1024 - kTailBytes) / stage_bytes);
+  p.stages = pair_stages(plan.bn, plan.halves);
   p.sk_tiles = plan.sk_tiles;
   p.total_tiles = plan.p_tiles * plan.q_tiles;
   p.partials = a.partials;
@@ -992,7 +1018,7 @@ cudaError_t launch_pair(const GemmLocalArgs& a, const Plan& plan, cudaStream_t s
   static const cudaError_t opted =
       cudaFuncSetAttribute(gemm_pair_kernel<SWAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
   if (opted != cudaSuccess) return opted;
-  return launch(gemm_pair_kernel<SWAP>, p, 2 * plan.pairs, 2, 1024 + (size_t)p.stages * stage_bytes + kTailBytes, stream, map_p, map_q, map_out);
+  return launch(gemm_pair_kernel<SWAP>, p, 2 * plan.pairs, 2, (size_t)pair_smem(plan.bn, plan.halves), stream, map_p, map_q, map_out);
 }
 
 template <bool SWAP, bool PAIR>
@@ -1001,24 +1027,27 @@ cudaError_t launch_tile(const GemmLocalArgs& a, const Plan& plan, cudaStream_t s
   CUtensorMap map_p, map_q, map_out;
   const int q_rows = PAIR ? plan.bn / 2 : plan.bn;
   if (!common_params(p, a, plan, plan.rows, q_rows, &map_p, &map_q, &map_out)) return cudaErrorInvalidValue;
-  const int stage_bytes = (plan.rows + q_rows) * kBK * 2;
-  const int room = kMaxDynamicSmem - 1024 - kTailBytes;
-  const int parts = plan.splits > 1 ? plan.splits * ((plan.bn / 8 + plan.splits - 1) / plan.splits) * 8 * kPRows * 4 : 0;
-  // the parts of a split tile in memory of their own, unless too little would be left for the pipeline
-  p.part_bytes = (room - parts) / stage_bytes >= 5 ? parts : 0;
-  p.stages = std::min(kMaxStages, (room - p.part_bytes) / stage_bytes);
-  p.stage_area = p.stages * stage_bytes;  // (a multiple of 1024, as the slabs behind it need)
-  if (p.part_bytes == 0) p.stage_area = std::max(p.stage_area, parts);
-  if (p.stages < 2 || p.stage_area + p.part_bytes > room) return cudaErrorInvalidValue;
+  const TileMemory mem = tile_memory(plan.rows, plan.bn, plan.splits, PAIR);
+  p.part_bytes = mem.part_bytes;
+  p.stages = mem.stages;
+  p.stage_area = mem.stage_area;
+  p.tmem_cols = mem.tmem_cols;
+  if (p.stages < 2 || mem.smem > kMaxDynamicSmem) return cudaErrorInvalidValue;
   static const cudaError_t opted =
       cudaFuncSetAttribute(gemm_tile_kernel<SWAP, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
   static const cudaError_t opted2 = cudaFuncSetAttribute(gemm_tile_kernel<SWAP, PAIR>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (opted != cudaSuccess || opted2 != cudaSuccess) return opted != cudaSuccess ? opted : opted2;
   return launch(gemm_tile_kernel<SWAP, PAIR>, p, plan.p_tiles * plan.q_tiles * ctas_of(plan), ctas_of(plan),
-                1024 + (size_t)p.stage_area + kTailBytes + p.part_bytes, stream, map_p, map_q, map_out);
+                (size_t)mem.smem, stream, map_p, map_q, map_out);
 }
 
 }  // namespace
+
+SmShare gemm_tile_share(int rows, int bn, int splits, bool pair) {
+  const TileMemory t = tile_memory(rows, bn, splits, pair);
+  return {t.smem, t.tmem_cols};
+}
+SmShare gemm_pair_share(int bn, int halves) { return {pair_smem(bn, halves), kTmemCols}; }
 
 bool gemm_local_cuts_tiles(int M, int N, int K, int sms) {
   const Plan& plan = cached_plan(M, N, K, sms);

@@ -100,6 +100,16 @@ constexpr int kGemmLocalCounters = kGemmLocalMaxPairs * 2 * 2 * 8;
 cudaError_t launch_gemm_local(const GemmLocalArgs& args, cudaStream_t stream);
 bool gemm_local_cuts_tiles(int M, int N, int K, int sms);  // whether the launch has a use for `partials`
 
+// What a CTA takes of its SM, by tile.  Two CTAs may meet on an SM (calls on two streams, or the next call's early
+// start) wherever their shared memory fits; a CTA that then had to wait for tensor memory might wait for one that waits
+// for it at a cluster barrier.  So whatever fits by shared memory has to fit by columns (512 per SM).
+struct SmShare {
+  int smem, tmem_cols;
+};
+SmShare gemm_tile_share(int rows, int bn, int splits, bool pair);
+SmShare gemm_pair_share(int bn, int halves);
+SmShare gemm_rs_share(int block_n, bool cta_pair);
+
 // How many clusters of `size` (1..16) CTAs that each fill an SM's shared memory are resident at once.
 int gemm_cluster_capacity(int size);
 

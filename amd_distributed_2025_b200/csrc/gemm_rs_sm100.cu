@@ -1223,6 +1223,17 @@ GemmRsPlan gemm_rs_plan(int M, int N, int K, int world_size, int block_n, int ct
   return make_plan(M, N, K, world_size, sms, block_n, cta_pair, splits);
 }
 
+SmShare gemm_rs_share(int block_n, bool cta_pair) {
+  if (cta_pair) {
+    if (block_n == 256) return {Cfg<256, 2>::kSmemBytes, Cfg<256, 2>::kTmemCols};
+    if (block_n == 192) return {Cfg<192, 2>::kSmemBytes, Cfg<192, 2>::kTmemCols};
+    return {Cfg<128, 2>::kSmemBytes, Cfg<128, 2>::kTmemCols};
+  }
+  if (block_n == 256) return {Cfg<256, 1>::kSmemBytes, Cfg<256, 1>::kTmemCols};
+  if (block_n == 128) return {Cfg<128, 1>::kSmemBytes, Cfg<128, 1>::kTmemCols};
+  return {Cfg<64, 1>::kSmemBytes, Cfg<64, 1>::kTmemCols};
+}
+
 cudaError_t launch_gemm_rs(const GemmRsArgs& a, cudaStream_t stream) {
   if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.world_size < 1 || a.M % a.world_size != 0) return cudaErrorInvalidValue;
   if (a.K % 8 != 0 || a.N % 8 != 0) return cudaErrorInvalidValue;

@@ -375,3 +375,24 @@ def test_closed_operators_launch_nothing():
         op(a, w, bias)
     torch.cuda.synchronize()
     assert float(torch.ones(4, device="cuda").sum()) == 4.0
+
+
+@pytest.mark.parametrize("m,n,k", [(32, 136, 1000), (8, 64, 1024), (17, 128, 904)])
+def test_gemm_small_clusters_of_two_streams_share_sms(m, n, k):
+    """Tiles so small that CTAs of two launches meet on an SM: both find their tensor memory there."""
+    from amd_distributed_2025_b200.models import gemm_rs
+
+    a, w, bias = contract.make_gemm_rs_inputs(0, 1, m, n, k, True, 3, device="cuda")
+    op = gemm_rs.get_op(m, n, k)
+    want = op(a, w, bias)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    outs = []
+    for _ in range(50):
+        for s in streams:
+            with torch.cuda.stream(s):
+                outs.append(op(a, w, bias))
+    torch.cuda.synchronize()
+    op.check()
+    assert all(torch.equal(o, want) for o in outs)
+    assert oracle.relative_error(want, (a.float() @ w.float().T).bfloat16().float() + bias.float()) < 5e-3

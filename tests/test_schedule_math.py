@@ -168,3 +168,28 @@ def test_gemm_reducers_cover_every_staged_output_vector_exactly_once(world_size)
                 assert len(seen) == len(expect_rows) * (n // 8), (m, n, k, world_size, grid, rank, cuts, parts)
                 assert {r for r, _ in seen} == set(expect_rows)
                 assert 1 <= cuts <= 16 or not items
+
+
+def test_ctas_that_fit_on_an_sm_by_shared_memory_fit_by_tensor_memory():
+    """A CTA that finds no tensor memory waits without a limit, and the CTA it waits for may be waiting for it at a
+    cluster barrier: every tile shape of the GEMM kernels, next to every other one."""
+    from amd_distributed_2025_b200.ops import _ext
+
+    ext = _ext.load()
+    shares = [ext.gemm_tile_share(rows, bn, splits, pair)
+              for rows in range(8, 129, 8) for bn in range(32, 257, 32) for pair in (False, True)
+              for splits in range(1, (8 if pair else 16) + 1)]
+    shares += [ext.gemm_pair_share(bn, 1) for bn in range(32, 257, 32)] + [ext.gemm_pair_share(256, 2)]
+    shares += [ext.gemm_rs_share(bn, pair) for bn, pair in ((64, False), (128, False), (256, False), (128, True), (192, True), (256, True))]
+    shares += [ext.fp8_gemm_share(bn, splits) for bn in (64, 128) for splits in range(1, 9)]
+    sm, reserved = 228 * 1024, 1024  # of an SM in all, and what each resident CTA takes on top of its own
+    least = {}  # columns -> the smallest shared memory that comes with them
+    for smem, cols in shares:
+        assert 32 <= cols <= 512 and cols & (cols - 1) == 0
+        least[cols] = min(smem, least.get(cols, sm))
+
+    def pack(room, kinds):  # most columns that CTAs of these kinds take together in this much shared memory
+        return max([0] + [cols + pack(room - smem - reserved, kinds[i:]) for i, (cols, smem) in enumerate(kinds)
+                          if smem + reserved <= room])
+
+    assert pack(sm, sorted(least.items())) <= 512
