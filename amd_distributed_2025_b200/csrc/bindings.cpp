@@ -618,6 +618,11 @@ class GemmRsEngine {
     mcast_ = std::move(region);
   }
   bool nvls() const { return (bool)mcast_; }
+  std::vector<at::Tensor> local_workspaces() const {  // where tiles cut along K meet, one per stream or graph
+    std::vector<at::Tensor> out;
+    for (const auto& ws : workspaces_) out.push_back(ws.keep);
+    return out;
+  }
   void set_trace(const c10::optional<at::Tensor>& trace) {
     trace_ = nullptr;
     trace_keep_ = at::Tensor();
@@ -767,6 +772,8 @@ class GemmRsEngine {
   // Cut tiles meet in a workspace, one per stream because calls on two streams may overlap, and one more per graph
   // that a stream is captured into, because the graph may be replayed on another (its counters are then zeroed by the
   // graph itself).  At most four of either kind are kept with the operator; null (no tile is cut then) beyond them.
+  // A kernel that gave up on a wait may have counted itself in at a tile that its other contributor never reached: no
+  // workspace outlives the reset of the status record.
   struct LocalWorkspace {
     cudaStream_t stream;
     unsigned long long capture;  // 0: calls that run at once
@@ -779,6 +786,10 @@ class GemmRsEngine {
     unsigned long long capture = 0;
     if (cudaStreamGetCaptureInfo(stream, &capturing, &capture) != cudaSuccess || capturing == cudaStreamCaptureStatusInvalidated) return nullptr;
     if (capturing == cudaStreamCaptureStatusNone) capture = 0;
+    if (workspaces_of_reset_ != heap_->status_resets()) {
+      workspaces_.clear();
+      workspaces_of_reset_ = heap_->status_resets();
+    }
     for (const auto& ws : workspaces_)
       if (ws.stream == stream && ws.capture == capture) return &ws;
     const auto same_kind = [&](const LocalWorkspace& ws) { return (ws.capture != 0) == (capture != 0); };
@@ -825,6 +836,7 @@ class GemmRsEngine {
   at::Tensor trace_keep_;
   std::vector<PlanEntry> plans_;
   std::vector<LocalWorkspace> workspaces_;
+  uint64_t workspaces_of_reset_ = 0;
   int sms_ = 148;
   std::shared_ptr<b200::McastRegion> mcast_;
 };
@@ -1368,6 +1380,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("plan", &GemmRsEngine::plan)
       .def("set_trace", &GemmRsEngine::set_trace)
       .def("restart_epochs", &GemmRsEngine::restart_epochs)
+      .def("local_workspaces", &GemmRsEngine::local_workspaces)
       .def("set_mcast", &GemmRsEngine::set_mcast)
       .def_property_readonly("nvls", &GemmRsEngine::nvls)
       .def_property_readonly("epoch", &GemmRsEngine::epoch)

@@ -142,6 +142,7 @@ void SymmHeap::reset_status() {
   std::memset(status_host_, 0, sizeof(StatusWord));
   check(cudaMemset(sync_counters_, 0, 64 * sizeof(uint32_t)), "cudaMemset(sync counters)");
   check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
+  ++status_resets_;
 }
 
 // ---------------------------------------------------------------------------------------

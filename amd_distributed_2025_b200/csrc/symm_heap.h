@@ -54,6 +54,8 @@ class SymmHeap {
   StatusWord status_sync() const;
   // Clears both copies and the kernels' grid-sync counters; call only when idle.
   void reset_status();
+  // How often that happened: what else a failed kernel may have left half done is then to be made new.
+  uint64_t status_resets() const { return status_resets_; }
 
   // Local scratch words used by kernels' intra-GPU barriers; zero between launches.
   uint32_t* sync_counters() const { return sync_counters_; }
@@ -63,6 +65,7 @@ class SymmHeap {
   uint64_t bytes_;
   void* base_[kMaxWorldSize];
   bool peers_open_;
+  uint64_t status_resets_ = 0;
   StatusBlock* status_dev_;
   StatusWord* status_host_;  // mapped pinned
   uint32_t* sync_counters_;

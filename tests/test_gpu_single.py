@@ -396,3 +396,22 @@ def test_gemm_small_clusters_of_two_streams_share_sms(m, n, k):
     op.check()
     assert all(torch.equal(o, want) for o in outs)
     assert oracle.relative_error(want, (a.float() @ w.float().T).bfloat16().float() + bias.float()) < 5e-3
+
+
+@pytest.mark.parametrize("clear", ["reset_status", "recover"])
+def test_workspace_of_cut_tiles_does_not_outlive_a_failure(clear):
+    """A kernel that gave up may leave a tile's counter behind; the next call must not take it for its other half."""
+    from amd_distributed_2025_b200.models import gemm_rs
+
+    m, n, k = 4162, 1248, 4280  # tiles cut along K
+    a, w, bias = contract.make_gemm_rs_inputs(0, 1, m, n, k, True, 17, device="cuda")
+    op = gemm_rs.GemmRS(1 << 20, 1 << 12, rank=0, world_size=1)
+    want = op(a, w, bias)
+    (old,) = op.engine.local_workspaces()
+    assert torch.equal(op(a, w, bias), want) and op.engine.local_workspaces()[0].data_ptr() == old.data_ptr()
+    op.ws.reset_status() if clear == "reset_status" else op.recover()
+    assert torch.equal(op(a, w, bias), want)
+    (new,) = op.engine.local_workspaces()
+    assert new.data_ptr() != old.data_ptr()
+    op.check()
+    op.close()
