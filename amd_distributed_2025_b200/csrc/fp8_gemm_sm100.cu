@@ -32,6 +32,7 @@
 
 #include "fp8_gemm.h"
 #include "gemm_rs.h"
+#include "per_device.h"
 #include "signal.cuh"
 #include "sm100_ptx.cuh"
 #include "tensor_map.h"
@@ -606,9 +607,9 @@ cudaError_t launch_fp8_gemm(const Fp8GemmArgs& a, cudaStream_t stream) {
       !make_tensor_map(&map_b, a.b, (uint64_t)a.N, (uint64_t)a.K, 1, (uint32_t)plan.bn / 2, kBlockK, 128) ||
       (p.tma_out && !make_tensor_map(&map_c, a.c, (uint64_t)a.M, (uint64_t)a.N, 2, 32, 32, 64)))
     return cudaErrorInvalidValue;
-  static const cudaError_t opted = cudaFuncSetAttribute(fp8_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
-  static const cudaError_t opted2 = cudaFuncSetAttribute(fp8_gemm_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (opted != cudaSuccess || opted2 != cudaSuccess) return opted != cudaSuccess ? opted : opted2;
+  static OncePerDevice once;
+  const cudaError_t opted = once([] { return opt_in(fp8_gemm_kernel, kMaxDynamicSmem, true); });
+  if (opted != cudaSuccess) return opted;
   const int total = p.m_tiles * p.n_tiles;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * plan.splits * (plan.splits > 1 ? total : plan.clusters)));

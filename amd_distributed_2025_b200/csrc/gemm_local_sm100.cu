@@ -33,6 +33,7 @@
 #include <cmath>
 
 #include "gemm_rs.h"
+#include "per_device.h"
 #include "signal.cuh"
 #include "sm100_ptx.cuh"
 #include "tensor_map.h"
@@ -781,8 +782,7 @@ int gemm_cluster_capacity(int size) {
   int& n = cache[dev & 15].n[size];
   if (n > 0) return n;
   auto kernel = gemm_tile_kernel<true, false>;
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  opt_in(kernel, kMaxDynamicSmem, true);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(size * 16));
   cfg.blockDim = dim3(kThreads);
@@ -1015,8 +1015,8 @@ cudaError_t launch_pair(const GemmLocalArgs& a, const Plan& plan, cudaStream_t s
   p.partials = a.partials;
   p.far_part = (int64_t)(kGemmLocalPartialBytes / 2 / 16);
   p.counters = a.counters;
-  static const cudaError_t opted =
-      cudaFuncSetAttribute(gemm_pair_kernel<SWAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+  static OncePerDevice once;
+  const cudaError_t opted = once([] { return opt_in(gemm_pair_kernel<SWAP>, kMaxDynamicSmem, false); });
   if (opted != cudaSuccess) return opted;
   return launch(gemm_pair_kernel<SWAP>, p, 2 * plan.pairs, 2, (size_t)pair_smem(plan.bn, plan.halves), stream, map_p, map_q, map_out);
 }
@@ -1033,10 +1033,9 @@ cudaError_t launch_tile(const GemmLocalArgs& a, const Plan& plan, cudaStream_t s
   p.stage_area = mem.stage_area;
   p.tmem_cols = mem.tmem_cols;
   if (p.stages < 2 || mem.smem > kMaxDynamicSmem) return cudaErrorInvalidValue;
-  static const cudaError_t opted =
-      cudaFuncSetAttribute(gemm_tile_kernel<SWAP, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
-  static const cudaError_t opted2 = cudaFuncSetAttribute(gemm_tile_kernel<SWAP, PAIR>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (opted != cudaSuccess || opted2 != cudaSuccess) return opted != cudaSuccess ? opted : opted2;
+  static OncePerDevice once;
+  const cudaError_t opted = once([] { return opt_in(gemm_tile_kernel<SWAP, PAIR>, kMaxDynamicSmem, true); });
+  if (opted != cudaSuccess) return opted;
   return launch(gemm_tile_kernel<SWAP, PAIR>, p, plan.p_tiles * plan.q_tiles * ctas_of(plan), ctas_of(plan),
                 (size_t)mem.smem, stream, map_p, map_q, map_out);
 }

@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "per_device.h"
 #include "signal.cuh"
 #include "sm100_ptx.cuh"
 #include "symm_heap.h"
@@ -102,11 +103,10 @@ cudaError_t launch_link_probe(const SymmHeap& heap, int peer, uint64_t src_offse
       dst_offset < kHeapHeaderBytes)
     return cudaErrorInvalidValue;
   const size_t smem = mode == 1 ? (size_t)kProbeWarps * 2 * kProbeMaxChunk : 0;
-  static bool opted_in = false;
-  if (mode == 1 && !opted_in) {
-    cudaError_t e = cudaFuncSetAttribute(link_probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static OncePerDevice once;
+  if (mode == 1) {
+    const cudaError_t e = once([smem] { return opt_in(link_probe_kernel, (int)smem, false); });
     if (e != cudaSuccess) return e;
-    opted_in = true;
   }
   const uint8_t* src = static_cast<const uint8_t*>(heap.local_base()) + src_offset;
   uint8_t* dst = reinterpret_cast<uint8_t*>(heap.peer_base(peer)) + dst_offset;

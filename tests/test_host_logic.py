@@ -403,3 +403,43 @@ def test_closed_moe_layer_raises_and_hands_nothing_to_the_engine(mode):
         with pytest.raises(RuntimeError):
             call()
     assert launched == []
+
+
+def test_once_per_device_runs_on_every_device_and_again_after_a_failure(tmp_path):
+    """Opt-ins to large shared memory belong to a device, not to the process (csrc/per_device.h against a fake runtime)."""
+    import os
+    import subprocess
+
+    from amd_distributed_2025_b200.ops import _ext
+
+    (tmp_path / "cuda_runtime.h").write_text("""
+#pragma once
+typedef int cudaError_t;
+enum { cudaSuccess = 0, cudaFuncAttributeMaxDynamicSharedMemorySize = 8, cudaFuncAttributeNonPortableClusterSizeAllowed = 14 };
+extern int device;
+inline cudaError_t cudaGetDevice(int* d) { *d = device; return device < 0 ? 101 : 0; }
+template <typename K> cudaError_t cudaFuncSetAttribute(K, int, int) { return 0; }
+""")
+    (tmp_path / "main.cpp").write_text("""
+#include <cstdio>
+#include "per_device.h"
+int device = 0;
+int main() {
+  static b200::OncePerDevice once;
+  const int plan[][2] = {{0, 0}, {0, 0}, {1, 0}, {0, 0}, {1, 0}, {2, 7}, {2, 0}, {2, 0}, {63, 0}, {64, 0}, {64, 0}, {-1, 0}};
+  for (auto& p : plan) {
+    device = p[0];
+    int ran = 0;
+    const int rc = once([&] { ran = 1; return p[1]; });
+    std::printf("%d%d ", ran, rc);
+  }
+}
+""")
+    exe = str(tmp_path / "once")
+    subprocess.run(["g++", "-std=c++17", "-I", str(tmp_path), "-I", _ext.CSRC_DIR, str(tmp_path / "main.cpp"), "-o", exe], check=True)
+    out = subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split()
+    # device 0 once, device 1 once, device 2 again after its failure; beyond 64 devices every time; no device: an error
+    assert out == ["10", "00", "10", "00", "00", "17", "10", "00", "10", "10", "10", "0101"]
+    for path in _ext._source_files():  # no setting of a device is made by the initialiser of a variable of the process
+        text = open(path, encoding="utf-8").read()
+        assert not [s for s in text.split(";") if "static" in s and "=" in s and "cudaFuncSetAttribute" in s.split("=", 1)[1]], os.path.basename(path)

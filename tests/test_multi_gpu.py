@@ -263,3 +263,25 @@ def test_multicast_region_sums_in_the_switch(ws):
         pytest.skip("NVLink multicast unavailable: " + "; ".join(sorted({r.get("why", "") for r in res if not r["available"]})))
     for r in res:
         assert r["ok"], r
+
+
+def test_one_process_uses_the_kernels_on_two_devices():
+    """Opt-ins and plans are per device: the same calls on a second GPU of one process."""
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    from amd_distributed_2025_b200.models import gemm_rs
+    from amd_distributed_2025_b200.ops.fp8_gemm import fp8_gemm
+
+    for dev in (0, 1, 0):
+        with torch.cuda.device(dev):
+            g = torch.Generator(device="cuda").manual_seed(1)
+            a = torch.randn(256, 512, device="cuda", generator=g).to(torch.float8_e4m3fn)
+            s = torch.ones(256, 4, device="cuda")
+            c = fp8_gemm(a, a, s, s[:2].contiguous())
+            assert float((c.float() - a.float() @ a.float().T).abs().max()) < 1.0
+            for m, n, k in ((64, 2880, 360), (2048, 2880, 2880), (4162, 1248, 4280)):
+                x = torch.randn(m, k, device="cuda", generator=g).bfloat16()
+                w = torch.randn(n, k, device="cuda", generator=g).bfloat16()
+                y = gemm_rs.GemmRS(1 << 20, 1 << 12, rank=0, world_size=1)(x, w)
+                want = x.float() @ w.float().T
+                assert float((y.float() - want).abs().max()) < 1e-2 * float(want.abs().max())
