@@ -9,6 +9,8 @@
 #include <pybind11/stl.h>
 #include <torch/extension.h>
 
+#include <atomic>
+#include <cstring>
 #include <memory>
 #include <string>
 #include <vector>
@@ -852,6 +854,38 @@ int device_sms(int device) {
   return sms.at((size_t)device);
 }
 
+// Where fp8_gemm leaves the record of an expired wait: one word per device, in mapped host memory, for the life of the
+// process (the operation has no object of its own to hold it).
+b200::StatusWord* fp8_status(int device) {
+  constexpr int kDevices = 64;
+  static b200::StatusWord* const words = [] {
+    // (the first call may come while a stream is being captured, which an allocation would break off in any other mode)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cuda_check(cudaThreadExchangeStreamCaptureMode(&mode), "fp8_gemm status");
+    void* w = nullptr;
+    const cudaError_t e = cudaHostAlloc(&w, kDevices * sizeof(b200::StatusWord), cudaHostAllocMapped | cudaHostAllocPortable);
+    cuda_check(cudaThreadExchangeStreamCaptureMode(&mode), "fp8_gemm status");
+    cuda_check(e, "fp8_gemm status");
+    std::memset(w, 0, kDevices * sizeof(b200::StatusWord));
+    return static_cast<b200::StatusWord*>(w);
+  }();
+  TORCH_CHECK(device >= 0 && device < kDevices, "device index out of range");
+  return words + device;
+}
+
+uint32_t fp8_status_code(int device) { return reinterpret_cast<const volatile b200::StatusWord*>(fp8_status(device))->code; }
+
+// The record of a device, which is cleared: an expired wait leaves nothing behind that a later call could trip over.
+py::dict fp8_gemm_take_status(int device) {
+  b200::StatusWord* w = fp8_status(device);
+  const uint32_t code = fp8_status_code(device);
+  std::atomic_thread_fence(std::memory_order_acquire);
+  b200::StatusWord copy = *w;
+  copy.code = code;
+  if (code != 0) std::memset(w, 0, sizeof(*w));
+  return status_to_dict(copy);
+}
+
 void run_fp8_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& a_scale, const at::Tensor& b_scale,
                   const at::Tensor& c, int64_t timeout_ns) {
   b200::Fp8GemmArgs g;
@@ -868,12 +902,15 @@ void run_fp8_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& a_
   g.bs_stride_n = b_scale.stride(0);
   g.bs_stride_k = b_scale.stride(1);
   g.timeout_ns = (uint64_t)timeout_ns;
+  g.status = fp8_status(a.get_device());
   g.sms = device_sms(a.get_device());
   cuda_check(b200::launch_fp8_gemm(g, at::cuda::getCurrentCUDAStream()), "fp8_gemm launch");
 }
 
-void fp8_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& a_scale, const at::Tensor& b_scale,
-              at::Tensor c, int64_t timeout_ns) {
+// Returns 0 after the launch, or the code of a failure that an earlier call on the device recorded (nothing is launched
+// then; the caller takes the record and turns it into an exception).
+int fp8_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& a_scale, const at::Tensor& b_scale,
+             at::Tensor c, int64_t timeout_ns) {
   TORCH_CHECK(a.is_cuda() && b.is_cuda() && a.dim() == 2 && b.dim() == 2 && a.size(1) == b.size(1),
               "a [M, K] and b [N, K] must be CUDA matrices with equal K");
   TORCH_CHECK(a.scalar_type() == at::kFloat8_e4m3fn && b.scalar_type() == at::kFloat8_e4m3fn, "a and b must be float8_e4m3fn");
@@ -887,7 +924,9 @@ void fp8_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& a_scal
   TORCH_CHECK(c.scalar_type() == at::kBFloat16 && c.is_contiguous() && c.size(0) == M && c.size(1) == N, "c must be bf16 [M, N]");
   TORCH_CHECK(K % 16 == 0, "K must be a multiple of 16");
   c10::cuda::CUDAGuard guard(a.device());
+  if (const uint32_t code = fp8_status_code(a.get_device())) return (int)code;
   run_fp8_gemm(a, b, a_scale, b_scale, c, timeout_ns);
+  return 0;
 }
 
 // The common call (operands and scales as the kernel wants them, result to be allocated) without a look at it from
@@ -905,6 +944,7 @@ c10::optional<at::Tensor> fp8_gemm_try(const at::Tensor& a, const at::Tensor& b,
       a_scale.get_device() != a.get_device() || b_scale.get_device() != a.get_device())
     return c10::nullopt;
   c10::cuda::CUDAGuard guard(a.device());
+  if (fp8_status_code(a.get_device()) != 0) return c10::nullopt;
   at::Tensor c = at::detail::empty_cuda({M, N}, at::kBFloat16, a.device(), c10::nullopt);
   run_fp8_gemm(a, b, a_scale, b_scale, c, timeout_ns);
   return c;
@@ -1448,6 +1488,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_rs", &gemm_rs);
   m.def("fp8_gemm", &fp8_gemm);
   m.def("fp8_gemm_try", &fp8_gemm_try);
+  m.def("fp8_gemm_take_status", &fp8_gemm_take_status);
+  m.def("fp8_wait_selftest", [](int device, int64_t timeout_ns) {
+    c10::cuda::CUDAGuard guard(device);
+    cuda_check(b200::launch_fp8_wait_selftest(fp8_status(device), (uint64_t)timeout_ns, at::cuda::getCurrentCUDAStream()),
+               "fp8 wait_selftest launch");
+  });
   // (shared memory, tensor-memory columns) of a CTA, by tile
   m.def("gemm_tile_share", [](int rows, int bn, int splits, bool pair) {
     const b200::SmShare s = b200::gemm_tile_share(rows, bn, splits, pair);

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "status.h"
+
 namespace b200 {
 
 struct Fp8GemmArgs {
@@ -15,6 +17,7 @@ struct Fp8GemmArgs {
   int M, N, K;
   long long as_stride_m, as_stride_k, bs_stride_n, bs_stride_k;  // element strides of the scale tensors
   uint64_t timeout_ns;
+  StatusWord* status;  // mapped host memory: where a kernel that gave up on a wait leaves its record
   int sms;
 };
 
@@ -22,5 +25,8 @@ struct Fp8GemmArgs {
 int fp8_gemm_smem(int bn, int splits);
 
 cudaError_t launch_fp8_gemm(const Fp8GemmArgs& args, cudaStream_t stream);
+
+// Self-test of the bounded wait: one warp waits for a barrier that nothing signals and leaves its record.
+cudaError_t launch_fp8_wait_selftest(StatusWord* status, uint64_t timeout_ns, cudaStream_t stream);
 
 }  // namespace b200

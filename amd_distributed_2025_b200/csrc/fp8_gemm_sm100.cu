@@ -69,6 +69,7 @@ struct Fp8Params {
   int splits;            // pairs of a cluster that share a tile
   int tma_out;           // 1: rows of C are whole 16-byte pieces: results leave through TMA
   uint64_t timeout_ns;   // of a pipeline wait
+  StatusWord* status;    // mapped host memory
 };
 
 // Instruction descriptor of tcgen05.mma.kind::f8f6f4 with e4m3 A and B (both K-major) and fp32
@@ -88,7 +89,8 @@ __device__ __forceinline__ void umma_fp8_pair(uint32_t tmem_d, uint64_t desc_a, 
       : "memory");
 }
 
-__device__ __forceinline__ bool fp8_wait(uint32_t bar, uint32_t parity, volatile int* abort, const Fp8Params& p) {
+// `detail` (not 0) tells which wait it was that expired: a hundred for the kind of barrier, plus its index.
+__device__ __forceinline__ bool fp8_wait(uint32_t bar, uint32_t parity, volatile int* abort, const Fp8Params& p, int detail) {
   uint64_t t0 = 0;  // (the clock takes longer to read than most waits last)
   for (uint32_t spins = 1; !ptx::mbar_try_wait(bar, parity); ++spins) {
     if ((spins & 255u) == 0) {
@@ -96,12 +98,18 @@ __device__ __forceinline__ bool fp8_wait(uint32_t bar, uint32_t parity, volatile
       const uint64_t now = global_timer_ns();
       if (t0 == 0) t0 = now;
       if (now - t0 > p.timeout_ns) {
-        *abort = 1;
+        *abort = detail;
         return false;
       }
     }
   }
   return true;
+}
+
+// A CTA in which a wait expired says so, once, on its way out: what it computed is of no use.
+__device__ __forceinline__ void record_expired(const Fp8Params& p, int detail) {
+  if (p.status != nullptr && reinterpret_cast<volatile StatusWord*>(p.status)->code == STATUS_OK)
+    store_status(p.status, STATUS_TIMEOUT, PHASE_GEMM_PIPELINE, -1, detail, 0, 0);
 }
 
 // acc[0..1] += v[0..1] * s
@@ -229,7 +237,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const int ay = mt * 256 + cta * kRows;
       const int by = nt * p.bn + cta * b_rows;
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (!fp8_wait(empty_bar(stage), phase ^ 1u, &abort_flag, p)) break;
+        if (!fp8_wait(empty_bar(stage), phase ^ 1u, &abort_flag, p, 100 + (int)stage)) break;
         const uint32_t sa = base + stage * stage_bytes;
         if (ptx::elect_one()) {
           if (cta == 0) ptx::mbar_arrive_expect_tx(full_bar(stage), 2 * stage_bytes);
@@ -251,12 +259,12 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       for (int tile = first_tile; tile < total && !abort_flag; tile += tile_step) {
         bool ok = true;
         for (int kb = kb0; kb < kb1 && ok; kb += kStep) {
-          ok = fp8_wait(tempty_bar(buf), buf_phase ^ 1u, &abort_flag, p);
+          ok = fp8_wait(tempty_bar(buf), buf_phase ^ 1u, &abort_flag, p, 200 + (int)buf);
           ptx::tcgen05_fence_after();
 #pragma unroll
           for (int i = 0; i < kStep; ++i) {
             if (kb + i >= kb1) break;
-            ok = ok && fp8_wait(full_bar(stage), phase, &abort_flag, p);
+            ok = ok && fp8_wait(full_bar(stage), phase, &abort_flag, p, 300 + (int)stage);
             if (!ok) break;
             ptx::tcgen05_fence_after();
             const uint32_t sa = base + stage * stage_bytes;
@@ -296,7 +304,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       tile_coords(tile, mt, nt);
       const int m0 = mt * 256 + cta * kRows;
       for (int kb = kb0; kb < kb1; kb += kGroup) {
-        if (!fp8_wait(sempty_bar(slot), phase ^ 1u, &abort_flag, p)) break;
+        if (!fp8_wait(sempty_bar(slot), phase ^ 1u, &abort_flag, p, 500 + (int)slot)) break;
         const uint32_t at = scales + slot * kScaleBytes;
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -348,7 +356,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       float2 last = make_float2(0.f, 0.f);  // scale of v[1]: it is added while the next block's v[0] is on its way
       for (int kb = kb0; kb < kb1; kb += kGroup) {
         // (where a wait expires, the numbers are of no use any more; the loop still ends, and `alive` is asked after it)
-        alive &= fp8_wait(sfull_bar(slot), slot_phase, &abort_flag, p);
+        alive &= fp8_wait(sfull_bar(slot), slot_phase, &abort_flag, p, 600 + (int)slot);
         __syncwarp();
         float sa[kGroup], sb[2 * kGroup];
         const uint32_t at = scales + slot * kScaleBytes;
@@ -364,7 +372,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
         for (int i0 = 0; i0 < kGroup; i0 += kStep) {
           if (kb + i0 >= kb1) break;
-          alive &= fp8_wait(tfull_bar(buf), buf_phase, &abort_flag, p);
+          alive &= fp8_wait(tfull_bar(buf), buf_phase, &abort_flag, p, 400 + (int)buf);
           __syncwarp();
           ptx::tcgen05_fence_after();
           if (rows_in) {
@@ -506,6 +514,21 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   ptx::cluster_sync_all();  // no CTA retires while another may still signal its barriers or read its memory
   ptx::tcgen05_fence_after();
   if (warp == 1) ptx::tmem_dealloc_pair(tmem_base, kTmemCols);
+  if (tid == 0 && abort_flag) record_expired(p, abort_flag);
+}
+
+__global__ void fp8_wait_selftest_kernel(const Fp8Params p) {
+  __shared__ volatile int abort_flag;
+  __shared__ alignas(8) uint64_t bar;
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    ptx::mbar_init(ptx::smem_u32(&bar), 1);
+    ptx::fence_mbar_init();
+  }
+  __syncthreads();
+  fp8_wait(ptx::smem_u32(&bar), 0, &abort_flag, p, 900);  // nobody arrives
+  __syncthreads();
+  if (threadIdx.x == 0 && abort_flag) record_expired(p, abort_flag);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -598,6 +621,7 @@ cudaError_t launch_fp8_gemm(const Fp8GemmArgs& a, cudaStream_t stream) {
   p.band = std::min(8, p.m_tiles);
   p.tma_out = (a.N % 8 == 0 && (reinterpret_cast<uintptr_t>(a.c) & 15u) == 0) ? 1 : 0;
   p.timeout_ns = a.timeout_ns;
+  p.status = a.status;
   const Fp8Memory mem = fp8_memory(plan.bn, plan.splits);
   p.stages = mem.stages;
   p.stage_area = mem.stage_area;
@@ -626,6 +650,14 @@ cudaError_t launch_fp8_gemm(const Fp8GemmArgs& a, cudaStream_t stream) {
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, fp8_gemm_kernel, map_a, map_b, map_c, p);
+}
+
+cudaError_t launch_fp8_wait_selftest(StatusWord* status, uint64_t timeout_ns, cudaStream_t stream) {
+  Fp8Params p = {};
+  p.timeout_ns = timeout_ns;
+  p.status = status;
+  fp8_wait_selftest_kernel<<<1, 32, 0, stream>>>(p);
+  return cudaGetLastError();
 }
 
 }  // namespace b200

@@ -72,6 +72,18 @@ __device__ __forceinline__ uint32_t ld_relaxed_gpu_u32(const uint32_t* p) {
   return v;
 }
 
+// The host's copy of a record: the fields first, then the code that says they are there.
+__device__ __forceinline__ void store_status(volatile StatusWord* h, uint32_t code, uint32_t phase, int peer, int detail,
+                                             uint64_t epoch, uint64_t seen) {
+  h->phase = phase;
+  h->peer = peer;
+  h->detail = detail;
+  h->epoch = epoch;
+  h->seen = seen;
+  __threadfence_system();
+  h->code = code;
+}
+
 // First error wins; later errors are dropped so the original cause survives.
 __device__ __forceinline__ void record_status(StatusBlock* st, uint32_t code, uint32_t phase, int peer,
                                               int detail, uint64_t epoch, uint64_t seen) {
@@ -82,17 +94,7 @@ __device__ __forceinline__ void record_status(StatusBlock* st, uint32_t code, ui
     st->word.detail = detail;
     st->word.epoch = epoch;
     st->word.seen = seen;
-    StatusWord* h = st->host_mirror;
-    if (h != nullptr) {
-      volatile StatusWord* hv = h;
-      hv->phase = phase;
-      hv->peer = peer;
-      hv->detail = detail;
-      hv->epoch = epoch;
-      hv->seen = seen;
-      __threadfence_system();
-      hv->code = code;
-    }
+    if (st->host_mirror != nullptr) store_status(st->host_mirror, code, phase, peer, detail, epoch, seen);
     __threadfence_system();
   }
 }

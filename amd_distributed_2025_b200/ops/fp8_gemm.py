@@ -17,6 +17,8 @@ from typing import Optional, Tuple
 
 import torch
 
+from ..utils.status import StatusError, describe_status
+
 BLOCK = 128
 
 
@@ -43,7 +45,10 @@ def fp8_gemm(
     timeout_ms: float = 2000.0,
 ) -> torch.Tensor:
     """``a [M, K]``, ``b [N, K]`` in ``float8_e4m3fn``; ``a_scale [M, ceil(K/128)]``,
-    ``b_scale [ceil(N/128), ceil(K/128)]`` fp32; returns (and fills, if given) bf16 ``c [M, N]``."""
+    ``b_scale [ceil(N/128), ceil(K/128)]`` fp32; returns (and fills, if given) bf16 ``c [M, N]``.
+
+    The kernel's waits are limited to ``timeout_ms``.  A call in which one expires has no result; as nothing here waits
+    for the GPU, that is raised (``StatusError``) by ``check()`` or by the next call on the device, once."""
     from . import _ext
 
     ext = _ext.load()
@@ -57,8 +62,25 @@ def fp8_gemm(
         b = b.contiguous()
     if c is None:
         c = torch.empty((a.shape[0], b.shape[0]), dtype=torch.bfloat16, device=a.device)
-    ext.fp8_gemm(a, b, a_scale, b_scale, c, int(timeout_ms * 1e6))
+    while ext.fp8_gemm(a, b, a_scale, b_scale, c, int(timeout_ms * 1e6)):
+        _raise_recorded(ext, a.device)  # (returns if another thread has raised it meanwhile: launch after all)
     return c
+
+
+def _raise_recorded(ext, device: torch.device) -> None:
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    status = ext.fp8_gemm_take_status(index)
+    if status["code"] != 0:
+        raise StatusError(f"an earlier fp8_gemm on cuda:{index} has no result: " + describe_status(status, 0), status)
+
+
+def check(device: Optional[torch.device] = None) -> None:
+    """Wait for the device and raise ``StatusError`` if a call on it gave up on a wait; this clears the record."""
+    from . import _ext
+
+    device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+    torch.cuda.synchronize(device)
+    _raise_recorded(_ext.load(), device)
 
 
 def custom_kernel(data: Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]) -> torch.Tensor:

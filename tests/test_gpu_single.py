@@ -415,3 +415,45 @@ def test_workspace_of_cut_tiles_does_not_outlive_a_failure(clear):
     assert new.data_ptr() != old.data_ptr()
     op.check()
     op.close()
+
+
+def test_fp8_gemm_expired_wait_leaves_a_record():
+    from amd_distributed_2025_b200.ops import fp8_gemm as f
+    from amd_distributed_2025_b200.utils.status import StatusError
+
+    ext = _ext()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a = torch.randn(128, 256, device="cuda", generator=g).to(torch.float8_e4m3fn)
+    s = torch.ones(128, 2, device="cuda")
+    want = f.fp8_gemm(a, a, s, s[:1])
+    f.check()
+    for ask in (f.check, lambda: f.fp8_gemm(a, a, s, s[:1]), lambda: f.fp8_gemm(a, a, s, s[:1], c=torch.empty_like(want))):
+        ext.fp8_wait_selftest(0, 1_000_000)  # a barrier nobody arrives on, 1 ms
+        torch.cuda.synchronize()
+        with pytest.raises(StatusError) as err:
+            ask()
+        assert err.value.code == "timeout" and err.value.phase == "gemm_pipeline" and err.value.status["detail"] == 900
+        assert torch.equal(f.fp8_gemm(a, a, s, s[:1]), want)
+        f.check()
+
+
+def test_fp8_gemm_first_call_of_a_process_may_be_captured():
+    """Nothing that the first call sets up (opt-ins, plan, the record's memory) breaks a capture off."""
+    import os
+    import subprocess
+    import sys
+
+    code = """
+import torch
+from amd_distributed_2025_b200.ops.fp8_gemm import fp8_gemm, fp8_gemm_reference
+a = torch.randn(256, 512, device="cuda").to(torch.float8_e4m3fn)
+s, t = torch.rand(256, 4, device="cuda"), torch.rand(2, 4, device="cuda")
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    c = fp8_gemm(a, a, s, t)
+graph.replay()
+torch.cuda.synchronize()
+want = fp8_gemm_reference(a, a, s, t)
+assert float((c.float() - want).abs().max()) < 1e-2 * float(want.abs().max())
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))

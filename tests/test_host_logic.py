@@ -443,3 +443,33 @@ int main() {
     for path in _ext._source_files():  # no setting of a device is made by the initialiser of a variable of the process
         text = open(path, encoding="utf-8").read()
         assert not [s for s in text.split(";") if "static" in s and "=" in s and "cudaFuncSetAttribute" in s.split("=", 1)[1]], os.path.basename(path)
+
+
+@pytest.mark.parametrize("given", [False, True])
+def test_fp8_gemm_raises_what_an_earlier_call_recorded(monkeypatch, given):
+    """An expired wait of the fp8 kernel: raised once by the next call, which launches nothing, then forgotten."""
+    from amd_distributed_2025_b200.ops import _ext, fp8_gemm as f
+
+    class Native:
+        record, launched = 1, 0
+
+        def fp8_gemm_try(self, a, b, a_scale, b_scale, timeout_ns):
+            return None
+
+        def fp8_gemm(self, a, b, a_scale, b_scale, c, timeout_ns):
+            self.launched += self.record == 0
+            return self.record
+
+        def fp8_gemm_take_status(self, index):
+            code, self.record = self.record, 0
+            return {"code": code, "phase": 6, "peer": -1, "detail": 302, "epoch": 0, "seen": 0}
+
+    native = Native()
+    monkeypatch.setattr(_ext, "load", lambda *a, **k: native)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    a, s = torch.zeros(16, 32), torch.ones(16, 1)
+    c = torch.empty(16, 16, dtype=torch.bfloat16) if given else None
+    with pytest.raises(StatusError) as err:
+        f.fp8_gemm(a, a, s, s[:1], c)
+    assert err.value.code == "timeout" and err.value.phase == "gemm_pipeline" and native.launched == 0
+    assert f.fp8_gemm(a, a, s, s[:1], c).shape == (16, 16) and native.launched == 1
