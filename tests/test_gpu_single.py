@@ -457,3 +457,107 @@ want = fp8_gemm_reference(a, a, s, t)
 assert float((c.float() - want).abs().max()) < 1e-2 * float(want.abs().max())
 """
     subprocess.run([sys.executable, "-c", code], check=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+
+
+def _captured_case(op, size):
+    """(buffers to refill, how to fill them, the call) of a one-rank operator."""
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    normal = lambda *shape, dtype=torch.float32: torch.randn(*shape, device="cuda", generator=gen).to(dtype)  # noqa: E731
+    if op.startswith("moe"):
+        from amd_distributed_2025_b200.models import moe_all2all
+
+        E, k, H, T = size
+        cfg, data, _, _ = contract.make_moe_inputs(E, k, H, T, 5, 0, 1, device="cuda", dtype=torch.bfloat16, fixed_num_tokens=T)
+        layer = moe_all2all.MoEAllToAll(cfg, 0, 1, mode="dedup")
+        bufs = [data.x, data.indices, data.weights]
+        fill = lambda: [normal(T, H, dtype=torch.bfloat16), torch.argsort(normal(T, E), 1)[:, :k].int(), normal(T, k)]  # noqa: E731
+        if op == "moe_forward":
+            return bufs, fill, lambda: [layer.forward(*bufs, 3.0)], layer
+        out = torch.empty(T, H, dtype=torch.bfloat16, device="cuda")
+
+        def layered():
+            counts, ex, meta = layer.dispatch(bufs[0], bufs[1])
+            layer.combine(out, bufs[2], meta, ex, counts, T)
+            return [out, counts]
+
+        return bufs, fill, layered, layer
+    m, n, k = size
+    if op == "fp8":
+        from amd_distributed_2025_b200.ops.fp8_gemm import fp8_gemm
+
+        fill = lambda: [normal(m, k).to(torch.float8_e4m3fn), normal(n, k).to(torch.float8_e4m3fn),  # noqa: E731
+                        normal(m, (k + 127) // 128), normal((n + 127) // 128, (k + 127) // 128)]
+        bufs = fill()
+        return bufs, fill, lambda: [fp8_gemm(*bufs)], None
+    from amd_distributed_2025_b200.models import gemm_rs
+
+    gemm = gemm_rs.GemmRS(1 << 20, 1 << 12, rank=0, world_size=1)
+    fill = lambda: [normal(m, k, dtype=torch.bfloat16), normal(n, k, dtype=torch.bfloat16), normal(n, dtype=torch.bfloat16)]  # noqa: E731
+    bufs = fill()
+    return bufs, fill, lambda: [gemm(*bufs), gemm(*bufs, bias_mode="once")], gemm
+
+
+@pytest.mark.parametrize(
+    "op,size",
+    [
+        ("moe_forward", (64, 4, 512, 96)),
+        ("moe_layer", (64, 4, 512, 96)),
+        ("gemm", (64, 2880, 360)),  # clusters that share a tile
+        ("gemm", (4162, 1248, 4280)),  # tiles cut along K, which meet in a workspace of the graph's own
+        ("fp8", (300, 619, 400)),
+    ],
+)
+def test_one_rank_operators_replayed_from_graphs(op, size):
+    """Captured once, replayed with other inputs, on another stream, and with calls outside the graph in between."""
+    bufs, fill, call, owner = _captured_case(op, size)
+    call()
+    graphs = []
+    for _ in range(6):  # more graphs than the GEMM keeps workspaces for
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            outs = call()
+        graphs.append((g, outs))
+    side = torch.cuda.Stream()
+    for turn, (g, outs) in enumerate(graphs + graphs[:2]):
+        for b, v in zip(bufs, fill()):
+            b.copy_(v)
+        if turn % 2:
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                g.replay()
+                g.replay()
+            torch.cuda.current_stream().wait_stream(side)
+        else:
+            g.replay()
+        got = [o.clone() for o in outs]
+        want = call()
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), turn
+    if owner is not None:
+        owner.check()
+        owner.close()
+
+
+def test_gemm_cut_tiles_on_more_streams_than_workspaces():
+    """Calls on several streams at once: the first four streams get a workspace each, the others run whole tiles."""
+    from amd_distributed_2025_b200.models import gemm_rs
+
+    m, n, k = 4162, 1248, 4280
+    a, w, bias = contract.make_gemm_rs_inputs(0, 1, m, n, k, True, 17, device="cuda")
+    op = gemm_rs.GemmRS(1 << 20, 1 << 12, rank=0, world_size=1)
+    cut = op(a, w, bias, "once")
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(6)]
+    outs = [[] for _ in streams]
+    for _ in range(4):
+        for s, got in zip(streams, outs):
+            with torch.cuda.stream(s):
+                got.append(op(a, w, bias, "once"))
+    torch.cuda.synchronize()
+    op.check()
+    assert len(op.engine.local_workspaces()) == 4
+    truth = a.float() @ w.float().T + bias.float()
+    for i, got in enumerate(outs):
+        assert all(torch.equal(o, got[0]) for o in got)
+        assert i >= 3 or torch.equal(got[0], cut)
+        assert oracle.relative_error(got[0], truth) < 5e-3
+    op.close()
