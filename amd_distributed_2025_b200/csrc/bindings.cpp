@@ -33,6 +33,11 @@ void cuda_check(cudaError_t e, const char* what) {
   TORCH_CHECK(e == cudaSuccess, what, ": ", cudaGetErrorString(e));
 }
 
+// A kernel can read device memory and pinned host memory; an ordinary host tensor would fault the GPU.
+void check_reachable(const at::Tensor& t, const char* what) {
+  TORCH_CHECK(t.is_cuda() || t.is_pinned(), what, " must be a CUDA tensor");
+}
+
 int dtype_code(at::ScalarType t) {
   switch (t) {
     case at::kHalf: return 0;
@@ -102,6 +107,7 @@ void moe_dispatch(SymmHeap& heap, const at::Tensor& x, const at::Tensor& indices
   TORCH_CHECK(blk_hist.scalar_type() == at::kInt && blk_hist.is_contiguous() &&
                   blk_hist.numel() >= std::max<int64_t>(count_blocks, 1) * num_experts,
               "blk_hist scratch too small");
+  for (const at::Tensor& t : {blk_hist, local_rank, route, expert_num_tokens}) check_reachable(t, "scratch and results");
   TORCH_CHECK(local_rank.scalar_type() == at::kInt && local_rank.is_contiguous() && local_rank.numel() >= n,
               "local_rank scratch too small");
   TORCH_CHECK(route.scalar_type() == at::kInt && route.is_contiguous() && route.numel() >= 2 * n,
@@ -148,6 +154,9 @@ void moe_expert_scale(const at::Tensor& expert_x, at::Tensor expert_y, const at:
                       double scale) {
   TORCH_CHECK(expert_x.dim() == 3 && expert_y.sizes() == expert_x.sizes(), "expert_x / expert_y shapes differ");
   TORCH_CHECK(expert_x.is_contiguous() && expert_y.is_contiguous(), "expert buffers must be contiguous");
+  check_reachable(expert_x, "expert_x");
+  check_reachable(expert_y, "expert_y");
+  check_reachable(expert_num_tokens, "expert_num_tokens");
   c10::cuda::CUDAGuard guard(expert_x.device());
   cuda_check(b200::launch_moe_expert_scale(expert_x.data_ptr(), expert_y.data_ptr(),
                                            expert_num_tokens.data_ptr<int32_t>(), (int)expert_x.size(0),
@@ -164,6 +173,8 @@ void moe_combine(SymmHeap& heap, at::Tensor out, const at::Tensor& weights, cons
   TORCH_CHECK(weights.scalar_type() == at::kFloat && weights.is_contiguous() && weights.dim() == 2,
               "weights must be contiguous fp32 [T, k]");
   TORCH_CHECK(out.size(0) >= num_tokens && weights.size(0) >= num_tokens, "out/weights have fewer rows than tokens");
+  check_reachable(weights, "weights");
+  check_reachable(route, "route");
   const int64_t k = weights.size(1);
   TORCH_CHECK(route.scalar_type() == at::kInt && route.numel() >= 2 * num_tokens * k, "route too small");
   c10::cuda::CUDAGuard guard(heap.device());
@@ -542,11 +553,13 @@ void gemm_rs(SymmHeap& heap, const at::Tensor& a, const at::Tensor& w, const c10
   const int64_t M = a.size(0), N = w.size(0), K = a.size(1);
   TORCH_CHECK(M % ws == 0, "M must be divisible by world_size");
   TORCH_CHECK(out.scalar_type() == at::kBFloat16 && out.size(0) == M / ws && out.size(1) == N, "out must be bf16 [M/ws, N]");
+  check_reachable(out, "out");
   TORCH_CHECK(K % 8 == 0, "K per rank must be a multiple of 8 (16-byte rows for TMA)");
   TORCH_CHECK(N % 8 == 0, "N must be a multiple of 8 (16-byte vector epilogue)");
   const void* bias_ptr = nullptr;
   if (bias.has_value() && bias->defined()) {
     TORCH_CHECK(bias->scalar_type() == at::kBFloat16 && bias->numel() == N && bias->is_contiguous(), "bias must be bf16 [N]");
+    check_reachable(*bias, "bias");
     bias_ptr = bias->data_ptr();
   }
   c10::cuda::CUDAGuard guard(heap.device());
@@ -662,11 +675,13 @@ class GemmRsEngine {
     const int64_t M = a.size(0), N = w.size(0), K = a.size(1);
     TORCH_CHECK(M % ws == 0, "M must be divisible by world_size");
     TORCH_CHECK(out.scalar_type() == at::kBFloat16 && out.size(0) == M / ws && out.size(1) == N, "out must be bf16 [M/ws, N]");
+    check_reachable(out, "out");
     TORCH_CHECK(K % 8 == 0, "K per rank must be a multiple of 8 (16-byte rows for TMA)");
     TORCH_CHECK(N % 8 == 0, "N must be a multiple of 8 (16-byte vector epilogue)");
     const void* bias_ptr = nullptr;
     if (bias.has_value() && bias->defined()) {
       TORCH_CHECK(bias->scalar_type() == at::kBFloat16 && bias->numel() == N && bias->is_contiguous(), "bias must be bf16 [N]");
+      check_reachable(*bias, "bias");
       bias_ptr = bias->data_ptr();
     }
     c10::cuda::CUDAGuard guard(heap_->device());
@@ -923,6 +938,9 @@ int fp8_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& a_scale
               "b_scale must be fp32 [ceil(N/128), ceil(K/128)]");
   TORCH_CHECK(c.scalar_type() == at::kBFloat16 && c.is_contiguous() && c.size(0) == M && c.size(1) == N, "c must be bf16 [M, N]");
   TORCH_CHECK(K % 16 == 0, "K must be a multiple of 16");
+  check_reachable(a_scale, "a_scale");
+  check_reachable(b_scale, "b_scale");
+  check_reachable(c, "c");
   c10::cuda::CUDAGuard guard(a.device());
   if (const uint32_t code = fp8_status_code(a.get_device())) return (int)code;
   run_fp8_gemm(a, b, a_scale, b_scale, c, timeout_ns);

@@ -561,3 +561,29 @@ def test_gemm_cut_tiles_on_more_streams_than_workspaces():
         assert i >= 3 or torch.equal(got[0], cut)
         assert oracle.relative_error(got[0], truth) < 5e-3
     op.close()
+
+
+def test_host_tensors_are_refused_before_a_launch():
+    """A kernel that is given the address of an ordinary host tensor faults: scales, bias, results, weights, expert rows."""
+    from amd_distributed_2025_b200.models import gemm_rs, moe_all2all
+    from amd_distributed_2025_b200.ops.fp8_gemm import fp8_gemm
+
+    a = torch.ones(128, 256, device="cuda").to(torch.float8_e4m3fn)
+    s, t = torch.ones(128, 2, device="cuda"), torch.ones(1, 2, device="cuda")
+    x, w, bias = contract.make_gemm_rs_inputs(0, 1, 64, 512, 256, True, 5, device="cuda")
+    op = gemm_rs.get_op(64, 512, 256)
+    cfg, data, _, _ = contract.make_moe_inputs(16, 2, 256, 8, 3, 0, 1, device="cuda", fixed_num_tokens=8)
+    layer = moe_all2all.MoEAllToAll(cfg, 0, 1, mode="direct")
+    counts, ex, meta = layer.dispatch(data.x, data.indices)
+    y = torch.empty(8, 256, dtype=cfg.out_dtype, device="cuda")
+    for call in (lambda: fp8_gemm(a, a, s.cpu(), t), lambda: fp8_gemm(a, a, s, t.cpu()),
+                 lambda: fp8_gemm(a, a, s, t, c=torch.empty(128, 128, dtype=torch.bfloat16)),
+                 lambda: op(x, w, bias.cpu()), lambda: op(x, w, bias, out=torch.empty(64, 512, dtype=torch.bfloat16)),
+                 lambda: layer.combine(y, data.weights.cpu(), meta, ex, counts), lambda: layer.combine(y, data.weights, meta, ex.cpu(), counts)):
+        with pytest.raises(RuntimeError):
+            call()
+    want = op(x, w, bias)
+    assert torch.equal(op(x, w, bias.cpu().pin_memory()), want)  # memory that the GPU can read stays accepted
+    torch.cuda.synchronize()
+    layer.check()
+    layer.close()
