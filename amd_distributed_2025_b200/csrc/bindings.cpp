@@ -782,6 +782,7 @@ class GemmRsEngine {
     g.timeout_ns = (uint64_t)timeout_ns_;
     g.status = heap_->status_device();
     g.trace = trace_;
+    g.trace_ctas = trace_ == nullptr ? 0 : (int)std::min<int64_t>(trace_keep_.numel() / 8, 1 << 20);
     g.sms = sms_;
     ++epoch_;
     cuda_check(b200::launch_gemm_local(g, stream), "gemm_local launch");
@@ -1526,6 +1527,21 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return py::make_tuple(s.smem, s.tmem_cols);
   });
   m.def("fp8_gemm_share", [](int bn, int splits) { return py::make_tuple(b200::fp8_gemm_smem(bn, splits), 512); });
+  m.def("gemm_local_plan", [](int M, int N, int K, int sms) {  // one rank
+    TORCH_CHECK(M > 0 && N > 0 && K > 0, "sizes must be positive");
+    const b200::GemmLocalPlan p = b200::gemm_local_plan(M, N, K, sms);
+    py::dict d;
+    d["kernel"] = p.persistent ? "pair" : "tile";
+    d["swap"] = p.swap;
+    d["cta_pair"] = p.pair;
+    d["rows"] = p.rows;
+    d["bn"] = p.bn;
+    d["splits"] = p.splits;
+    d["halves"] = p.halves;
+    d["cut_tiles"] = p.cut_tiles;
+    d["ctas"] = p.ctas;
+    return d;
+  }, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("sms") = 148);
   m.def("gemm_rs_plan", [](int64_t M, int64_t N, int64_t K, int64_t ws, int64_t block_n, int64_t cta_pair, int64_t splits) {
     const b200::GemmRsPlan p = b200::gemm_rs_plan((int)M, (int)N, (int)K, (int)ws, (int)block_n, (int)cta_pair, (int)splits);
     py::dict d;

@@ -75,11 +75,12 @@ struct LocalParams {
   uint32_t* counters; // pair kernel: [sk_tiles][cta][epilogue warp], zero between launches
   uint64_t timeout_ns;
   StatusBlock* status;
-  uint64_t* trace;    // optional [gridDim.x][8]: 0 start, 1 ready, 2 tiles done, 3 exit
+  int trace_ctas;     // CTAs that `trace` has room for: a grid of several waves has more than an SM each
+  uint64_t* trace;    // optional [trace_ctas][8]: 0 start, 1 ready, 2 tiles done, 3 exit
 };
 
 __device__ __forceinline__ void stamp(const LocalParams& p, int slot) {
-  if (p.trace != nullptr) p.trace[(size_t)blockIdx.x * 8 + slot] = global_timer_ns();
+  if (p.trace != nullptr && (int)blockIdx.x < p.trace_ctas) p.trace[(size_t)blockIdx.x * 8 + slot] = global_timer_ns();
 }
 
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* abort, const LocalParams& p, int detail) {
@@ -977,6 +978,7 @@ bool common_params(LocalParams& p, const GemmLocalArgs& a, const Plan& plan, int
   p.timeout_ns = a.timeout_ns;
   p.status = a.status;
   p.trace = a.trace;
+  p.trace_ctas = a.trace_ctas;
   return make_tensor_map(map_p, swap ? a.w : a.a, (uint64_t)p.P, (uint64_t)a.K, 2, (uint32_t)p_rows, kBK, 128) &&
          make_tensor_map(map_q, swap ? a.a : a.w, (uint64_t)p.Q, (uint64_t)a.K, 2, (uint32_t)q_rows, kBK, 128) &&
          make_tensor_map(map_out, a.out, (uint64_t)a.M, (uint64_t)a.N, 2, 32, swap ? 32 : 64, swap ? 0 : 128);
@@ -1047,6 +1049,12 @@ SmShare gemm_tile_share(int rows, int bn, int splits, bool pair) {
   return {t.smem, t.tmem_cols};
 }
 SmShare gemm_pair_share(int bn, int halves) { return {pair_smem(bn, halves), kTmemCols}; }
+
+GemmLocalPlan gemm_local_plan(int M, int N, int K, int sms) {
+  const Plan& p = cached_plan(M, N, K, sms);
+  const int ctas = p.persistent ? 2 * p.pairs : p.p_tiles * p.q_tiles * ctas_of(p);
+  return {p.persistent, p.swap, p.persistent || p.pair, p.rows, p.bn, p.splits, p.halves, p.sk_tiles, ctas};
+}
 
 bool gemm_local_cuts_tiles(int M, int N, int K, int sms) {
   const Plan& plan = cached_plan(M, N, K, sms);

@@ -87,7 +87,8 @@ struct GemmLocalArgs {
   uint32_t* counters;  // kGemmLocalCounters words, zero between launches; calls in flight at once need their own
   uint64_t timeout_ns;
   StatusBlock* status;
-  uint64_t* trace;
+  uint64_t* trace;  // [trace_ctas][8]
+  int trace_ctas;
   int sms;
 };
 
@@ -98,6 +99,12 @@ constexpr uint64_t kGemmLocalPartialBytes = (uint64_t)kGemmLocalMaxPairs * 2 * 2
 constexpr int kGemmLocalCounters = kGemmLocalMaxPairs * 2 * 2 * 8;
 
 cudaError_t launch_gemm_local(const GemmLocalArgs& args, cudaStream_t stream);
+// How the launch will run (a pure function of its arguments and the device's cluster capacities).
+struct GemmLocalPlan {
+  bool persistent, swap, pair;  // pair kernel or tile kernel; weight on the 128-row side; a CTA pair per tile
+  int rows, bn, splits, halves, cut_tiles, ctas;
+};
+GemmLocalPlan gemm_local_plan(int M, int N, int K, int sms);
 bool gemm_local_cuts_tiles(int M, int N, int K, int sms);  // whether the launch has a use for `partials`
 
 // What a CTA takes of its SM, by tile.  Two CTAs may meet on an SM (calls on two streams, or the next call's early

@@ -587,3 +587,20 @@ def test_host_tensors_are_refused_before_a_launch():
     torch.cuda.synchronize()
     layer.check()
     layer.close()
+
+
+def test_gemm_stamps_stay_inside_the_trace_tensor():
+    """A grid of several waves has more CTAs than the trace has rows: those beyond it leave no stamps."""
+    from amd_distributed_2025_b200.models import gemm_rs
+
+    op = gemm_rs.GemmRS(1 << 20, 1 << 12, rank=0, world_size=1)
+    buf = torch.zeros(2048, 8, dtype=torch.int64, device="cuda")
+    op.engine.set_trace(buf[:160])  # (any CTA's row would lie in `buf`)
+    m, n, k = 16, 32000, 4096
+    plan = _ext().gemm_local_plan(m, n, k, torch.cuda.get_device_properties(0).multi_processor_count)
+    assert 160 < plan["ctas"] <= 2048
+    a, w, _ = contract.make_gemm_rs_inputs(0, 1, m, n, k, False, 1, device="cuda")
+    op(a, w)
+    torch.cuda.synchronize()
+    assert bool((buf[:160, :4] > 0).all()) and int(buf[160:].abs().sum()) == 0
+    op.close()
