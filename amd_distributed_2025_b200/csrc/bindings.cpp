@@ -1534,6 +1534,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     d["kernel"] = p.persistent ? "pair" : "tile";
     d["swap"] = p.swap;
     d["cta_pair"] = p.pair;
+    d["own_parts"] = p.own_parts;
     d["rows"] = p.rows;
     d["bn"] = p.bn;
     d["splits"] = p.splits;

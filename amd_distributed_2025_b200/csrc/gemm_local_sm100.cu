@@ -1053,7 +1053,8 @@ SmShare gemm_pair_share(int bn, int halves) { return {pair_smem(bn, halves), kTm
 GemmLocalPlan gemm_local_plan(int M, int N, int K, int sms) {
   const Plan& p = cached_plan(M, N, K, sms);
   const int ctas = p.persistent ? 2 * p.pairs : p.p_tiles * p.q_tiles * ctas_of(p);
-  return {p.persistent, p.swap, p.persistent || p.pair, p.rows, p.bn, p.splits, p.halves, p.sk_tiles, ctas};
+  const bool own_parts = !p.persistent && tile_memory(p.rows, p.bn, p.splits, p.pair).part_bytes > 0;
+  return {p.persistent, p.swap, p.persistent || p.pair, own_parts, p.rows, p.bn, p.splits, p.halves, p.sk_tiles, ctas};
 }
 
 bool gemm_local_cuts_tiles(int M, int N, int K, int sms) {

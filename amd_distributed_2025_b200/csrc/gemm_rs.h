@@ -102,6 +102,7 @@ cudaError_t launch_gemm_local(const GemmLocalArgs& args, cudaStream_t stream);
 // How the launch will run (a pure function of its arguments and the device's cluster capacities).
 struct GemmLocalPlan {
   bool persistent, swap, pair;  // pair kernel or tile kernel; weight on the 128-row side; a CTA pair per tile
+  bool own_parts;               // the parts of a shared tile have memory of their own (else the pipeline's)
   int rows, bn, splits, halves, cut_tiles, ctas;
 };
 GemmLocalPlan gemm_local_plan(int M, int N, int K, int sms);
