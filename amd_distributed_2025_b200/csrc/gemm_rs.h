@@ -87,7 +87,7 @@ struct GemmLocalArgs {
   uint32_t* counters;  // kGemmLocalCounters words, zero between launches; calls in flight at once need their own
   uint64_t timeout_ns;
   StatusBlock* status;
-  uint64_t* trace;  // [trace_ctas][8]
+  uint64_t* trace;   // [trace_ctas][8]; a launch of more CTAs leaves no stamps
   int trace_ctas;
   int sms;
 };

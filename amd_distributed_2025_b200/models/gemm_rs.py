@@ -181,7 +181,8 @@ class GemmRS:
     def enable_trace(self, on: bool = True) -> None:
         """Record per-CTA phase time stamps (ns) of the next calls into ``self.trace``: columns =
         kernel start, pipeline ready, GEMM tiles done, exit, first own tile reached, its
-        peers' rows arrived, last own tile stored."""
+        peers' rows arrived, last own tile stored.  (On one rank a launch of more than 160 CTAs, several
+        waves of small tiles, leaves none.)"""
         self.trace = torch.zeros((160, 8), dtype=torch.int64, device=self.device) if on else None
         self.engine.set_trace(self.trace)
 

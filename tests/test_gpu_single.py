@@ -640,7 +640,7 @@ def test_host_tensors_are_refused_before_a_launch():
 
 
 def test_gemm_stamps_stay_inside_the_trace_tensor():
-    """A grid of several waves has more CTAs than the trace has rows: those beyond it leave no stamps."""
+    """A grid of several waves has more CTAs than the trace has rows: it leaves no stamps then."""
     from amd_distributed_2025_b200.models import gemm_rs
 
     op = gemm_rs.GemmRS(1 << 20, 1 << 12, rank=0, world_size=1)
@@ -652,5 +652,9 @@ def test_gemm_stamps_stay_inside_the_trace_tensor():
     a, w, _ = contract.make_gemm_rs_inputs(0, 1, m, n, k, False, 1, device="cuda")
     op(a, w)
     torch.cuda.synchronize()
-    assert bool((buf[:160, :4] > 0).all()) and int(buf[160:].abs().sum()) == 0
+    assert int(buf.abs().sum()) == 0
+    op.engine.set_trace(buf)
+    op(a, w)
+    torch.cuda.synchronize()
+    assert bool((buf[: plan["ctas"], :4] > 0).all()) and int(buf[plan["ctas"]:].abs().sum()) == 0
     op.close()
