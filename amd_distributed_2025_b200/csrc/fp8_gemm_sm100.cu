@@ -15,13 +15,14 @@
 // than the products.  Pairs are persistent; where there are fewer tiles than pairs, a cluster of pairs shares a tile,
 // each over its part of K, and the parts meet in distributed shared memory.
 //
-// What bounds it: the epilogue.  For a K block a warp spends some 300 cycles on reading and scaling 64 columns, 130 on
+// What bounds it: the epilogue, closely followed by the operands (a CTA brings in 192 rows for a K block of a 128-column
+// tile; without its epilogue 4096 x 4096 x 2048 still takes 34 us) and, in a row of calls, by power.  For a K block a warp spends some 300 cycles on reading and scaling 64 columns, 130 on
 // the signal that frees the buffer and 130 on the wait for the next, against 256 cycles of multiplication; meeting once
 // for two blocks halves the last two, and the read of a chunk runs beside the sums of the one before.  Tried and slower
-// at 4096 x 4096 x 2048: 256 columns in halves with split registers (40.6 us; few tiles, long ends), sixteen epilogue
-// warps (52 us; the waits doubled), warp-wide waits (40.8 us).
-// On a B200, us, with one block a buffer and scales through registers -> now: 4096 x 4096 x 2048 40.9 -> 37.8,
-// 8192 x 8192 x 4096 293 -> 268, 2048^3 14.5 -> 13.0, 512 x 512 x 8192 12.6 -> 10.7, 64 x 4096 x 4096 11.6 -> 10.2.
+// at 4096 x 4096 x 2048, all timed while the GPU was cool: 256 columns in halves with split registers (40.6 us; few
+// tiles, long ends), sixteen epilogue warps (52 us; the waits doubled), warp-wide waits (40.8 us).
+// On a B200, us, while cool (in a row of calls 4096 x 4096 x 2048 takes 44), with one block a buffer and scales through
+// registers -> now: 4096 x 4096 x 2048 40.9 -> 37.8, 8192 x 8192 x 4096 293 -> 268, 2048^3 14.5 -> 13.0, 512 x 512 x 8192 12.6 -> 10.7, 64 x 4096 x 4096 11.6 -> 10.2.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -106,7 +107,8 @@ __device__ __forceinline__ bool fp8_wait(uint32_t bar, uint32_t parity, volatile
   return true;
 }
 
-// A CTA in which a wait expired says so, once, on its way out: what it computed is of no use.
+// A CTA in which a wait expired says so on its way out (every warp that knows of it does, and one is enough): what it
+// computed is of no use.
 __device__ __forceinline__ void record_expired(const Fp8Params& p, int detail) {
   if (p.status != nullptr && reinterpret_cast<volatile StatusWord*>(p.status)->code == STATUS_OK)
     store_status(p.status, STATUS_TIMEOUT, PHASE_GEMM_PIPELINE, -1, detail, 0, 0);
@@ -507,6 +509,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   if (abort_flag) {
     const uint64_t t0 = global_timer_ns();
     while (global_timer_ns() - t0 < 200000) __nanosleep(1000);
+    if (lane == 0) record_expired(p, abort_flag);
   }
   __syncwarp();
   ptx::tcgen05_fence_before();
@@ -514,7 +517,6 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   ptx::cluster_sync_all();  // no CTA retires while another may still signal its barriers or read its memory
   ptx::tcgen05_fence_after();
   if (warp == 1) ptx::tmem_dealloc_pair(tmem_base, kTmemCols);
-  if (tid == 0 && abort_flag) record_expired(p, abort_flag);
 }
 
 __global__ void fp8_wait_selftest_kernel(const Fp8Params p) {
