@@ -13,12 +13,12 @@
 //   gemm_pair_kernel   larger ones: persistent CTA pairs (cta_group::2) on tiles of 256 P rows; the last wave, which
 //                      would leave pairs idle, is dealt out by k-blocks instead of by tiles.  The largest ones run
 //                      against the power limit: there a tile is 512 columns, both accumulators wide, and a quarter
-//                      less operand traffic buys clock (8192 x 8192 x 28672 in a row of calls: 2980 us at 1100 MHz with
-//                      256 columns, 2846 us at 1280 MHz with 512; cuBLAS 2863 us at 1245 MHz).
+//                      less operand traffic buys clock (8192 x 8192 x 28672 in a row of calls: 1280 MHz instead of the
+//                      1100 with 256 columns, and 4.5 % less time).
 //
 // Multi-rank kernel before -> these kernels, one rank, us in a row of calls: 64 x 2880 x 360 10.2 -> 4.6 (latency: a launch
 // and its call), 64 x 7168 x 18432 71 -> 49 (memory, 5.9 TB/s while cool), 256 x 5120 x 12800 58 -> 41 (34 while cool:
-// memory, then the meeting of the parts), 2048 x 2880 x 2880 45 -> 34 (power), 8192 x 8192 x 28672 3040 -> 2770 (power).
+// memory, then the meeting of the parts), 2048 x 2880 x 2880 45 -> 34 (120 tiles on 74 pairs), 8192 x 8192 x 28672 3135 -> 2792 (power).
 //
 // Warp roles of both (320 threads): 0 TMA producer, 1 MMA issuer, 2..9 epilogue, two per tensor-memory lane quarter.
 // Shared memory keeps CTAs of the pair kernel, which take all of the tensor memory, alone on their SM.  Small tiles of
@@ -943,7 +943,8 @@ Plan make_local_plan(int M, int N, int K, int sms) {
   return best;
 }
 
-// A program comes back with the same few shapes: the search above costs more than a short kernel.
+// A program comes back with the same few shapes: the search above (2 to 6 us) costs more than a short kernel.  Each
+// thread keeps 64 plans, one to a slot of the hash; shapes that share a slot are searched anew whenever they alternate.
 const Plan& cached_plan(int M, int N, int K, int sms) {
   struct Entry {
     int M = 0, N = 0, K = 0, sms = 0, dev = -1;

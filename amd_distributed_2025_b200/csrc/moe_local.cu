@@ -6,8 +6,9 @@
 // by the route table.  The layouts are those of the multi-rank kernels (rows of an expert in
 // (token, k) order; 5-int metadata; per-expert counts).
 //
-// Both kernels may start before the previous kernel of the stream has ended (programmatic dependent launch), so
-// what that kernel may have written is read through L2 (ld.global.cg) and only after grid_dep_wait().
+// Both kernels may start before the previous kernel of the stream has ended (programmatic dependent launch): nothing
+// is read or written before grid_dep_wait(), which makes that kernel's stores visible.  Ids, routes, weights and whole
+// vectors are read past L1 (ld.global.cg), as nothing comes back for them; ragged rows, element by element, are not.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -430,10 +431,15 @@ cudaError_t combine_typed(const MoeLocalCombineParams& p, int grid, cudaStream_t
 
 }  // namespace
 
-// A CTA reads the ids of every earlier token, so that work grows with the square of the entries; at 32768
-// entries it is 128 KiB of L2 reads per SM, a few microseconds beside 200 MB of row stores.  Beyond that the
-// kernel with a grid barrier counts every entry once.  (8192 experts: the counts fill 32 KiB of the 48 KiB of
-// shared memory that need no opt-in.)
+// A CTA reads the ids of every earlier token, so that work grows with the square of the entries, where the kernel
+// with a grid barrier counts every entry once.  The line lies at the most entries that the task's generator draws, the
+// range this kernel is tested over; the two do not cross there.  bf16, us, forward / dispatch + combine, on either side:
+//   entries                                32768        65536: here, with barrier     131072: here, with barrier
+//   64 experts, top-8, rows of 8 KiB     70 / 116     135 / 230      344 / 244        266 / 451      668 / 470
+//   256 experts, top-8, rows of 2 KiB    22 / 39       44 / 71       142 / 120         85 / 129      240 / 192
+//   64 experts, top-8, rows of 512 B     13 / 18       23 / 34        66 / 55          42 / 71       115 / 95
+//   64 experts, top-4, rows of 128 B     14 / 23       24 / 41        82 / 72          44 / 74       139 / 118
+// (8192 experts: the counts fill 32 KiB of the 48 KiB of shared memory that need no opt-in.)
 bool moe_local_dispatch_applies(int64_t num_entries, int num_experts) {
   return num_entries <= 32768 && num_experts <= 8192;
 }

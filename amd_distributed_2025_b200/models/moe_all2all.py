@@ -326,9 +326,10 @@ class MoEAllToAll:
     def forward(self, dp_x: torch.Tensor, indices: torch.Tensor, weights: torch.Tensor, scale: float) -> torch.Tensor:
         """dispatch -> ``expert_y = expert_x * scale`` -> combine, launched back to back from
         one native call.  In "dedup" mode the scale is applied while the landed rows are
-        replicated into the expert buffers (two launches); on one rank it and the weighted sum are
-        formed from the rows as they are stored to ``expert_x`` (one launch, ``expert_y`` is not
-        written); in "direct" mode it is the three kernels of the separate methods."""
+        replicated into the expert buffers (two launches).  On one rank, up to 32768 (token, k) entries,
+        it and the weighted sum are formed from the rows as they are stored to ``expert_x`` (one launch);
+        ``self.expert_y`` is not written then, as it is beyond that size and in "direct" mode.  In "direct"
+        mode it is the three kernels of the separate methods."""
         if self._native is not None and self.monitor is None:
             y = self._native.try_forward(dp_x, indices, weights, scale)
             if y is not None:
