@@ -173,7 +173,8 @@ struct MoeLocalDispatchParams {
   StatusBlock* status;
   uint64_t* trace_d;         // optional stamps, slots as in the multi-rank kernels
   uint64_t* trace_c;
-  int32_t vec, pieces, piece_vecs, cap, hist_copies;  // filled in by the launcher
+  int32_t vec, pieces, piece_vecs, cap;  // filled in by the launcher
+  float lean;                // how much longer the runs of the first CTAs are than those of the last
 };
 
 struct MoeLocalCombineParams {

@@ -59,142 +59,110 @@ __device__ __forceinline__ int4 pack_pairs(const float2* acc) {
   return pack_vec<T>(reinterpret_cast<const float*>(acc));
 }
 
-// What a CTA of the dispatch kernel owns.
+// What a CTA of the dispatch kernel owns: items [lo, hi) and the entries [i0, i0 + m) of the tokens they touch.
 struct Share {
-  int lo, hi;   // items
-  int t0;       // first token
-  int32_t* rows;  // shared memory: final row of every entry of tokens t0, t0 + 1, ..., or -1
+  int lo, hi, t0, i0, m;
+  int32_t* total;  // shared memory: entries [0, i0 + m) of each expert
+  int32_t* ids;    // shared memory: expert of each own entry, or -1; then three words of -2
+  int32_t* rows;   // shared memory: final row of each own entry, or -1
 };
 
-// First half of the dispatch kernel: the CTA's share, the final rows of its entries (in shared memory), and
-// the route table, metadata and counts in global memory.  Called by all threads; ends with the rows visible.
-//
-// Work is T x P items (token, piece of its row); CTA b owns the items [b I / G, (b + 1) I / G) and so the
-// tokens they touch.  It counts the entries of all EARLIER tokens per expert by reading their ids itself (at
-// most 128 KiB, out of L2) instead of meeting the other CTAs on a barrier, and ranks its own entries with one
-// warp.  Neighbouring CTAs may share a token; its metadata belongs to the CTA with its first piece.
-template <int THREADS>
-__device__ __forceinline__ void assign_rows(const MoeLocalDispatchParams& p, int32_t* smem, Share& sh) {
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int E = p.num_experts;
-  const int k = p.k;
-  const int P = p.pieces;
-  const int copies = p.hist_copies;
-  int32_t* s_hist = smem;  // [copies][E]; after the count, row 0 holds the sums
-  int32_t* s_ids = smem + copies * E;
-  int32_t* s_rows = s_ids + p.cap;
-  const int t1 = (sh.hi + P - 1) / P;
-  const int i0 = sh.t0 * k;
-  const int m = sh.hi > sh.lo ? t1 * k - i0 : 0;  // own entries
-  sh.rows = s_rows;
-
-  for (int e = tid; e < copies * E; e += THREADS) s_hist[e] = 0;
-  for (int j = tid; j < m; j += THREADS) {
-    int e = __ldcg(p.indices + i0 + j);
-    if (e < 0 || e >= E) {
-      record_status(p.status, STATUS_BAD_INDEX, PHASE_NONE, -1, i0 + j, p.epoch, (uint64_t)(int64_t)e);
-      e = -1;
-    }
-    s_ids[j] = e;
-  }
-  __syncthreads();
-  {
-    // skewed routing has many lanes of a warp add to the same expert: spread them over the copies
-    int32_t* hist = s_hist + (lane & (copies - 1)) * E;
-    auto count = [&](int e) {
-      if (e >= 0 && e < E) atomicAdd(&hist[e], 1);
-    };
-    int done = 0;
-    if ((reinterpret_cast<uintptr_t>(p.indices) & 15u) == 0) {
-      const int4* ids4 = reinterpret_cast<const int4*>(p.indices);
-      const int n4 = i0 >> 2;
-      constexpr int kFly = 8;  // loads in flight per thread
-      for (int q0 = tid; q0 < n4; q0 += THREADS * kFly) {
-        int4 a[kFly];
-#pragma unroll
-        for (int u = 0; u < kFly; ++u) {
-          const int q = q0 + u * THREADS;
-          a[u] = q < n4 ? __ldcg(ids4 + q) : make_int4(-1, -1, -1, -1);
-        }
-#pragma unroll
-        for (int u = 0; u < kFly; ++u) {
-          count(a[u].x);
-          count(a[u].y);
-          count(a[u].z);
-          count(a[u].w);
-        }
-      }
-      done = n4 << 2;
-    }
-    for (int i = done + tid; i < i0; i += THREADS) count(__ldcg(p.indices + i));
-  }
-  __syncthreads();
-  if (copies > 1) {
-    for (int e = tid; e < E; e += THREADS) {
-      int sum = s_hist[e];
-      for (int c = 1; c < copies; ++c) sum += s_hist[c * E + e];
-      s_hist[e] = sum;
-    }
-    __syncthreads();
-  }
-  stamp_cta0(p.trace_d, 1);
-  if (tid < 32) {
-    for (int base = 0; base < m; base += 32) {
-      const int j = base + lane;
-      const int e = j < m ? s_ids[j] : -1;
-      const unsigned active = __ballot_sync(0xffffffffu, e >= 0);
-      int slot = -1;
-      if (e >= 0) {
-        const unsigned same = __match_any_sync(active, e);
-        const int before = __popc(same & ((1u << lane) - 1u));
-        const int cur = s_hist[e];
-        __syncwarp(active);
-        slot = cur + before;
-        if (before == 0) s_hist[e] = cur + __popc(same);
-      }
-      __syncwarp();
-      int row = -1;
-      if (e >= 0) {
-        if (slot < p.max_recv) row = e * p.max_recv + slot;
-        else record_status(p.status, STATUS_BAD_INDEX, PHASE_NONE, 0, i0 + j, p.epoch, (uint64_t)slot);
-      }
-      if (j < m) s_rows[j] = row;
-    }
-  }
-  __syncthreads();
-  stamp_cta0(p.trace_d, 2);
-
-  // route table, metadata rows (global expert, source rank, token, k, 0) and counts
-  const int j_lo = ((sh.lo + P - 1) / P) * k - i0;  // entries of tokens whose first piece is this CTA's
-  for (int j = max(j_lo, 0) + tid; j < m; j += THREADS) {
-    const int row = s_rows[j];
-    const int i = i0 + j;
-    p.route[i] = make_int2(row >= 0 ? 0 : -1, row);
-    if (row >= 0) {
-      int32_t* meta = p.expert_meta + (size_t)row * kMetaDim;
-      meta[0] = s_ids[j];
-      meta[1] = 0;
-      meta[2] = i / k;
-      meta[3] = i % k;
-      meta[4] = 0;
-    }
-  }
-  if (blockIdx.x == gridDim.x - 1)
-    for (int e = tid; e < E; e += THREADS) p.expert_num_tokens[e] = min(s_hist[e], p.max_recv);
-  stamp_cta0(p.trace_d, 3);
-  stamp_cta0(p.trace_d, 4);
-  stamp_cta0(p.trace_d, 5);
+// Where CTA b's run of items starts: runs get shorter towards the last CTA by `lean` of their mean either way.
+__device__ __forceinline__ int first_item(const MoeLocalDispatchParams& p, int b) {
+  const int items = p.num_tokens * p.pieces;
+  if (b >= (int)gridDim.x) return items;
+  const float x = (float)b / (float)gridDim.x;
+  return (int)((float)items * x * (1.f + p.lean * (1.f - x)));
 }
 
-__device__ __forceinline__ Share share_of_cta(const MoeLocalDispatchParams& p) {
+// Work is T x P items (token, piece of its row), dealt out to the CTAs in runs.  Neighbouring CTAs may share a
+// token; its metadata belongs to the CTA with its first piece.
+__device__ __forceinline__ Share share_of_cta(const MoeLocalDispatchParams& p, int32_t* smem) {
   Share sh;
-  const long long items = (long long)p.num_tokens * p.pieces;
-  sh.lo = (int)(items * blockIdx.x / gridDim.x);
-  sh.hi = (int)(items * (blockIdx.x + 1) / gridDim.x);
+  sh.lo = first_item(p, (int)blockIdx.x);
+  sh.hi = first_item(p, (int)blockIdx.x + 1);
   sh.t0 = sh.lo / p.pieces;
-  sh.rows = nullptr;
+  sh.i0 = sh.t0 * p.k;
+  sh.m = sh.hi > sh.lo ? (sh.hi + p.pieces - 1) / p.pieces * p.k - sh.i0 : 0;
+  sh.total = smem;
+  sh.ids = smem + ((p.num_experts + 3) & ~3);
+  sh.rows = sh.ids + p.cap;
   return sh;
+}
+
+// Counts the entries of every expert up to the CTA's last one, by reading the ids itself (at most 128 KiB, out of L2)
+// instead of meeting the other CTAs on a barrier, and keeps its own ids.
+template <int FLY>
+__device__ __forceinline__ void count_entries(const MoeLocalDispatchParams& p, const Share& sh) {
+  const int tid = threadIdx.x, threads = blockDim.x;
+  auto count = [&](int i, int e) {
+    const bool valid = (uint32_t)e < (uint32_t)p.num_experts;
+    if (valid) atomicAdd(sh.total + e, 1);
+    if (i >= sh.i0) {
+      if (!valid) record_status(p.status, STATUS_BAD_INDEX, PHASE_NONE, -1, i, p.epoch, (uint64_t)(int64_t)e);
+      sh.ids[i - sh.i0] = valid ? e : -1;
+    }
+  };
+  const int n = sh.i0 + sh.m;
+  int done = 0;
+  if ((reinterpret_cast<uintptr_t>(p.indices) & 15u) == 0) {
+    const int4* ids4 = reinterpret_cast<const int4*>(p.indices);
+    const int n4 = n >> 2;
+    for (int q0 = tid; q0 < n4; q0 += threads * FLY) {
+      int4 a[FLY];  // loads in flight per thread
+#pragma unroll
+      for (int u = 0; u < FLY; ++u)
+        if (q0 + u * threads < n4) a[u] = __ldcg(ids4 + q0 + u * threads);
+#pragma unroll
+      for (int u = 0; u < FLY; ++u) {
+        const int q = q0 + u * threads;
+        if (q >= n4) break;
+        count(4 * q, a[u].x);
+        count(4 * q + 1, a[u].y);
+        count(4 * q + 2, a[u].z);
+        count(4 * q + 3, a[u].w);
+      }
+    }
+    done = n4 << 2;
+  }
+  for (int i = done + tid; i < n; i += threads) count(i, __ldcg(p.indices + i));
+}
+
+// Final rows of the own entries, a lane each.  An expert's rows are in (token, k) order: the slot of an entry is the
+// count up to the CTA's end less the own entries of that expert from it on.
+__device__ __forceinline__ void assign_rows(const MoeLocalDispatchParams& p, const Share& sh) {
+  const int lane = threadIdx.x & 31;
+  for (int j0 = (int)threadIdx.x - lane; j0 < sh.m; j0 += blockDim.x) {
+    const int j = j0 + lane;
+    const int e = j < sh.m ? sh.ids[j] : -1;
+    const int before = e >= 0 ? sh.total[e] : 0;
+    int from_here = __popc(__match_any_sync(0xffffffffu, e) & (0xffffffffu << lane));
+#pragma unroll 4
+    for (int i = j0 + 32; i < sh.m; i += 4) {
+      const int4 later = *reinterpret_cast<const int4*>(sh.ids + i);
+      from_here += (later.x == e) + (later.y == e) + (later.z == e) + (later.w == e);
+    }
+    const int slot = before - from_here;
+    if (j < sh.m) sh.rows[j] = e >= 0 && slot < p.max_recv ? e * p.max_recv + slot : -1;
+  }
+}
+
+// Route table and metadata rows (global expert, source rank, token, k, 0) of a token.
+__device__ __forceinline__ void write_metadata(const MoeLocalDispatchParams& p, const Share& sh, int t, int lane) {
+  if (lane >= p.k) return;
+  const int i = t * p.k + lane;
+  const int e = sh.ids[i - sh.i0], row = sh.rows[i - sh.i0];
+  p.route[i] = make_int2(row >= 0 ? 0 : -1, row);
+  if (row >= 0) {
+    int32_t* meta = p.expert_meta + (size_t)row * kMetaDim;
+    meta[0] = e;
+    meta[1] = 0;
+    meta[2] = t;
+    meta[3] = lane;
+    meta[4] = 0;
+  } else if (e >= 0) {
+    record_status(p.status, STATUS_BAD_INDEX, PHASE_NONE, 0, i, p.epoch, (uint64_t)p.max_recv);
+  }
 }
 
 __device__ __forceinline__ void final_stamps(const MoeLocalDispatchParams& p, bool fused) {
@@ -215,25 +183,35 @@ __device__ __forceinline__ void final_stamps(const MoeLocalDispatchParams& p, bo
 //
 // Every warp takes one 1 KiB piece at a time through registers; the first is on its way while the slots are
 // worked out, the next is asked for before the stores of the current one.  Large problems are bound by the row
-// stores: 268 MB (4096 tokens, top-6, hidden 4096) in 55 us, where a bare copy of the same pattern takes 48 to
+// stores: 268 MB (4096 tokens, top-6, hidden 4096) in 52 us, where a bare copy of the same pattern takes 48 to
 // 51.  Moving the pieces through shared memory with bulk copies measured 53 us there but 67 us (against 59)
-// for dispatch + combine of 2047 tokens.  Small ones are bound by the chain ids -> counts -> slots -> stores.
-template <typename T, bool FUSED, int THREADS>
-__global__ void __launch_bounds__(THREADS) moe_local_dispatch_kernel(const MoeLocalDispatchParams p) {
-  constexpr int kThreads = THREADS, kWarps = kThreads / 32;
+// for dispatch + combine of 2047 tokens.
+//
+// Small ones are bound by latency.  Index arithmetic and zeroing run before grid_dep_wait(), beside the previous
+// kernel; then all loads (ids of earlier and own entries, the first row piece, its weights) leave together, so that one
+// memory latency lies before the first store, and ranks come from one warp match.  With own ids, earlier ids and weights
+// asked for one after the other, and one warp ranking 32 entries at a time: 11 tokens, top-2 4.4 us in a graph, now 3.1;
+// 128 tokens, top-8, 256 experts 6.6, now 5.1; 101 tokens, top-4 4.2, now 3.3; 32 tokens, rows of 1 KiB 3.8, now 2.7.
+// Ranks worked out by every warp for itself cost 8.8 us at 128 tokens, clusters that share the counting 5.2 (pairs, and
+// nothing for plain copies) to 8.4 (eight CTAs), L2 prefetches before the wait changed nothing, and neither did
+// stores with an evict-first policy.
+template <typename T, bool FUSED>
+__global__ void __launch_bounds__(FUSED ? 512 : 1024, 1) moe_local_dispatch_kernel(const MoeLocalDispatchParams p) {
   constexpr int kLaneVecs = kPieceVecs / 32;
   static_assert(kLaneVecs == 2, "the copy loop is written for two vectors per lane");
   extern __shared__ __align__(128) uint8_t smem_local[];
   const int lane = threadIdx.x & 31;
+  const int threads = blockDim.x, warps = threads >> 5;
   const int k = p.k;
   const int P = p.pieces;
   ptx::grid_dep_launch();
-  ptx::grid_dep_wait();
-  stamp_cta0(p.trace_d, 0);
-  Share sh = share_of_cta(p);
+  const Share sh = share_of_cta(p, reinterpret_cast<int32_t*>(smem_local));
+  for (int i = threadIdx.x; i < (int)(sh.ids - sh.total); i += threads) sh.total[i] = 0;
+  if (threadIdx.x < 3) sh.ids[sh.m + threadIdx.x] = -2;
   const int nv = (int)(p.row_bytes >> 4);
   int item = sh.lo + (int)(threadIdx.x >> 5);
   int4 next[kLaneVecs];
+  float next_w = 0.f;
   auto load_piece = [&](int item) {
     const int t = item / P;
     const int v0 = (item - t * P) * p.piece_vecs;
@@ -242,10 +220,25 @@ __global__ void __launch_bounds__(THREADS) moe_local_dispatch_kernel(const MoeLo
 #pragma unroll
     for (int u = 0; u < kLaneVecs; ++u)
       if (v0 + lane + 32 * u < v1) next[u] = __ldcg(src + v0 + lane + 32 * u);
+    if (FUSED && lane < k) next_w = __ldcg(p.weights + (size_t)t * k + lane);
   };
+  __syncthreads();
+  ptx::grid_dep_wait();
+  stamp_cta0(p.trace_d, 0);
   if (p.vec && item < sh.hi) load_piece(item);
-
-  assign_rows<kThreads>(p, reinterpret_cast<int32_t*>(smem_local), sh);
+  count_entries<4>(p, sh);
+  __syncthreads();
+  stamp_cta0(p.trace_d, 1);
+  assign_rows(p, sh);
+  __syncthreads();
+  stamp_cta0(p.trace_d, 2);
+  if (blockIdx.x == gridDim.x - 1) {
+    for (int e = threadIdx.x; e < p.num_experts; e += threads)
+      p.expert_num_tokens[e] = min(sh.total[e], p.max_recv);
+  }
+  stamp_cta0(p.trace_d, 3);
+  stamp_cta0(p.trace_d, 4);
+  stamp_cta0(p.trace_d, 5);
   if (FUSED) {
     stamp_cta0(p.trace_c, 0);
     stamp_cta0(p.trace_c, 1);
@@ -253,17 +246,18 @@ __global__ void __launch_bounds__(THREADS) moe_local_dispatch_kernel(const MoeLo
   uint8_t* ex = reinterpret_cast<uint8_t*>(p.expert_x);
   if (p.vec) {
     constexpr int N = Vec16<T>::N;
-    for (; item < sh.hi; item += kWarps) {
+    for (; item < sh.hi; item += warps) {
       const int4 r0 = next[0], r1 = next[1];
-      if (item + kWarps < sh.hi) load_piece(item + kWarps);  // ahead of this piece's stores in the memory queue
+      const float w_lane = next_w;
+      if (item + warps < sh.hi) load_piece(item + warps);  // ahead of this piece's stores in the memory queue
       const int t = item / P;
-      const int v0 = (item - t * P) * p.piece_vecs;
+      const int piece = item - t * P;
+      const int v0 = piece * p.piece_vecs;
       const int v1 = min(nv, v0 + p.piece_vecs);
       const int32_t* rows = sh.rows + (t - sh.t0) * k;
+      if (piece == 0) write_metadata(p, sh, t, lane);
       float2 y[kLaneVecs][N / 2], acc[kLaneVecs][N / 2];
-      float w_lane = 0.f;
       if (FUSED) {
-        if (lane < k) w_lane = __ldcg(p.weights + (size_t)t * k + lane);
         expert_output<T>(r0, p.scale, y[0]);
         expert_output<T>(r1, p.scale, y[1]);
 #pragma unroll
@@ -294,20 +288,25 @@ __global__ void __launch_bounds__(THREADS) moe_local_dispatch_kernel(const MoeLo
   } else {
     // rows that are not whole aligned 16-byte vectors: element by element
     const int hidden = (int)(p.row_bytes / sizeof(T));
-    for (; item < sh.hi; item += kWarps) {  // P == 1: an item is a token
+    for (; item < sh.hi; item += warps) {  // P == 1: an item is a token
       const T* src = reinterpret_cast<const T*>(p.x) + (size_t)item * hidden;
       const int32_t* rows = sh.rows + (item - sh.t0) * k;
-      for (int h = lane; h < hidden; h += 32) {
-        const T v = src[h];
+      const float w_lane = FUSED && lane < k ? __ldcg(p.weights + (size_t)item * k + lane) : 0.f;
+      write_metadata(p, sh, item, lane);
+      for (int h0 = 0; h0 < hidden; h0 += 32) {  // same trip count for every lane: the shuffles need them all
+        const int h = h0 + lane;
+        const bool in = h < hidden;
+        const T v = in ? src[h] : from_f32<T>(0.f);
         float acc = 0.f;
         const float y = FUSED ? to_f32(from_f32<T>(to_f32(v) * p.scale)) : 0.f;
         for (int kk = 0; kk < k; ++kk) {
           const int row = rows[kk];
+          const float w = FUSED ? __shfl_sync(0xffffffffu, w_lane, kk) : 0.f;
           if (row < 0) continue;
-          reinterpret_cast<T*>(p.expert_x)[(size_t)row * hidden + h] = v;
-          if (FUSED) acc = fmaf(y, __ldcg(p.weights + (size_t)item * k + kk), acc);
+          if (in) reinterpret_cast<T*>(p.expert_x)[(size_t)row * hidden + h] = v;
+          if (FUSED) acc = fmaf(y, w, acc);
         }
-        if (FUSED) reinterpret_cast<T*>(p.out)[(size_t)item * hidden + h] = from_f32<T>(acc);
+        if (FUSED && in) reinterpret_cast<T*>(p.out)[(size_t)item * hidden + h] = from_f32<T>(acc);
       }
     }
   }
@@ -417,9 +416,8 @@ void cut_row(uint32_t row_bytes, bool vec, int most, int32_t* pieces, int32_t* p
 
 template <typename T>
 cudaError_t dispatch_typed(const MoeLocalDispatchParams& p, int threads, int grid, size_t smem, cudaStream_t stream) {
-  if (p.out == nullptr) return ptx::launch_dependent(moe_local_dispatch_kernel<T, false, 256>, grid, 256, smem, stream, p);
-  if (threads == 256) return ptx::launch_dependent(moe_local_dispatch_kernel<T, true, 256>, grid, 256, smem, stream, p);
-  return ptx::launch_dependent(moe_local_dispatch_kernel<T, true, 512>, grid, 512, smem, stream, p);
+  return p.out == nullptr ? ptx::launch_dependent(moe_local_dispatch_kernel<T, false>, grid, threads, smem, stream, p)
+                          : ptx::launch_dependent(moe_local_dispatch_kernel<T, true>, grid, threads, smem, stream, p);
 }
 
 template <typename T>
@@ -450,17 +448,24 @@ cudaError_t launch_moe_local_dispatch(MoeLocalDispatchParams p, int sms, cudaStr
           (reinterpret_cast<uintptr_t>(p.expert_x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
   cut_row(p.row_bytes, p.vec != 0, kPieceVecs, &p.pieces, &p.piece_vecs);
   const int64_t items = (int64_t)p.num_tokens * p.pieces;
-  // Plain copies keep the most stores in flight with four CTAs of eight warps per SM (2047 tokens to 16376 rows
-  // of 8 KiB: 59 us with combine, 71 with half the warps, 95 with a quarter).  Where the result is formed on the
-  // way, the fewer CTAs the less of the counting is repeated: 16 warps per SM (4096 tokens, top-6: 55 us; 57 to
-  // 62 with 32 warps), or eight when no warp gets more than two pieces (128 tokens: 6.6 us, 7.2 with 16 warps).
+  // 32 warps per SM keep the most stores in flight where rows are only copied (2047 tokens to 16376 rows of 8 KiB: 30 us,
+  // 44 with half the warps).  Every CTA counts for itself, so few large ones repeat less of that: it pays from some
+  // 6000 entries on (4000 tokens, top-2, rows of 1 KiB, with combine: 9.2 us with 2 x 16 warps, 10.0 with 4 x 8; 606 items
+  // 6.6 and 5.6).  Where the result is formed on the way there is one CTA per SM: 16 warps when each gets more than one
+  // piece (4096 tokens, top-6, rows of 8 KiB: 52 us; 58 to 60 with 32 warps), eight when that is two rounds or less
+  // (128 tokens, 12 pieces per SM: 5.1 us, 6.1 with 16 warps), ten in between (300 tokens, 16 pieces: 6.2, 6.9 and 6.8).
   const bool fused = p.out != nullptr;
-  const int threads = fused && items > 16 * (int64_t)sms ? 512 : 256;
+  const int64_t entries = (int64_t)p.num_tokens * p.k;
+  const int threads = fused ? (items > 20 * (int64_t)sms ? 512 : items > 14 * (int64_t)sms ? 320 : 256) : (entries > 6144 ? 512 : 256);
   const int warps = threads / 32;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((items + warps - 1) / warps, (int64_t)(fused ? 1 : 4) * sms));
-  p.cap = (int32_t)((items + grid - 1) / grid / p.pieces + 2) * p.k;
-  p.hist_copies = (p.num_tokens * p.k > 4096 && p.num_experts <= 1024) ? 4 : 1;
-  const size_t smem = ((size_t)p.hist_copies * p.num_experts + 2 * (size_t)p.cap) * sizeof(int32_t);
+  const int ctas = fused ? sms : (32 / warps) * sms;
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((items + warps - 1) / warps, ctas));
+  // The later a CTA's tokens, the longer it counts before its first store.  Where counting is short against the stores, a
+  // tenth evens that out (4096 tokens, top-6, rows of 8 KiB: 54.5 -> 52.2 us; 1000, top-4, 4 KiB: 6.0 -> 5.9), where it is
+  // not, two tenths (4096 tokens, top-8, rows of 1 KiB: 13.4 us, with a tenth 12.8, with two 12.2).
+  p.lean = !fused || threads < 512 ? 0.f : entries > 16384 && p.row_bytes <= 2048 ? 0.2f : 0.1f;
+  p.cap = ((int32_t)((int64_t)((1.0 + p.lean) * items / grid + 16) / p.pieces + 2) * p.k + 6) & ~3;  // (and three words, in groups of four)
+  const size_t smem = ((size_t)((p.num_experts + 3) & ~3) + 2 * (size_t)p.cap) * sizeof(int32_t);
   if (smem > 48 * 1024) return cudaErrorInvalidValue;
   switch (p.dtype) {
     case 0: return dispatch_typed<__half>(p, threads, grid, smem, stream);

@@ -126,6 +126,61 @@ def test_moe_one_rank_kernels_at_the_edges_of_their_ranges(E, k, H, T, M, dtype)
     layer.close()
 
 
+@pytest.mark.parametrize(
+    "E,k,H,T,dtype",
+    [
+        (31, 3, 4096, 259, torch.bfloat16),  # forward: 14 pieces per SM, eight warps ...
+        (31, 3, 4096, 260, torch.bfloat16),  # ... one piece more, ten
+        (40, 5, 4096, 370, torch.bfloat16),  # 20 pieces per SM, ten warps ...
+        (40, 5, 4096, 371, torch.bfloat16),  # ... one more, sixteen, and shorter runs for later CTAs
+        (7, 6, 256, 1024, torch.float16),  # plain dispatch: the most entries that eight warps per CTA take ...
+        (7, 6, 256, 1025, torch.float16),  # ... and sixteen; more own entries than one warp ranks at a time
+        (130, 5, 1030, 3301, torch.bfloat16),  # rows that are no whole vectors, 16505 entries, own ones not a multiple of 4
+        (3, 15, 512, 2184, torch.float32),  # experts that appear several times in a token, nearly 32768 entries
+    ],
+)
+def test_moe_one_rank_shares_of_the_ctas(E, k, H, T, dtype):
+    """Where the launcher deals the work out differently, with ids on any address: rows, metadata and counts exactly."""
+    from amd_distributed_2025_b200.models import moe_all2all
+
+    cfg = contract.MoEConfig(E, k, H, T * (k if k > E else 1), dtype, dtype)
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, H, device="cuda", generator=gen).to(dtype)
+    w = torch.rand(T, k, device="cuda", generator=gen)
+    if k > E:
+        ids = torch.randint(0, E, (T, k), device="cuda", generator=gen)
+    else:
+        ids = torch.rand(T, E, device="cuda", generator=gen).pow(3).argsort(1)[:, :k]
+    layer = moe_all2all.MoEAllToAll(cfg, 0, 1, mode="dedup")
+    for shift in (0, 1):  # (ids on a 16-byte boundary, and off it)
+        idx = torch.empty(T * k + 4, dtype=torch.int32, device="cuda")[shift : shift + T * k].view(T, k).copy_(ids)
+        y = layer.forward(x, idx, w, 2.0)
+        layer.check()
+        assert oracle.relative_error(y, (x * 2.0).double() * w.double().sum(1, keepdim=True)) < 5e-3
+        for fused in (True, False):
+            if not fused:
+                layer.expert_x.zero_()
+                layer.expert_meta.zero_()
+                layer.dispatch(x, idx)
+            counts, ex, meta = layer.expert_num_tokens, layer.expert_x, layer.expert_meta
+            flat = ids.flatten()
+            order = torch.sort(flat, stable=True).indices
+            assert torch.equal(counts.long(), torch.bincount(flat, minlength=E))
+            slot = torch.arange(T * k, device="cuda") - (torch.cumsum(counts.long(), 0) - counts.long())[flat[order]]
+            assert torch.equal(ex[flat[order], slot], x[order // k])
+            want = torch.stack([flat[order], 0 * order, order // k, order % k, 0 * order], dim=1)
+            assert torch.equal(meta[flat[order], slot].long(), want)
+    bad = idx.clone()
+    bad[T - 2, k - 1] = E  # known to the last CTAs only as one of their own
+    y = layer.forward(x, bad, w, 1.0)
+    with pytest.raises(Exception, match="bad_index"):
+        layer.check()
+    keep = torch.arange(T, device="cuda") != T - 2
+    assert oracle.relative_error(y[keep], (x.double() * w.double().sum(1, keepdim=True))[keep]) < 5e-3
+    layer.ws.reset_status()
+    layer.close()
+
+
 def test_moe_dedup_fp32_partial_rows_and_phase_stamps():
     from amd_distributed_2025_b200.models import moe_all2all
 
