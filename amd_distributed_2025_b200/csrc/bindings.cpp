@@ -1526,6 +1526,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     const b200::SmShare s = b200::gemm_rs_share(block_n, cta_pair);
     return py::make_tuple(s.smem, s.tmem_cols);
   });
+  m.def("fp8_gemm_plan", [](int M, int N, int K, int sms) {
+    const b200::Fp8GemmPlan p = b200::fp8_gemm_plan(M, N, K, sms);
+    return py::make_tuple(p.bn, p.splits);
+  });
   m.def("fp8_gemm_share", [](int bn, int splits) { return py::make_tuple(b200::fp8_gemm_smem(bn, splits), 512); });
   m.def("gemm_local_plan", [](int M, int N, int K, int sms) {  // one rank
     TORCH_CHECK(M > 0 && N > 0 && K > 0, "sizes must be positive");

@@ -24,6 +24,12 @@ struct Fp8GemmArgs {
 // Shared memory of a CTA (it takes all of the tensor memory).
 int fp8_gemm_smem(int bn, int splits);
 
+// The tile width and the pairs that share a tile's K, as planned for a problem (for tests).
+struct Fp8GemmPlan {
+  int bn, splits;
+};
+Fp8GemmPlan fp8_gemm_plan(int M, int N, int K, int sms);
+
 cudaError_t launch_fp8_gemm(const Fp8GemmArgs& args, cudaStream_t stream);
 
 // Self-test of the bounded wait: one warp waits for a barrier that nothing signals and leaves its record.

@@ -25,6 +25,12 @@ __device__ __forceinline__ bool elect_one() {
   return one != 0;
 }
 
+// A warpgroup gives registers up, or takes some that others gave up (all of its warps, once; waits until there are enough).
+template <int REGS>
+__device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS)); }
+template <int REGS>
+__device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS)); }
+
 // ---- mbarrier -------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -230,6 +236,29 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, uint32_t cta) 
       "mapa.shared::cluster.u32 remote, %0, %1;\n\t"
       "mbarrier.arrive.shared::cluster.b64 _, [remote];\n\t}"
       ::"r"(bar), "r"(cta)
+      : "memory");
+}
+// The same place in CTA `cta`, as an address for the whole cluster.
+__device__ __forceinline__ uint32_t map_cluster(uint32_t smem_addr, uint32_t cta) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(cta));
+  return r;
+}
+// Arrivals of one lane without a branch: the warp stays converged.
+__device__ __forceinline__ void mbar_arrive_if(bool arrives, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.u32 p, %0, 0;\n\t"
+      "@p mbarrier.arrive.shared::cta.b64 _, [%1];\n\t}"
+      ::"r"((uint32_t)arrives), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_remote_if(bool arrives, uint32_t cluster_bar) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.u32 p, %0, 0;\n\t"
+      "@p mbarrier.arrive.shared::cluster.b64 _, [%1];\n\t}"
+      ::"r"((uint32_t)arrives), "r"(cluster_bar)
       : "memory");
 }
 // 16 bytes to the same shared-memory offset of CTA `cta` of the cluster.

@@ -182,6 +182,7 @@ def test_ctas_that_fit_on_an_sm_by_shared_memory_fit_by_tensor_memory():
     shares += [ext.gemm_pair_share(bn, 1) for bn in range(32, 257, 32)] + [ext.gemm_pair_share(256, 2)]
     shares += [ext.gemm_rs_share(bn, pair) for bn, pair in ((64, False), (128, False), (256, False), (128, True), (192, True), (256, True))]
     shares += [ext.fp8_gemm_share(bn, splits) for bn in (64, 128) for splits in range(1, 9)]
+    shares += [ext.fp8_gemm_share(bn, 1) for bn in (192, 256)]
     sm, reserved = 228 * 1024, 1024  # of an SM in all, and what each resident CTA takes on top of its own
     least = {}  # columns -> the smallest shared memory that comes with them
     for smem, cols in shares:
