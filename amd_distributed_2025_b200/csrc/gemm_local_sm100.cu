@@ -17,8 +17,11 @@
 //                      1100 with 256 columns, and 4.5 % less time).
 //
 // Multi-rank kernel before -> these kernels, one rank, us in a row of calls: 64 x 2880 x 360 10.2 -> 4.6 (latency: a launch
-// and its call), 64 x 7168 x 18432 71 -> 49 (memory, 5.9 TB/s while cool), 256 x 5120 x 12800 58 -> 41 (34 while cool:
-// memory, then the meeting of the parts), 2048 x 2880 x 2880 45 -> 34 (120 tiles on 74 pairs), 8192 x 8192 x 28672 3135 -> 2792 (power).
+// and its call), 64 x 7168 x 18432 71 -> 47 (memory, 5.9 TB/s while cool), 256 x 5120 x 12800 58 -> 38 (memory, then the
+// meeting of the parts), 2048 x 2880 x 2880 45 -> 31 (144 tiles on 74 pairs, power), 8192 x 8192 x 28672 3135 -> 2675
+// (power).  Widths are multiples of 32 columns; with multiples of 64 only, 256 x 5120 x 12800 was three parts of 256 columns
+// on 120 CTAs (40 us; two parts of 160 on 128 are less to exchange), 2048 x 2880 x 2880 120 tiles of 192 (33.5 us).
+// Tried and level: as many pipeline stages as a part has k-blocks, which lets two launches share an SM.
 //
 // Warp roles of both (320 threads): 0 TMA producer, 1 MMA issuer, 2..9 epilogue, two per tensor-memory lane quarter.
 // Shared memory keeps CTAs of the pair kernel, which take all of the tensor memory, alone on their SM.  Small tiles of
@@ -67,6 +70,7 @@ struct LocalParams {
   int splits;         // tile kernel: CTAs (or pairs) of a cluster that share a tile
   int part_bytes;     // tile kernel: shared memory of its own for their parts (0: they take the pipeline's)
   int tmem_cols;      // tile kernel: tensor-memory columns of its one accumulator
+  int group;          // chunks of 32 columns that leave together: 2, or 1 (swapped, or `bn` is an odd number of chunks)
   int stage_area;     // tile kernel: bytes of the pipeline's stages, and of the parts where these share them
   int sk_tiles, total_tiles;  // pair kernel
   int halves;         // pair kernel: 2 = a tile is twice `bn` columns, one accumulator for each half
@@ -165,28 +169,28 @@ __device__ __forceinline__ float bias_of_word(const LocalParams& p, const uint32
   return p.bias_mode == 2 ? b * p.bias_scale : b;
 }
 
-// One column group of a warp's 32 rows -- 64 columns, or 32 when swapped -- from fp32 to the result: bias, rounding,
+// One column group of a warp's 32 rows -- p.group chunks of 32 columns -- from fp32 to the result: bias, rounding,
 // through the warp's slab, out by TMA (which clips what lies outside the result).  chunk(c, v) gives 32 columns.
 template <bool SWAP, typename F>
 __device__ __forceinline__ void emit_group(const LocalParams& p, const CUtensorMap* map_out, Emit& em, int g, int prow, int qrow,
                                            float lane_bias, int lane, F&& chunk) {
-  constexpr int kGroupChunks = SWAP ? 1 : 2;
-  const uint32_t buf = SWAP ? em.slab + (em.stores & 1u) * (kSlabBytes / 2) : em.slab;
+  const int group = SWAP ? 1 : p.group;
+  const uint32_t buf = group == 1 ? em.slab + (em.stores & 1u) * (kSlabBytes / 2) : em.slab;
   ++em.stores;
   if (!SWAP && p.bias_mode != 0) {
-    const int n = qrow + g * 64 + 2 * lane;  // N is a multiple of 8: both values or none
+    const int n = qrow + g * group * 32 + 2 * lane;  // N is a multiple of 8: both values or none
     const uint32_t two = n < p.Q ? *reinterpret_cast<const uint32_t*>(p.bias + n) : 0u;
     asm volatile("st.shared.b32 [%0], %1;" ::"r"(em.bias + (uint32_t)lane * 4u), "r"(two) : "memory");
   }
   if (lane == 0) {  // the store that used this buffer has read it
-    if (SWAP) ptx::bulk_wait_group_read<1>();
+    if (group == 1) ptx::bulk_wait_group_read<1>();
     else ptx::bulk_wait_group_read<0>();
   }
   __syncwarp();
 #pragma unroll 1
-  for (int cc = 0; cc < kGroupChunks; ++cc) {
+  for (int cc = 0; cc < group; ++cc) {
     float v[32];
-    chunk(g * kGroupChunks + cc, v);
+    chunk(g * group + cc, v);
     if (SWAP) {
       // lane = feature, v[j] = token j of the chunk.  Two lanes exchange values so that each writes the feature
       // pair of one of two tokens: rows of 64 bytes, 16 words per token, no bank conflict.
@@ -216,8 +220,9 @@ __device__ __forceinline__ void emit_group(const LocalParams& p, const CUtensorM
         }
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {  // 16-byte piece cc * 4 + j of row `lane`, at the place the 128-byte swizzle wants it
-        const uint32_t at = buf + (uint32_t)lane * 128u + (uint32_t)(((cc * 4 + j) ^ (lane & 7)) << 4);
+      for (int j = 0; j < 4; ++j) {  // 16-byte piece cc * 4 + j of row `lane`, at the place the 128 (64)-byte swizzle wants it
+        const uint32_t at = group == 2 ? buf + (uint32_t)lane * 128u + (uint32_t)(((cc * 4 + j) ^ (lane & 7)) << 4)
+                                       : buf + (uint32_t)lane * 64u + (uint32_t)((j ^ ((lane >> 1) & 3)) << 4);
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(pack2(v[8 * j], v[8 * j + 1])),
                      "r"(pack2(v[8 * j + 2], v[8 * j + 3])), "r"(pack2(v[8 * j + 4], v[8 * j + 5])),
                      "r"(pack2(v[8 * j + 6], v[8 * j + 7]))
@@ -228,7 +233,7 @@ __device__ __forceinline__ void emit_group(const LocalParams& p, const CUtensorM
   ptx::fence_proxy_async_smem();
   __syncwarp();
   if (lane == 0) {
-    const int x = SWAP ? prow : qrow + g * 64;
+    const int x = SWAP ? prow : qrow + g * group * 32;
     const int y = SWAP ? qrow + g * 32 : prow;
     if (x < (SWAP ? p.P : p.Q) && y < (SWAP ? p.Q : p.P)) ptx::tma_store_2d(map_out, buf, x, y);
     ptx::bulk_commit_group();
@@ -429,8 +434,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
     const int q = warp & 3;       // tensor-memory lane quarter this warp may read
     const int half = ew >> 2;
     const int chunks = p.bn / 32;
-    // column groups: 2 chunks of 32 (normal), 1 (swapped); this warp takes every second one
-    constexpr int kGroupChunks = SWAP ? 1 : 2;
+    const int group = SWAP ? 1 : p.group;  // this warp takes every second group of so many chunks
     Emit em{slabs + (uint32_t)ew * kSlabBytes, bias_smem + (uint32_t)ew * 128u};
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     const size_t part_vecs = (size_t)chunks * 8 * kPRows;  // float4s of one CTA's half of a tile
@@ -469,7 +473,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
         // be there at once.
         float4* dst = part + (seg.kb0 > 0 ? 0 : (size_t)p.far_part);
         for (int c = 0; c < chunks; ++c) {
-          if (((c / kGroupChunks) & 1) != half) continue;
+          if (((group == 1 ? c : c / 2) & 1) != half) continue;
           float v[32];
           load_chunk(acc_addr + c * 32, v);
 #pragma unroll
@@ -500,9 +504,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
 #pragma unroll
         for (int j = 0; j < 8; ++j) ahead[j] = __ldcg(theirs + (size_t)(c * 8 + j) * kPRows);
       };
-      if (cut && half * kGroupChunks < chunks) ask(half * kGroupChunks);
+      if (cut && half * group < chunks) ask(half * group);
 #pragma unroll 1
-      for (int g = half; g * kGroupChunks < chunks; g += 2) {
+      for (int g = half; g * group < chunks; g += 2) {
         emit_group<SWAP>(p, &map_out, em, g, prow, qrow, lane_bias, lane, [&](int c, float (&v)[32]) {
           if (own_in_tmem) {
             load_chunk(acc_addr + c * 32, v);
@@ -518,7 +522,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
               v[4 * j + 2] += ahead[j].z;
               v[4 * j + 3] += ahead[j].w;
             }
-            const int next = (c + 1) / kGroupChunks == g ? c + 1 : (g + 2) * kGroupChunks;
+            const int next = group == 2 && c == 2 * g ? c + 1 : (g + 2) * group;
             if (next < chunks) ask(next);
           }
         });
@@ -684,7 +688,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
     ptx::tcgen05_fence_after();
     if (splits == 1 && alive && q * 32 < p.rows) {  // not split: whole groups of 32 rows
       Emit em{slabs + (uint32_t)ew * kSlabBytes, bias_smem + (uint32_t)ew * 128u};
-      for (int g = half; g * (SWAP ? 1 : 2) < p.bn / 32; g += 2)
+      for (int g = half; g * (SWAP ? 1 : p.group) < p.bn / 32; g += 2)
         emit_group<SWAP>(p, &map_out, em, g, prow, q0, lane_bias, lane,
                          [&](int c, float (&v)[32]) { load_chunk(lane_addr + c * 32, v); });
       if (lane == 0) ptx::bulk_wait_group_read<0>();
@@ -840,17 +844,19 @@ int grid_ctas(const Plan& p) { return p.persistent ? 2 * p.pairs : p.p_tiles * p
 
 // Time model in ns.  What it charges persistent pairs, measured on a B200:
 //   a 128-byte row of a k-block takes an SM 1 ns to bring in, 1.6 when the rows of the matrix do not start on cache lines;
-//   128 x 256 x 64 takes a tensor core 280 ns, all tensor cores together do 1.55 PFLOP/s (the power limit); a k-block
-//   costs its issuing warp 150 ns; 6.6 TB/s of HBM; then what a launch costs before and after its k-blocks.
+//   128 x 256 x 64 takes a tensor core 280 ns, all tensor cores together do 1.45 PFLOP/s in a row of calls (the power
+//   limit; 1.55 where a launch comes alone); a k-block costs its issuing warp 150 ns; 6.6 TB/s of HBM; then what a launch
+//   costs before and after its k-blocks.
 // The tile kernel's terms are fitted (below).
 Plan make_local_plan(int M, int N, int K, int sms) {
   const int num_kb = (K + kBK - 1) / kBK;
-  const double dram_ns = 2.0 * ((double)M * K + (double)N * K + (double)M * N) / 6600.0;
+  const double operand_bytes = 2.0 * ((double)M * K + (double)N * K);
+  const double dram_ns = (operand_bytes + 2.0 * M * N) / 6600.0;
   const double row_ns = K % kBK == 0 ? 1.0 : 1.6;
   // ... and the narrower the tile, the more of the power goes into moving operands: `rows_per_col` is what a CTA brings
   // in per k-block, relative to a pair's 256 rows for 256 columns
-  auto power_ns = [&](double rows, double cols, double rows_per_col) {
-    return 2.0 * rows * cols * num_kb * kBK / 1.55e6 * (1.0 + 0.26 * (rows_per_col - 1.0));
+  auto power_ns = [&](double rows, double cols, double rows_per_col, double pflops) {
+    return 2.0 * rows * cols * num_kb * kBK / (pflops * 1e6) * (1.0 + 0.26 * (rows_per_col - 1.0));
   };
   Plan best;
   auto keep = [&](const Plan& p) {
@@ -888,7 +894,7 @@ Plan make_local_plan(int M, int N, int K, int sms) {
       // also waits for its turn in the SM.
       const double kb_ns = std::max({(K % kBK == 0 ? 0.55 : 1.15) * (p.rows + q_rows), 246.0 * bn / 256.0, 140.0, 1200.0 / stages});
       const double limits[3] = {waves * kbs * kb_ns, dram_ns * 0.825,
-                                power_ns((double)p.p_tiles * halves * 128, (double)p.q_tiles * bn, (128.0 + q_rows) / bn)};
+                                power_ns((double)p.p_tiles * halves * 128, (double)p.q_tiles * bn, (128.0 + q_rows) / bn, 1.55)};
       double cubes = 0.0;
       for (double t : limits) cubes += t * t * t;
       const double ends_ns = (s == 1 ? 2580.0 + 6.6 * bn : 3980.0 + 30.0 * std::max(bn - 64, 0) + 70.0 * s) + (pair ? 220.0 : 0.0);
@@ -908,27 +914,31 @@ Plan make_local_plan(int M, int N, int K, int sms) {
     const int64_t tiles = (int64_t)p.p_tiles * p.q_tiles;
     p.pairs = (int)std::min<int64_t>(tiles, std::min(sms / 2, kGemmLocalMaxPairs));
     if (halves == 1 && tiles == p.pairs) return;  // one wave: the tile kernel's pairs do the same 8 % faster
-    const double power = power_ns(p.p_tiles * 256.0, (double)p.q_tiles * cols, (128.0 + cols / 2) / cols);
-    const double kb_ns = std::max({row_ns * (128 + cols / 2), 280.0 * cols / 256.0, 150.0});
-    const double waves = std::ceil((double)tiles / p.pairs);
+    // A wave takes as long as one of its tiles, or as the power for all of them: a last wave of few tiles has power to
+    // spare, and its tiles still take their time (2048 x 5120 x 12800: 231 us in 2.2 waves of 256 columns, 214 in 2.9 of 192).
+    const double wave_ns = power_ns(256.0 * p.pairs, cols, (128.0 + cols / 2) / cols, 1.45);
+    const double tile_ns = num_kb * std::max({row_ns * (128 + cols / 2), 280.0 * cols / 256.0, 150.0});
+    const int64_t whole = tiles / p.pairs, last = tiles % p.pairs;
+    const int64_t waves = whole + (last > 0 ? 1 : 0);
     p.sk_tiles = 0;
-    p.ns = std::max({waves * num_kb * kb_ns, power, dram_ns}) + 3400.0 + 9.0 * cols;
-    // With both accumulators in one tile, 5.5 us of its epilogue do not run beside products (all pairs store at once), and
-    // the long tiles of a last wave that is not full cost more than the power its idle pairs leave to the others:
-    // 4096 x 8192 x 14336, 3.5 waves, takes 647 us this way and 620 us with 256 columns.
-    if (halves == 2) p.ns = std::max(waves * num_kb * kb_ns, power * waves * p.pairs / tiles) + waves * 5500.0 + 3400.0 + 9.0 * cols;
+    p.ns = std::max(whole * std::max(tile_ns, wave_ns) + (last > 0 ? std::max(tile_ns, wave_ns * last / p.pairs) : 0.0), dram_ns) + 3400.0 +
+           9.0 * cols;
+    // With both accumulators in one tile, 5.5 us of its epilogue do not run beside products (all pairs store at once).
+    if (halves == 2) p.ns += waves * 5500.0;
     keep(p);
-    if (halves == 1 && tiles > p.pairs && tiles % p.pairs != 0) {
-      p.sk_tiles = (int)(tiles % p.pairs) + p.pairs;
+    if (halves == 1 && whole > 0 && last != 0) {
+      p.sk_tiles = (int)last + p.pairs;
       // The parts of the cut tiles go through memory: 5 us in all, and time by how many pairs' work is cut up.  (With 2.5 us
       // 2348 x 2144 x 1504 was cut and took 21.4 us where whole tiles of 192 columns take 16.5; of 240 drawn sizes, the 24
-      // that are still cut gain 7 % on whole tiles.)
-      const double cut = (double)(tiles % p.pairs) / p.pairs;
-      p.ns = std::max({(double)tiles / p.pairs * num_kb * kb_ns * (1.05 + 0.3 * cut), power, dram_ns}) + 3400.0 + 9.0 * bn + 5000.0;
+      // that are still cut gain 7 % on whole tiles.)  Pairs at work on different parts of K share no operands: what L2 does
+      // not hold comes from memory for every tile (1923 x 5056 x 19824: 429 us cut, 335 in whole tiles of 192 columns).
+      const double cut = (double)last / p.pairs;
+      const double apart_ns = operand_bytes > 126e6 ? 0.4 * p.sk_tiles * num_kb * (256.0 + cols) * kBK * 2 / 6600.0 : 0.0;
+      p.ns = std::max((double)tiles / p.pairs * std::max(tile_ns, wave_ns) * (1.05 + 0.3 * cut), dram_ns) + apart_ns + 3400.0 + 9.0 * bn + 5000.0;
       keep(p);
     }
   };
-  for (int bn : {64, 128, 192, 256}) {
+  for (int bn = 64; bn <= 256; bn += 32) {
     for (bool pair : {false, true}) consider_tile(false, pair, bn);
     consider_pair(false, bn, 1);
   }
@@ -974,6 +984,7 @@ bool common_params(LocalParams& p, const GemmLocalArgs& a, const Plan& plan, int
   p.q_tiles = plan.q_tiles;
   p.band = std::min(8, plan.p_tiles);
   p.bn = plan.bn;
+  p.group = swap || plan.bn % 64 != 0 ? 1 : 2;
   p.rows = plan.rows;
   p.splits = plan.splits;
   p.timeout_ns = a.timeout_ns;
@@ -983,7 +994,7 @@ bool common_params(LocalParams& p, const GemmLocalArgs& a, const Plan& plan, int
   p.trace = grid_ctas(plan) <= a.trace_ctas ? a.trace : nullptr;
   return make_tensor_map(map_p, swap ? a.w : a.a, (uint64_t)p.P, (uint64_t)a.K, 2, (uint32_t)p_rows, kBK, 128) &&
          make_tensor_map(map_q, swap ? a.a : a.w, (uint64_t)p.Q, (uint64_t)a.K, 2, (uint32_t)q_rows, kBK, 128) &&
-         make_tensor_map(map_out, a.out, (uint64_t)a.M, (uint64_t)a.N, 2, 32, swap ? 32 : 64, swap ? 0 : 128);
+         make_tensor_map(map_out, a.out, (uint64_t)a.M, (uint64_t)a.N, 2, 32, (uint32_t)p.group * 32, swap ? 0 : p.group * 64);
 }
 
 template <typename K>

@@ -350,6 +350,42 @@ def test_gemm_one_rank_reaches_every_path(kind, m, n, k):
         pytest.skip("right, but planned here as: " + " ".join(got))
 
 
+@pytest.mark.parametrize(
+    "kind,m,n,k",
+    [
+        ("tile normal single", 206, 4792, 64),  # one k-block; the last column tile holds 88 of 96 columns
+        ("tile normal single shared own", 384, 1040, 1736),
+        ("tile normal single shared pipeline", 362, 744, 3472),
+        ("tile normal pair", 242, 4760, 264),
+        ("tile normal pair shared own", 396, 1040, 2088),
+        ("tile normal pair shared pipeline", 646, 1104, 2952),  # three parts of 160 columns: 56, 56 and 48 to finish
+        ("pair normal", 7639, 520, 72),
+        ("pair normal", 2048, 2880, 2880),  # 160 columns: five chunks, three for one half of the warps
+        ("pair normal cut", 6345, 656, 1888),  # 224 columns, left in the workspace chunk by chunk
+    ],
+)
+def test_gemm_one_rank_widths_of_an_odd_number_of_chunks(kind, m, n, k):
+    """Tiles of 96, 160 and 224 columns, whose groups leave chunk by chunk."""
+    plan = _ext().gemm_local_plan(m, n, k, torch.cuda.get_device_properties(0).multi_processor_count)
+    test_gemm_one_rank_reaches_every_path(kind, m, n, k)
+    if plan["bn"] % 64 == 0:
+        pytest.skip(f"right, but planned here with {plan['bn']} columns")
+
+
+@pytest.mark.parametrize(
+    "kind,m,n,k",
+    [
+        ("tile normal single", 134, 1040, 256),
+        ("tile normal single shared pipeline", 1088, 608, 2600),
+        ("tile normal pair shared own", 389, 768, 848),
+        ("pair normal", 5477, 712, 256),
+    ],
+)
+def test_gemm_one_rank_reaches_the_widths_of_whole_groups(kind, m, n, k):
+    """The same paths at multiples of 64 columns."""
+    test_gemm_one_rank_reaches_every_path(kind, m, n, k)
+
+
 @pytest.mark.parametrize("m,n,k,has_bias", [(64, 2880, 360, True), (512, 4096, 1536, True), (2048, 2880, 360, True)])
 def test_gemm_world1_reference_inputs_pass_reference_checker(m, n, k, has_bias):
     """Operands from the reference generator (uniform +-0.01) against the library path."""
