@@ -314,12 +314,15 @@ __global__ void __launch_bounds__(FUSED ? 512 : 1024, 1) moe_local_dispatch_kern
 }
 
 // out[t] = sum over k (ascending) of w[t, k] * expert_y[row(t, k)], fp32, rounded once; a token none of whose
-// entries was delivered gets a zero row.  One warp per (token, piece of the row).  Eight 16-byte loads per
-// lane are in flight whatever k is: KB rows of 8 / KB vectors each.  Bound by the gather of k rows.
+// entries was delivered gets a zero row.  One warp per (token, piece of the row), 1 KiB of KB rows at a
+// time: KB is k, or k in equal rounds of at most four.  Bound by the gather of k rows.  What counts is that a request is
+// 1 KiB of a row and that no round is partly idle, not how many loads a lane has in flight: eight whatever k is, as
+// 512 bytes of eight rows or 2 KiB of two, took (combine alone, us) 12.1 at 600 tokens, top-8, rows of 8 KiB, now 10.4;
+// 11.3 at 1500, top-6, 4 KiB, now 10.1; 4.3 at 4000, top-2, 1 KiB, now 3.3; 7.4 at 1000, top-3, 8 KiB, now 6.8.
 template <typename T, int KB>
 __global__ void __launch_bounds__(256) moe_local_combine_kernel(const MoeLocalCombineParams p) {
   constexpr int N = Vec16<T>::N;
-  constexpr int U = 8 / KB;
+  constexpr int U = 2;
   const int lane = threadIdx.x & 31;
   const int k = p.k;
   const int P = p.pieces;
@@ -422,9 +425,13 @@ cudaError_t dispatch_typed(const MoeLocalDispatchParams& p, int threads, int gri
 
 template <typename T>
 cudaError_t combine_typed(const MoeLocalCombineParams& p, int grid, cudaStream_t stream) {
-  if (p.k <= 2) return ptx::launch_dependent(moe_local_combine_kernel<T, 2>, grid, 256, 0, stream, p);
-  if (p.k <= 4) return ptx::launch_dependent(moe_local_combine_kernel<T, 4>, grid, 256, 0, stream, p);
-  return ptx::launch_dependent(moe_local_combine_kernel<T, 8>, grid, 256, 0, stream, p);
+  const int rounds = (p.k + 3) / 4;
+  switch ((p.k + rounds - 1) / rounds) {
+    case 1: return ptx::launch_dependent(moe_local_combine_kernel<T, 1>, grid, 256, 0, stream, p);
+    case 2: return ptx::launch_dependent(moe_local_combine_kernel<T, 2>, grid, 256, 0, stream, p);
+    case 3: return ptx::launch_dependent(moe_local_combine_kernel<T, 3>, grid, 256, 0, stream, p);
+    default: return ptx::launch_dependent(moe_local_combine_kernel<T, 4>, grid, 256, 0, stream, p);
+  }
 }
 
 }  // namespace

@@ -181,6 +181,35 @@ def test_moe_one_rank_shares_of_the_ctas(E, k, H, T, dtype):
     layer.close()
 
 
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 7, 8, 9, 13, 15])
+@pytest.mark.parametrize("H,dtype", [(520, torch.bfloat16), (1000, torch.float32), (130, torch.float16)])
+def test_moe_one_rank_combine_rounds(k, H, dtype):
+    """Every number of rows that combine gathers at a time, and what is left of the last round; pieces that end short, and
+    rows that are no whole vectors.  fp32 sums of k products, rounded once."""
+    from amd_distributed_2025_b200.models import moe_all2all
+
+    T, E = 67, 16
+    cfg = contract.MoEConfig(E, k, H, T, dtype, dtype)
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    x = torch.randn(T, H, device="cuda", generator=gen).to(dtype)
+    w = torch.rand(T, k, device="cuda", generator=gen)
+    ids = torch.rand(T, E, device="cuda", generator=gen).argsort(1)[:, :k].int().contiguous()
+    layer = moe_all2all.MoEAllToAll(cfg, 0, 1, mode="dedup")
+    counts, ex, meta = layer.dispatch(x, ids)
+    ey = torch.randn(ex.shape, device="cuda", generator=gen).to(dtype)
+    out = layer.combine(torch.empty(T, H, dtype=dtype, device="cuda"), w, meta, ey, counts, T)
+    rows = torch.empty(T * k, H, dtype=torch.float64, device="cuda")
+    m = meta.long()
+    for e in range(E):
+        n = int(counts[e])
+        rows[m[e, :n, 2] * k + m[e, :n, 3]] = ey[e, :n].double()
+    want = (rows.view(T, k, H) * w.double()[:, :, None]).sum(1)
+    layer.check()
+    eps = {torch.bfloat16: 2.0**-8, torch.float16: 2.0**-11, torch.float32: 2.0**-23 * (k + 1)}[dtype]
+    assert oracle.relative_error(out, want) < eps
+    layer.close()
+
+
 def test_moe_dedup_fp32_partial_rows_and_phase_stamps():
     from amd_distributed_2025_b200.models import moe_all2all
 
