@@ -424,8 +424,8 @@ cudaError_t dispatch_typed(const MoeLocalDispatchParams& p, int threads, int gri
 }
 
 template <typename T>
-cudaError_t combine_typed(const MoeLocalCombineParams& p, int grid, cudaStream_t stream) {
-  const int rounds = (p.k + 3) / 4;
+cudaError_t combine_typed(const MoeLocalCombineParams& p, int grid, int most, cudaStream_t stream) {
+  const int rounds = (p.k + most - 1) / most;
   switch ((p.k + rounds - 1) / rounds) {
     case 1: return ptx::launch_dependent(moe_local_combine_kernel<T, 1>, grid, 256, 0, stream, p);
     case 2: return ptx::launch_dependent(moe_local_combine_kernel<T, 2>, grid, 256, 0, stream, p);
@@ -493,12 +493,15 @@ cudaError_t launch_moe_local_combine(MoeLocalCombineParams p, int sms, cudaStrea
   const int64_t row_vecs = p.row_bytes >> 4;
   const bool plenty = p.num_tokens * row_vecs >= 2 * kPieceVecs * 32 * (int64_t)sms;
   cut_row(p.row_bytes, p.vec != 0, plenty ? 2 * kPieceVecs : kPieceVecs, &p.pieces, &p.piece_vecs);
+  // Four rows at a time, three where every warp stays busy: 2047 tokens, top-8, rows of 8 KiB 26.4 us against 27.1; 4000,
+  // top-7, 4 KiB 24.1 and 24.4, top-4, 8 KiB (then two) 28.8 and 30.0; 600 tokens, top-8, 8 KiB 11.5 against 10.4.
+  const int most = plenty ? 3 : 4;
   const int64_t warps = (int64_t)p.num_tokens * p.pieces;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((warps + 7) / 8, 4 * (int64_t)sms));
   switch (p.dtype) {
-    case 0: return combine_typed<__half>(p, grid, stream);
-    case 1: return combine_typed<__nv_bfloat16>(p, grid, stream);
-    case 2: return combine_typed<float>(p, grid, stream);
+    case 0: return combine_typed<__half>(p, grid, most, stream);
+    case 1: return combine_typed<__nv_bfloat16>(p, grid, most, stream);
+    case 2: return combine_typed<float>(p, grid, most, stream);
     default: return cudaErrorInvalidValue;
   }
 }
