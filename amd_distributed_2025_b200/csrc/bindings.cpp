@@ -7,6 +7,8 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <pybind11/stl.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
 
 #include <atomic>
@@ -258,6 +260,7 @@ class MoeDedupEngine {
   bool bulk_landing = true;  // rows cross NVLink as bulk copies through shared memory (else 16-byte stores)
   int64_t dispatch_epoch() const { return dispatch_epoch_; }
   int64_t combine_epoch() const { return combine_epoch_; }
+  int64_t num_tokens() const { return num_tokens_; }  // of the last dispatch
   void set_timeout_ns(int64_t t) { timeout_ns_ = t; }
   void set_trace(const c10::optional<at::Tensor>& dispatch_trace, const c10::optional<at::Tensor>& combine_trace) {
     trace_d_ = check_trace(dispatch_trace);
@@ -776,16 +779,21 @@ class GemmRsEngine {
     g.bias_scale = (float)bias_scale;
     g.bias_at_source = bias_at_source ? 1 : 0;
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
-    const LocalWorkspace* ws = b200::gemm_local_cuts_tiles(g.M, g.N, g.K, sms_) ? local_workspace(stream) : nullptr;
-    g.partials = ws ? ws->partials : nullptr;
-    g.counters = ws ? ws->counters : nullptr;
+    g.partials = nullptr;
+    g.counters = nullptr;
     g.timeout_ns = (uint64_t)timeout_ns_;
     g.status = heap_->status_device();
     g.trace = trace_;
     g.trace_ctas = trace_ == nullptr ? 0 : (int)std::min<int64_t>(trace_keep_.numel() / 8, 1 << 20);
     g.sms = sms_;
     ++epoch_;
-    cuda_check(b200::launch_gemm_local(g, stream), "gemm_local launch");
+    const auto workspace = [&](b200::GemmLocalArgs& args) {
+      if (const LocalWorkspace* ws = local_workspace(stream)) {
+        args.partials = ws->partials;
+        args.counters = ws->counters;
+      }
+    };
+    cuda_check(b200::launch_gemm_local(g, heap_->device(), workspace, stream), "gemm_local launch");
   }
   // Cut tiles meet in a workspace, one per stream because calls on two streams may overlap, and one more per graph
   // that a stream is captured into, because the graph may be replayed on another (its counters are then zeroed by the
@@ -967,6 +975,167 @@ c10::optional<at::Tensor> fp8_gemm_try(const at::Tensor& a, const at::Tensor& b,
   at::Tensor c = at::detail::empty_cuda({M, N}, at::kBFloat16, a.device(), c10::nullopt);
   run_fp8_gemm(a, b, a_scale, b_scale, c, timeout_ns);
   return c;
+}
+
+// ---------------------------------------------------------------------------------------
+// The calls that a short kernel waits for
+// ---------------------------------------------------------------------------------------
+// One rank's whole calls, as methods and functions of the C API: pybind11 takes 0.3 us to look at the arguments of a call,
+// and what Python does around the call of a layer 0.7 us, beside 1.9 us for the launch.  (Host time a call, us: forward
+// 4.8, now 4.1; dispatch + combine 6.6, now 5.7; gemm_rs 4.8, now 4.4; fp8_gemm 5.3, now 4.2.)
+
+const at::Tensor& tensor_arg(PyObject* o) {
+  if (!THPVariable_Check(o)) throw py::type_error(std::string("expected a torch.Tensor, got ") + Py_TYPE(o)->tp_name);
+  return THPVariable_Unpack(o);
+}
+void count_args(Py_ssize_t got, Py_ssize_t want) {
+  if (got != want) throw py::type_error("expected " + std::to_string(want) + " arguments, got " + std::to_string(got));
+}
+double double_arg(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw py::error_already_set();
+  return v;
+}
+PyObject* wrap(const c10::optional<at::Tensor>& t) {
+  if (!t.has_value()) Py_RETURN_NONE;
+  return THPVariable_Wrap(*t);
+}
+// Runs a call; a C++ exception becomes a Python one.
+template <typename F>
+PyObject* guarded(F&& call) {
+  HANDLE_TH_ERRORS
+  try {
+    return call();
+  } catch (py::error_already_set& e) {
+    e.restore();
+    return nullptr;
+  } catch (py::builtin_exception& e) {
+    e.set_error();
+    return nullptr;
+  }
+  END_HANDLE_TH_ERRORS
+}
+template <typename T>
+T& native(PyObject* o) {
+  return *py::handle(o).cast<T*>();
+}
+
+PyObject* moe_try_forward(PyObject* self, PyObject* const* a, Py_ssize_t n) {  // (x, indices, weights, scale) -> result or None
+  return guarded([&] {
+    count_args(n, 4);
+    return wrap(native<MoeDedupEngine>(self).try_forward(tensor_arg(a[0]), tensor_arg(a[1]), tensor_arg(a[2]), double_arg(a[3])));
+  });
+}
+PyObject* moe_try_dispatch(PyObject* self, PyObject* const* a, Py_ssize_t n) {  // (x, indices) -> bool
+  return guarded([&] {
+    count_args(n, 2);
+    return PyBool_FromLong(native<MoeDedupEngine>(self).try_dispatch(tensor_arg(a[0]), tensor_arg(a[1])));
+  });
+}
+PyObject* moe_try_combine(PyObject* self, PyObject* const* a, Py_ssize_t n) {  // (out, weights, expert_y, num_tokens or -1) -> bool
+  return guarded([&] {
+    count_args(n, 4);
+    const int64_t tokens = PyLong_AsLongLong(a[3]);
+    if (tokens == -1 && PyErr_Occurred()) throw py::error_already_set();
+    return PyBool_FromLong(native<MoeDedupEngine>(self).try_combine(tensor_arg(a[0]), tensor_arg(a[1]), tensor_arg(a[2]), tokens));
+  });
+}
+PyObject* gemm_try_run(PyObject* self, PyObject* const* a, Py_ssize_t n) {  // (a, w, bias or None, bias_at_source) -> result or None
+  return guarded([&] {
+    count_args(n, 4);
+    c10::optional<at::Tensor> bias;
+    if (a[2] != Py_None) bias = tensor_arg(a[2]);
+    const int at_source = PyObject_IsTrue(a[3]);
+    if (at_source < 0) throw py::error_already_set();
+    return wrap(native<GemmRsEngine>(self).try_run(tensor_arg(a[0]), tensor_arg(a[1]), bias, at_source != 0));
+  });
+}
+PyObject* fp8_try(PyObject*, PyObject* const* a, Py_ssize_t n) {  // (a, b, a_scale, b_scale, timeout_ns) -> result or None
+  return guarded([&] {
+    count_args(n, 5);
+    const int64_t timeout_ns = PyLong_AsLongLong(a[4]);
+    if (timeout_ns == -1 && PyErr_Occurred()) throw py::error_already_set();
+    return wrap(fp8_gemm_try(tensor_arg(a[0]), tensor_arg(a[1]), tensor_arg(a[2]), tensor_arg(a[3]), timeout_ns));
+  });
+}
+
+// custom_kernel of the MoE task, from its input tuple (cfg, data, rank, world_size) and the table of layers (by the key
+// that get_layer builds): the result, or None where the general way has to be gone (no layer yet, a monitor, several
+// ranks, inputs that are not as the kernel wants them, anything unexpected in the tuple).
+PyObject* moe_forward_try(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    count_args(n, 2);
+    struct Names {
+      PyObject* key[6];
+      PyObject *x, *indices, *weights, *native, *monitor, *num_tokens, *no_group;
+    };
+    static const Names names = [] {
+      Names s;
+      const char* key[6] = {"num_experts", "experts_per_token", "hidden_dim", "max_num_tokens", "in_dtype", "out_dtype"};
+      for (int i = 0; i < 6; ++i) s.key[i] = PyUnicode_InternFromString(key[i]);
+      s.x = PyUnicode_InternFromString("x");
+      s.indices = PyUnicode_InternFromString("indices");
+      s.weights = PyUnicode_InternFromString("weights");
+      s.native = PyUnicode_InternFromString("_native");
+      s.monitor = PyUnicode_InternFromString("monitor");
+      s.num_tokens = PyUnicode_InternFromString("_num_tokens");
+      s.no_group = PyLong_FromVoidPtr(Py_None);  // id(None)
+      return s;
+    }();
+    const auto none = [] {  // (an attribute that is missing is for the general way to complain about)
+      PyErr_Clear();
+      Py_RETURN_NONE;
+    };
+    const auto attr = [](PyObject* o, PyObject* name) { return py::reinterpret_steal<py::object>(PyObject_GetAttr(o, name)); };
+    if (!PyTuple_Check(a[0]) || PyTuple_GET_SIZE(a[0]) != 4 || !PyDict_Check(a[1])) return none();
+    PyObject* const cfg = PyTuple_GET_ITEM(a[0], 0);
+    PyObject* const data = PyTuple_GET_ITEM(a[0], 1);
+    PyObject* const rank = PyTuple_GET_ITEM(a[0], 2);
+    PyObject* const world = PyTuple_GET_ITEM(a[0], 3);
+    py::object key = py::reinterpret_steal<py::object>(PyTuple_New(10));
+    if (!key) throw py::error_already_set();
+    for (int i = 0; i < 6; ++i) {
+      PyObject* v = PyObject_GetAttr(cfg, names.key[i]);
+      if (v == nullptr) return none();
+      PyTuple_SET_ITEM(key.ptr(), i, v);
+    }
+    PyObject* const rest[4] = {rank, world, names.no_group, Py_None};
+    for (int i = 0; i < 4; ++i) {
+      Py_INCREF(rest[i]);
+      PyTuple_SET_ITEM(key.ptr(), 6 + i, rest[i]);
+    }
+    const py::object layer = py::reinterpret_borrow<py::object>(PyDict_GetItemWithError(a[1], key.ptr()));
+    if (!layer) return none();
+    const py::object monitor = attr(layer.ptr(), names.monitor), engine = attr(layer.ptr(), names.native);
+    if (!monitor || !engine || !monitor.is_none() || !py::isinstance<MoeDedupEngine>(engine)) return none();
+    const py::object x = attr(data, names.x), indices = attr(data, names.indices), weights = attr(data, names.weights);
+    if (!x || !indices || !weights || !THPVariable_Check(x.ptr()) || !THPVariable_Check(indices.ptr()) || !THPVariable_Check(weights.ptr()))
+      return none();
+    const double r = PyFloat_AsDouble(rank);
+    if (r == -1.0 && PyErr_Occurred()) return none();
+    const auto y = native<MoeDedupEngine>(engine.ptr())
+                       .try_forward(THPVariable_Unpack(x.ptr()), THPVariable_Unpack(indices.ptr()), THPVariable_Unpack(weights.ptr()), 1.0 + r);
+    if (!y.has_value()) return none();
+    if (PyObject_SetAttr(layer.ptr(), names.num_tokens, Py_None) != 0) throw py::error_already_set();  // (the engine knows)
+    return THPVariable_Wrap(*y);
+  });
+}
+
+#define B200_CALL(name, function) {name, (PyCFunction)(void (*)(void))function, METH_FASTCALL, nullptr}
+PyMethodDef kMoeCalls[] = {B200_CALL("try_forward", moe_try_forward), B200_CALL("try_dispatch", moe_try_dispatch),
+                           B200_CALL("try_combine", moe_try_combine), {nullptr, nullptr, 0, nullptr}};
+PyMethodDef kGemmCalls[] = {B200_CALL("try_run", gemm_try_run), {nullptr, nullptr, 0, nullptr}};
+PyMethodDef kModuleCalls[] = {B200_CALL("fp8_gemm_try", fp8_try), B200_CALL("moe_forward_try", moe_forward_try), {nullptr, nullptr, 0, nullptr}};
+#undef B200_CALL
+
+template <typename T>
+void add_methods(PyMethodDef* defs) {
+  const py::handle type = py::type::of<T>();
+  for (; defs->ml_name != nullptr; ++defs) {
+    const py::object method = py::reinterpret_steal<py::object>(PyDescr_NewMethod(reinterpret_cast<PyTypeObject*>(type.ptr()), defs));
+    if (!method) throw py::error_already_set();
+    type.attr(defs->ml_name) = method;
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1413,9 +1582,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            py::arg("fuse_scale") = false, py::arg("scale") = 1.0)
       .def("combine", &MoeDedupEngine::combine, py::arg("out"), py::arg("weights"), py::arg("expert_y") = py::none())
       .def("forward", &MoeDedupEngine::forward)
-      .def("try_forward", &MoeDedupEngine::try_forward)
-      .def("try_dispatch", &MoeDedupEngine::try_dispatch)
-      .def("try_combine", &MoeDedupEngine::try_combine)
       .def("set_trace", &MoeDedupEngine::set_trace, py::arg("dispatch_trace") = py::none(), py::arg("combine_trace") = py::none())
       .def("set_timeout_ns", &MoeDedupEngine::set_timeout_ns)
       .def_readwrite("bulk_landing", &MoeDedupEngine::bulk_landing)
@@ -1423,7 +1589,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("chunk_min_ranks", &MoeDedupEngine::chunk_min_ranks)
       .def_readwrite("chunk_min_bytes", &MoeDedupEngine::chunk_min_bytes)
       .def_property_readonly("dispatch_epoch", &MoeDedupEngine::dispatch_epoch)
-      .def_property_readonly("combine_epoch", &MoeDedupEngine::combine_epoch);
+      .def_property_readonly("combine_epoch", &MoeDedupEngine::combine_epoch)
+      .def_property_readonly("num_tokens", &MoeDedupEngine::num_tokens);
+  add_methods<MoeDedupEngine>(kMoeCalls);
   m.def("moe_dedup_dispatch_max_blocks", [](int device, int num_experts, int num_entries, int bulk_landing) {
     c10::cuda::CUDAGuard guard(device);
     return b200::moe_dedup_dispatch_max_blocks(device, num_experts, num_entries, bulk_landing);
@@ -1435,7 +1603,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            py::arg("counter_bytes"), py::arg("timeout_ns"))
       .def("run", &GemmRsEngine::run, py::arg("a"), py::arg("w"), py::arg("bias"), py::arg("out"),
            py::arg("bias_at_source") = true, py::arg("bias_scale") = 1.0)
-      .def("try_run", &GemmRsEngine::try_run)
       .def("plan", &GemmRsEngine::plan)
       .def("set_trace", &GemmRsEngine::set_trace)
       .def("restart_epochs", &GemmRsEngine::restart_epochs)
@@ -1452,6 +1619,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("tma_store", &GemmRsEngine::tma_store)
       .def_readwrite("force_staged", &GemmRsEngine::force_staged)
       .def_readwrite("checked", &GemmRsEngine::checked);
+  add_methods<GemmRsEngine>(kGemmCalls);
 
   py::class_<b200::McastRegion, std::shared_ptr<b200::McastRegion>>(m, "McastRegion")
       .def(py::init([](int rank, int world_size, int64_t bytes, int device) {
@@ -1506,7 +1674,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_forward", &moe_forward);
   m.def("gemm_rs", &gemm_rs);
   m.def("fp8_gemm", &fp8_gemm);
-  m.def("fp8_gemm_try", &fp8_gemm_try);
+  if (PyModule_AddFunctions(m.ptr(), kModuleCalls) != 0) throw py::error_already_set();
   m.def("fp8_gemm_take_status", &fp8_gemm_take_status);
   m.def("fp8_wait_selftest", [](int device, int64_t timeout_ns) {
     c10::cuda::CUDAGuard guard(device);

@@ -39,6 +39,7 @@
 #include "fp8_gemm.h"
 #include "gemm_rs.h"
 #include "per_device.h"
+#include "plan_cache.h"
 #include "signal.cuh"
 #include "sm100_ptx.cuh"
 #include "tensor_map.h"
@@ -649,16 +650,10 @@ Fp8Plan make_fp8_plan(int M, int N, int K, int sms) {
 }
 
 const Fp8Plan& cached_plan(int M, int N, int K, int sms) {
-  struct Entry {
-    int M = 0, N = 0, K = 0, sms = 0, dev = -1;
-    Fp8Plan plan;
-  };
-  static thread_local Entry cache[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  Entry& e = cache[((uint32_t)M * 31u + (uint32_t)N * 7u + (uint32_t)K) * 2654435761u >> 26];
-  if (e.M != M || e.N != N || e.K != K || e.sms != sms || e.dev != dev) e = Entry{M, N, K, sms, dev, make_fp8_plan(M, N, K, sms)};
-  return e.plan;
+  static thread_local PlanCache<Fp8Plan> cache;
+  int device = 0;
+  cudaGetDevice(&device);
+  return cache.get(M, N, K, sms, device, make_fp8_plan);
 }
 
 template <int CHUNKS>

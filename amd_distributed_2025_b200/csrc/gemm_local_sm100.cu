@@ -37,6 +37,7 @@
 
 #include "gemm_rs.h"
 #include "per_device.h"
+#include "plan_cache.h"
 #include "signal.cuh"
 #include "sm100_ptx.cuh"
 #include "tensor_map.h"
@@ -953,19 +954,14 @@ Plan make_local_plan(int M, int N, int K, int sms) {
   return best;
 }
 
-// A program comes back with the same few shapes: the search above (2 to 6 us) costs more than a short kernel.  Each
-// thread keeps 64 plans, one to a slot of the hash; shapes that share a slot are searched anew whenever they alternate.
+const Plan& cached_plan(int M, int N, int K, int sms, int device) {
+  static thread_local PlanCache<Plan> cache;
+  return cache.get(M, N, K, sms, device, make_local_plan);
+}
 const Plan& cached_plan(int M, int N, int K, int sms) {
-  struct Entry {
-    int M = 0, N = 0, K = 0, sms = 0, dev = -1;
-    Plan plan;
-  };
-  static thread_local Entry cache[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  Entry& e = cache[((uint32_t)M * 31u + (uint32_t)N * 7u + (uint32_t)K) * 2654435761u >> 26];
-  if (e.M != M || e.N != N || e.K != K || e.sms != sms || e.dev != dev) e = Entry{M, N, K, sms, dev, make_local_plan(M, N, K, sms)};
-  return e.plan;
+  int device = 0;
+  cudaGetDevice(&device);
+  return cached_plan(M, N, K, sms, device);
 }
 
 bool common_params(LocalParams& p, const GemmLocalArgs& a, const Plan& plan, int p_rows, int q_rows, CUtensorMap* map_p,
@@ -1068,15 +1064,11 @@ GemmLocalPlan gemm_local_plan(int M, int N, int K, int sms) {
   return {p.persistent, p.swap, p.persistent || p.pair, own_parts, p.rows, p.bn, p.splits, p.halves, p.sk_tiles, grid_ctas(p)};
 }
 
-bool gemm_local_cuts_tiles(int M, int N, int K, int sms) {
-  const Plan& plan = cached_plan(M, N, K, sms);
-  return plan.persistent && plan.sk_tiles > 0;
-}
-
-cudaError_t launch_gemm_local(const GemmLocalArgs& a, cudaStream_t stream) {
+cudaError_t launch_gemm_local(GemmLocalArgs& a, int device, const std::function<void(GemmLocalArgs&)>& workspace, cudaStream_t stream) {
   if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.K % 8 != 0 || a.N % 8 != 0) return cudaErrorInvalidValue;
-  Plan plan = cached_plan(a.M, a.N, a.K, a.sms);
+  Plan plan = cached_plan(a.M, a.N, a.K, a.sms, device);
   if (plan.persistent) {
+    if (plan.sk_tiles > 0) workspace(a);
     if (a.partials == nullptr) plan.sk_tiles = 0;
     return plan.swap ? launch_pair<true>(a, plan, stream) : launch_pair<false>(a, plan, stream);
   }

@@ -21,6 +21,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
+
 #include "status.h"
 
 namespace b200 {
@@ -98,7 +100,8 @@ constexpr uint64_t kGemmLocalPartialBytes = (uint64_t)kGemmLocalMaxPairs * 2 * 2
 // per cut tile (at most two per pair): one per CTA and epilogue warp
 constexpr int kGemmLocalCounters = kGemmLocalMaxPairs * 2 * 2 * 8;
 
-cudaError_t launch_gemm_local(const GemmLocalArgs& args, cudaStream_t stream);
+// `device`: the current one.  workspace(args) is asked for `partials` and `counters` where the plan has a use for them.
+cudaError_t launch_gemm_local(GemmLocalArgs& args, int device, const std::function<void(GemmLocalArgs&)>& workspace, cudaStream_t stream);
 // How the launch will run (a pure function of its arguments and the device's cluster capacities).
 struct GemmLocalPlan {
   bool persistent, swap, pair;  // pair kernel or tile kernel; weight on the 128-row side; a CTA pair per tile
@@ -106,7 +109,6 @@ struct GemmLocalPlan {
   int rows, bn, splits, halves, cut_tiles, ctas;
 };
 GemmLocalPlan gemm_local_plan(int M, int N, int K, int sms);
-bool gemm_local_cuts_tiles(int M, int N, int K, int sms);  // whether the launch has a use for `partials`
 
 // What a CTA takes of its SM, by tile.  Two CTAs may meet on an SM (calls on two streams, or the next call's early
 // start) wherever their shared memory fits; a CTA that then had to wait for tensor memory might wait for one that waits

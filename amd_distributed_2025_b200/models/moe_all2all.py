@@ -135,7 +135,7 @@ class MoEAllToAll:
         self._local_rank = torch.zeros(n_max, **i32)
         self._route = torch.full((n_max, 2), -1, **i32)
         self.expert_num_tokens = torch.zeros(self.num_local_experts, **i32)
-        self._num_tokens = 0
+        self._num_tokens: Optional[int] = 0  # of the last dispatch (None: the engine knows)
         self._dispatch_pending = False  # a dispatch whose combine has not run yet
         self._off_counts = self.ws.offset("counts")
         self._off_expert_x = self.ws.offset("expert_x")
@@ -157,6 +157,8 @@ class MoEAllToAll:
             self.engine.chunk_min_bytes = int(os.environ.get("B200_MOE_CHUNK_MIN_BYTES", str(8 << 20)))
             if world_size == 1:
                 self._native = self.engine
+                global _forward_try
+                _forward_try = ext.moe_forward_try
         self._dispatched = (self.expert_num_tokens, self.expert_x, self.expert_meta)
         self.trace: Optional[Tuple[torch.Tensor, torch.Tensor]] = None
 
@@ -207,7 +209,7 @@ class MoEAllToAll:
     # -- dispatch ----------------------------------------------------------------------
     def dispatch(self, dp_x: torch.Tensor, indices: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
         if self._native is not None and self.monitor is None and self._native.try_dispatch(dp_x, indices):
-            self._num_tokens = dp_x.shape[0]
+            self._num_tokens = None
             self._dispatch_pending = True
             return self._dispatched
         cfg = self.cfg
@@ -277,8 +279,9 @@ class MoEAllToAll:
                 and self._native.try_combine(out_tokens, weights, expert_y, -1 if num_tokens is None else num_tokens)):
             self._dispatch_pending = False
             return out_tokens
-        n = self._num_tokens if num_tokens is None else int(num_tokens)
-        if n != self._num_tokens:
+        known = self.engine.num_tokens if self._num_tokens is None else self._num_tokens
+        n = known if num_tokens is None else int(num_tokens)
+        if n != known:
             raise ValueError("num_tokens differs from the preceding dispatch")
         self._guard()
         self._dispatch_pending = False
@@ -333,7 +336,7 @@ class MoEAllToAll:
         if self._native is not None and self.monitor is None:
             y = self._native.try_forward(dp_x, indices, weights, scale)
             if y is not None:
-                self._num_tokens = dp_x.shape[0]
+                self._num_tokens = None
                 self._dispatch_pending = False
                 return y
         cfg = self.cfg
@@ -382,6 +385,7 @@ class MoEAllToAll:
 # --------------------------------------------------------------------------------------
 
 _LAYERS: Dict[tuple, MoEAllToAll] = {}
+_forward_try = None  # custom_kernel's common call, once the first one-rank layer has loaded the extension
 
 
 def get_layer(cfg: MoEConfig, rank: int, world_size: int, group=None, mode: Optional[str] = None) -> MoEAllToAll:
@@ -425,6 +429,10 @@ def custom_kernel(data: MoEInput, backend: str = "auto", mode: Optional[str] = N
     otherwise; "shm" and "torch" force the latter two.  ``mode`` picks the protocol ("dedup" or
     "direct"; default on GPUs ``B200_MOE_MODE`` or "dedup", on CPU ranks ``B200_HOST_MOE_MODE`` or
     "direct")."""
+    if _forward_try is not None and mode is None and backend == "auto":
+        y = _forward_try(data, _LAYERS)
+        if y is not None:
+            return y
     cfg, rank_data, rank, world_size = data
     x = rank_data.x
     if backend == "shm" or (backend == "auto" and not x.is_cuda and _cpu_ranks_share_a_node()):

@@ -106,6 +106,8 @@ def _import_so():
 def load(allow_build: bool = True):
     """Return the extension module, building it first if no up-to-date binary exists."""
     global _module
+    if _module is not None:  # (set once, and last)
+        return _module
     with _lock:
         if _module is not None:
             return _module

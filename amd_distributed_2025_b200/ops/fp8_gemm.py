@@ -18,6 +18,7 @@ from typing import Optional, Tuple
 import torch
 
 from ..utils.status import StatusError, describe_status
+from . import _ext
 
 BLOCK = 128
 
@@ -49,8 +50,6 @@ def fp8_gemm(
 
     The kernel's waits are limited to ``timeout_ms``.  A call in which one expires has no result; as nothing here waits
     for the GPU, that is raised (``StatusError``) by ``check()`` or by the next call on the device, once."""
-    from . import _ext
-
     ext = _ext.load()
     if c is None:
         c = ext.fp8_gemm_try(a, b, a_scale, b_scale, int(timeout_ms * 1e6))
@@ -76,8 +75,6 @@ def _raise_recorded(ext, device: torch.device) -> None:
 
 def check(device: Optional[torch.device] = None) -> None:
     """Wait for the device and raise ``StatusError`` if a call on it gave up on a wait; this clears the record."""
-    from . import _ext
-
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     torch.cuda.synchronize(device)
     _raise_recorded(_ext.load(), device)

@@ -210,6 +210,40 @@ def test_moe_one_rank_combine_rounds(k, H, dtype):
     layer.close()
 
 
+def test_moe_whole_calls_and_the_general_way_agree():
+    """custom_kernel, dispatch and combine through the engine's own calls: the layer of each configuration, token counts
+    known to what follows, nothing kept of the arguments, wrong ones refused."""
+    import sys
+
+    from amd_distributed_2025_b200.models import moe_all2all
+
+    inputs = [contract.make_moe_inputs(E, k, H, 24, 5 + H, 0, 1, device="cuda", dtype=dtype, fixed_num_tokens=T, weights="softmax")
+              for E, k, H, T, dtype in ((16, 2, 256, 24, torch.float16), (16, 2, 256, 24, torch.float32), (8, 3, 264, 7, torch.float16))]
+    want = [oracle.moe_expected_output(cfg, data, 1) for cfg, data, _, _ in inputs]
+    held = None
+    for _ in range(3):
+        for item, w in zip(inputs, want):  # each its own layer, also right after another's call
+            y = moe_all2all.custom_kernel(item)
+            assert oracle.check_moe_output(y, w)[0]
+        del y, item, w
+        if held is None:  # (the layers, made by the first round, hold their configurations)
+            held = [sys.getrefcount(v) for cfg, d, _, _ in inputs for v in (cfg, d, d.x, d.indices, d.weights)]
+    assert held == [sys.getrefcount(v) for cfg, d, _, _ in inputs for v in (cfg, d, d.x, d.indices, d.weights)]
+    cfg, data, _, _ = inputs[2]
+    layer = moe_all2all.get_layer(cfg, 0, 1)
+    counts, ex, meta = layer.dispatch(data.x, data.indices)
+    wide = torch.empty(7, 2 * 264, dtype=torch.float16, device="cuda")[:, :264]  # rows apart: the general way
+    with pytest.raises(ValueError):
+        layer.combine(wide, data.weights, meta, ex, counts, 6)
+    layer.combine(wide, data.weights, meta, ex, counts)
+    assert oracle.check_moe_output(wide.contiguous(), want[2])[0]
+    for bad in ((data.x,), (data.x, None), (data.x, 3)):
+        with pytest.raises(TypeError):
+            layer.engine.try_dispatch(*bad)
+    moe_all2all.release_layers()  # the layers are gone: new ones
+    assert oracle.check_moe_output(moe_all2all.custom_kernel(inputs[0]), want[0])[0]
+
+
 def test_moe_dedup_fp32_partial_rows_and_phase_stamps():
     from amd_distributed_2025_b200.models import moe_all2all
 

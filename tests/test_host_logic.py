@@ -445,6 +445,41 @@ int main() {
         assert not [s for s in text.split(";") if "static" in s and "=" in s and "cudaFuncSetAttribute" in s.split("=", 1)[1]], os.path.basename(path)
 
 
+def test_plan_cache_keeps_sizes_apart(tmp_path):
+    """csrc/plan_cache.h: what `make` gave for the size, the SM count and the device at hand, and slots that do not meet for
+    two layers of one model at the same batch size."""
+    import os
+    import subprocess
+
+    from amd_distributed_2025_b200.ops import _ext
+
+    (tmp_path / "main.cpp").write_text("""
+#include <cstdio>
+#include "plan_cache.h"
+struct Plan { int id = -1; };
+int main() {
+  static b200::PlanCache<Plan> cache;
+  int made = 0;
+  auto make = [&](int M, int N, int K, int sms) { ++made; return Plan{M * 1000003 + N * 1009 + K * 7 + sms}; };
+  int wrong = 0, shared = 0;
+  for (int round = 0; round < 2; ++round)
+    for (int M = 1; M <= 600; ++M)
+      for (int dev = 0; dev < 2; ++dev) {
+        wrong += cache.get(M, 512, 64, 148, dev, make).id != M * 1000003 + 512 * 1009 + 64 * 7 + 148;
+        wrong += cache.get(M, 64, 512, 132, dev, make).id != M * 1000003 + 64 * 1009 + 512 * 7 + 132;
+      }
+  made = 0;
+  for (int i = 0; i < 5; ++i) cache.get(7, 8, 9, 148, 0, make);
+  for (int M = 1; M <= 512; ++M) shared += b200::PlanCache<Plan>::slot(M, 7168, 18432) == b200::PlanCache<Plan>::slot(M, 2112, 7168);
+  std::printf("%d %d %d", wrong, made, shared);
+}
+""")
+    exe = str(tmp_path / "plans")
+    subprocess.run(["g++", "-std=c++17", "-I", _ext.CSRC_DIR, str(tmp_path / "main.cpp"), "-o", exe], check=True)
+    wrong, made, shared = map(int, subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split())
+    assert wrong == 0 and made == 1 and shared <= 12  # (512 / 256 slots by chance)
+
+
 @pytest.mark.parametrize("given", [False, True])
 def test_fp8_gemm_raises_what_an_earlier_call_recorded(monkeypatch, given):
     """An expired wait of the fp8 kernel: raised once by the next call, which launches nothing, then forgotten."""
