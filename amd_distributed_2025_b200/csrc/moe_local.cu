@@ -16,6 +16,7 @@
 
 #include "moe.h"
 #include "moe_common.cuh"
+#include "per_device.h"
 #include "signal.cuh"
 #include "sm100_ptx.cuh"
 
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(FUSED ? 512 : 1024, 1) moe_local_dispatch_kern
   const int threads = blockDim.x, warps = threads >> 5;
   const int k = p.k;
   const int P = p.pieces;
-  ptx::grid_dep_launch();
+  if (!FUSED) ptx::grid_dep_launch();
   const Share sh = share_of_cta(p, reinterpret_cast<int32_t*>(smem_local));
   for (int i = threadIdx.x; i < (int)(sh.ids - sh.total); i += threads) sh.total[i] = 0;
   if (threadIdx.x < 3) sh.ids[sh.m + threadIdx.x] = -2;
@@ -243,6 +244,7 @@ __global__ void __launch_bounds__(FUSED ? 512 : 1024, 1) moe_local_dispatch_kern
     stamp_cta0(p.trace_c, 0);
     stamp_cta0(p.trace_c, 1);
   }
+  if (FUSED) ptx::grid_dep_launch();  // (its CTAs would only stand in line for the SMs before: 0.1 us)
   uint8_t* ex = reinterpret_cast<uint8_t*>(p.expert_x);
   if (p.vec) {
     constexpr int N = Vec16<T>::N;
@@ -417,10 +419,19 @@ void cut_row(uint32_t row_bytes, bool vec, int most, int32_t* pieces, int32_t* p
   *piece_vecs = (nv + *pieces - 1) / *pieces;
 }
 
+// Shared memory that keeps a CTA of forward alone on its SM.  A launch of one CTA per SM starts while the one before it
+// still runs; where two fit, the scheduler may put two on each SM that happens to be free, none on the others, and the next
+// launch into the gaps, call after call: 128 tokens, top-8 took 7.05 us in a row of calls, 5.3 with one CTA to an SM (129 and
+// 136 likewise, 140 never).
+constexpr int kAloneBytes = 116 * 1024;
+
 template <typename T>
 cudaError_t dispatch_typed(const MoeLocalDispatchParams& p, int threads, int grid, size_t smem, cudaStream_t stream) {
-  return p.out == nullptr ? ptx::launch_dependent(moe_local_dispatch_kernel<T, false>, grid, threads, smem, stream, p)
-                          : ptx::launch_dependent(moe_local_dispatch_kernel<T, true>, grid, threads, smem, stream, p);
+  if (p.out == nullptr) return ptx::launch_dependent(moe_local_dispatch_kernel<T, false>, grid, threads, smem, stream, p);
+  static OncePerDevice once;
+  const cudaError_t opted = once([] { return opt_in(moe_local_dispatch_kernel<T, true>, kAloneBytes, false); });
+  if (opted != cudaSuccess) return opted;
+  return ptx::launch_dependent(moe_local_dispatch_kernel<T, true>, grid, threads, std::max<size_t>(smem, kAloneBytes), stream, p);
 }
 
 template <typename T>
