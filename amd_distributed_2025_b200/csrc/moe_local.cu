@@ -205,7 +205,6 @@ __global__ void __launch_bounds__(FUSED ? 512 : 1024, 1) moe_local_dispatch_kern
   const int threads = blockDim.x, warps = threads >> 5;
   const int k = p.k;
   const int P = p.pieces;
-  if (!FUSED) ptx::grid_dep_launch();
   const Share sh = share_of_cta(p, reinterpret_cast<int32_t*>(smem_local));
   for (int i = threadIdx.x; i < (int)(sh.ids - sh.total); i += threads) sh.total[i] = 0;
   if (threadIdx.x < 3) sh.ids[sh.m + threadIdx.x] = -2;
@@ -244,7 +243,10 @@ __global__ void __launch_bounds__(FUSED ? 512 : 1024, 1) moe_local_dispatch_kern
     stamp_cta0(p.trace_c, 0);
     stamp_cta0(p.trace_c, 1);
   }
-  if (FUSED) ptx::grid_dep_launch();  // (its CTAs would only stand in line for the SMs before: 0.1 us)
+  // The next launch is let in when the stores begin (its CTAs would only stand in line for the SMs before: 0.1 us); behind
+  // plain copies, combine as a rule, not before the CTAs leave: several of its CTAs fit on an SM, and early ones gather where
+  // a dispatch CTA has just left (111 tokens, top-7, 2 KiB, dispatch + combine 8.1 us, now 6.9; 2000, top-2, 2 KiB 8.2, now 7.8).
+  if (FUSED) ptx::grid_dep_launch();
   uint8_t* ex = reinterpret_cast<uint8_t*>(p.expert_x);
   if (p.vec) {
     constexpr int N = Vec16<T>::N;
