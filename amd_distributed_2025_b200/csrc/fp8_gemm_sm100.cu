@@ -622,7 +622,8 @@ Fp8Memory fp8_memory(int bn, int splits) {
 
 // Time model in ns, fitted to 480 timed plans of 120 drawn sizes (0.6 % from the best width of each): a K block of a tile
 // takes its pair `kb_ns` whatever limits it; then power, memory, and what a launch costs before and after its blocks.  A
-// launch that leaves half of the SMs idle is set up beside the one before it.
+// launch that leaves half of the SMs idle is set up beside the one before it, which shows most where there is one row of
+// tiles (57 x 4640 x 752: 74 CTAs 5.5 us in a row of calls, 146 6.1; but 3409 x 328 x 336: 56 CTAs 6.4, 84 5.5).
 Fp8Plan make_fp8_plan(int M, int N, int K, int sms) {
   const int k_blocks = (K + kBlockK - 1) / kBlockK;
   const double dram_ns = ((double)M * K + (double)N * K + 2.0 * M * N) / 6600.0;
@@ -642,7 +643,7 @@ Fp8Plan make_fp8_plan(int M, int N, int K, int sms) {
       const double power_ns = 2.0 * ((M + 255) / 256) * 256.0 * ((N + bn - 1) / bn) * bn * (double)k_blocks * kBlockK / 2.6e6;
       p.ns = std::max({waves * kbs * kb_ns, power_ns, dram_ns}) +
              (s == 1 ? 2490.0 + 5.6 * bn : 5060.0 + 23.5 * std::max(bn - 64, 0) + 86.0 * s) + (waves - 1) * 7.8 * bn +
-             (4 * s * p.clusters > sms ? 910.0 : 0.0);
+             (4 * s * p.clusters > sms ? (M <= 256 ? 910.0 : 450.0) : 0.0);
       if (p.ns < best.ns) best = p;
     }
   }
