@@ -279,6 +279,7 @@ class MoEAllToAll:
                 and self._native.try_combine(out_tokens, weights, expert_y, -1 if num_tokens is None else num_tokens)):
             self._dispatch_pending = False
             return out_tokens
+        self._require_open()  # (a closed layer has no engine to ask)
         known = self.engine.num_tokens if self._num_tokens is None else self._num_tokens
         n = known if num_tokens is None else int(num_tokens)
         if n != known:

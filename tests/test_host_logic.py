@@ -367,15 +367,18 @@ def test_second_dedup_dispatch_without_combine_waits_for_all_ranks(monkeypatch):
     assert calls[6:] == ["dispatch"]
 
 
+@pytest.mark.parametrize("last_call", [None, "dispatch", "forward"])
 @pytest.mark.parametrize("mode", ["dedup", "direct"])
-def test_closed_moe_layer_raises_and_hands_nothing_to_the_engine(mode):
-    """The workspace of a closed layer is freed memory: no call may reach a launch."""
+def test_closed_moe_layer_raises_and_hands_nothing_to_the_engine(mode, last_call):
+    """The workspace of a closed layer is freed memory: no call may reach a launch, whatever the layer did before."""
     from amd_distributed_2025_b200.models import moe_all2all as m
     from amd_distributed_2025_b200.parallel.symm_mem import SlabLayout, SymmetricWorkspace
 
     launched = []
 
     class Engine:
+        num_tokens = 4
+
         def __getattr__(self, name):
             return lambda *a, **k: launched.append(name) or True
 
@@ -397,10 +400,17 @@ def test_closed_moe_layer_raises_and_hands_nothing_to_the_engine(mode):
     layer.expert_num_tokens = layer.expert_meta = None
     layer.expert_x = layer.expert_y = torch.zeros(8, 4, 16)
     x, idx, w, y = torch.zeros(4, 16), torch.zeros(4, 2, dtype=torch.int32), torch.zeros(4, 2), torch.zeros(4, 16)
+    if layer._native is not None:  # (the token count of a native call is known to the engine alone)
+        if last_call == "dispatch":
+            layer.dispatch(x, idx)
+        elif last_call == "forward":
+            layer.forward(x, idx, w, 1.0)
+    launched.clear()
     layer.close()
     for call in (lambda: layer.expert_scale(2.0), lambda: layer.forward(x, idx, w, 1.0), lambda: layer.dispatch(x, idx),
-                 lambda: layer.combine(y, w, None, torch.zeros(8, 4, 16), None, 4)):
-        with pytest.raises(RuntimeError):
+                 lambda: layer.combine(y, w, None, torch.zeros(8, 4, 16), None, 4),
+                 lambda: layer.combine(y, w, None, torch.zeros(8, 4, 16), None)):
+        with pytest.raises(RuntimeError, match="closed"):
             call()
     assert launched == []
 
