@@ -1032,11 +1032,16 @@ PyObject* moe_try_dispatch(PyObject* self, PyObject* const* a, Py_ssize_t n) {  
     return PyBool_FromLong(native<MoeDedupEngine>(self).try_dispatch(tensor_arg(a[0]), tensor_arg(a[1])));
   });
 }
-PyObject* moe_try_combine(PyObject* self, PyObject* const* a, Py_ssize_t n) {  // (out, weights, expert_y, num_tokens or -1) -> bool
-  return guarded([&] {
+PyObject* moe_try_combine(PyObject* self, PyObject* const* a, Py_ssize_t n) {  // (out, weights, expert_y, num_tokens or None) -> bool
+  return guarded([&]() -> PyObject* {
     count_args(n, 4);
-    const int64_t tokens = PyLong_AsLongLong(a[3]);
-    if (tokens == -1 && PyErr_Occurred()) throw py::error_already_set();
+    int64_t tokens = -1;  // the engine's
+    if (a[3] != Py_None) {
+      if (!PyLong_Check(a[3])) Py_RETURN_FALSE;  // (the general way converts it)
+      int overflow = 0;
+      tokens = PyLong_AsLongLongAndOverflow(a[3], &overflow);
+      if (tokens < 0 || overflow != 0) Py_RETURN_FALSE;  // (... or refuses it)
+    }
     return PyBool_FromLong(native<MoeDedupEngine>(self).try_combine(tensor_arg(a[0]), tensor_arg(a[1]), tensor_arg(a[2]), tokens));
   });
 }

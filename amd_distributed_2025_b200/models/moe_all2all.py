@@ -276,7 +276,7 @@ class MoEAllToAll:
         instead, which equals the reference's ``+=`` onto a caller-provided buffer).
         """
         if (self._native is not None and self.monitor is None and not accumulate
-                and self._native.try_combine(out_tokens, weights, expert_y, -1 if num_tokens is None else num_tokens)):
+                and self._native.try_combine(out_tokens, weights, expert_y, num_tokens)):
             self._dispatch_pending = False
             return out_tokens
         self._require_open()  # (a closed layer has no engine to ask)

@@ -244,6 +244,29 @@ def test_moe_whole_calls_and_the_general_way_agree():
     assert oracle.check_moe_output(moe_all2all.custom_kernel(inputs[0]), want[0])[0]
 
 
+@pytest.mark.parametrize("mode", ["dedup", "direct"])
+def test_moe_combine_takes_the_dispatched_token_count_or_none(mode):
+    """Every number but that of the dispatch is refused, negative ones too; whatever int() takes is taken."""
+    import numpy
+
+    from amd_distributed_2025_b200.models import moe_all2all
+
+    cfg, data, _, _ = contract.make_moe_inputs(8, 2, 64, 9, 3, 0, 1, device="cuda", dtype=torch.float16, fixed_num_tokens=5)
+    layer = moe_all2all.MoEAllToAll(cfg, 0, 1, mode=mode)
+    counts, ex, meta = layer.dispatch(data.x, data.indices)
+    ey = ex.clone()
+    want = oracle.moe_expected_output(cfg, data, 1)  # (one rank scales by 1 + 0)
+    for bad in (-1, -5, 0, 4, 6, 2**70, -(2**70)):
+        with pytest.raises(ValueError, match="num_tokens"):
+            layer.combine(torch.empty(5, 64, dtype=torch.float16, device="cuda"), data.weights, meta, ey, counts, bad)
+    for good in (None, 5, 5.0, numpy.int64(5), torch.tensor(5)):
+        out = torch.empty(5, 64, dtype=torch.float16, device="cuda")
+        layer.combine(out, data.weights, meta, ey, counts, good)
+        assert oracle.check_moe_output(out, want)[0]
+    layer.check()
+    layer.close()
+
+
 def test_moe_dedup_fp32_partial_rows_and_phase_stamps():
     from amd_distributed_2025_b200.models import moe_all2all
 
