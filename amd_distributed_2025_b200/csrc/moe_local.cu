@@ -65,7 +65,7 @@ struct Share {
   int lo, hi, t0, i0, m;
   int32_t* total;  // shared memory: entries [0, i0 + m) of each expert
   int32_t* ids;    // shared memory: expert of each own entry, or -1; then three words of -2
-  int32_t* rows;   // shared memory: final row of each own entry, or -1
+  int32_t* rows;   // shared memory: final row of each own entry; -1 where it has no expert, -2 - slot where the slot does not fit
 };
 
 // Where CTA b's run of items starts: runs get shorter towards the last CTA by `lean` of their mean either way.
@@ -144,7 +144,7 @@ __device__ __forceinline__ void assign_rows(const MoeLocalDispatchParams& p, con
       from_here += (later.x == e) + (later.y == e) + (later.z == e) + (later.w == e);
     }
     const int slot = before - from_here;
-    if (j < sh.m) sh.rows[j] = e >= 0 && slot < p.max_recv ? e * p.max_recv + slot : -1;
+    if (j < sh.m) sh.rows[j] = e < 0 ? -1 : slot < p.max_recv ? e * p.max_recv + slot : -2 - slot;
   }
 }
 
@@ -152,17 +152,17 @@ __device__ __forceinline__ void assign_rows(const MoeLocalDispatchParams& p, con
 __device__ __forceinline__ void write_metadata(const MoeLocalDispatchParams& p, const Share& sh, int t, int lane) {
   if (lane >= p.k) return;
   const int i = t * p.k + lane;
-  const int e = sh.ids[i - sh.i0], row = sh.rows[i - sh.i0];
-  p.route[i] = make_int2(row >= 0 ? 0 : -1, row);
+  const int row = sh.rows[i - sh.i0];
+  p.route[i] = row >= 0 ? make_int2(0, row) : make_int2(-1, -1);
   if (row >= 0) {
     int32_t* meta = p.expert_meta + (size_t)row * kMetaDim;
-    meta[0] = e;
+    meta[0] = sh.ids[i - sh.i0];
     meta[1] = 0;
     meta[2] = t;
     meta[3] = lane;
     meta[4] = 0;
-  } else if (e >= 0) {
-    record_status(p.status, STATUS_BAD_INDEX, PHASE_NONE, 0, i, p.epoch, (uint64_t)p.max_recv);
+  } else if (row < -1) {
+    record_status(p.status, STATUS_BAD_INDEX, PHASE_NONE, 0, i, p.epoch, (uint64_t)(int64_t)(-2 - row));
   }
 }
 

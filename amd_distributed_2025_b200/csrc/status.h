@@ -37,7 +37,7 @@ struct StatusWord {
   int32_t peer;     // peer rank the wait was on, or -1
   int32_t detail;   // kernel specific (block id, expert id, ...)
   uint64_t epoch;   // call number of the failing wait
-  uint64_t seen;    // last value read from the flag
+  uint64_t seen;    // last value read from the flag; with STATUS_BAD_INDEX the id, slot or row that was out of range
 };
 
 // Device-resident status record.  `word` is updated with device atomics; when a failure

@@ -322,6 +322,43 @@ def test_moe_bad_expert_id_is_reported_not_faulted(mode):
     layer.close()
 
 
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("H", [64, 65])  # rows of whole vectors, and not
+def test_moe_one_rank_entries_that_do_not_fit_their_expert(fused, H):
+    """A token that names an expert twice can send it more rows than the layer has room for: the others are delivered,
+    and the record says which entry had which slot."""
+    from amd_distributed_2025_b200.models import moe_all2all
+    from amd_distributed_2025_b200.utils.status import StatusError
+
+    T, k = 4, 8  # room for four rows an expert
+    cfg = contract.MoEConfig(2, k, H, T, torch.float32, torch.float32)
+    gen = torch.Generator(device="cuda").manual_seed(H)
+    x = torch.randn(T, H, device="cuda", generator=gen)
+    w = torch.rand(T, k, device="cuda", generator=gen)
+    ids = torch.zeros(T, k, dtype=torch.int32, device="cuda")  # expert 0: entry i is its row i ...
+    ids[1, 6] = ids[3, 7] = 1  # ... but for two that go to expert 1, after which it is row i - 1
+    layer = moe_all2all.MoEAllToAll(cfg, 0, 1, mode="dedup")
+    assert layer.max_recv == T
+    if fused:
+        y = layer.forward(x, ids, w, 2.0)
+        served = torch.zeros(T, k, dtype=torch.float64, device="cuda")
+        served[0, :4] = served[1, 6] = served[3, 7] = 1.0
+        want = 2.0 * x.double() * (w.double() * served).sum(1, keepdim=True)
+        assert oracle.relative_error(y, want) < 1e-6
+        counts, ex, meta = layer.expert_num_tokens, layer.expert_x, layer.expert_meta
+    else:
+        counts, ex, meta = layer.dispatch(x, ids)
+    with pytest.raises(StatusError) as err:
+        layer.check()
+    entry, slot = err.value.status["detail"], err.value.status["seen"]
+    assert err.value.code == "bad_index" and 4 <= entry < 31 and entry != 14 and slot == entry - (entry > 14)
+    assert counts.tolist() == [4, 2]
+    assert torch.equal(ex[0], x[[0, 0, 0, 0]]) and torch.equal(ex[1, :2], x[[1, 3]])
+    assert meta[0].tolist() == [[0, 0, 0, j, 0] for j in range(4)] and meta[1, :2].tolist() == [[1, 0, 1, 6, 0], [1, 0, 3, 7, 0]]
+    layer.ws.reset_status()
+    layer.close()
+
+
 @pytest.mark.parametrize(
     "m,n,k,has_bias",
     [
