@@ -8,6 +8,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "moe_runs.h"
 #include "status.h"
 
 namespace b200 {
@@ -174,7 +175,7 @@ struct MoeLocalDispatchParams {
   uint64_t* trace_d;         // optional stamps, slots as in the multi-rank kernels
   uint64_t* trace_c;
   int32_t vec, pieces, piece_vecs, cap;  // filled in by the launcher
-  float lean;                // how much longer the runs of the first CTAs are than those of the last
+  int32_t slope;             // of the CTAs' runs of items (moe_runs.h)
 };
 
 struct MoeLocalCombineParams {

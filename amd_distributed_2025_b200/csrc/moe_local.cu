@@ -68,20 +68,13 @@ struct Share {
   int32_t* rows;   // shared memory: final row of each own entry; -1 where it has no expert, -2 - slot where the slot does not fit
 };
 
-// Where CTA b's run of items starts: runs get shorter towards the last CTA by `lean` of their mean either way.
-__device__ __forceinline__ int first_item(const MoeLocalDispatchParams& p, int b) {
-  const int items = p.num_tokens * p.pieces;
-  if (b >= (int)gridDim.x) return items;
-  const float x = (float)b / (float)gridDim.x;
-  return (int)((float)items * x * (1.f + p.lean * (1.f - x)));
-}
-
-// Work is T x P items (token, piece of its row), dealt out to the CTAs in runs.  Neighbouring CTAs may share a
-// token; its metadata belongs to the CTA with its first piece.
+// Work is T x P items (token, piece of its row), dealt out to the CTAs in runs (moe_runs.h).  Neighbouring CTAs may share
+// a token; its metadata belongs to the CTA with its first piece.
 __device__ __forceinline__ Share share_of_cta(const MoeLocalDispatchParams& p, int32_t* smem) {
   Share sh;
-  sh.lo = first_item(p, (int)blockIdx.x);
-  sh.hi = first_item(p, (int)blockIdx.x + 1);
+  const MoeRuns runs(p.num_tokens * p.pieces, (int)gridDim.x, p.slope);
+  sh.lo = runs.start((int)blockIdx.x);
+  sh.hi = runs.start((int)blockIdx.x + 1);
   sh.t0 = sh.lo / p.pieces;
   sh.i0 = sh.t0 * p.k;
   sh.m = sh.hi > sh.lo ? (sh.hi + p.pieces - 1) / p.pieces * p.k - sh.i0 : 0;
@@ -468,6 +461,7 @@ cudaError_t launch_moe_local_dispatch(MoeLocalDispatchParams p, int sms, cudaStr
           (reinterpret_cast<uintptr_t>(p.expert_x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
   cut_row(p.row_bytes, p.vec != 0, kPieceVecs, &p.pieces, &p.piece_vecs);
   const int64_t items = (int64_t)p.num_tokens * p.pieces;
+  if (items > INT32_MAX) return cudaErrorInvalidValue;  // (2 TB of rows)
   // 32 warps per SM keep the most stores in flight where rows are only copied (2047 tokens to 16376 rows of 8 KiB: 30 us,
   // 44 with half the warps).  Every CTA counts for itself, so few large ones repeat less of that: it pays from some
   // 6000 entries on (4000 tokens, top-2, rows of 1 KiB, with combine: 9.2 us with 2 x 16 warps, 10.0 with 4 x 8; 606 items
@@ -483,8 +477,10 @@ cudaError_t launch_moe_local_dispatch(MoeLocalDispatchParams p, int sms, cudaStr
   // The later a CTA's tokens, the longer it counts before its first store.  Where counting is short against the stores, a
   // tenth evens that out (4096 tokens, top-6, rows of 8 KiB: 54.5 -> 52.2 us; 1000, top-4, 4 KiB: 6.0 -> 5.9), where it is
   // not, two tenths (4096 tokens, top-8, rows of 1 KiB: 13.4 us, with a tenth 12.8, with two 12.2).
-  p.lean = !fused || threads < 512 ? 0.f : entries > 16384 && p.row_bytes <= 2048 ? 0.2f : 0.1f;
-  p.cap = ((int32_t)((int64_t)((1.0 + p.lean) * items / grid + 16) / p.pieces + 2) * p.k + 6) & ~3;  // (and three words, in groups of four)
+  const double lean = !fused || threads < 512 ? 0.0 : entries > 16384 && p.row_bytes <= 2048 ? 0.2 : 0.1;
+  p.slope = moe_run_slope((int32_t)items, grid, lean);
+  const int32_t longest = MoeRuns((int32_t)items, grid, p.slope).longest();
+  p.cap = (int32_t)(moe_run_entries(longest, p.pieces, p.k) + 6) & ~3;  // (and three words, in groups of four)
   const size_t smem = ((size_t)((p.num_experts + 3) & ~3) + 2 * (size_t)p.cap) * sizeof(int32_t);
   if (smem > 48 * 1024) return cudaErrorInvalidValue;
   switch (p.dtype) {

@@ -455,6 +455,56 @@ int main() {
         assert not [s for s in text.split(";") if "static" in s and "=" in s and "cudaFuncSetAttribute" in s.split("=", 1)[1]], os.path.basename(path)
 
 
+def test_moe_runs_tile_the_items_and_fit_their_memory(tmp_path):
+    """csrc/moe_runs.h: every item belongs to one CTA, from none to 2^31 - 1 of them, and no run is longer, or touches more
+    entries, than the launcher cuts shared memory to."""
+    import subprocess
+
+    from amd_distributed_2025_b200.ops import _ext
+
+    (tmp_path / "main.cpp").write_text("""
+#include <cstdio>
+#include <random>
+#include "moe_runs.h"
+int main() {
+  long long wrong = 0, loose = 0, lopsided = 0;
+  std::mt19937_64 rng(1);
+  for (int i = 0; i < 200000; ++i) {
+    const int bits = (int)(rng() % 32);
+    const int items = i < 600 ? i : i < 610 ? 2147483647 - (i - 600) : (int)((rng() & ((1ull << bits) - 1)));
+    const int ctas = i % 3 == 0 ? 148 : 1 + (int)(rng() % 600);
+    const double lean = (i % 4) * 0.1;
+    const long long pieces = 1 + (long long)(rng() % 30);
+    const b200::MoeRuns r(items, ctas, b200::moe_run_slope(items, ctas, lean));
+    wrong += r.start(0) != 0 || r.start(ctas) != items;
+    int longest = 0;
+    long long entries = 0;
+    for (int b = 0; b < ctas; ++b) {
+      const int lo = r.start(b), hi = r.start(b + 1);
+      wrong += hi < lo;
+      if (hi - lo > longest) longest = hi - lo;
+      if (hi > lo) {
+        const long long tokens = (hi + pieces - 1) / pieces - lo / pieces;
+        if (tokens > entries) entries = tokens;
+      }
+    }
+    wrong += longest > r.longest() || entries > b200::moe_run_entries(r.longest(), pieces, 1);
+    loose += r.longest() > longest + 2;
+    const double mean = (double)items / ctas;  // the first run is longer by `lean` and the last one shorter, to the unit
+    if (mean >= 5 && ctas > 1 && r.slope < 2147483647) {
+      const double gain = lean * mean * (ctas - 1) / ctas;
+      lopsided += r.start(1) < mean + gain - 3 || r.start(1) > mean + gain + 3 || items - r.start(ctas - 1) > mean - gain + 3;
+    }
+  }
+  std::printf("%lld %lld %lld", wrong, loose, lopsided);
+}
+""")
+    exe = str(tmp_path / "runs")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-fsanitize=undefined", "-fno-sanitize-recover", "-I", _ext.CSRC_DIR,
+                    str(tmp_path / "main.cpp"), "-o", exe], check=True)
+    assert subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split() == ["0", "0", "0"]
+
+
 def test_plan_cache_keeps_sizes_apart(tmp_path):
     """csrc/plan_cache.h: what `make` gave for the size, the SM count and the device at hand, and slots that do not meet for
     two layers of one model at the same batch size."""
