@@ -1704,6 +1704,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return py::make_tuple(p.bn, p.splits);
   });
   m.def("fp8_gemm_share", [](int bn, int splits) { return py::make_tuple(b200::fp8_gemm_smem(bn, splits), 512); });
+  // how many clusters of so many CTAs of the tile kernel fit on the current device at once: what its planner goes by
+  m.def("gemm_cluster_capacity", [](int size) {
+    TORCH_CHECK(size >= 2 && size <= 16, "clusters have 2 to 16 CTAs");
+    return b200::gemm_cluster_capacity(size);
+  });
   m.def("gemm_local_plan", [](int M, int N, int K, int sms) {  // one rank
     TORCH_CHECK(M > 0 && N > 0 && K > 0, "sizes must be positive");
     const b200::GemmLocalPlan p = b200::gemm_local_plan(M, N, K, sms);

@@ -13,6 +13,18 @@ def _ext():
     return _ext.load()
 
 
+# The planners of the one-rank GEMM and of the fp8 GEMM are functions of the problem's size, the number of SMs and how many
+# clusters of 2, 3 .. 16 CTAs fit on the device at once.  Sizes that are to reach a certain path are chosen for this part.
+_PART = (148, (74, 45, 33, 26, 22, 15, 15, 15, 11, 7, 7, 7, 7, 7, 7))
+
+
+def _check_plan(got, want):
+    part = (torch.cuda.get_device_properties(0).multi_processor_count, tuple(_ext().gemm_cluster_capacity(i) for i in range(2, 17)))
+    if part != _PART:
+        pytest.skip(f"right, and planned here as {got}: this part has {part}, the size is chosen for {_PART}")
+    assert got == want
+
+
 def test_extension_is_loaded_from_tree():
     mod = _ext()
     assert mod.__file__.endswith("_C/b200_ext.so")
@@ -393,9 +405,9 @@ def test_gemm_world1_matches_fp32_reference(m, n, k, has_bias):
         (33, 520, 1032),  # ragged in all three: rows of W start between cache lines
         (30, 512, 29568),  # a few tiles, K shared by a large cluster
         (90, 2048, 2752),  # ... by a small one
-        (256, 5120, 6400),  # CTA pairs, one tile each
-        (700, 2208, 1112),  # several tiles along M, short last ones
-        (129, 8192, 264),  # one row more than a tile
+        (256, 5120, 6400),  # CTA pairs, two of them to a tile
+        (700, 2208, 1112),  # CTA pairs, one tile each; several along M, short last ones
+        (129, 8192, 264),  # one row more than a tile: swapped, on pairs
         (2048, 2880, 2880),  # persistent pairs, whole tiles
         (2560, 4096, 1032),  # ... ragged along K
         (4162, 1248, 4280),  # ... and tiles cut along K, ragged
@@ -428,22 +440,24 @@ def test_gemm_one_rank_schedules(m, n, k):
     [  # kernel, which operand has the 128 rows, CTAs, where the parts of a shared tile meet / accumulators / cut tiles
         ("tile normal single", 202, 656, 256),
         ("tile normal single shared own", 4, 512, 1152),
-        ("tile normal single shared pipeline", 1066, 536, 2512),
+        ("tile normal single shared pipeline", 1058, 624, 3104),
         ("tile normal pair", 386, 688, 328),
         ("tile normal pair shared own", 388, 736, 912),
-        ("tile normal pair shared pipeline", 221, 1240, 7984),
+        ("tile normal pair shared pipeline", 1528, 528, 5152),
         ("tile swapped single", 1, 512, 256),
         ("tile swapped single shared own", 1, 512, 904),
         ("tile swapped single shared pipeline", 67, 1856, 3880),
         ("tile swapped pair", 206, 1168, 344),
         ("tile swapped pair shared own", 1, 4416, 5792),
-        ("tile swapped pair shared pipeline", 921, 656, 2576),
-        ("pair normal", 2739, 800, 256),
-        ("pair normal cut", 7454, 520, 1368),
-        ("pair normal two accumulators", 7556, 864, 2616),
+        ("tile swapped pair shared pipeline", 632, 512, 5384),
+        ("pair normal", 1822, 3352, 104),
+        ("pair normal cut", 1180, 4088, 2584),
+        ("pair normal two accumulators", 4759, 5240, 4424),  # three waves
+        ("pair normal two accumulators", 3441, 1944, 3344),
         ("pair swapped", 411, 7280, 256),
         ("pair swapped cut", 522, 7568, 1936),
-        ("pair swapped two accumulators", 6119, 1160, 2440),
+        ("pair swapped two accumulators", 2551, 6744, 3984),  # two waves
+        ("pair swapped two accumulators", 1465, 4688, 3816),
     ],
 )
 def test_gemm_one_rank_reaches_every_path(kind, m, n, k):
@@ -469,8 +483,7 @@ def test_gemm_one_rank_reaches_every_path(kind, m, n, k):
             got += ["shared", "own" if p["own_parts"] else "pipeline"]
     else:
         got += ["cut"] * (p["cut_tiles"] > 0) + ["two accumulators"] * (p["halves"] == 2)
-    if " ".join(got) != kind:  # (cluster capacities differ between parts of the same name)
-        pytest.skip("right, but planned here as: " + " ".join(got))
+    _check_plan(" ".join(got), kind)
 
 
 @pytest.mark.parametrize(
@@ -489,10 +502,8 @@ def test_gemm_one_rank_reaches_every_path(kind, m, n, k):
 )
 def test_gemm_one_rank_widths_of_an_odd_number_of_chunks(kind, m, n, k):
     """Tiles of 96, 160 and 224 columns, whose groups leave chunk by chunk."""
-    plan = _ext().gemm_local_plan(m, n, k, torch.cuda.get_device_properties(0).multi_processor_count)
     test_gemm_one_rank_reaches_every_path(kind, m, n, k)
-    if plan["bn"] % 64 == 0:
-        pytest.skip(f"right, but planned here with {plan['bn']} columns")
+    assert _ext().gemm_local_plan(m, n, k, _PART[0])["bn"] % 64 == 32
 
 
 @pytest.mark.parametrize(
@@ -507,6 +518,7 @@ def test_gemm_one_rank_widths_of_an_odd_number_of_chunks(kind, m, n, k):
 def test_gemm_one_rank_reaches_the_widths_of_whole_groups(kind, m, n, k):
     """The same paths at multiples of 64 columns."""
     test_gemm_one_rank_reaches_every_path(kind, m, n, k)
+    assert _ext().gemm_local_plan(m, n, k, _PART[0])["bn"] % 64 == 0
 
 
 @pytest.mark.parametrize("m,n,k,has_bias", [(64, 2880, 360, True), (512, 4096, 1536, True), (2048, 2880, 360, True)])
@@ -523,18 +535,17 @@ def test_gemm_world1_reference_inputs_pass_reference_checker(m, n, k, has_bias):
     assert oracle.relative_error(out, truth) < 5e-3
 
 
-@pytest.mark.parametrize("block_n,cta_pair,splits",
-                         [(64, 0, 1), (128, 0, 1), (256, 0, 1), (128, 1, 1), (192, 1, 1), (256, 1, 1),
-                          (256, 1, 3), (192, 1, 2), (128, 0, 4)])
-@pytest.mark.parametrize("m,n,k", [(384, 1024, 832), (128, 256, 64), (1000, 2880, 360), (2048, 2048, 2048)])
-def test_gemm_tile_shapes_single_cta_and_cta_pair(block_n, cta_pair, splits, m, n, k):
+@pytest.mark.parametrize(
+    "m,n,k,block_n,cta_pair,splits",
+    [(*size, *tile) for size in ((384, 1024, 832), (128, 256, 64), (1000, 2880, 360), (2048, 2048, 2048))
+     for tile in ((64, 0, 1), (128, 0, 1), (256, 0, 1), (128, 1, 1), (192, 1, 1), (256, 1, 1), (256, 1, 3), (192, 1, 2), (128, 0, 4))
+     if tile[2] <= (size[2] + 63) // 64])  # (no more K slices than k-blocks)
+def test_gemm_tile_shapes_single_cta_and_cta_pair(m, n, k, block_n, cta_pair, splits):
     """Every tile width, as single CTAs and as CTA pairs (256-row tiles, odd block counts
     and ragged edges included), gives the same GEMM."""
     from amd_distributed_2025_b200.models import gemm_rs
 
     a, w, bias = contract.make_gemm_rs_inputs(0, 1, m, n, k, True, 9, device="cuda")
-    if splits > (k + 63) // 64:
-        pytest.skip("more K slices than k-blocks")
     op = gemm_rs.get_op(m, n, k)
     op.block_n, op.cta_pair, op.splits = block_n, cta_pair, splits
     try:
@@ -587,6 +598,29 @@ def test_fp8_gemm_schedules(m, n, k):
 
 
 @pytest.mark.parametrize(
+    "bn,splits,m,n,k",
+    [
+        (64, 1, 2638, 784, 144),  # several waves; two K blocks, the second one ragged
+        (64, 2, 788, 326, 3408),
+        (64, 4, 518, 179, 2032),
+        (64, 5, 154, 120, 1840),  # 16 columns for each of the five, but none for the last
+        (64, 7, 129, 112, 2384),  # one row in the second CTA of the pair
+        (64, 8, 176, 110, 2944),
+        (128, 1, 361, 2824, 176),
+        (128, 1, 3687, 1096, 144),  # several waves
+        (128, 1, 2803, 1556, 16),  # part of a K block
+        (128, 2, 270, 1896, 5824),
+        (128, 3, 139, 2335, 5088),  # 48, 48 and 32 columns to finish; rows of C are no whole 16-byte pieces
+        (128, 4, 338, 750, 5440),
+    ],
+)
+def test_fp8_gemm_narrow_tiles(bn, splits, m, n, k):
+    """Tiles of 64 and 128 columns, whole and shared."""
+    _fp8_gemm_against_fp64(m, n, k)
+    _check_plan(_ext().fp8_gemm_plan(m, n, k, _PART[0]), (bn, splits))
+
+
+@pytest.mark.parametrize(
     "bn,m,n,k",
     [
         (192, 1000, 3003, 656),  # one wave: rows and columns end inside a tile, rows of C are no whole 16-byte pieces
@@ -594,11 +628,17 @@ def test_fp8_gemm_schedules(m, n, k):
         (256, 640, 5003, 656),
         (256, 257, 9000, 400),  # one row in the second row of tiles; four K blocks: one set of scales
         (256, 3000, 5904, 528),  # several waves, five K blocks: one of them in a set of its own
-        (256, 4096, 4096, 128),  # one K block
+        (256, 1118, 6664, 128),  # one K block, several waves
     ],
 )
 def test_fp8_gemm_wide_tiles(bn, m, n, k):
-    """Tiles of 192 and 256 columns against fp64.  A sum rounds once to bf16 (2^-9 of it at most); partial sums are fp32."""
+    """Tiles of 192 and 256 columns."""
+    _fp8_gemm_against_fp64(m, n, k)
+    _check_plan(_ext().fp8_gemm_plan(m, n, k, _PART[0]), (bn, 1))
+
+
+def _fp8_gemm_against_fp64(m, n, k):
+    """A sum rounds once to bf16 (2^-9 of it at most); partial sums are fp32."""
     from amd_distributed_2025_b200.ops.fp8_gemm import fp8_gemm
 
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
@@ -613,9 +653,6 @@ def test_fp8_gemm_wide_tiles(bn, m, n, k):
     assert torch.equal(out, fp8_gemm(a, b, a_scale, b_scale))
     assert oracle.relative_error(out, want) < 2.0**-9
     assert float(((out.double() - want).abs() - want.abs() * 2.0**-8).max()) < 1e-4 * float(want.abs().max())
-    plan = _ext().fp8_gemm_plan(m, n, k, torch.cuda.get_device_properties(0).multi_processor_count)
-    if k > 128 and plan[0] != bn:  # (cluster capacities differ between parts of the same name)
-        pytest.skip(f"right, but planned here with {plan[0]} columns")
 
 
 @pytest.mark.parametrize("tma_store", [True, False])
