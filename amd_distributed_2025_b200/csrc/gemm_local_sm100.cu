@@ -777,14 +777,18 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
 // ---------------------------------------------------------------------------------------
 constexpr int kMaxSplits = 16;
 
-int gemm_cluster_capacity(int size) {
-  struct PerDevice {
-    int n[kMaxSplits + 1] = {0};
-  };
-  static thread_local PerDevice cache[16];
+namespace {
+struct ClusterCapacities {
+  int n[kMaxSplits + 1] = {0};  // by size; 0: not asked for yet
+};
+ClusterCapacities& cluster_capacities() {  // of the current device
+  static thread_local ClusterCapacities cache[16];
   int dev = 0;
   cudaGetDevice(&dev);
-  int& n = cache[dev & 15].n[size];
+  return cache[dev & 15];
+}
+int cluster_capacity(ClusterCapacities& known, int size) {
+  int& n = known.n[size];
   if (n > 0) return n;
   auto kernel = gemm_tile_kernel<true, false>;
   opt_in(kernel, kMaxDynamicSmem, true);
@@ -805,6 +809,10 @@ int gemm_cluster_capacity(int size) {
   }
   return n;
 }
+}  // namespace
+
+int gemm_cluster_capacity(int size) { return cluster_capacity(cluster_capacities(), size); }
+
 namespace {
 
 struct Plan {
@@ -849,6 +857,8 @@ int grid_ctas(const Plan& p) { return p.persistent ? 2 * p.pairs : p.p_tiles * p
 //   limit; 1.55 where a launch comes alone); a k-block costs its issuing warp 150 ns; 6.6 TB/s of HBM; then what a launch
 //   costs before and after its k-blocks.
 // The tile kernel's terms are fitted (below).
+// A size that is new to the thread pays for the search: 1.5 to 2.6 us, because a candidate whose lower bound is above the best
+// so far is not worked out, and the current device is asked for once (10 to 13 us without the two; the same plans).
 Plan make_local_plan(int M, int N, int K, int sms) {
   const int num_kb = (K + kBK - 1) / kBK;
   const double operand_bytes = 2.0 * ((double)M * K + (double)N * K);
@@ -860,6 +870,7 @@ Plan make_local_plan(int M, int N, int K, int sms) {
     return 2.0 * rows * cols * num_kb * kBK / (pflops * 1e6) * (1.0 + 0.26 * (rows_per_col - 1.0));
   };
   Plan best;
+  ClusterCapacities& capacities = cluster_capacities();
   auto keep = [&](const Plan& p) {
     if (p.ns < best.ns) best = p;
   };
@@ -871,10 +882,12 @@ Plan make_local_plan(int M, int N, int K, int sms) {
     const int P = swap ? N : M;
     const int halves = pair ? 2 : 1;  // tile height in units of `rows`
     p.q_tiles = ((swap ? M : N) + bn - 1) / bn;
-    for (int s = 1; s <= kMaxSplits / halves; ++s) {
-      if (s > 1 && s > num_kb) continue;
+    const int q_rows = bn / halves;
+    for (int s = 1; s <= std::min(kMaxSplits / halves, num_kb); ++s) {
+      const double ends_ns = (s == 1 ? 2580.0 + 6.6 * bn : 3980.0 + 30.0 * std::max(bn - 64, 0) + 70.0 * s) + (pair ? 220.0 : 0.0);
+      if (s > 1 && dram_ns * 0.825 + ends_ns >= best.ns) break;  // (and no larger s does better)
       p.splits = s;
-      const int cap = ctas_of(p) == 1 ? sms : gemm_cluster_capacity(ctas_of(p));
+      const int cap = ctas_of(p) == 1 ? sms : cluster_capacity(capacities, ctas_of(p));
       // Lower tiles when that many clusters fit at once and full ones would leave SMs without work: a share of the
       // weight for everybody.  (Not split, tiles end on the 32 rows of an epilogue warp.)
       p.rows = 128;
@@ -885,10 +898,9 @@ Plan make_local_plan(int M, int N, int K, int sms) {
       }
       p.p_tiles = (P + halves * p.rows - 1) / (halves * p.rows);
       const int64_t tiles = (int64_t)p.p_tiles * p.q_tiles;
-      const double waves = std::ceil((double)tiles / cap);
-      if (waves > 4) continue;
+      if (tiles > 4 * (int64_t)cap) continue;
+      const int waves = ((int)tiles + cap - 1) / cap;
       const int kbs = (num_kb + s - 1) / s;
-      const int q_rows = bn / halves;
       const int stages = std::min(kMaxStages, (kMaxDynamicSmem - 1024 - kTailBytes) / ((p.rows + q_rows) * kBK * 2));
       // Fitted to 2179 timed plans of 190 drawn sizes (the plan it picks is 3 % from the best of each size).  What limits
       // a tile's main loop does not add up, but does not hide behind one another either: a copy that waits for memory
@@ -896,9 +908,9 @@ Plan make_local_plan(int M, int N, int K, int sms) {
       const double kb_ns = std::max({(K % kBK == 0 ? 0.55 : 1.15) * (p.rows + q_rows), 246.0 * bn / 256.0, 140.0, 1200.0 / stages});
       const double limits[3] = {waves * kbs * kb_ns, dram_ns * 0.825,
                                 power_ns((double)p.p_tiles * halves * 128, (double)p.q_tiles * bn, (128.0 + q_rows) / bn, 1.55)};
+      if (std::max({limits[0], limits[1], limits[2]}) + ends_ns + (waves - 1) * 4000.0 >= best.ns) continue;  // (it is more than that)
       double cubes = 0.0;
       for (double t : limits) cubes += t * t * t;
-      const double ends_ns = (s == 1 ? 2580.0 + 6.6 * bn : 3980.0 + 30.0 * std::max(bn - 64, 0) + 70.0 * s) + (pair ? 220.0 : 0.0);
       p.ns = std::cbrt(cubes) + ends_ns + (waves - 1) * 4000.0;
       keep(p);
     }

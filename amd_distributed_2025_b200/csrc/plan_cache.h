@@ -1,6 +1,6 @@
-// Plans of the problem sizes that a thread has seen: a program comes back with the same few, and a search (5 to 10 us)
-// costs more than a short kernel.  Each thread keeps one plan to a slot of the hash; sizes that share a slot are searched
-// anew whenever they alternate.
+// Plans of the problem sizes that a thread has seen: a program comes back with the same few, and a search (1.5 to 2.6 us
+// for the bf16 GEMM) takes as long as a short kernel.  Each thread keeps one plan to a slot of the hash; sizes that share a
+// slot are searched anew whenever they alternate.
 #pragma once
 #include <cstdint>
 
