@@ -152,10 +152,15 @@ __device__ __forceinline__ float with_bias(float v, float b, int mode) {
   return v + b;
 }
 
-// Where an epilogue warp stands: its slab and bias values in shared memory, and how many groups it has sent off.
+// Where an epilogue warp stands: its slab and bias values in shared memory, how many groups it has sent off, and (not
+// swapped) the lane's two bias values of the group that is next.  These are asked for a group ahead, the first ones before
+// the accumulator is waited for: asked for when the group's turn came, each group waited for memory once more, and narrow
+// groups made that worse.  (us with a bias, then -> now; without one: 2558 x 1368 x 416 9.5 -> 8.7; 7.4, 3515 x 1048 x 744
+// 12.2 -> 11.4; 10.1, 5256 x 576 x 360 9.1 -> 8.9; 7.3.  The rest is arithmetic.)
 struct Emit {
   uint32_t slab, bias;
   uint32_t stores = 0;
+  uint32_t two = 0;
 };
 
 __device__ __forceinline__ float bias_of_lane(const LocalParams& p, int feature) {
@@ -170,6 +175,12 @@ __device__ __forceinline__ float bias_of_word(const LocalParams& p, const uint32
   return p.bias_mode == 2 ? b * p.bias_scale : b;
 }
 
+// The lane's bias values of group g (N is a multiple of 8: both or none).
+__device__ __forceinline__ uint32_t ask_bias(const LocalParams& p, int qrow, int g, int lane) {
+  const int n = qrow + g * p.group * 32 + 2 * lane;
+  return p.bias_mode != 0 && n < p.Q ? *reinterpret_cast<const uint32_t*>(p.bias + n) : 0u;
+}
+
 // One column group of a warp's 32 rows -- p.group chunks of 32 columns -- from fp32 to the result: bias, rounding,
 // through the warp's slab, out by TMA (which clips what lies outside the result).  chunk(c, v) gives 32 columns.
 template <bool SWAP, typename F>
@@ -179,9 +190,8 @@ __device__ __forceinline__ void emit_group(const LocalParams& p, const CUtensorM
   const uint32_t buf = group == 1 ? em.slab + (em.stores & 1u) * (kSlabBytes / 2) : em.slab;
   ++em.stores;
   if (!SWAP && p.bias_mode != 0) {
-    const int n = qrow + g * group * 32 + 2 * lane;  // N is a multiple of 8: both values or none
-    const uint32_t two = n < p.Q ? *reinterpret_cast<const uint32_t*>(p.bias + n) : 0u;
-    asm volatile("st.shared.b32 [%0], %1;" ::"r"(em.bias + (uint32_t)lane * 4u), "r"(two) : "memory");
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(em.bias + (uint32_t)lane * 4u), "r"(em.two) : "memory");
+    em.two = ask_bias(p, qrow, g + 2, lane);
   }
   if (lane == 0) {  // the store that used this buffer has read it
     if (group == 1) ptx::bulk_wait_group_read<1>();
@@ -448,6 +458,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
       const int prow = pt * 256 + (int)cta * kPRows + q * 32;
       const int qrow = p.halves == 1 ? qt * p.bn : (2 * qt + (int)acc) * p.bn;
       const float lane_bias = SWAP ? bias_of_lane(p, prow + lane) : 0.f;
+      if (!SWAP) em.two = ask_bias(p, qrow, half, lane);
       // A cut tile has two contributors: the pair that starts it, as its last piece of cut work, and the next pair,
       // as its first.  Whoever comes second, warp by warp, finds the other's accumulator in the workspace and
       // finishes the tile; nobody waits.  (A sum of two terms is the same in either order.)
@@ -685,10 +696,11 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
   if (warp >= 2) {
     const int prow = p0 + q * 32;
     const float lane_bias = SWAP ? bias_of_lane(p, prow + lane) : 0.f;
+    Emit em{slabs + (uint32_t)ew * kSlabBytes, bias_smem + (uint32_t)ew * 128u};
+    if (!SWAP && splits == 1) em.two = ask_bias(p, q0, half, lane);
     alive = wait_bar(done_bar, 0, &abort_flag, p, 400);
     ptx::tcgen05_fence_after();
     if (splits == 1 && alive && q * 32 < p.rows) {  // not split: whole groups of 32 rows
-      Emit em{slabs + (uint32_t)ew * kSlabBytes, bias_smem + (uint32_t)ew * 128u};
       for (int g = half; g * (SWAP ? 1 : p.group) < p.bn / 32; g += 2)
         emit_group<SWAP>(p, &map_out, em, g, prow, q0, lane_bias, lane,
                          [&](int c, float (&v)[32]) { load_chunk(lane_addr + c * 32, v); });
