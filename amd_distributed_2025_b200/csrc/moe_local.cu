@@ -312,10 +312,11 @@ __global__ void __launch_bounds__(FUSED ? 512 : 1024, 1) moe_local_dispatch_kern
 
 // out[t] = sum over k (ascending) of w[t, k] * expert_y[row(t, k)], fp32, rounded once; a token none of whose
 // entries was delivered gets a zero row.  One warp per (token, piece of the row), 1 KiB of KB rows at a
-// time: KB is k, or k in equal rounds of at most four.  Bound by the gather of k rows.  What counts is that a request is
-// 1 KiB of a row and that no round is partly idle, not how many loads a lane has in flight: eight whatever k is, as
-// 512 bytes of eight rows or 2 KiB of two, took (combine alone, us) 12.1 at 600 tokens, top-8, rows of 8 KiB, now 10.4;
-// 11.3 at 1500, top-6, 4 KiB, now 10.1; 4.3 at 4000, top-2, 1 KiB, now 3.3; 7.4 at 1000, top-3, 8 KiB, now 6.8.
+// time: KB is k, or k in equal rounds (the launcher says of how many at most).  Bound by the gather of k rows.  What counts
+// is that a request is 1 KiB of a row and that no round is partly idle, not how many loads a lane has in flight: eight
+// whatever k is, as 512 bytes of eight rows or 2 KiB of two, took (combine alone, rows in L2, us) 8.1 at 600 tokens, top-8,
+// rows of 8 KiB, now 6.9; 9.8 at 1500, top-6, 4 KiB, now 7.4; 4.4 at 4000, top-2, 1 KiB, now 3.2; 6.2 at 1000, top-3,
+// 8 KiB, now 5.7.
 template <typename T, int KB>
 __global__ void __launch_bounds__(256) moe_local_combine_kernel(const MoeLocalCombineParams p) {
   constexpr int N = Vec16<T>::N;
@@ -496,15 +497,23 @@ cudaError_t launch_moe_local_combine(MoeLocalCombineParams p, int sms, cudaStrea
   if (p.num_tokens == 0) return cudaSuccess;
   p.vec = (p.row_bytes & 15u) == 0 && (reinterpret_cast<uintptr_t>(p.expert_y) & 15u) == 0 &&
           (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
-  // 2 KiB pieces when every resident warp (four CTAs of eight per SM) gets one, else 1 KiB ones: 2047 tokens of
-  // 8 KiB 58.6 us against 59.7 with dispatch, 3000 of 4000 bytes 17.1 against 18.9, but 300 of 8 KiB 17.0
-  // against 13.5.
-  const int64_t row_vecs = p.row_bytes >> 4;
-  const bool plenty = p.num_tokens * row_vecs >= 2 * kPieceVecs * 32 * (int64_t)sms;
-  cut_row(p.row_bytes, p.vec != 0, plenty ? 2 * kPieceVecs : kPieceVecs, &p.pieces, &p.piece_vecs);
-  // Four rows at a time, three where every warp stays busy: 2047 tokens, top-8, rows of 8 KiB 26.4 us against 27.1; 4000,
-  // top-7, 4 KiB 24.1 and 24.4, top-4, 8 KiB (then two) 28.8 and 30.0; 600 tokens, top-8, 8 KiB 11.5 against 10.4.
-  const int most = plenty ? 3 : 4;
+  // What counts is how full the last round of the resident warps (four CTAs of eight per SM) is, and how many dependent
+  // loads an item takes: few where there is about one item a warp, many short items where there are several.
+  // Up to three entries a token, gathered at once: 2 KiB pieces as soon as every warp gets one (2250 tokens, top-1, rows
+  // of 8 KiB 5.6 us against 6.2 with 1 KiB ones, top-3 9.9 and 11.0; but 1599, top-3 9.1 and 8.2).
+  // More of them: 1 KiB pieces, and rows two at a time from 1.75 items a warp on, else up to four (us, two / up to four):
+  //   items a warp                     1.4          1.7          1.85         2.0          2.7          6
+  //   top-4, rows of 14 KiB        6.3 / 5.8    6.4 / 6.6    6.5 / 7.5    6.5 / 8.0    9.5 / 10.6   34.2 / 40.6
+  //   top-7, rows of 8 KiB         9.5 / 8.2   10.0 / 9.8   10.4 / 12.2  10.6 / 13.2  14.7 / 15.5  41.6 / 47.8
+  //   top-8, rows of 5760 bytes   10.3 / 8.8   10.7 / 12.4  11.4 / 14.4  14.2 / 15.5  18.0 / 18.2  45.5 / 53.2
+  // (Combine alone; with dispatch before it, 623 tokens, top-8, rows of 14 KiB 32.3 and 35.6.  2 KiB pieces of three rows at
+  // a time, as from two items a warp on before: 779 of these tokens 42.5, this way 40.0; 2724 tokens, top-12, rows of 4 KiB
+  // 62.3, 60.0; 1185, top-4, 14 KiB 32.8, 33.2; of 80 counts of tokens they are ahead at 22, by 2 % at most.)
+  const int64_t resident = 32 * (int64_t)sms;
+  cut_row(p.row_bytes, p.vec != 0, kPieceVecs, &p.pieces, &p.piece_vecs);
+  if (p.k <= 3 && p.num_tokens * (int64_t)(p.row_bytes >> 4) >= 2 * kPieceVecs * resident)
+    cut_row(p.row_bytes, p.vec != 0, 2 * kPieceVecs, &p.pieces, &p.piece_vecs);
+  const int most = p.k > 3 && 4 * (int64_t)p.num_tokens * p.pieces >= 7 * resident ? 2 : 4;
   const int64_t warps = (int64_t)p.num_tokens * p.pieces;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((warps + 7) / 8, 4 * (int64_t)sms));
   switch (p.dtype) {

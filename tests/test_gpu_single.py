@@ -197,10 +197,25 @@ def test_moe_one_rank_shares_of_the_ctas(E, k, H, T, dtype):
 @pytest.mark.parametrize("H,dtype", [(520, torch.bfloat16), (1000, torch.float32), (130, torch.float16)])
 def test_moe_one_rank_combine_rounds(k, H, dtype):
     """Every number of rows that combine gathers at a time, and what is left of the last round; pieces that end short, and
-    rows that are no whole vectors.  fp32 sums of k products, rounded once."""
+    rows that are no whole vectors."""
+    _combine_against_fp64(67, 16, k, H, dtype)
+
+
+@pytest.mark.parametrize("T,k,H", [
+    (1183, 3, 4096), (1184, 3, 4096),  # up to three rows: pieces of 1 KiB, and of 2 KiB where each of 4736 warps has one
+    (1169, 2, 4152),  # ... the last one 104 bytes long
+    (1035, 4, 4096), (1036, 4, 4096),  # more: up to four at a time, and two from 8288 pieces of 1 KiB on
+    (1036, 7, 4088), (2072, 13, 2048),  # a last piece that ends short; an odd number of rows
+])
+def test_moe_one_rank_combine_many_tokens(T, k, H):
+    """Where every warp of combine has one piece of a row and more."""
+    _combine_against_fp64(T, k + 1, k, H, torch.bfloat16)
+
+
+def _combine_against_fp64(T, E, k, H, dtype):
+    """fp32 sums of k products, rounded once."""
     from amd_distributed_2025_b200.models import moe_all2all
 
-    T, E = 67, 16
     cfg = contract.MoEConfig(E, k, H, T, dtype, dtype)
     gen = torch.Generator(device="cuda").manual_seed(k)
     x = torch.randn(T, H, device="cuda", generator=gen).to(dtype)
