@@ -145,11 +145,11 @@ __device__ __forceinline__ void assign_rows(const MoeLocalDispatchParams& p, con
 __device__ __forceinline__ void write_metadata(const MoeLocalDispatchParams& p, const Share& sh, int t, int lane) {
   if (lane >= p.k) return;
   const int i = t * p.k + lane;
-  const int row = sh.rows[i - sh.i0];
+  const int e = sh.ids[i - sh.i0], row = sh.rows[i - sh.i0];
   p.route[i] = row >= 0 ? make_int2(0, row) : make_int2(-1, -1);
   if (row >= 0) {
     int32_t* meta = p.expert_meta + (size_t)row * kMetaDim;
-    meta[0] = sh.ids[i - sh.i0];
+    meta[0] = e;
     meta[1] = 0;
     meta[2] = t;
     meta[3] = lane;
@@ -468,17 +468,22 @@ cudaError_t launch_moe_local_dispatch(MoeLocalDispatchParams p, int sms, cudaStr
   // 6000 entries on (4000 tokens, top-2, rows of 1 KiB, with combine: 9.2 us with 2 x 16 warps, 10.0 with 4 x 8; 606 items
   // 6.6 and 5.6).  Where the result is formed on the way there is one CTA per SM: 16 warps when each gets more than one
   // piece (4096 tokens, top-6, rows of 8 KiB: 52 us; 58 to 60 with 32 warps), eight when that is two rounds or less
-  // (128 tokens, 12 pieces per SM: 5.1 us, 6.1 with 16 warps), ten in between (300 tokens, 16 pieces: 6.2, 6.9 and 6.8).
+  // (128 tokens, 12 pieces per SM: 5.3 us, 6.0 with 16 warps), ten in between (us with 8, 10 and 16 warps: 300 tokens, 16
+  // pieces, 6.1, 5.6, 6.0; 180 tokens, 17 pieces, 7.4, 6.8, 7.3; 600 tokens, 16 pieces, 4.9, 4.3, 4.7; but at the ends of
+  // the range 520 tokens, 14 pieces, 4.5, 4.3, 4.1 and 740 tokens, 20 pieces, 5.2, 5.0, 4.7).
   const bool fused = p.out != nullptr;
   const int64_t entries = (int64_t)p.num_tokens * p.k;
   const int threads = fused ? (items > 20 * (int64_t)sms ? 512 : items > 14 * (int64_t)sms ? 320 : 256) : (entries > 6144 ? 512 : 256);
   const int warps = threads / 32;
   const int ctas = fused ? sms : (32 / warps) * sms;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((items + warps - 1) / warps, ctas));
-  // The later a CTA's tokens, the longer it counts before its first store.  Where counting is short against the stores, a
-  // tenth evens that out (4096 tokens, top-6, rows of 8 KiB: 54.5 -> 52.2 us; 1000, top-4, 4 KiB: 6.0 -> 5.9), where it is
-  // not, two tenths (4096 tokens, top-8, rows of 1 KiB: 13.4 us, with a tenth 12.8, with two 12.2).
-  const double lean = !fused || threads < 512 ? 0.0 : entries > 16384 && p.row_bytes <= 2048 ? 0.2 : 0.1;
+  // The later a CTA's tokens, the longer it counts before its first store.  With three entries a token and more, a tenth
+  // evens that out (4096 tokens, top-6, rows of 8 KiB: 55.5 us without, 53.0 with, 54.7 with two tenths; 2000, top-4, 8 KiB
+  // 17.8, 17.5, 18.1; 1500, top-3, 8 KiB 12.3, 11.8; but 1500, top-3, 14 KiB 18.8, 19.3), two tenths where counting is long
+  // against the stores (4096, top-8, 1 KiB 13.6, 13.2, 12.4; 4096, top-8, 512 bytes 11.0, 10.9, 10.5; between the two, 2000,
+  // top-8, 2 KiB 10.8, 10.4, 10.0).  With one or two, nothing on the average of 36 sizes, and up to 7 % lost (800 tokens,
+  // top-1, 14 KiB 7.3 without, 7.8 with a tenth; 1500, top-2, 14 KiB 15.1, 15.6; 3000, top-2, 4 KiB 10.6, 10.3).
+  const double lean = !fused || threads < 512 || p.k < 3 ? 0.0 : entries > 16384 && p.row_bytes <= 2048 ? 0.2 : 0.1;
   p.slope = moe_run_slope((int32_t)items, grid, lean);
   const int32_t longest = MoeRuns((int32_t)items, grid, p.slope).longest();
   p.cap = (int32_t)(moe_run_entries(longest, p.pieces, p.k) + 6) & ~3;  // (and three words, in groups of four)

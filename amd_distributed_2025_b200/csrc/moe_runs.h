@@ -16,22 +16,22 @@ namespace b200 {
 // CTAs' shared memory is cut to it.
 struct MoeRuns {
   int32_t ctas, mean, rest;  // items = mean * ctas + rest
-  int32_t slope;             // 2^16 times what the first of very many runs gains, over `ctas`
+  int32_t slope;             // 2^20 times what the first of very many runs gains, over `ctas`
 
   // (Made anew by every CTA: a launch costs the host 0.3 us more with 168 bytes of parameters than with 152.)
   B200_HOST_DEVICE MoeRuns(int32_t items, int32_t n, int32_t s) : ctas(n), mean(items / n), rest(items % n), slope(s) {}
   B200_HOST_DEVICE int32_t start(int32_t b) const {
-    return b * mean + (b < rest ? b : rest) + (int32_t)(((int64_t)slope * b * (ctas - b)) >> 16);
+    return b * mean + (b < rest ? b : rest) + (int32_t)(((int64_t)slope * b * (ctas - b)) >> 20);
   }
-  B200_HOST_DEVICE int32_t longest() const { return mean + 2 + (int32_t)(((int64_t)slope * (ctas - 1)) >> 16); }
+  B200_HOST_DEVICE int32_t longest() const { return mean + 2 + (int32_t)(((int64_t)slope * (ctas - 1)) >> 20); }
 };
 
 // The slope at which the first run gains the fraction `lean` (up to a half) of the mean, and the last one loses it.  None
 // for runs of fewer than four items, the last of which could end before it starts.
 inline int32_t moe_run_slope(int32_t items, int32_t ctas, double lean) {
   const int32_t mean = items / ctas;
-  const double slope = mean < 4 ? 0.0 : lean * 65536.0 * mean / ctas;
-  return slope < 2147483647.0 ? (int32_t)slope : 2147483647;
+  const double slope = mean < 4 ? 0.0 : lean * 1048576.0 * mean / ctas;
+  return slope < 2147483647.0 ? (int32_t)slope : 2147483647;  // (less of a lean beyond 2^27 items)
 }
 
 // Entries of the tokens that a run of `longest` items may touch: the first and the last token may be shared with neighbours.

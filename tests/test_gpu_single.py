@@ -145,6 +145,8 @@ def test_moe_one_rank_kernels_at_the_edges_of_their_ranges(E, k, H, T, M, dtype)
         (31, 3, 4096, 260, torch.bfloat16),  # ... one piece more, ten
         (40, 5, 4096, 370, torch.bfloat16),  # 20 pieces per SM, ten warps ...
         (40, 5, 4096, 371, torch.bfloat16),  # ... one more, sixteen, and shorter runs for later CTAs
+        (40, 2, 4096, 371, torch.bfloat16),  # ... and equal ones with two entries a token
+        (9, 3, 512, 3000, torch.float16),  # 20 pieces and a bit per SM, runs of 22 down to 18
         (7, 6, 256, 1024, torch.float16),  # plain dispatch: the most entries that eight warps per CTA take ...
         (7, 6, 256, 1025, torch.float16),  # ... and sixteen; more own entries than one warp ranks at a time
         (130, 5, 1030, 3301, torch.bfloat16),  # rows that are no whole vectors, 16505 entries, own ones not a multiple of 4
