@@ -742,7 +742,8 @@ class GemmRsEngine {
   // nothing was done, take the checked path.
   c10::optional<at::Tensor> try_run(const at::Tensor& a, const at::Tensor& w, const c10::optional<at::Tensor>& bias,
                                     bool bias_at_source) {
-    if (heap_->world_size() != 1 || !heap_->peers_open() || heap_->status_host().code != 0 || !a.is_cuda() || !w.is_cuda() || a.dim() != 2 || w.dim() != 2 ||
+    if (heap_->world_size() != 1 || !heap_->peers_open() || heap_->status_host().code != 0 || !a.is_cuda() ||
+        !w.is_cuda() || a.dim() != 2 || w.dim() != 2 ||
         a.scalar_type() != at::kBFloat16 || w.scalar_type() != at::kBFloat16 || !a.is_contiguous() || !w.is_contiguous() ||
         a.get_device() != heap_->device() || w.get_device() != heap_->device())
       return c10::nullopt;
@@ -750,7 +751,8 @@ class GemmRsEngine {
     if (M <= 0 || N <= 0 || K <= 0 || K != w.size(1) || K % 8 != 0 || N % 8 != 0) return c10::nullopt;
     const void* bias_ptr = nullptr;
     if (bias.has_value() && bias->defined()) {
-      if (!bias->is_cuda() || bias->scalar_type() != at::kBFloat16 || bias->numel() != N || !bias->is_contiguous()) return c10::nullopt;
+      if (!bias->is_cuda() || bias->scalar_type() != at::kBFloat16 || bias->numel() != N || !bias->is_contiguous())
+        return c10::nullopt;
       bias_ptr = bias->const_data_ptr();
     }
     c10::cuda::CUDAGuard guard(heap_->device());
@@ -764,10 +766,11 @@ class GemmRsEngine {
   static bool aligned16(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15u) == 0; }
   // the one-rank kernel plans for itself: any knob set by hand means the multi-rank kernel
   bool local_applies(const at::Tensor& a, const at::Tensor& w, const at::Tensor& out) const {
-    return heap_->world_size() == 1 && !force_staged && max_ctas == 0 && block_n == 0 && cta_pair < 0 && splits == 0 && debug == 0 &&
-           aligned16(a) && aligned16(w) && aligned16(out);
+    return heap_->world_size() == 1 && !force_staged && max_ctas == 0 && block_n == 0 && cta_pair < 0 && splits == 0 &&
+           debug == 0 && aligned16(a) && aligned16(w) && aligned16(out);
   }
-  void run_local(const at::Tensor& a, const at::Tensor& w, const void* bias, const at::Tensor& out, bool bias_at_source, double bias_scale) {
+  void run_local(const at::Tensor& a, const at::Tensor& w, const void* bias, const at::Tensor& out, bool bias_at_source,
+                 double bias_scale) {
     b200::GemmLocalArgs g;
     g.a = a.const_data_ptr();
     g.w = w.const_data_ptr();
@@ -810,7 +813,9 @@ class GemmRsEngine {
   const LocalWorkspace* local_workspace(cudaStream_t stream) {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     unsigned long long capture = 0;
-    if (cudaStreamGetCaptureInfo(stream, &capturing, &capture) != cudaSuccess || capturing == cudaStreamCaptureStatusInvalidated) return nullptr;
+    if (cudaStreamGetCaptureInfo(stream, &capturing, &capture) != cudaSuccess ||
+        capturing == cudaStreamCaptureStatusInvalidated)
+      return nullptr;
     if (capturing == cudaStreamCaptureStatusNone) capture = 0;
     if (workspaces_of_reset_ != heap_->status_resets()) {
       workspaces_.clear();
@@ -872,7 +877,8 @@ class GemmRsEngine {
 int device_sms(int device) {
   static const std::vector<int> sms = [] {
     std::vector<int> v;
-    for (int d = 0; d < (int)at::cuda::device_count(); ++d) v.push_back(at::cuda::getDeviceProperties(d)->multiProcessorCount);
+    for (int d = 0; d < (int)at::cuda::device_count(); ++d)
+      v.push_back(at::cuda::getDeviceProperties(d)->multiProcessorCount);
     return v;
   }();
   return sms.at((size_t)device);
@@ -958,11 +964,11 @@ int fp8_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& a_scale
 
 // The common call (operands and scales as the kernel wants them, result to be allocated) without a look at it from
 // Python.  None: nothing was done, take the checked path.
-c10::optional<at::Tensor> fp8_gemm_try(const at::Tensor& a, const at::Tensor& b, const at::Tensor& a_scale, const at::Tensor& b_scale,
-                                       int64_t timeout_ns) {
-  if (!a.is_cuda() || !b.is_cuda() || !a_scale.is_cuda() || !b_scale.is_cuda() || a.dim() != 2 || b.dim() != 2 || a_scale.dim() != 2 ||
-      b_scale.dim() != 2 || a.scalar_type() != at::kFloat8_e4m3fn || b.scalar_type() != at::kFloat8_e4m3fn || !a.is_contiguous() ||
-      !b.is_contiguous() || a_scale.scalar_type() != at::kFloat || b_scale.scalar_type() != at::kFloat)
+c10::optional<at::Tensor> fp8_gemm_try(const at::Tensor& a, const at::Tensor& b, const at::Tensor& a_scale,
+                                       const at::Tensor& b_scale, int64_t timeout_ns) {
+  if (!a.is_cuda() || !b.is_cuda() || !a_scale.is_cuda() || !b_scale.is_cuda() || a.dim() != 2 || b.dim() != 2 ||
+      a_scale.dim() != 2 || b_scale.dim() != 2 || a.scalar_type() != at::kFloat8_e4m3fn ||
+      b.scalar_type() != at::kFloat8_e4m3fn || !a.is_contiguous() || !b.is_contiguous() || a_scale.scalar_type() != at::kFloat || b_scale.scalar_type() != at::kFloat)
     return c10::nullopt;
   const int64_t M = a.size(0), N = b.size(0), K = a.size(1);
   const int64_t kb = (K + 127) / 128;
@@ -1020,10 +1026,12 @@ T& native(PyObject* o) {
   return *py::handle(o).cast<T*>();
 }
 
-PyObject* moe_try_forward(PyObject* self, PyObject* const* a, Py_ssize_t n) {  // (x, indices, weights, scale) -> result or None
+// (x, indices, weights, scale) -> result or None
+PyObject* moe_try_forward(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     count_args(n, 4);
-    return wrap(native<MoeDedupEngine>(self).try_forward(tensor_arg(a[0]), tensor_arg(a[1]), tensor_arg(a[2]), double_arg(a[3])));
+    return wrap(native<MoeDedupEngine>(self).try_forward(tensor_arg(a[0]), tensor_arg(a[1]), tensor_arg(a[2]),
+                                                         double_arg(a[3])));
   });
 }
 PyObject* moe_try_dispatch(PyObject* self, PyObject* const* a, Py_ssize_t n) {  // (x, indices) -> bool
@@ -1032,7 +1040,8 @@ PyObject* moe_try_dispatch(PyObject* self, PyObject* const* a, Py_ssize_t n) {  
     return PyBool_FromLong(native<MoeDedupEngine>(self).try_dispatch(tensor_arg(a[0]), tensor_arg(a[1])));
   });
 }
-PyObject* moe_try_combine(PyObject* self, PyObject* const* a, Py_ssize_t n) {  // (out, weights, expert_y, num_tokens or None) -> bool
+// (out, weights, expert_y, num_tokens or None) -> bool
+PyObject* moe_try_combine(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     count_args(n, 4);
     int64_t tokens = -1;  // the engine's
@@ -1042,10 +1051,12 @@ PyObject* moe_try_combine(PyObject* self, PyObject* const* a, Py_ssize_t n) {  /
       tokens = PyLong_AsLongLongAndOverflow(a[3], &overflow);
       if (tokens < 0 || overflow != 0) Py_RETURN_FALSE;  // (... or refuses it)
     }
-    return PyBool_FromLong(native<MoeDedupEngine>(self).try_combine(tensor_arg(a[0]), tensor_arg(a[1]), tensor_arg(a[2]), tokens));
+    return PyBool_FromLong(
+        native<MoeDedupEngine>(self).try_combine(tensor_arg(a[0]), tensor_arg(a[1]), tensor_arg(a[2]), tokens));
   });
 }
-PyObject* gemm_try_run(PyObject* self, PyObject* const* a, Py_ssize_t n) {  // (a, w, bias or None, bias_at_source) -> result or None
+// (a, w, bias or None, bias_at_source) -> result or None
+PyObject* gemm_try_run(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     count_args(n, 4);
     c10::optional<at::Tensor> bias;
@@ -1091,7 +1102,9 @@ PyObject* moe_forward_try(PyObject*, PyObject* const* a, Py_ssize_t n) {
       PyErr_Clear();
       Py_RETURN_NONE;
     };
-    const auto attr = [](PyObject* o, PyObject* name) { return py::reinterpret_steal<py::object>(PyObject_GetAttr(o, name)); };
+    const auto attr = [](PyObject* o, PyObject* name) {
+      return py::reinterpret_steal<py::object>(PyObject_GetAttr(o, name));
+    };
     if (!PyTuple_Check(a[0]) || PyTuple_GET_SIZE(a[0]) != 4 || !PyDict_Check(a[1])) return none();
     PyObject* const cfg = PyTuple_GET_ITEM(a[0], 0);
     PyObject* const data = PyTuple_GET_ITEM(a[0], 1);
@@ -1114,12 +1127,14 @@ PyObject* moe_forward_try(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const py::object monitor = attr(layer.ptr(), names.monitor), engine = attr(layer.ptr(), names.native);
     if (!monitor || !engine || !monitor.is_none() || !py::isinstance<MoeDedupEngine>(engine)) return none();
     const py::object x = attr(data, names.x), indices = attr(data, names.indices), weights = attr(data, names.weights);
-    if (!x || !indices || !weights || !THPVariable_Check(x.ptr()) || !THPVariable_Check(indices.ptr()) || !THPVariable_Check(weights.ptr()))
+    if (!x || !indices || !weights || !THPVariable_Check(x.ptr()) || !THPVariable_Check(indices.ptr()) ||
+        !THPVariable_Check(weights.ptr()))
       return none();
     const double r = PyFloat_AsDouble(rank);
     if (r == -1.0 && PyErr_Occurred()) return none();
     const auto y = native<MoeDedupEngine>(engine.ptr())
-                       .try_forward(THPVariable_Unpack(x.ptr()), THPVariable_Unpack(indices.ptr()), THPVariable_Unpack(weights.ptr()), 1.0 + r);
+                       .try_forward(THPVariable_Unpack(x.ptr()), THPVariable_Unpack(indices.ptr()),
+                                    THPVariable_Unpack(weights.ptr()), 1.0 + r);
     if (!y.has_value()) return none();
     if (PyObject_SetAttr(layer.ptr(), names.num_tokens, Py_None) != 0) throw py::error_already_set();  // (the engine knows)
     return THPVariable_Wrap(*y);
@@ -1130,14 +1145,16 @@ PyObject* moe_forward_try(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyMethodDef kMoeCalls[] = {B200_CALL("try_forward", moe_try_forward), B200_CALL("try_dispatch", moe_try_dispatch),
                            B200_CALL("try_combine", moe_try_combine), {nullptr, nullptr, 0, nullptr}};
 PyMethodDef kGemmCalls[] = {B200_CALL("try_run", gemm_try_run), {nullptr, nullptr, 0, nullptr}};
-PyMethodDef kModuleCalls[] = {B200_CALL("fp8_gemm_try", fp8_try), B200_CALL("moe_forward_try", moe_forward_try), {nullptr, nullptr, 0, nullptr}};
+PyMethodDef kModuleCalls[] = {B200_CALL("fp8_gemm_try", fp8_try), B200_CALL("moe_forward_try", moe_forward_try),
+                              {nullptr, nullptr, 0, nullptr}};
 #undef B200_CALL
 
 template <typename T>
 void add_methods(PyMethodDef* defs) {
   const py::handle type = py::type::of<T>();
   for (; defs->ml_name != nullptr; ++defs) {
-    const py::object method = py::reinterpret_steal<py::object>(PyDescr_NewMethod(reinterpret_cast<PyTypeObject*>(type.ptr()), defs));
+    const py::object method =
+        py::reinterpret_steal<py::object>(PyDescr_NewMethod(reinterpret_cast<PyTypeObject*>(type.ptr()), defs));
     if (!method) throw py::error_already_set();
     type.attr(defs->ml_name) = method;
   }

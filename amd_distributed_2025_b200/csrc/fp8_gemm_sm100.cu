@@ -18,14 +18,17 @@
 // distributed shared memory.
 //
 // What bounds it, in cycles per K block: tiles of up to 128 columns the operands (192 rows for 128 columns: 500 without
-// the epilogue, where the products alone take 300); wider ones the chain of one epilogue warp -- the wait for the products
-// (about 110), two reads with 128 packed additions (250), the signal that frees the buffer and the next step's scales
-// (150), a sixteenth of the result's way out (130): 960 for 256 columns, products alone 560.  So the chain is kept short:
-// one lane signals by predicate, not by branch; the wide tile fetches its next scales before it adds.  In a row of
-// calls power decides, and wide tiles move a third less operand data.
+// the epilogue, where the products alone take 300); wider ones the chain of one epilogue warp.  By its own clock, at
+// 4096 x 4096 x 2048 on tiles of 256 columns: 1000 cycles a K block, where the products alone take 560 -- 150 waiting for
+// the products, 320 for two reads with 64 packed additions each, 55 for the signal that frees the buffer, 200 for the
+// scales of the next step, and 275 between the stamps that have no name -- and 2480 a tile, 2030 of them the result's way
+// out: four waves of 18500 cycles are the 37.7 us that it takes cool.  So the chain is kept short: one lane signals by
+// predicate, not by branch; the wide tile fetches its next scales before it adds.  In a long row of calls the clock goes
+// down to 1700 MHz (42 us), and wide tiles move a third less operand data.
 // On a B200, us, cool / in a row of calls, tiles of up to 128 columns with branches -> now:
 //   4096 x 4096 x 2048 38.1 / 45.8 -> 37.2 / 43.5   8192 x 8192 x 4096 268 / 310 -> 241 / 281   2048^3 13.4 -> 12.4
-//   3545 x 4512 x 3824 78.5 / 90.5 -> 65 / 76       2048 x 5000 x 8192 84 / 102 -> 79 / 95      1024 x 4096 x 4096 21.1 -> 19.7
+//   3545 x 4512 x 3824 78.5 / 90.5 -> 65 / 76       2048 x 5000 x 8192 84 / 102 -> 79 / 95
+//   1024 x 4096 x 4096 21.1 -> 19.7
 // Tried and slower: sixteen epilogue warps (52 us at 4096 x 4096 x 2048, the waits doubled), warp-wide waits (40.8), chunks
 // read one by one (47.5), results by 32-byte stores (44.8), the last wave's tiles in halves for twice the pairs (level).
 #include <cuda.h>
@@ -74,7 +77,7 @@ struct Fp8Params {
   __nv_bfloat16* c;      // [m, n] row-major
   int M, N, k_blocks;
   long long as_stride_m, as_stride_k, bs_stride_n, bs_stride_k;
-  int m_tiles, n_tiles, band, bn, stages, stage_area;
+  int m_tiles, n_tiles, band, stages, stage_area;
   int splits;            // pairs of a cluster that share a tile
   int tma_out;           // 1: rows of C are whole 16-byte pieces: results leave through TMA
   uint64_t timeout_ns;   // of a pipeline wait
@@ -99,7 +102,8 @@ __device__ __forceinline__ void umma_fp8_pair(uint32_t tmem_d, uint64_t desc_a, 
 }
 
 // `detail` (not 0) tells which wait it was that expired: a hundred for the kind of barrier, plus its index.
-__device__ __forceinline__ bool fp8_wait(uint32_t bar, uint32_t parity, volatile int* abort, const Fp8Params& p, int detail) {
+__device__ __forceinline__ bool fp8_wait(uint32_t bar, uint32_t parity, volatile int* abort, const Fp8Params& p,
+                                         int detail) {
   uint64_t t0 = 0;  // (the clock takes longer to read than most waits last)
   for (uint32_t spins = 1; !ptx::mbar_try_wait(bar, parity); ++spins) {
     if ((spins & 255u) == 0) {
@@ -142,7 +146,10 @@ __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
 }
 
 __device__ __forceinline__ void ld_shared_f4(float* to, uint32_t from) {
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(to[0]), "=f"(to[1]), "=f"(to[2]), "=f"(to[3]) : "r"(from) : "memory");
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(to[0]), "=f"(to[1]), "=f"(to[2]), "=f"(to[3])
+               : "r"(from)
+               : "memory");
 }
 
 __device__ __forceinline__ uint32_t pack2(float2 f) {
@@ -323,7 +330,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       // ---- scales: two rows per lane, four K blocks at a time, sixteen under way ------------------------------
       const int l = (warp - 2) * 32 + lane;
       // how many neighbouring scales of a row one copy may take: addresses, group starts and the end of the row allow it
-      const uint64_t ends = reinterpret_cast<uintptr_t>(p.a_scale) / 4 | (uint64_t)p.as_stride_m | (uint64_t)kb0 | (uint64_t)p.k_blocks;
+      const uint64_t ends =
+          reinterpret_cast<uintptr_t>(p.a_scale) / 4 | (uint64_t)p.as_stride_m | (uint64_t)kb0 | (uint64_t)p.k_blocks;
       const int wide = p.as_stride_k != 1 || ends % 2 != 0 ? 1 : ends % 4 != 0 ? 2 : 4;
       uint32_t slot = 0, phase = 0;
       for (int tile = first_tile; tile < total && !abort_flag; tile += tile_step) {
@@ -346,14 +354,16 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               cp_async<8>(to + 8u, as + min(kb + 2, p.k_blocks - 2));
             } else {
 #pragma unroll
-              for (int i = 0; i < kGroup; ++i) cp_async<4>(to + 4u * i, as + (long long)min(kb + i, p.k_blocks - 1) * p.as_stride_k);
+              for (int i = 0; i < kGroup; ++i)
+                cp_async<4>(to + 4u * i, as + (long long)min(kb + i, p.k_blocks - 1) * p.as_stride_k);
             }
           }
-          if (l < 2 * kMaxChunks * kGroup) {  // block l / 8, chunk l % 8: the first half's CHUNKS in words 0.., the second's in 4..
+          if (l < 2 * kMaxChunks * kGroup) {  // block l / 8, chunk l % 8: the first half's in words 0.., the second's in 4..
             const int chunk = (l & 4 ? CHUNKS : 0) + (l & 3);
             const int n = min(nt * kBn + chunk * 32, p.N - 1);
+            const int block = min(kb + (l >> 3), p.k_blocks - 1);
             cp_async<4>(at + (uint32_t)(kGroup * kRows + l) * 4u,
-                       p.b_scale + (long long)(n >> 7) * p.bs_stride_n + (long long)min(kb + (l >> 3), p.k_blocks - 1) * p.bs_stride_k);
+                        p.b_scale + (long long)(n >> 7) * p.bs_stride_n + (long long)block * p.bs_stride_k);
           }
           cp_async_arrive(sfull_bar(slot));
           if (++slot == kScaleSlots) {
@@ -409,7 +419,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       };
       auto fetch_columns = [&]() {
 #pragma unroll
-        for (int i = 0; i < kStep; ++i) ld_shared_f4(sb[i], column_at + slot * kScaleBytes + (uint32_t)((g + i) * 2 * kMaxChunks * 4));
+        for (int i = 0; i < kStep; ++i)
+          ld_shared_f4(sb[i], column_at + slot * kScaleBytes + (uint32_t)((g + i) * 2 * kMaxChunks * 4));
       };
       auto next_step = [&](bool more) {
         g += kStep;
@@ -451,7 +462,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
               for (int d = 0; d < 2; ++d)
                 if (c + d < kChunks)
-                  ptx::tmem_ld_32x32b_x32(lane_addr + buf * buf_cols + (c + d) / CHUNKS * block_cols + (c + d) % CHUNKS * 32, v[d]);
+                  ptx::tmem_ld_32x32b_x32(
+                      lane_addr + buf * buf_cols + (c + d) / CHUNKS * block_cols + (c + d) % CHUNKS * 32, v[d]);
               if (c == 0) {
 #pragma unroll
                 for (int i = 0; i < kStep; ++i)
@@ -495,9 +507,10 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           for (int i = i0; i < i0 + 2 && i < CHUNKS; ++i) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {  // 16-byte piece j of row `lane`, at the place the 64-byte swizzle wants it
-              const uint32_t at = slab + (uint32_t)(i - i0) * 2048u + (uint32_t)lane * 64u + (uint32_t)((j ^ ((lane >> 1) & 3)) << 4);
-              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(pack2(acc[i][4 * j])), "r"(pack2(acc[i][4 * j + 1])),
-                           "r"(pack2(acc[i][4 * j + 2])), "r"(pack2(acc[i][4 * j + 3]))
+              const uint32_t at = slab + (uint32_t)(i - i0) * 2048u + (uint32_t)lane * 64u +
+                                  (uint32_t)((j ^ ((lane >> 1) & 3)) << 4);
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(pack2(acc[i][4 * j])),
+                           "r"(pack2(acc[i][4 * j + 1])), "r"(pack2(acc[i][4 * j + 2])), "r"(pack2(acc[i][4 * j + 3]))
                            : "memory");
             }
           }
@@ -544,8 +557,9 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           const int owner = col / per;
           const uint32_t to = (uint32_t)(2 * owner + cta);
           const uint32_t at = base + (uint32_t)((rank * (per / 4) + (col - owner * per) / 4) * kRows + q * 32 + lane) * 16u;
-          ptx::st_cluster_v4(at, to, acc[i][4 * j].x, acc[i][4 * j].y, acc[i][4 * j + 1].x, acc[i][4 * j + 1].y);
-          ptx::st_cluster_v4(at + kRows * 16u, to, acc[i][4 * j + 2].x, acc[i][4 * j + 2].y, acc[i][4 * j + 3].x, acc[i][4 * j + 3].y);
+          const float2* a = &acc[i][4 * j];
+          ptx::st_cluster_v4(at, to, a[0].x, a[0].y, a[1].x, a[1].y);
+          ptx::st_cluster_v4(at + kRows * 16u, to, a[2].x, a[2].y, a[3].x, a[3].y);
         }
       }
     }
@@ -640,7 +654,7 @@ Fp8Plan make_fp8_plan(int M, int N, int K, int sms) {
       if (s > 1 && waves > 1) break;
       p.clusters = (int)std::min<int64_t>(tiles, cap);
       const int kbs = (k_blocks + s - 1) / s;
-      const double power_ns = 2.0 * ((M + 255) / 256) * 256.0 * ((N + bn - 1) / bn) * bn * (double)k_blocks * kBlockK / 2.6e6;
+      const double power_ns = 2.0 * ((M + 255) / 256) * 256.0 * ((N + bn - 1) / bn) * bn * k_blocks * kBlockK / 2.6e6;
       p.ns = std::max({waves * kbs * kb_ns, power_ns, dram_ns}) +
              (s == 1 ? 2490.0 + 5.6 * bn : 5060.0 + 23.5 * std::max(bn - 64, 0) + 86.0 * s) + (waves - 1) * 7.8 * bn +
              (4 * s * p.clusters > sms ? (M <= 256 ? 910.0 : 450.0) : 0.0);
@@ -658,7 +672,7 @@ const Fp8Plan& cached_plan(int M, int N, int K, int sms) {
 }
 
 template <int CHUNKS>
-cudaError_t launch(const Fp8GemmArgs& a, const Fp8Plan& plan, const Fp8Params& p, const CUtensorMap& map_a, const CUtensorMap& map_b,
+cudaError_t launch(const Fp8Plan& plan, const Fp8Params& p, const CUtensorMap& map_a, const CUtensorMap& map_b,
                    const CUtensorMap& map_c, cudaStream_t stream) {
   static OncePerDevice once;
   const cudaError_t opted = once([] { return opt_in(fp8_gemm_kernel<CHUNKS>, kMaxDynamicSmem, CHUNKS <= 2); });
@@ -707,7 +721,6 @@ cudaError_t launch_fp8_gemm(const Fp8GemmArgs& a, cudaStream_t stream) {
   p.as_stride_k = a.as_stride_k;
   p.bs_stride_n = a.bs_stride_n;
   p.bs_stride_k = a.bs_stride_k;
-  p.bn = plan.bn;
   p.splits = plan.splits;
   p.m_tiles = (a.M + 255) / 256;
   p.n_tiles = (a.N + plan.bn - 1) / plan.bn;
@@ -725,10 +738,10 @@ cudaError_t launch_fp8_gemm(const Fp8GemmArgs& a, cudaStream_t stream) {
       (p.tma_out && !make_tensor_map(&map_c, a.c, (uint64_t)a.M, (uint64_t)a.N, 2, 32, 32, 64)))
     return cudaErrorInvalidValue;
   switch (plan.bn) {
-    case 64: return launch<1>(a, plan, p, map_a, map_b, map_c, stream);
-    case 128: return launch<2>(a, plan, p, map_a, map_b, map_c, stream);
-    case 192: return launch<3>(a, plan, p, map_a, map_b, map_c, stream);
-    default: return launch<4>(a, plan, p, map_a, map_b, map_c, stream);
+    case 64: return launch<1>(plan, p, map_a, map_b, map_c, stream);
+    case 128: return launch<2>(plan, p, map_a, map_b, map_c, stream);
+    case 192: return launch<3>(plan, p, map_a, map_b, map_c, stream);
+    default: return launch<4>(plan, p, map_a, map_b, map_c, stream);
   }
 }
 

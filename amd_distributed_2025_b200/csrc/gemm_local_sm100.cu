@@ -16,10 +16,10 @@
 //                      less operand traffic buys clock (8192 x 8192 x 28672 in a row of calls: 1280 MHz instead of the
 //                      1100 with 256 columns, and 4.5 % less time).
 //
-// Multi-rank kernel before -> these kernels, one rank, us in a row of calls: 64 x 2880 x 360 10.2 -> 4.6 (latency: a launch
-// and its call), 64 x 7168 x 18432 71 -> 47 (memory, 5.9 TB/s while cool), 256 x 5120 x 12800 58 -> 38 (memory, then the
-// meeting of the parts), 2048 x 2880 x 2880 45 -> 31 (144 tiles on 74 pairs, power), 8192 x 8192 x 28672 3135 -> 2675
-// (power).  Widths are multiples of 32 columns; with multiples of 64 only, 256 x 5120 x 12800 was three parts of 256 columns
+// Multi-rank kernel before -> these kernels, one rank, us in a row of calls (cool, then the SM clock of a long row, held
+// down at 985 W): 64 x 2880 x 360 10.2 -> 4.2 (latency: a launch and its call), 64 x 7168 x 18432 71 -> 48 (46, 1550 MHz;
+// memory, 5.9 TB/s), 256 x 5120 x 12800 58 -> 40 (35, 1455 MHz; memory, then the meeting of the parts), 2048 x 2880 x 2880
+// 45 -> 31 (27, 1500 MHz; 144 tiles on 74 pairs), 8192 x 8192 x 28672 3135 -> 2787 (2430, 1297 MHz).  Widths are multiples of 32 columns; with multiples of 64 only, 256 x 5120 x 12800 was three parts of 256 columns
 // on 120 CTAs (40 us; two parts of 160 on 128 are less to exchange), 2048 x 2880 x 2880 120 tiles of 192 (33.5 us).
 // Tried and level: as many pipeline stages as a part has k-blocks, which lets two launches share an SM.
 //
@@ -87,7 +87,8 @@ __device__ __forceinline__ void stamp(const LocalParams& p, int slot) {
   if (p.trace != nullptr) p.trace[(size_t)blockIdx.x * 8 + slot] = global_timer_ns();
 }
 
-__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* abort, const LocalParams& p, int detail) {
+__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* abort, const LocalParams& p,
+                                         int detail) {
   if (ptx::mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = global_timer_ns();
   uint32_t spins = 0;
@@ -184,8 +185,8 @@ __device__ __forceinline__ uint32_t ask_bias(const LocalParams& p, int qrow, int
 // One column group of a warp's 32 rows -- p.group chunks of 32 columns -- from fp32 to the result: bias, rounding,
 // through the warp's slab, out by TMA (which clips what lies outside the result).  chunk(c, v) gives 32 columns.
 template <bool SWAP, typename F>
-__device__ __forceinline__ void emit_group(const LocalParams& p, const CUtensorMap* map_out, Emit& em, int g, int prow, int qrow,
-                                           float lane_bias, int lane, F&& chunk) {
+__device__ __forceinline__ void emit_group(const LocalParams& p, const CUtensorMap* map_out, Emit& em, int g, int prow,
+                                           int qrow, float lane_bias, int lane, F&& chunk) {
   const int group = SWAP ? 1 : p.group;
   const uint32_t buf = group == 1 ? em.slab + (em.stores & 1u) * (kSlabBytes / 2) : em.slab;
   ++em.stores;
@@ -215,8 +216,8 @@ __device__ __forceinline__ void emit_group(const LocalParams& p, const CUtensorM
         const float mine = odd ? v[j + 1] : v[j];
         const float other = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
         const uint32_t word = odd ? pack2(other, mine) : pack2(mine, other);
-        asm volatile("st.shared.b32 [%0], %1;" ::"r"(buf + (uint32_t)(j + (odd ? 1 : 0)) * 64u + (uint32_t)(lane >> 1) * 4u), "r"(word)
-                     : "memory");
+        const uint32_t at = buf + (uint32_t)(j + (odd ? 1 : 0)) * 64u + (uint32_t)(lane >> 1) * 4u;
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(word) : "memory");
       }
     } else {
       if (p.bias_mode != 0) {
@@ -231,7 +232,7 @@ __device__ __forceinline__ void emit_group(const LocalParams& p, const CUtensorM
         }
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {  // 16-byte piece cc * 4 + j of row `lane`, at the place the 128 (64)-byte swizzle wants it
+      for (int j = 0; j < 4; ++j) {  // 16-byte piece cc * 4 + j of row `lane`, where the 128 (64)-byte swizzle wants it
         const uint32_t at = group == 2 ? buf + (uint32_t)lane * 128u + (uint32_t)(((cc * 4 + j) ^ (lane & 7)) << 4)
                                        : buf + (uint32_t)lane * 64u + (uint32_t)((j ^ ((lane >> 1) & 3)) << 4);
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(pack2(v[8 * j], v[8 * j + 1])),
@@ -742,8 +743,12 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
         for (int m = 0; m < splits; ++m) {  // ascending k
           const uint32_t from = at + (uint32_t)m * (uint32_t)(per / 4) * kPRows * 16u;
           float f[8];
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]) : "r"(from));
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "r"(from + kPRows * 16u));
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3])
+                       : "r"(from));
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7])
+                       : "r"(from + kPRows * 16u));
 #pragma unroll
           for (int e = 0; e < 8; ++e) v[e] += f[e];
         }
@@ -753,7 +758,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             if (qc + e >= p.Q) break;
-            p.out[(size_t)(qc + e) * p.N + prow] = __float2bfloat16_rn(p.bias_mode ? with_bias(v[e], lane_bias, p.bias_mode) : v[e]);
+            const float f = p.bias_mode ? with_bias(v[e], lane_bias, p.bias_mode) : v[e];
+            p.out[(size_t)(qc + e) * p.N + prow] = __float2bfloat16_rn(f);
           }
         } else if (qc < p.Q) {  // N is a multiple of 8: all eight or none
           if (p.bias_mode != 0) {
@@ -857,7 +863,9 @@ TileMemory tile_memory(int rows, int bn, int splits, bool pair) {
 }
 
 int pair_stage_bytes(int bn, int halves) { return kPBytes + halves * bn * kBK; }
-int pair_stages(int bn, int halves) { return std::min(kMaxStages, (kMaxDynamicSmem - 1024 - kTailBytes) / pair_stage_bytes(bn, halves)); }
+int pair_stages(int bn, int halves) {
+  return std::min(kMaxStages, (kMaxDynamicSmem - 1024 - kTailBytes) / pair_stage_bytes(bn, halves));
+}
 int pair_smem(int bn, int halves) { return 1024 + pair_stages(bn, halves) * pair_stage_bytes(bn, halves) + kTailBytes; }
 
 int ctas_of(const Plan& p) { return p.splits * (p.pair ? 2 : 1); }  // CTAs that share a tile
@@ -869,8 +877,8 @@ int grid_ctas(const Plan& p) { return p.persistent ? 2 * p.pairs : p.p_tiles * p
 //   limit; 1.55 where a launch comes alone); a k-block costs its issuing warp 150 ns; 6.6 TB/s of HBM; then what a launch
 //   costs before and after its k-blocks.
 // The tile kernel's terms are fitted (below).
-// A size that is new to the thread pays for the search: 1.5 to 2.6 us, because a candidate whose lower bound is above the best
-// so far is not worked out, and the current device is asked for once (10 to 13 us without the two; the same plans).
+// A size that is new to the thread pays for the search: 1.5 to 2.6 us, because a candidate whose lower bound is above the
+// best so far is not worked out, and the current device is asked for once (10 to 13 us without the two; the same plans).
 Plan make_local_plan(int M, int N, int K, int sms) {
   const int num_kb = (K + kBK - 1) / kBK;
   const double operand_bytes = 2.0 * ((double)M * K + (double)N * K);
@@ -896,7 +904,8 @@ Plan make_local_plan(int M, int N, int K, int sms) {
     p.q_tiles = ((swap ? M : N) + bn - 1) / bn;
     const int q_rows = bn / halves;
     for (int s = 1; s <= std::min(kMaxSplits / halves, num_kb); ++s) {
-      const double ends_ns = (s == 1 ? 2580.0 + 6.6 * bn : 3980.0 + 30.0 * std::max(bn - 64, 0) + 70.0 * s) + (pair ? 220.0 : 0.0);
+      const double ends_ns =
+          (s == 1 ? 2580.0 + 6.6 * bn : 3980.0 + 30.0 * std::max(bn - 64, 0) + 70.0 * s) + (pair ? 220.0 : 0.0);
       if (s > 1 && dram_ns * 0.825 + ends_ns >= best.ns) break;  // (and no larger s does better)
       p.splits = s;
       const int cap = ctas_of(p) == 1 ? sms : cluster_capacity(capacities, ctas_of(p));
@@ -917,10 +926,12 @@ Plan make_local_plan(int M, int N, int K, int sms) {
       // Fitted to 2179 timed plans of 190 drawn sizes (the plan it picks is 3 % from the best of each size).  What limits
       // a tile's main loop does not add up, but does not hide behind one another either: a copy that waits for memory
       // also waits for its turn in the SM.
-      const double kb_ns = std::max({(K % kBK == 0 ? 0.55 : 1.15) * (p.rows + q_rows), 246.0 * bn / 256.0, 140.0, 1200.0 / stages});
+      const double kb_ns =
+          std::max({(K % kBK == 0 ? 0.55 : 1.15) * (p.rows + q_rows), 246.0 * bn / 256.0, 140.0, 1200.0 / stages});
       const double limits[3] = {waves * kbs * kb_ns, dram_ns * 0.825,
-                                power_ns((double)p.p_tiles * halves * 128, (double)p.q_tiles * bn, (128.0 + q_rows) / bn, 1.55)};
-      if (std::max({limits[0], limits[1], limits[2]}) + ends_ns + (waves - 1) * 4000.0 >= best.ns) continue;  // (it is more than that)
+                                power_ns(p.p_tiles * halves * 128.0, (double)p.q_tiles * bn, (128.0 + q_rows) / bn, 1.55)};
+      const double largest = std::max({limits[0], limits[1], limits[2]});
+      if (largest + ends_ns + (waves - 1) * 4000.0 >= best.ns) continue;  // (it is more than that)
       double cubes = 0.0;
       for (double t : limits) cubes += t * t * t;
       p.ns = std::cbrt(cubes) + ends_ns + (waves - 1) * 4000.0;
@@ -940,14 +951,15 @@ Plan make_local_plan(int M, int N, int K, int sms) {
     p.pairs = (int)std::min<int64_t>(tiles, std::min(sms / 2, kGemmLocalMaxPairs));
     if (halves == 1 && tiles == p.pairs) return;  // one wave: the tile kernel's pairs do the same 8 % faster
     // A wave takes as long as one of its tiles, or as the power for all of them: a last wave of few tiles has power to
-    // spare, and its tiles still take their time (2048 x 5120 x 12800: 231 us in 2.2 waves of 256 columns, 214 in 2.9 of 192).
+    // spare, and its tiles still take their time (2048 x 5120 x 12800: 231 us in 2.2 waves of 256 columns, 214 in 2.9 of
+    // 192).
     const double wave_ns = power_ns(256.0 * p.pairs, cols, (128.0 + cols / 2) / cols, 1.45);
     const double tile_ns = num_kb * std::max({row_ns * (128 + cols / 2), 280.0 * cols / 256.0, 150.0});
     const int64_t whole = tiles / p.pairs, last = tiles % p.pairs;
     const int64_t waves = whole + (last > 0 ? 1 : 0);
     p.sk_tiles = 0;
-    p.ns = std::max(whole * std::max(tile_ns, wave_ns) + (last > 0 ? std::max(tile_ns, wave_ns * last / p.pairs) : 0.0), dram_ns) + 3400.0 +
-           9.0 * cols;
+    const double last_ns = last > 0 ? std::max(tile_ns, wave_ns * last / p.pairs) : 0.0;
+    p.ns = std::max(whole * std::max(tile_ns, wave_ns) + last_ns, dram_ns) + 3400.0 + 9.0 * cols;
     // With both accumulators in one tile, 5.5 us of its epilogue do not run beside products (all pairs store at once).
     if (halves == 2) p.ns += waves * 5500.0;
     keep(p);
@@ -959,7 +971,8 @@ Plan make_local_plan(int M, int N, int K, int sms) {
       // not hold comes from memory for every tile (1923 x 5056 x 19824: 429 us cut, 335 in whole tiles of 192 columns).
       const double cut = (double)last / p.pairs;
       const double apart_ns = operand_bytes > 126e6 ? 0.4 * p.sk_tiles * num_kb * (256.0 + cols) * kBK * 2 / 6600.0 : 0.0;
-      p.ns = std::max((double)tiles / p.pairs * std::max(tile_ns, wave_ns) * (1.05 + 0.3 * cut), dram_ns) + apart_ns + 3400.0 + 9.0 * bn + 5000.0;
+      const double tiles_ns = (double)tiles / p.pairs * std::max(tile_ns, wave_ns) * (1.05 + 0.3 * cut);
+      p.ns = std::max(tiles_ns, dram_ns) + apart_ns + 3400.0 + 9.0 * bn + 5000.0;
       keep(p);
     }
   };
@@ -1018,8 +1031,8 @@ bool common_params(LocalParams& p, const GemmLocalArgs& a, const Plan& plan, int
 }
 
 template <typename K>
-cudaError_t launch(K kernel, const LocalParams& p, int ctas, int cluster, size_t smem, cudaStream_t stream, const CUtensorMap& map_p,
-                   const CUtensorMap& map_q, const CUtensorMap& map_out) {
+cudaError_t launch(K kernel, const LocalParams& p, int ctas, int cluster, size_t smem, cudaStream_t stream,
+                   const CUtensorMap& map_p, const CUtensorMap& map_q, const CUtensorMap& map_out) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ctas);
   cfg.blockDim = dim3(kThreads);
@@ -1053,7 +1066,8 @@ cudaError_t launch_pair(const GemmLocalArgs& a, const Plan& plan, cudaStream_t s
   static OncePerDevice once;
   const cudaError_t opted = once([] { return opt_in(gemm_pair_kernel<SWAP>, kMaxDynamicSmem, false); });
   if (opted != cudaSuccess) return opted;
-  return launch(gemm_pair_kernel<SWAP>, p, grid_ctas(plan), 2, (size_t)pair_smem(plan.bn, plan.halves), stream, map_p, map_q, map_out);
+  const size_t smem = (size_t)pair_smem(plan.bn, plan.halves);
+  return launch(gemm_pair_kernel<SWAP>, p, grid_ctas(plan), 2, smem, stream, map_p, map_q, map_out);
 }
 
 template <bool SWAP, bool PAIR>
@@ -1071,7 +1085,8 @@ cudaError_t launch_tile(const GemmLocalArgs& a, const Plan& plan, cudaStream_t s
   static OncePerDevice once;
   const cudaError_t opted = once([] { return opt_in(gemm_tile_kernel<SWAP, PAIR>, kMaxDynamicSmem, true); });
   if (opted != cudaSuccess) return opted;
-  return launch(gemm_tile_kernel<SWAP, PAIR>, p, grid_ctas(plan), ctas_of(plan), (size_t)mem.smem, stream, map_p, map_q, map_out);
+  return launch(gemm_tile_kernel<SWAP, PAIR>, p, grid_ctas(plan), ctas_of(plan), (size_t)mem.smem, stream, map_p, map_q,
+                map_out);
 }
 
 }  // namespace
@@ -1085,10 +1100,12 @@ SmShare gemm_pair_share(int bn, int halves) { return {pair_smem(bn, halves), kTm
 GemmLocalPlan gemm_local_plan(int M, int N, int K, int sms) {
   const Plan& p = cached_plan(M, N, K, sms);
   const bool own_parts = !p.persistent && tile_memory(p.rows, p.bn, p.splits, p.pair).part_bytes > 0;
-  return {p.persistent, p.swap, p.persistent || p.pair, own_parts, p.rows, p.bn, p.splits, p.halves, p.sk_tiles, grid_ctas(p)};
+  return {p.persistent, p.swap, p.persistent || p.pair, own_parts, p.rows, p.bn, p.splits, p.halves, p.sk_tiles,
+          grid_ctas(p)};
 }
 
-cudaError_t launch_gemm_local(GemmLocalArgs& a, int device, const std::function<void(GemmLocalArgs&)>& workspace, cudaStream_t stream) {
+cudaError_t launch_gemm_local(GemmLocalArgs& a, int device, const std::function<void(GemmLocalArgs&)>& workspace,
+                              cudaStream_t stream) {
   if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.K % 8 != 0 || a.N % 8 != 0) return cudaErrorInvalidValue;
   Plan plan = cached_plan(a.M, a.N, a.K, a.sms, device);
   if (plan.persistent) {

@@ -6,8 +6,8 @@
 // by the route table.  The layouts are those of the multi-rank kernels (rows of an expert in
 // (token, k) order; 5-int metadata; per-expert counts).
 //
-// Both kernels may start before the previous kernel of the stream has ended (programmatic dependent launch): nothing
-// is read or written before grid_dep_wait(), which makes that kernel's stores visible.  Ids, routes, weights and whole
+// Both kernels may start before the previous kernel of the stream has ended (programmatic dependent launch): no global
+// memory is read or written before grid_dep_wait(), which makes that kernel's stores visible.  Ids, routes, weights and whole
 // vectors are read past L1 (ld.global.cg), as nothing comes back for them; ragged rows, element by element, are not.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -238,8 +238,9 @@ __global__ void __launch_bounds__(FUSED ? 512 : 1024, 1) moe_local_dispatch_kern
     stamp_cta0(p.trace_c, 1);
   }
   // The next launch is let in when the stores begin (its CTAs would only stand in line for the SMs before: 0.1 us); behind
-  // plain copies, combine as a rule, not before the CTAs leave: several of its CTAs fit on an SM, and early ones gather where
-  // a dispatch CTA has just left (111 tokens, top-7, 2 KiB, dispatch + combine 8.1 us, now 6.9; 2000, top-2, 2 KiB 8.2, now 7.8).
+  // plain copies, combine as a rule, not before the CTAs leave: several of its CTAs fit on an SM, and early ones gather
+  // where a dispatch CTA has just left (111 tokens, top-7, 2 KiB, dispatch + combine 8.1 us, now 6.9; 2000, top-2, 2 KiB
+  // 8.2, now 7.8).
   if (FUSED) ptx::grid_dep_launch();
   uint8_t* ex = reinterpret_cast<uint8_t*>(p.expert_x);
   if (p.vec) {
@@ -393,7 +394,8 @@ __global__ void __launch_bounds__(256) moe_local_combine_kernel(const MoeLocalCo
         for (int kk = 0; kk < k; ++kk) {
           const int rq = __shfl_sync(0xffffffffu, row, kk);
           const float wq = __shfl_sync(0xffffffffu, w, kk);
-          if (rq >= 0 && h < hidden) acc = fmaf(to_f32(reinterpret_cast<const T*>(p.expert_y)[(size_t)rq * hidden + h]), wq, acc);
+          const T* src = reinterpret_cast<const T*>(p.expert_y) + (size_t)max(rq, 0) * hidden;
+          if (rq >= 0 && h < hidden) acc = fmaf(to_f32(src[h]), wq, acc);
         }
         if (h < hidden) reinterpret_cast<T*>(p.out)[(size_t)t * hidden + h] = from_f32<T>(acc);
       }
@@ -418,8 +420,12 @@ void cut_row(uint32_t row_bytes, bool vec, int most, int32_t* pieces, int32_t* p
 
 // Shared memory that keeps a CTA of forward alone on its SM.  A launch of one CTA per SM starts while the one before it
 // still runs; where two fit, the scheduler may put two on each SM that happens to be free, none on the others, and the next
-// launch into the gaps, call after call: 128 tokens, top-8 took 7.05 us in a row of calls, 5.3 with one CTA to an SM (129 and
-// 136 likewise, 140 never).
+// launch into the gaps, call after call: 128 tokens, top-8 took 7.05 us in a row of calls, 5.3 with one CTA to an SM (129
+// and 136 likewise, 140 never).  What that costs: beside a kernel on another stream that holds most of the shared memory,
+// forward waits for whole SMs (beside a library GEMM of 4096^3, us a call: 128 tokens 26, two CTAs to an SM 9; 11 tokens
+// 4.7 and 4.4; 1000 tokens of 4 KiB 27 either way; beside an elementwise kernel over 512 MB 25 either way).  The other
+// remedy, to let the next launch in only when the CTAs leave, costs a row of calls less than 0.1 us at 128 tokens, but 2 to
+// 7 % in a graph and at most sizes.
 constexpr int kAloneBytes = 116 * 1024;
 
 template <typename T>
@@ -428,7 +434,8 @@ cudaError_t dispatch_typed(const MoeLocalDispatchParams& p, int threads, int gri
   static OncePerDevice once;
   const cudaError_t opted = once([] { return opt_in(moe_local_dispatch_kernel<T, true>, kAloneBytes, false); });
   if (opted != cudaSuccess) return opted;
-  return ptx::launch_dependent(moe_local_dispatch_kernel<T, true>, grid, threads, std::max<size_t>(smem, kAloneBytes), stream, p);
+  const size_t alone = std::max<size_t>(smem, kAloneBytes);
+  return ptx::launch_dependent(moe_local_dispatch_kernel<T, true>, grid, threads, alone, stream, p);
 }
 
 template <typename T>
@@ -446,12 +453,13 @@ cudaError_t combine_typed(const MoeLocalCombineParams& p, int grid, int most, cu
 
 // A CTA reads the ids of every earlier token, so that work grows with the square of the entries, where the kernel
 // with a grid barrier counts every entry once.  The line lies at the most entries that the task's generator draws, the
-// range this kernel is tested over; the two do not cross there.  bf16, us, forward / dispatch + combine, on either side:
-//   entries                                32768        65536: here, with barrier     131072: here, with barrier
-//   64 experts, top-8, rows of 8 KiB     70 / 116     135 / 230      344 / 244        266 / 451      668 / 470
-//   256 experts, top-8, rows of 2 KiB    22 / 39       44 / 71       142 / 120         85 / 129      240 / 192
-//   64 experts, top-8, rows of 512 B     13 / 18       23 / 34        66 / 55          42 / 71       115 / 95
-//   64 experts, top-4, rows of 128 B     14 / 23       24 / 41        82 / 72          44 / 74       139 / 118
+// range this kernel is tested over, and beyond which forward() writes expert_y; the two do not cross there, nor at four
+// times as many.  bf16, us, forward / dispatch + combine, this kernel and the one with the barrier:
+//   entries                                 32768                  65536                  131072
+//   64 experts, top-8, rows of 8 KiB    66/111  194/152       133/225  340/241       265/437  651/454
+//   256 experts, top-8, rows of 2 KiB   19/36    96/85         40/64   143/120        85/121  235/191
+//   64 experts, top-8, rows of 512 B    11/16    47/42         19/29    68/57         41/57   119/99
+//   64 experts, top-4, rows of 128 B    12/16    52/47         21/26    78/68         41/49   135/114
 // (8192 experts: the counts fill 32 KiB of the 48 KiB of shared memory that need no opt-in.)
 bool moe_local_dispatch_applies(int64_t num_entries, int num_experts) {
   return num_entries <= 32768 && num_experts <= 8192;
@@ -474,7 +482,8 @@ cudaError_t launch_moe_local_dispatch(MoeLocalDispatchParams p, int sms, cudaStr
   // the range 520 tokens, 14 pieces, 4.5, 4.3, 4.1 and 740 tokens, 20 pieces, 5.2, 5.0, 4.7).
   const bool fused = p.out != nullptr;
   const int64_t entries = (int64_t)p.num_tokens * p.k;
-  const int threads = fused ? (items > 20 * (int64_t)sms ? 512 : items > 14 * (int64_t)sms ? 320 : 256) : (entries > 6144 ? 512 : 256);
+  const int threads = !fused ? (entries > 6144 ? 512 : 256)
+                             : (items > 20 * (int64_t)sms ? 512 : items > 14 * (int64_t)sms ? 320 : 256);
   const int warps = threads / 32;
   const int ctas = fused ? sms : (32 / warps) * sms;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((items + warps - 1) / warps, ctas));

@@ -1,4 +1,5 @@
-// How the one-rank MoE dispatch deals its items (a token's row in pieces: tokens x pieces of them, in order) out to the CTAs.
+// How the one-rank MoE dispatch deals its items (a token's row in pieces: tokens x pieces of them, in order) out to the
+// CTAs.
 #pragma once
 #include <stdint.h>
 
@@ -35,6 +36,8 @@ inline int32_t moe_run_slope(int32_t items, int32_t ctas, double lean) {
 }
 
 // Entries of the tokens that a run of `longest` items may touch: the first and the last token may be shared with neighbours.
-inline int64_t moe_run_entries(int64_t longest, int64_t pieces, int64_t topk) { return ((longest + pieces - 2) / pieces + 1) * topk; }
+inline int64_t moe_run_entries(int64_t longest, int64_t pieces, int64_t topk) {
+  return ((longest + pieces - 2) / pieces + 1) * topk;
+}
 
 }  // namespace b200

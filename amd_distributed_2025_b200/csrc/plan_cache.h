@@ -13,7 +13,8 @@ class PlanCache {
   template <typename F>
   const Plan& get(int M, int N, int K, int sms, int device, F&& make) {
     Entry& e = entries_[slot(M, N, K)];
-    if (e.M != M || e.N != N || e.K != K || e.sms != sms || e.device != device) e = Entry{M, N, K, sms, device, make(M, N, K, sms)};
+    if (e.M != M || e.N != N || e.K != K || e.sms != sms || e.device != device)
+      e = Entry{M, N, K, sms, device, make(M, N, K, sms)};
     return e.plan;
   }
   static constexpr int kSlots = 256;
