@@ -148,6 +148,14 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
+// Two rounded products and their bias values, added and rounded again: the exact sum of two bf16 numbers either fits fp32
+// (exponents up to 16 apart) or rounds to the larger one either way, so this is with_bias() and a rounding, in one
+// instruction for both.
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t v, uint32_t b) {
+  const __nv_bfloat162 s = __hadd2_rn(*reinterpret_cast<const __nv_bfloat162*>(&v), *reinterpret_cast<const __nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&s);
+}
+
 __device__ __forceinline__ float with_bias(float v, float b, int mode) {
   if (mode == 1) return __bfloat162float(__float2bfloat16_rn(v)) + b;
   return v + b;
@@ -220,24 +228,32 @@ __device__ __forceinline__ void emit_group(const LocalParams& p, const CUtensorM
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(word) : "memory");
       }
     } else {
+      uint32_t w[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) w[j] = pack2(v[2 * j], v[2 * j + 1]);
       if (p.bias_mode != 0) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          uint32_t two[2];
-          asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];"
-                       : "=r"(two[0]), "=r"(two[1])
-                       : "r"(em.bias + (uint32_t)(cc * 32 + j) * 2u));
+        for (int j = 0; j < 4; ++j) {
+          uint32_t b[4];
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3])
+                       : "r"(em.bias + (uint32_t)(cc * 32 + j * 8) * 2u));
+          if (p.bias_mode == 1) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) v[j + e] = with_bias(v[j + e], bias_of_word(p, two, e), p.bias_mode);
+            for (int e = 0; e < 4; ++e) w[4 * j + e] = add_bf16x2(w[4 * j + e], b[e]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              w[4 * j + e] = pack2(v[8 * j + 2 * e] + bias_of_word(p, b, 2 * e), v[8 * j + 2 * e + 1] + bias_of_word(p, b, 2 * e + 1));
+          }
         }
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {  // 16-byte piece cc * 4 + j of row `lane`, where the 128 (64)-byte swizzle wants it
         const uint32_t at = group == 2 ? buf + (uint32_t)lane * 128u + (uint32_t)(((cc * 4 + j) ^ (lane & 7)) << 4)
                                        : buf + (uint32_t)lane * 64u + (uint32_t)((j ^ ((lane >> 1) & 3)) << 4);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(pack2(v[8 * j], v[8 * j + 1])),
-                     "r"(pack2(v[8 * j + 2], v[8 * j + 3])), "r"(pack2(v[8 * j + 4], v[8 * j + 5])),
-                     "r"(pack2(v[8 * j + 6], v[8 * j + 7]))
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(w[4 * j]), "r"(w[4 * j + 1]),
+                     "r"(w[4 * j + 2]), "r"(w[4 * j + 3])
                      : "memory");
       }
     }

@@ -538,6 +538,43 @@ def test_gemm_one_rank_reaches_the_widths_of_whole_groups(kind, m, n, k):
     assert _ext().gemm_local_plan(m, n, k, _PART[0])["bn"] % 64 == 0
 
 
+@pytest.mark.parametrize("m,n,k", [
+    (2048, 2880, 2880), (6345, 656, 1888), (4759, 5240, 4424), (242, 4760, 264), (134, 1040, 256), (646, 1104, 2952),  # normal
+    (411, 7280, 256), (206, 1168, 344),  # swapped
+])
+def test_gemm_one_rank_bias_is_added_to_the_rounded_product(m, n, k):
+    """Bit for bit what the library's bf16 addition makes of the product without a bias."""
+    from amd_distributed_2025_b200.models import gemm_rs
+
+    a, w, bias = contract.make_gemm_rs_inputs(0, 1, m, n, k, True, 29, device="cuda")
+    bias = (bias.float() * 2.0 ** torch.randint(-30, 8, bias.shape, device="cuda").float()).bfloat16()
+    op = gemm_rs.get_op(m, n, k)
+    plain = op(a, w, None)
+    assert torch.equal(op(a, w, bias, "per_rank"), plain + bias)
+    op.check()
+
+
+def test_gemm_one_rank_bias_of_every_kind_of_number():
+    """Products and bias values of every bit pattern, infinities, NaNs, signed zeros and subnormal numbers among them."""
+    from amd_distributed_2025_b200.models import gemm_rs
+
+    m, n, k = 256, 8192, 64
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    a = torch.zeros(m, k, dtype=torch.bfloat16, device="cuda")
+    a[:, 0] = 1.0
+    for _ in range(4):
+        w = torch.zeros(n, k, dtype=torch.bfloat16, device="cuda")
+        w[:, 0] = torch.randint(-32768, 32768, (n,), device="cuda", generator=gen).short().view(torch.bfloat16)
+        bias = torch.randint(-32768, 32768, (n,), device="cuda", generator=gen).short().view(torch.bfloat16)
+        near = torch.rand(n, device="cuda", generator=gen) < 0.5  # exponents that are close, or the sum is one of the two
+        bias = torch.where(near, (w[:, 0].float() * -1.007).bfloat16(), bias)
+        op = gemm_rs.get_op(m, n, k)
+        want = op(a, w, None) + bias
+        got = op(a, w, bias, "per_rank")
+        assert torch.equal(got.isnan(), want.isnan())
+        assert torch.equal(got[~want.isnan()].view(torch.int16), want[~want.isnan()].view(torch.int16))
+
+
 @pytest.mark.parametrize("m,n,k,has_bias", [(64, 2880, 360, True), (512, 4096, 1536, True), (2048, 2880, 360, True)])
 def test_gemm_world1_reference_inputs_pass_reference_checker(m, n, k, has_bias):
     """Operands from the reference generator (uniform +-0.01) against the library path."""
