@@ -968,7 +968,8 @@ c10::optional<at::Tensor> fp8_gemm_try(const at::Tensor& a, const at::Tensor& b,
                                        const at::Tensor& b_scale, int64_t timeout_ns) {
   if (!a.is_cuda() || !b.is_cuda() || !a_scale.is_cuda() || !b_scale.is_cuda() || a.dim() != 2 || b.dim() != 2 ||
       a_scale.dim() != 2 || b_scale.dim() != 2 || a.scalar_type() != at::kFloat8_e4m3fn ||
-      b.scalar_type() != at::kFloat8_e4m3fn || !a.is_contiguous() || !b.is_contiguous() || a_scale.scalar_type() != at::kFloat || b_scale.scalar_type() != at::kFloat)
+      b.scalar_type() != at::kFloat8_e4m3fn || !a.is_contiguous() || !b.is_contiguous() ||
+      a_scale.scalar_type() != at::kFloat || b_scale.scalar_type() != at::kFloat)
     return c10::nullopt;
   const int64_t M = a.size(0), N = b.size(0), K = a.size(1);
   const int64_t kb = (K + 127) / 128;

@@ -19,8 +19,9 @@
 // Multi-rank kernel before -> these kernels, one rank, us in a row of calls (cool, then the SM clock of a long row, held
 // down at 985 W): 64 x 2880 x 360 10.2 -> 4.2 (latency: a launch and its call), 64 x 7168 x 18432 71 -> 48 (46, 1550 MHz;
 // memory, 5.9 TB/s), 256 x 5120 x 12800 58 -> 40 (35, 1455 MHz; memory, then the meeting of the parts), 2048 x 2880 x 2880
-// 45 -> 31 (27, 1500 MHz; 144 tiles on 74 pairs), 8192 x 8192 x 28672 3135 -> 2787 (2430, 1297 MHz).  Widths are multiples of 32 columns; with multiples of 64 only, 256 x 5120 x 12800 was three parts of 256 columns
-// on 120 CTAs (40 us; two parts of 160 on 128 are less to exchange), 2048 x 2880 x 2880 120 tiles of 192 (33.5 us).
+// 45 -> 31 (27, 1500 MHz; 144 tiles on 74 pairs), 8192 x 8192 x 28672 3135 -> 2787 (2430, 1297 MHz).  Widths are multiples
+// of 32 columns; with multiples of 64 only, 256 x 5120 x 12800 was three parts of 256 columns on 120 CTAs (40 us; two parts
+// of 160 on 128 are less to exchange), 2048 x 2880 x 2880 120 tiles of 192 (33.5 us).
 // Tried and level: as many pipeline stages as a part has k-blocks, which lets two launches share an SM.
 //
 // Warp roles of both (320 threads): 0 TMA producer, 1 MMA issuer, 2..9 epilogue, two per tensor-memory lane quarter.
@@ -152,7 +153,8 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 // (exponents up to 16 apart) or rounds to the larger one either way, so this is with_bias() and a rounding, in one
 // instruction for both.
 __device__ __forceinline__ uint32_t add_bf16x2(uint32_t v, uint32_t b) {
-  const __nv_bfloat162 s = __hadd2_rn(*reinterpret_cast<const __nv_bfloat162*>(&v), *reinterpret_cast<const __nv_bfloat162*>(&b));
+  const __nv_bfloat162 s =
+      __hadd2_rn(*reinterpret_cast<const __nv_bfloat162*>(&v), *reinterpret_cast<const __nv_bfloat162*>(&b));
   return *reinterpret_cast<const uint32_t*>(&s);
 }
 
@@ -244,7 +246,8 @@ __device__ __forceinline__ void emit_group(const LocalParams& p, const CUtensorM
           } else {
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-              w[4 * j + e] = pack2(v[8 * j + 2 * e] + bias_of_word(p, b, 2 * e), v[8 * j + 2 * e + 1] + bias_of_word(p, b, 2 * e + 1));
+              w[4 * j + e] = pack2(v[8 * j + 2 * e] + bias_of_word(p, b, 2 * e),
+                                   v[8 * j + 2 * e + 1] + bias_of_word(p, b, 2 * e + 1));
           }
         }
       }

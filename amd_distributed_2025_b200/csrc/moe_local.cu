@@ -7,8 +7,8 @@
 // (token, k) order; 5-int metadata; per-expert counts).
 //
 // Both kernels may start before the previous kernel of the stream has ended (programmatic dependent launch): no global
-// memory is read or written before grid_dep_wait(), which makes that kernel's stores visible.  Ids, routes, weights and whole
-// vectors are read past L1 (ld.global.cg), as nothing comes back for them; ragged rows, element by element, are not.
+// memory is read or written before grid_dep_wait(), which makes that kernel's stores visible.  Ids, routes, weights and
+// whole vectors are read past L1 (ld.global.cg), as nothing comes back for them; ragged rows, element by element, are not.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
