@@ -106,9 +106,12 @@ def report(bench_line: Dict, peaks: Optional[Dict[str, float]] = None) -> Dict[s
             rows = _moe_remote_rows(spec, ws)
             row_bytes = spec["hidden_dim"] * 2
             link = moe_roofline_us(rows["out"], rows["in"], row_bytes, peaks)["roofline_us"]
-            # local floor: per entry one write each of expert_x and expert_y and one read of expert_y,
-            # per token one read of x and one write of the result
-            local_bytes = (3.0 * spec["experts_per_token"] + 2.0) * spec["tokens_per_rank"] * row_bytes
+            # local floor: per entry one write each of expert_x and expert_y and one read of expert_y, per token one
+            # read of x and one write of the result; one rank's forward() forms the result from the rows that it
+            # delivers and leaves expert_y alone (csrc/moe_local.cu, up to 32768 entries)
+            entries = spec["experts_per_token"] * spec["tokens_per_rank"]
+            passes = 1.0 if ws == 1 and entries <= 32768 else 3.0
+            local_bytes = (passes * entries + 2.0 * spec["tokens_per_rank"]) * row_bytes
             roof = max(link, local_bytes / (peaks["hbm_gbs"] * 1e9) * 1e6)
         out[name] = {"measured_us": measured["us"], "roofline_us": roof, "fraction_of_roofline": roof / measured["us"]}
     return out

@@ -128,6 +128,14 @@ def test_roofline_report_for_a_bench_line():
     assert 18.0 < rep["moe_decode"]["roofline_us"] < 28.0
 
 
+def test_roofline_of_one_rank_counts_what_its_forward_moves():
+    """A row in and one out for each token, and a row to each of its experts; nothing of their results."""
+    peaks = {"hbm_gbs": 6500.0, "bf16_tflops": 1600.0, "bf16_tflops_sustained": 1400.0, "nvlink_gbs_per_dir": 770.0}
+    rep = roofline.report({"n_gpus": 1, "per_config_us": {"moe_decode": {"us": 20.0}, "moe_prefill_zipf": {"us": 60.0}}}, peaks)
+    assert rep["moe_decode"]["roofline_us"] == pytest.approx(128 * (8 + 2) * 7168 * 2 / 6500e3)
+    assert rep["moe_prefill_zipf"]["roofline_us"] == pytest.approx(4096 * (6 + 2) * 4096 * 2 / 6500e3)
+
+
 def test_report_table_has_ratios_geomeans_and_the_speed_of_light_column():
     from amd_distributed_2025_b200.harness import report
 
