@@ -634,10 +634,11 @@ Fp8Memory fp8_memory(int bn, int splits) {
   return m;
 }
 
-// Time model in ns, fitted to 480 timed plans of 120 drawn sizes (0.6 % from the best width of each): a K block of a tile
-// takes its pair `kb_ns` whatever limits it; then power, memory, and what a launch costs before and after its blocks.  A
-// launch that leaves half of the SMs idle is set up beside the one before it, which shows most where there is one row of
-// tiles (57 x 4640 x 752: 74 CTAs 5.5 us in a row of calls, 146 6.1; but 3409 x 328 x 336: 56 CTAs 6.4, 84 5.5).
+// Time model in ns, fitted to 480 timed plans of 120 drawn sizes (0.6 % from the best width of each, with 910 ns in the last
+// term throughout; the 450 are from rows of calls and came later): a K block of a tile takes its pair `kb_ns` whatever
+// limits it; then power, memory, and what a launch costs before and after its blocks.  A launch that leaves half of the SMs
+// idle is set up beside the one before it, which shows most where there is one row of tiles (57 x 4640 x 752: 74 CTAs
+// 5.5 us in a row of calls, 146 6.1; but 3409 x 328 x 336: 56 CTAs 6.4, 84 5.5).
 Fp8Plan make_fp8_plan(int M, int N, int K, int sms) {
   const int k_blocks = (K + kBlockK - 1) / kBlockK;
   const double dram_ns = ((double)M * K + (double)N * K + 2.0 * M * N) / 6600.0;

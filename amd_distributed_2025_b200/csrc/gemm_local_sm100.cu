@@ -19,7 +19,7 @@
 // Multi-rank kernel before -> these kernels, one rank, us in a row of calls (cool, then the SM clock of a long row, held
 // down at 985 W): 64 x 2880 x 360 10.2 -> 4.2 (latency: a launch and its call), 64 x 7168 x 18432 71 -> 48 (46, 1550 MHz;
 // memory, 5.9 TB/s), 256 x 5120 x 12800 58 -> 40 (35, 1455 MHz; memory, then the meeting of the parts), 2048 x 2880 x 2880
-// 45 -> 31 (27, 1500 MHz; 144 tiles on 74 pairs), 8192 x 8192 x 28672 3135 -> 2787 (2430, 1297 MHz).  Widths are multiples
+// 45 -> 31 (26, 1500 MHz; 144 tiles on 74 pairs), 8192 x 8192 x 28672 3135 -> 2787 (2430, 1297 MHz).  Widths are multiples
 // of 32 columns; with multiples of 64 only, 256 x 5120 x 12800 was three parts of 256 columns on 120 CTAs (40 us; two parts
 // of 160 on 128 are less to exchange), 2048 x 2880 x 2880 120 tiles of 192 (33.5 us).
 // Tried and level: as many pipeline stages as a part has k-blocks, which lets two launches share an SM.
